@@ -156,40 +156,40 @@ block_fp8_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
   if (warp >= Pair::kEpiWarps) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair::kRegsOther));
     if (warp == kProducerWarp) {
-      // ---------------------------------------------------------------- TMA producer (both CTAs)
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = pair; t < total_tiles && ok; t += npairs) {
-        int mt2, nt;
-        tile_coords(t, m_tiles2, p.n_tiles, p.group_m, p.per_group_div, mt2, nt);
-        const int a_row = mt2 * 2 * kBM + (int)rank * kBM;
-        const int b_row = nt * BN + (int)rank * 128;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % S;
-          ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-          if (!ok) break;
-          if (lane == 0) {
+      if (ptx::elect_one()) {
+        // ---------------------------------------------------------------- TMA producer (both CTAs)
+        uint32_t it = 0;
+        bool ok = true;
+        for (int t = pair; t < total_tiles && ok; t += npairs) {
+          int mt2, nt;
+          tile_coords(t, m_tiles2, p.n_tiles, p.group_m, p.per_group_div, mt2, nt);
+          const int a_row = mt2 * 2 * kBM + (int)rank * kBM;
+          const int b_row = nt * BN + (int)rank * 128;
+          for (int kb = 0; kb < num_kb; ++kb, ++it) {
+            const int s = it % S;
+            ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+            if (!ok) break;
             const uint32_t lf = ptx::mapa(full_bar(s), 0);
             ptx::mbar_expect_tx_cluster(lf, Pair::kStageA + Pair::kStageB);
             ptx::tma_load_2d_pair(sA + s * Pair::kStageA, &tmap_a, kb * kBK, a_row, lf);
             ptx::tma_load_2d_pair(sB + s * Pair::kStageB, &tmap_b, kb * kBK, b_row, lf);
           }
-          __syncwarp();
         }
       }
+      __syncwarp();
     } else if (warp == kMmaWarp && leader) {
-      // ---------------------------------------------------------------- MMA issuer (leader only)
-      constexpr uint32_t idesc = ptx::idesc_e4m3_f32(2 * kBM, BN);
-      uint32_t it = 0;
-      bool ok = true;
-      for (int t = pair; t < total_tiles && ok; t += npairs) {
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % S, b = it & 1;
-          ok = ptx::mbar_wait(tempty_bar(b), ((it >> 1) & 1) ^ 1, abort_flag) &&
-               ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-          if (!ok) break;
-          ptx::tc_fence_after();
-          if (lane == 0) {
+      if (ptx::elect_one()) {
+        // ---------------------------------------------------------------- MMA issuer (leader only)
+        constexpr uint32_t idesc = ptx::idesc_e4m3_f32(2 * kBM, BN);
+        uint32_t it = 0;
+        bool ok = true;
+        for (int t = pair; t < total_tiles && ok; t += npairs) {
+          for (int kb = 0; kb < num_kb; ++kb, ++it) {
+            const int s = it % S, b = it & 1;
+            ok = ptx::mbar_wait(tempty_bar(b), ((it >> 1) & 1) ^ 1, abort_flag) &&
+                 ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+            if (!ok) break;
+            ptx::tc_fence_after();
             const uint64_t da = ptx::smem_desc_sw128(sA + s * Pair::kStageA);
             const uint64_t db = ptx::smem_desc_sw128(sB + s * Pair::kStageB);
             const uint32_t d = tmem_base + b * BN;
@@ -199,9 +199,9 @@ block_fp8_gemm_2cta_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
             // CTA's promotion warp 0 releases its own shared-memory stage when it sees the barrier.
             ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
           }
-          __syncwarp();
         }
       }
+      __syncwarp();
     }
   } else {
     // ------------------------------------------------------------------ promotion warps (both CTAs)

@@ -307,30 +307,30 @@ block_fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   // the producer / MMA warpgroup hands registers to the promotion warpgroups
   if constexpr (Cfg::kRebalanceRegs) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsOther));
   if (warp == kProducerWarp) {
-    // ------------------------------------------------------------------ TMA producer
-    uint32_t it = 0;
-    bool ok = true;
-    for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-      const int t = fast_div(item, p.k_splits_div), ks = item - t * S_k;
-      const int kb0 = ks * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
-      int mt, nt;
-      tile_coords(t, m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
-      int b_row = nt * BN, b_row2 = 0;
-      if (MODE != GEMM_DENSE) {
-        const int e = p.expert_ids[mt];
-        if (e < 0) continue;
-        if (MODE == GEMM_GROUPED_SILU_QUANT) {
-          b_row = e * 2 * p.N + nt * 128;  // gate rows of this 128-wide output group
-          b_row2 = b_row + p.N;            // matching up rows
-        } else {
-          b_row += e * p.N;
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------ TMA producer
+      uint32_t it = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+        const int t = fast_div(item, p.k_splits_div), ks = item - t * S_k;
+        const int kb0 = ks * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
+        int mt, nt;
+        tile_coords(t, m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
+        int b_row = nt * BN, b_row2 = 0;
+        if (MODE != GEMM_DENSE) {
+          const int e = p.expert_ids[mt];
+          if (e < 0) continue;
+          if (MODE == GEMM_GROUPED_SILU_QUANT) {
+            b_row = e * 2 * p.N + nt * 128;  // gate rows of this 128-wide output group
+            b_row2 = b_row + p.N;            // matching up rows
+          } else {
+            b_row += e * p.N;
+          }
         }
-      }
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % S;
-        ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        if (lane == 0) {
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % S;
+          ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+          if (!ok) break;
           ptx::mbar_expect_tx(full_bar(s), Cfg::kStageA + Cfg::kStageB);
           ptx::tma_load_2d(sA + s * Cfg::kStageA, &tmap_a, kb * kBK, mt * kBM, full_bar(s));
           if (MODE == GEMM_GROUPED_SILU_QUANT) {
@@ -344,27 +344,27 @@ block_fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
             ptx::tma_load_2d(sB + s * Cfg::kStageB, &tmap_b, kb * kBK, b_row, full_bar(s));
           }
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------- MMA issuer
-    constexpr uint32_t idesc = ptx::idesc_e4m3_f32(kBM, BN);
-    uint32_t it = 0;
-    bool ok = true;
-    for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
-      const int t = fast_div(item, p.k_splits_div), ks = item - t * S_k;
-      const int kb0 = ks * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
-      int mt, nt;
-      tile_coords(t, m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
-      if (MODE != GEMM_DENSE && p.expert_ids[mt] < 0) continue;
-      for (int kb = kb0; kb < kb1; ++kb, ++it) {
-        const int s = it % S, b = it & 1;
-        ok = ptx::mbar_wait(tempty_bar(b), ((it >> 1) & 1) ^ 1, abort_flag) &&
-             ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc = ptx::idesc_e4m3_f32(kBM, BN);
+      uint32_t it = 0;
+      bool ok = true;
+      for (int item = blockIdx.x; item < total_items && ok; item += gridDim.x) {
+        const int t = fast_div(item, p.k_splits_div), ks = item - t * S_k;
+        const int kb0 = ks * p.kb_per_split, kb1 = min(num_kb, kb0 + p.kb_per_split);
+        int mt, nt;
+        tile_coords(t, m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
+        if (MODE != GEMM_DENSE && p.expert_ids[mt] < 0) continue;
+        for (int kb = kb0; kb < kb1; ++kb, ++it) {
+          const int s = it % S, b = it & 1;
+          ok = ptx::mbar_wait(tempty_bar(b), ((it >> 1) & 1) ^ 1, abort_flag) &&
+               ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+          if (!ok) break;
+          ptx::tc_fence_after();
           const uint64_t da = ptx::smem_desc_sw128(sA + s * Cfg::kStageA);
           const uint64_t db = ptx::smem_desc_sw128(sB + s * Cfg::kStageB);
           const uint32_t d = tmem_base + b * BN;
@@ -376,9 +376,9 @@ block_fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
           // here costs the issuing thread more than a hundred cycles per K block.)
           ptx::mma_commit(tfull_bar(b));
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   }
   } else {
     // ------------------------------------------------------------- promotion warps

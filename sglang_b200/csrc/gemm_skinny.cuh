@@ -116,43 +116,40 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   }
 
   if (warp == kProducerWarp) {
-    bool ok = true;
-    // Prologue: the weights do not depend on the previous kernel, the quantised activations do.
-    // The weight tiles of the first stages are requested before waiting for that kernel, so the
-    // weight stream starts while it is still finishing.
-    const int npro = min(S, kb1 - kb0);
-    if (lane == 0) {
+    if (ptx::elect_one()) {
+      bool ok = true;
+      // Prologue: the weights do not depend on the previous kernel, the quantised activations do.
+      // The weight tiles of the first stages are requested before waiting for that kernel, so the
+      // weight stream starts while it is still finishing.
+      const int npro = min(S, kb1 - kb0);
       for (int i = 0; i < npro; ++i) {
         ptx::mbar_expect_tx(full_bar(i), Cfg::kStageW + Cfg::kStageX);
         ptx::tma_load_2d(sW + i * Cfg::kStageW, &tmap_w, (kb0 + i) * kBK, n0, full_bar(i));
       }
       asm volatile("griddepcontrol.wait;" ::: "memory");
       for (int i = 0; i < npro; ++i) ptx::tma_load_2d(sX + i * Cfg::kStageX, &tmap_x, (kb0 + i) * kBK, m0, full_bar(i));
-    }
-    __syncwarp();
-    uint32_t it = npro;
-    for (int kb = kb0 + npro; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S;
-      ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-      if (!ok) break;
-      if (lane == 0) {
+      uint32_t it = npro;
+      for (int kb = kb0 + npro; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S;
+        ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+        if (!ok) break;
         ptx::mbar_expect_tx(full_bar(s), Cfg::kStageW + Cfg::kStageX);
         ptx::tma_load_2d(sW + s * Cfg::kStageW, &tmap_w, kb * kBK, n0, full_bar(s));
         ptx::tma_load_2d(sX + s * Cfg::kStageX, &tmap_x, kb * kBK, m0, full_bar(s));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
-    constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
-    bool ok = true;
-    uint32_t it = 0;
-    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S, b = it % NB;
-      ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
-           ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-      if (!ok) break;
-      ptx::tc_fence_after();
-      if (lane == 0) {
+    if (ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
+      bool ok = true;
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S, b = it % NB;
+        ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
+             ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+        if (!ok) break;
+        ptx::tc_fence_after();
         const uint64_t dw = ptx::smem_desc_sw128(sW + s * Cfg::kStageW);
         const uint64_t dx = ptx::smem_desc_sw128(sX + s * Cfg::kStageX);
         const uint32_t d = tmem_base + b * NT;
@@ -161,8 +158,8 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         ptx::mma_commit(empty_bar(s));
         ptx::mma_commit(tfull_bar(b));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else {
     // promotion warps: lane = weight row, columns = tokens
     const int n = n0 + warp * 32 + lane;

@@ -142,24 +142,24 @@ block_fp8_gemm_ue8m0_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
   const int groups = (num_kb + 3) / 4;  // scale groups (four K blocks each) per tile
 
   if (warp == Cfg::kProducerWarp) {
-    // ------------------------------------------------------------------ TMA producer
-    uint32_t it = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
-      int mt, nt;
-      tile_coords(t, p.m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
-        const int s = it % S;
-        ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------ TMA producer
+      uint32_t it = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+        int mt, nt;
+        tile_coords(t, p.m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const int s = it % S;
+          ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+          if (!ok) break;
           ptx::mbar_expect_tx(full_bar(s), Cfg::kStageA + Cfg::kStageB);
           ptx::tma_load_2d(sA + s * Cfg::kStageA, &tmap_a, kb * kBK, mt * kBM, full_bar(s));
           ptx::tma_load_2d(sB + s * Cfg::kStageB, &tmap_b, kb * kBK, nt * BN, full_bar(s));
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp == Cfg::kSfWarp) {
     // ------------------------------------------------------------------ scale loader
     // Atom layout expected by the 32x128b.warpx4 copy: row r of a 128-row atom at byte (r % 32) * 16 + (r / 32) * 4.
@@ -198,38 +198,35 @@ block_fp8_gemm_ue8m0_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
       }
     }
   } else if (warp == Cfg::kMmaWarp) {
-    // ------------------------------------------------------------------- MMA issuer
-    constexpr uint32_t idesc0 = ptx::idesc_e4m3_block_scaled(kBM, BN);
-    uint32_t it = 0, gi = 0, tile_no = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_no) {
-      const int as = tile_no & 1;
-      ok = ptx::mbar_wait(acc_empty_bar(as), ((tile_no >> 1) & 1) ^ 1, abort_flag);
-      if (!ok) break;
-      const uint32_t d = tmem_base + as * Cfg::kAccCols;
-      for (int kb = 0; kb < num_kb; ++kb, ++it) {
-        const int s = it % S;
-        if ((kb & 3) == 0) {
-          // scales of the next four K blocks: three 512-byte atoms into the scale columns of buffer gi & 1
-          const int slot = gi % SFS;
-          ok = ptx::mbar_wait(sf_full_bar(slot), (gi / SFS) & 1, abort_flag);
-          if (!ok) break;
-          ptx::tc_fence_after();
-          if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc0 = ptx::idesc_e4m3_block_scaled(kBM, BN);
+      uint32_t it = 0, gi = 0, tile_no = 0;
+      bool ok = true;
+      for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x, ++tile_no) {
+        const int as = tile_no & 1;
+        ok = ptx::mbar_wait(acc_empty_bar(as), ((tile_no >> 1) & 1) ^ 1, abort_flag);
+        if (!ok) break;
+        const uint32_t d = tmem_base + as * Cfg::kAccCols;
+        for (int kb = 0; kb < num_kb; ++kb, ++it) {
+          const int s = it % S;
+          if ((kb & 3) == 0) {
+            // scales of the next four K blocks: three 512-byte atoms into the scale columns of buffer gi & 1
+            const int slot = gi % SFS;
+            ok = ptx::mbar_wait(sf_full_bar(slot), (gi / SFS) & 1, abort_flag);
+            if (!ok) break;
+            ptx::tc_fence_after();
             const uint32_t src = sSF + slot * Cfg::kSfSlotBytes;
             const uint32_t buf = gi & 1;
             ptx::tmem_cp_32x128b_warpx4(tmem_base + Cfg::kSfaCol + buf * 4, ptx::smem_desc_sf_atom(src));
             ptx::tmem_cp_32x128b_warpx4(tmem_base + Cfg::kSfbCol + buf * 8, ptx::smem_desc_sf_atom(src + 512));
             ptx::tmem_cp_32x128b_warpx4(tmem_base + Cfg::kSfbCol + buf * 8 + 4, ptx::smem_desc_sf_atom(src + 1024));
             ptx::mma_commit(sf_empty_bar(slot));  // the slot is free once the copies have read it
+            ++gi;
           }
-          __syncwarp();
-          ++gi;
-        }
-        ok = ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-        if (!ok) break;
-        ptx::tc_fence_after();
-        if (lane == 0) {
+          ok = ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+          if (!ok) break;
+          ptx::tc_fence_after();
           const uint64_t da = ptx::smem_desc_sw128(sA + s * Cfg::kStageA);
           const uint64_t db = ptx::smem_desc_sw128(sB + s * Cfg::kStageB);
           const uint32_t buf = (gi - 1) & 1, byte = kb & 3;
@@ -242,9 +239,9 @@ block_fp8_gemm_ue8m0_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
           ptx::mma_commit(empty_bar(s));  // stage free once these MMAs have read it
           if (kb == num_kb - 1) ptx::mma_commit(acc_full_bar(as));  // the tile's accumulator is complete
         }
-        __syncwarp();
       }
     }
+    __syncwarp();
   } else if (warp < Cfg::kEpiWarps) {
     // ------------------------------------------------------------------- epilogue warps
     const int quarter = warp & 3, half = warp >> 2;  // TMEM lanes 32*quarter.., columns 112*half..

@@ -103,34 +103,34 @@ block_fp8_linear_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 
   if (warp == kProducerWarp) {
-    // ------------------------------------------------------------- weight stream (TMA)
-    // the weights do not depend on the kernel before this one: no griddepcontrol.wait here
-    bool ok = true;
-    uint32_t it = 0;
-    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S;
-      if (it >= (uint32_t)S) {
-        ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-      }
-      if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------- weight stream (TMA)
+      // the weights do not depend on the kernel before this one: no griddepcontrol.wait here
+      bool ok = true;
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S;
+        if (it >= (uint32_t)S) {
+          ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+        }
         ptx::mbar_expect_tx(full_bar(s), Cfg::kStageW);
         ptx::tma_load_2d(sW + s * Cfg::kStageW, &tmap_w, kb * kBK, n0, full_bar(s));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------- MMA issuer
-    constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
-    bool ok = true;
-    uint32_t it = 0;
-    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S, b = it % NB;
-      ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
-           ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-      if (!ok) break;
-      ptx::tc_fence_after();
-      if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
+      bool ok = true;
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S, b = it % NB;
+        ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
+             ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+        if (!ok) break;
+        ptx::tc_fence_after();
         const uint64_t dw = ptx::smem_desc_sw128(sW + s * Cfg::kStageW);
         const uint64_t dx = ptx::smem_desc_sw128(sX + s * Cfg::kStageX);
         const uint32_t d = tmem_base + b * NT;
@@ -139,8 +139,8 @@ block_fp8_linear_decode_kernel(const __grid_constant__ CUtensorMap tmap_w, const
         ptx::mma_commit(empty_bar(s));
         ptx::mma_commit(tfull_bar(b));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp >= kFirstQuantWarp) {
     // --------------------------------------------------- quantiser warps: x -> FP8 stages
     // They run ahead of the tensor core by up to S stages and fetch the rows of two K blocks at a time, so the

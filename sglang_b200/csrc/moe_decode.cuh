@@ -191,20 +191,20 @@ moe_decode_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeDeco
   const uint32_t tmem_base = *tmem_slot;
 
   if (warp == kProducerWarp) {
-    // ------------------------------------------------------------- weight stream (TMA)
-    // gate_up: rows [tile*64, +64) of the expert's gate half and of its up half (w1 is [E][2*n_out][K]);
-    // down: rows [tile*128, +128) of w2 [E][n_out][K]
-    const int row_a = STAGE == 1 ? expert * 2 * p.n_out + tile * 64 : expert * p.n_out + tile * 128;
-    const int row_b = row_a + p.n_out;
-    bool ok = true;
-    uint32_t it = 0;
-    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S;
-      if (it >= (uint32_t)S) {
-        ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-      }
-      if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------- weight stream (TMA)
+      // gate_up: rows [tile*64, +64) of the expert's gate half and of its up half (w1 is [E][2*n_out][K]);
+      // down: rows [tile*128, +128) of w2 [E][n_out][K]
+      const int row_a = STAGE == 1 ? expert * 2 * p.n_out + tile * 64 : expert * p.n_out + tile * 128;
+      const int row_b = row_a + p.n_out;
+      bool ok = true;
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S;
+        if (it >= (uint32_t)S) {
+          ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
+          if (!ok) break;
+        }
         ptx::mbar_expect_tx(full_bar(s), Cfg::kStageW);
         const uint32_t d = sW + s * Cfg::kStageW;
         if (STAGE == 1) {
@@ -214,20 +214,20 @@ moe_decode_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeDeco
           ptx::tma_load_2d(d, &tmap_w, kb * kBK, row_a, full_bar(s));
         }
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp == kMmaWarp) {
-    // ------------------------------------------------------------------- MMA issuer
-    constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
-    bool ok = true;
-    uint32_t it = 0;
-    for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
-      const int s = it % S, b = it % NB;
-      ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
-           ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
-      if (!ok) break;
-      ptx::tc_fence_after();
-      if (lane == 0) {
+    if (ptx::elect_one()) {
+      // ------------------------------------------------------------------- MMA issuer
+      constexpr uint32_t idesc = ptx::idesc_e4m3_f32(128, NT);
+      bool ok = true;
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
+        const int s = it % S, b = it % NB;
+        ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
+             ptx::mbar_wait(full_bar(s), (it / S) & 1, abort_flag);
+        if (!ok) break;
+        ptx::tc_fence_after();
         const uint64_t dw = ptx::smem_desc_sw128(sW + s * Cfg::kStageW);
         const uint64_t dx = ptx::smem_desc_sw128(sX + s * Cfg::kStageX);
         const uint32_t d = tmem_base + b * NT;
@@ -236,8 +236,8 @@ moe_decode_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const MoeDeco
         ptx::mma_commit(empty_bar(s));
         ptx::mma_commit(tfull_bar(b));
       }
-      __syncwarp();
     }
+    __syncwarp();
   } else if (warp >= kFirstQuantWarp) {
     // ------------------------------------ quantiser warps: token rows -> FP8 stages in shared memory
     // They run ahead of the tensor core by up to S stages and fetch the rows of two K blocks at a time, so the

@@ -21,6 +21,22 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
+// True in exactly one lane of a converged warp. The roles that issue tcgen05.mma or TMA run their WHOLE loop in
+// that one thread: behind `if (lane == 0)` the compiler cannot prove that the descriptors are warp-uniform, and a
+// K block of four MMAs plus its commit took 574 clocks to issue whatever the tile width; elected once per K block it
+// takes 387-412, elected once per role 260 (128x256x32 MMAs then run at their own 512 clocks per K block).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile(
+      "{\n\t"
+      ".reg .pred P;\n\t"
+      "elect.sync _|P, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, P;\n\t"
+      "}"
+      : "=r"(p));
+  return p != 0;
+}
+
 // ------------------------------------------------------------------------ mbarrier
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
