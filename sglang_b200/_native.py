@@ -6,6 +6,7 @@ nvcc, and if that fails the import error propagates. There is no CPU or torch fa
 from __future__ import annotations
 
 import ctypes
+import importlib.util
 import os
 import threading
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_long, c_size_t, c_uint32, c_void_p, POINTER
@@ -125,11 +126,12 @@ E_BAD_ARG, E_UNSUPPORTED, E_LAUNCH, E_WORKSPACE, E_TIMEOUT = -1, -2, -3, -4, -5
 
 _lock = threading.Lock()
 _lib = None
+host = None  # the CPython extension (csrc/host_ext.cpp), bound to the same library; set by load()
 
 
 def load() -> ctypes.CDLL:
     """Load (building first if needed) the native library and bind every declared symbol."""
-    global _lib
+    global _lib, host
     if _lib is not None:
         return _lib
     with _lock:
@@ -146,7 +148,11 @@ def load() -> ctypes.CDLL:
             fn = getattr(lib, name)  # AttributeError if the library lacks a declared symbol
             fn.restype = res
             fn.argtypes = args
-        _lib = lib
+        spec = importlib.util.spec_from_file_location("_host", os.path.join(_PKG, "_lib", "_host.so"))
+        ext = importlib.util.module_from_spec(spec)
+        spec.loader.exec_module(ext)
+        ext.bind(LIB_PATH)
+        host, _lib = ext, lib
     return _lib
 
 

@@ -17,6 +17,7 @@ PKG = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(PKG, "csrc")
 OUT_DIR = os.path.join(PKG, "_lib")
 LIB = os.path.join(OUT_DIR, "libb200_blockfp8.so")
+HOST_EXT = os.path.join(OUT_DIR, "_host.so")  # CPython extension: the operators' host path (csrc/host_ext.cpp)
 SOURCES = ["status.cu", "quant.cu", "align.cu", "gemm.cu", "moe.cu", "topk.cu", "comm.cu", "ep.cu"]
 
 NVCC_FLAGS = [
@@ -51,8 +52,30 @@ def _stamp(srcs) -> str:
     return h.hexdigest()
 
 
+def _build_host_ext() -> None:
+    """Compile the CPython extension against this interpreter's and this torch's headers (host code only; it looks
+    the C-ABI functions up in the library at run time)."""
+    import sysconfig
+
+    import torch
+
+    troot = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    tmp = f"{HOST_EXT}.{os.getpid()}.tmp"
+    cmd = ["g++", "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden", "-w",
+           f"-D_GLIBCXX_USE_CXX11_ABI={int(torch.compiled_with_cxx11_abi())}",
+           os.path.join(CSRC, "host_ext.cpp"), "-o", tmp,
+           *(f"-I{d}" for d in (os.path.join(troot, "include"), os.path.join(troot, "include/torch/csrc/api/include"),
+                                sysconfig.get_paths()["include"], os.path.join(cuda, "include"))),
+           f"-L{os.path.join(troot, 'lib')}", "-lc10", "-lc10_cuda", "-ltorch_cpu", "-ltorch_cuda", "-ltorch_python", "-ldl"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError(f"g++ failed for host_ext.cpp:\n{r.stdout}\n{r.stderr}")
+    os.replace(tmp, HOST_EXT)
+
+
 def _up_to_date(stamp: str, stamp_file: str) -> bool:
-    return os.path.exists(LIB) and os.path.exists(stamp_file) and open(stamp_file).read() == stamp
+    return os.path.exists(LIB) and os.path.exists(HOST_EXT) and os.path.exists(stamp_file) and open(stamp_file).read() == stamp
 
 
 def build(force: bool = False, verbose: bool = False) -> str:
@@ -84,8 +107,10 @@ def build(force: bool = False, verbose: bool = False) -> str:
                 print(r.stderr)
             return obj
 
-        with ThreadPoolExecutor(max_workers=min(len(srcs), os.cpu_count() or 1)) as ex:
+        with ThreadPoolExecutor(max_workers=min(len(srcs) + 1, os.cpu_count() or 1)) as ex:
+            host = ex.submit(_build_host_ext)
             objs = list(ex.map(compile_one, srcs))
+            host.result()
         tmp = f"{LIB}.{os.getpid()}.tmp"
         cmd = [nvcc, "-shared", "-o", tmp, *objs, "-gencode", "arch=compute_100a,code=sm_100a", "-cudart", "static"]
         r = subprocess.run(cmd, capture_output=True, text=True)

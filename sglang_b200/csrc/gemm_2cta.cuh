@@ -351,11 +351,7 @@ inline int launch_gemm_2cta(const void* A, const void* B, GemmParams p, cudaStre
   rc = make_tmap_out(&tc, p.C, 1, (uint64_t)p.M, (uint64_t)p.N, (int)sizeof(OutT), std::is_same<OutT, __nv_bfloat16>::value, "C");
   if (rc) return rc;
   auto k = block_fp8_gemm_2cta_kernel<OutT>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Pair::kSmemBytes);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", Pair::kSmemBytes, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, Pair::kSmemBytes, "GEMM kernel")) return rc_smem;
   k<<<2 * pairs, Pair::kThreads, Pair::kSmemBytes, st>>>(ta, tb, tc, p);
   return check_launch("block_fp8_gemm_2cta_kernel");
 }

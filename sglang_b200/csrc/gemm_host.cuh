@@ -91,6 +91,28 @@ inline int make_tmap_u8(CUtensorMap* m, const void* base, uint64_t rows, uint64_
 // through boxes of [32 rows x 128 bytes] with the 128-byte swizzle.
 inline int make_tmap_out(CUtensorMap* m, const void* base, uint64_t splits, uint64_t rows, uint64_t cols,
                          int elem_bytes, bool is_bf16, const char* what) {
+  // kept per thread like the operand maps above: the allocator hands the same few output buffers out again
+  struct Key {
+    const void* base;
+    uint64_t splits, rows, cols;
+    int elem_bytes, is_bf16;
+    bool operator==(const Key& o) const {
+      return base == o.base && splits == o.splits && rows == o.rows && cols == o.cols && elem_bytes == o.elem_bytes &&
+             is_bf16 == o.is_bf16;
+    }
+  };
+  struct Hash {
+    size_t operator()(const Key& k) const {
+      return (size_t)((uintptr_t)k.base * 0x9E3779B97F4A7C15ull) ^ (size_t)(k.rows * 31 + k.cols * 131 + k.splits);
+    }
+  };
+  static thread_local std::unordered_map<Key, CUtensorMap, Hash> cache;
+  const Key key{base, splits, rows, cols, elem_bytes, (int)is_bf16};
+  auto hit = cache.find(key);
+  if (hit != cache.end()) {
+    *m = hit->second;
+    return B200_OK;
+  }
   EncodeTiledFn enc = encode_tiled_fn();
   if (!enc) {
     set_error_detail("cuTensorMapEncodeTiled is not available from the driver");
@@ -111,6 +133,27 @@ inline int make_tmap_out(CUtensorMap* m, const void* base, uint64_t splits, uint
                      (unsigned long long)splits, (unsigned long long)rows, (unsigned long long)cols, elem_bytes, (int)r);
     return B200_E_LAUNCH;
   }
+  if (cache.size() >= 4096) cache.clear();
+  cache.emplace(key, *m);
+  return B200_OK;
+}
+
+// Lets kernel `k` use `smem` bytes of dynamic shared memory on the current device: one runtime call per kernel,
+// device and thread (the attribute lasts as long as the context), not one per launch.
+template <typename Kernel>
+inline int allow_smem(Kernel k, size_t smem, const char* what) {
+  static thread_local std::unordered_map<const void*, unsigned long long> done;  // bit d: set on device d
+  int dev = 0;
+  cudaGetDevice(&dev);
+  unsigned long long& mask = done[reinterpret_cast<const void*>(k)];
+  const unsigned long long bit = dev < 64 ? 1ull << dev : 0ull;
+  if (bit && (mask & bit)) return B200_OK;
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e != cudaSuccess) {
+    set_error_detail("%s: cudaFuncSetAttribute(smem=%zu): %s", what, smem, cudaGetErrorString(e));
+    return B200_E_LAUNCH;
+  }
+  mask |= bit;
   return B200_OK;
 }
 
@@ -129,13 +172,8 @@ template <int BN, int MODE, typename OutT, int FAN = 1>
 inline int launch_gemm_inst(const CUtensorMap& ta, const CUtensorMap& tb, const TmapOut<FAN>& tc, const GemmParams& p,
                             int grid, cudaStream_t st) {
   auto k = block_fp8_gemm_kernel<BN, MODE, OutT, FAN>;
-  // per device and cheap: set on every launch rather than caching per device
   const size_t smem = GemmLayout<BN, MODE, OutT>::kSmemBytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   k<<<grid, GemmCfg<BN>::kThreads, smem, st>>>(ta, tb, tc, p);
   return check_launch("block_fp8_gemm_kernel");
 }

@@ -236,11 +236,7 @@ template <int NT, typename OutT>
 inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, cudaStream_t st) {
   auto k = block_fp8_gemm_skinny_kernel<NT, OutT>;
   const size_t smem = SkinnyCfg<NT>::kSmemBytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   const int grid = p.n_tiles * p.t_tiles * p.k_splits;
   // programmatic dependent of the kernel before it (normally the activation quantiser, which
   // signals launch_dependents at once): set-up and the first weight loads overlap its tail
@@ -254,7 +250,7 @@ inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, cons
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, tw, tx, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, tw, tx, p);
   if (e != cudaSuccess) {
     set_error_detail("block_fp8_gemm_skinny_kernel: %s", cudaGetErrorString(e));
     return B200_E_LAUNCH;

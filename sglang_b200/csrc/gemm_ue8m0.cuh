@@ -312,11 +312,7 @@ inline int launch_gemm_ue8m0(const void* A, const void* B, Ue8m0Params p, cudaSt
   rc = make_tmap_u8(&tb, B, (uint64_t)p.N, (uint64_t)p.K, (uint32_t)Ue8m0Cfg::BN, "B (224-row tiles)");
   if (rc) return rc;
   auto k = block_fp8_gemm_ue8m0_kernel<OutT>;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Ue8m0Cfg::kSmemBytes);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", Ue8m0Cfg::kSmemBytes, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, Ue8m0Cfg::kSmemBytes, "GEMM kernel")) return rc_smem;
   k<<<grid, Ue8m0Cfg::kThreads, Ue8m0Cfg::kSmemBytes, st>>>(ta, tb, p);
   return check_launch("block_fp8_gemm_ue8m0_kernel");
 }

@@ -1,0 +1,399 @@
+// Host side of the operators as a CPython extension: argument checks, output allocation, workspace lookup and the
+// C-ABI calls of one operator in one native call. Through ctypes a quantise + GEMM pair cost 40 us of interpreter
+// time on the calling thread (20 arguments marshalled twice, three tensors allocated from Python), more than the
+// two kernels run for at decode and short-prompt sizes.
+//
+// Every function here handles the regular case only and returns None for anything else (another layout, dtype or
+// device, a tensor subclass, an unsupported shape): the Python wrapper then takes its general path, which also
+// raises the errors. Nothing is kept from one call to the next except the scratch buffers below.
+#include <dlfcn.h>
+
+#include <vector>
+
+#include <ATen/cuda/EmptyTensor.h>
+#include <ATen/ops/zeros.h>
+#include <c10/cuda/CUDAFunctions.h>
+#include <c10/cuda/CUDAGraphsC10Utils.h>
+#include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
+#include <torch/csrc/autograd/python_variable.h>
+
+#include "../../include/b200_blockfp8.h"
+
+namespace {
+
+using at::Tensor;
+
+// The library is the one the ctypes binding loaded (possibly another build of it), so its functions are looked up
+// there instead of being linked.
+struct Abi {
+  decltype(&b200_status_string) status_string;
+  decltype(&b200_last_error_detail) last_error_detail;
+  decltype(&b200_get_tuning) get_tuning;
+  decltype(&b200_per_token_group_quant_fp8) quant;
+  decltype(&b200_per_token_group_quant_fp8_ue8m0) quant_ue8m0;
+  decltype(&b200_w8a8_block_fp8_gemm_workspace_bytes) gemm_ws;
+  decltype(&b200_w8a8_block_fp8_gemm) gemm;
+  decltype(&b200_w8a8_block_fp8_gemm_ue8m0) gemm_ue8m0;
+  decltype(&b200_w8a8_block_fp8_linear_decode_workspace_bytes) decode_ws;
+  decltype(&b200_w8a8_block_fp8_linear_decode) decode;
+  decltype(&b200_fused_experts_fp8_workspace_bytes) experts_ws;
+  decltype(&b200_fused_experts_fp8) experts;
+  decltype(&b200_route_topk) route;
+} abi;
+
+PyObject* fail(int status, const char* what) {
+  PyObject* type = status == B200_E_BAD_ARG       ? PyExc_AssertionError
+                   : status == B200_E_UNSUPPORTED ? PyExc_NotImplementedError
+                                                  : PyExc_RuntimeError;
+  return PyErr_Format(type, "%s: %s: %s", what, abi.status_string(status), abi.last_error_detail());
+}
+
+// ------------------------------------------------------------------------------ scratch buffers
+// One grow-only scratch buffer (and one array of split-K tickets) per (device, stream); work on one stream is
+// ordered, so the next call may reuse it. A CUDA graph bakes the buffer's address into its nodes: once a call has
+// been seen under capture, a buffer that has to grow is kept alive instead of being given back to the allocator.
+struct Scratch {
+  int device;
+  void* stream;
+  Tensor buf, tickets;
+};
+// never destroyed: the process may end after the CUDA context. Callers hold the interpreter lock.
+std::vector<Scratch>& scratch = *new std::vector<Scratch>;
+std::vector<Tensor>& retired = *new std::vector<Tensor>;
+bool capture_seen = false;
+
+Tensor empty_on(int device, at::IntArrayRef size, at::ScalarType dtype) {
+  return Tensor(at::detail::empty_cuda(size, dtype, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt));
+}
+
+Scratch& scratch_of(int device, void* stream) {
+  for (auto& s : scratch)
+    if (s.device == device && s.stream == stream) return s;
+  scratch.push_back(Scratch{device, stream, {}, {}});
+  return scratch.back();
+}
+
+Tensor workspace(int device, void* stream, size_t bytes) {
+  Scratch& s = scratch_of(device, stream);
+  if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) capture_seen = true;
+  const size_t have = s.buf.defined() ? (size_t)s.buf.numel() : 0;
+  if (have < bytes) {
+    if (have && capture_seen) retired.push_back(s.buf);
+    const size_t want = bytes > have + have / 2 ? bytes : have + have / 2;
+    s.buf = Tensor();  // back to the allocator first: the larger block may take its place
+    s.buf = empty_on(device, {(int64_t)want}, at::kByte);
+  }
+  return s.buf;
+}
+
+void* tickets_of(int device, void* stream) {
+  Scratch& s = scratch_of(device, stream);
+  if (!s.tickets.defined())  // zero once; every call leaves them zero
+    s.tickets = at::zeros({4096}, at::TensorOptions().dtype(at::kInt).device(c10::kCUDA, (c10::DeviceIndex)device));
+  return s.tickets.data_ptr();
+}
+
+// ------------------------------------------------------------------------------------ arguments
+// A plain CUDA tensor on the current device, or null.
+const Tensor* plain(PyObject* o, int device) {
+  if (!THPVariable_CheckExact(o)) return nullptr;
+  const Tensor& t = THPVariable_Unpack(o);
+  return t.is_cuda() && t.layout() == at::kStrided && t.get_device() == device ? &t : nullptr;
+}
+const Tensor* plain(PyObject* o, int device, at::ScalarType dtype) {  // and contiguous, of one type
+  const Tensor* t = plain(o, device);
+  return t && t->scalar_type() == dtype && t->is_contiguous() ? t : nullptr;
+}
+bool is_2d(const Tensor& t, int64_t rows, int64_t cols) { return t.dim() == 2 && t.size(0) == rows && t.size(1) == cols; }
+int dtype_code(at::ScalarType t) {
+  return t == at::kBFloat16 ? B200_BF16 : t == at::kHalf ? B200_F16 : t == at::kFloat ? B200_F32 : -1;
+}
+at::ScalarType dtype_of_code(long code) {
+  return code == B200_BF16 ? at::kBFloat16 : code == B200_F16 ? at::kHalf : at::kFloat;
+}
+int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
+size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
+void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
+bool knob_off(const char* name) {
+  long v = -1;
+  abi.get_tuning(name, &v);
+  return v == 0;
+}
+constexpr auto kFp8 = at::kFloat8_e4m3fn;
+// Activation bytes up to which the quantised copy lives in the scratch buffer (no tensor to allocate); larger
+// copies are worth a block of the caching allocator, which other work can use in between.
+constexpr size_t kScratchActivation = 8u << 20;
+
+// linear(x, weight, weight_scale, decode_max_rows): quantise per 1x128 group, block-FP8 GEMM, result of x's type.
+PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 4) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor* x = plain(args[0], dev);
+  const Tensor* w = plain(args[1], dev, kFp8);
+  const Tensor* ws = plain(args[2], dev, at::kFloat);
+  const long decode_rows = PyLong_AsLong(args[3]);
+  if (!x || !w || !ws || x->dim() < 1 || w->dim() != 2 || !x->is_contiguous()) Py_RETURN_NONE;
+  const auto type = x->scalar_type();
+  const int code = dtype_code(type);
+  const int64_t K = x->size(-1), N = w->size(0);
+  if ((code != B200_BF16 && code != B200_F16) || w->size(1) != K || K == 0 || K % 128 || N == 0 || N % 8) Py_RETURN_NONE;
+  const int64_t M = x->numel() / K;
+  if (M == 0 || !is_2d(*ws, cdiv(N, 128), K / 128)) Py_RETURN_NONE;
+  c10::SmallVector<int64_t, 4> shape(x->sizes().begin(), x->sizes().end());
+  shape.back() = N;
+  Tensor out = empty_on(dev, shape, type);
+  void* st = stream_of(dev);
+  if (M <= decode_rows && N <= 4096 * 128 && !knob_off("linear_decode_fused")) {
+    const size_t need = abi.decode_ws(M, N, K);
+    const Tensor scratch_buf = need ? workspace(dev, st, need) : Tensor();
+    const int rc = abi.decode(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K, 1e-10f,
+                              need ? scratch_buf.data_ptr() : nullptr, need, tickets_of(dev, st), st);
+    if (rc) return fail(rc, "w8a8_block_fp8_linear (decode)");
+    return THPVariable_Wrap(std::move(out));
+  }
+  const size_t qb = align256((size_t)(M * K)), sb = align256((size_t)(M * (K / 128)) * 4), gb = abi.gemm_ws(M, N, K);
+  const bool inside = qb <= kScratchActivation;
+  const size_t need = gb + (inside ? qb + sb : 0);
+  Tensor q_own, s_own;
+  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
+  uint8_t* base = need ? static_cast<uint8_t*>(buf.data_ptr()) : nullptr;
+  uint8_t* q = base;
+  float* s = reinterpret_cast<float*>(base + qb);
+  uint8_t* gws = inside ? base + qb + sb : base;
+  if (!inside) {
+    q_own = empty_on(dev, {M, K}, kFp8);
+    s_own = empty_on(dev, {K / 128, M}, at::kFloat);
+    q = static_cast<uint8_t*>(q_own.data_ptr());
+    s = s_own.data_ptr<float>();
+  }
+  // scales column-major: the GEMM reads one contiguous run of row scales per K block
+  int rc = abi.quant(x->data_ptr(), code, q, s, M, K, 128, 1, M, 1e-10f, B200_QUANT_DIV_CORRECTED, st);
+  if (rc) return fail(rc, "per_token_group_quant_fp8");
+  rc = abi.gemm(q, s, 1, M, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), code, M, N, K, gb ? gws : nullptr, gb, st);
+  if (rc) return fail(rc, "w8a8_block_fp8_matmul");
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+PyObject* pair(Tensor a, Tensor b) {
+  PyObject* t = PyTuple_New(2);
+  if (!t) return nullptr;
+  PyTuple_SET_ITEM(t, 0, THPVariable_Wrap(std::move(a)));
+  PyTuple_SET_ITEM(t, 1, THPVariable_Wrap(std::move(b)));
+  return t;
+}
+
+// quant(x, group, column_major, tma_aligned, ue8m0, formula, eps) of a 2-D input -> (x_q, x_s)
+PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 7) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor* x = plain(args[0], dev);
+  const long group = PyLong_AsLong(args[1]);
+  const bool col = args[2] == Py_True, aligned = args[3] == Py_True, ue8m0 = args[4] == Py_True;
+  const long formula = PyLong_AsLong(args[5]);
+  const double eps = PyFloat_AsDouble(args[6]);
+  if (!x || PyErr_Occurred() || x->dim() != 2 || !x->is_contiguous() || group <= 0) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+  const int code = dtype_code(x->scalar_type());
+  const int64_t M = x->size(0), K = x->size(1);
+  if (code < 0 || M == 0 || K == 0 || K % group || (ue8m0 && !(col && aligned))) Py_RETURN_NONE;
+  const int64_t groups = K / group, padded = cdiv(M, 4) * 4;
+  Tensor q = empty_on(dev, {M, K}, kFp8);
+  void* st = stream_of(dev);
+  if (ue8m0) {  // four exponent bytes per word, row index contiguous, rows padded to 4
+    Tensor s = empty_on(dev, {cdiv(groups, 4), padded}, at::kInt);
+    const int rc = abi.quant_ue8m0(x->data_ptr(), code, q.data_ptr(), s.data_ptr(), M, K, (int)group, padded, 0, nullptr, 1, st);
+    if (rc) return fail(rc, "per_token_group_quant_fp8 (UE8M0)");
+    return pair(std::move(q), s.as_strided({M, cdiv(groups, 4)}, {1, padded}));
+  }
+  const int64_t ld = aligned ? padded : M;
+  Tensor s = col ? empty_on(dev, {groups, ld}, at::kFloat) : empty_on(dev, {M, groups}, at::kFloat);
+  const int rc = abi.quant(x->data_ptr(), code, q.data_ptr(), s.data_ptr<float>(), M, K, (int)group, col ? 1 : groups,
+                           col ? ld : 1, (float)eps, (int)formula, st);
+  if (rc) return fail(rc, "per_token_group_quant_fp8");
+  return pair(std::move(q), col ? s.as_strided({M, groups}, {1, ld}) : s);
+  END_HANDLE_TH_ERRORS
+}
+
+// matmul(A, B, As, Bs, out_dtype_code): 2-D operands, fp32 scales
+PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 5) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor *A = plain(args[0], dev, kFp8), *B = plain(args[1], dev, kFp8);
+  const Tensor *As = plain(args[2], dev), *Bs = plain(args[3], dev, at::kFloat);
+  const long code = PyLong_AsLong(args[4]);
+  if (!A || !B || !As || !Bs || A->dim() != 2 || B->dim() != 2 || As->scalar_type() != at::kFloat) Py_RETURN_NONE;
+  const int64_t M = A->size(0), K = A->size(1), N = B->size(0);
+  if (M == 0 || N == 0 || K == 0 || B->size(1) != K || !is_2d(*As, M, cdiv(K, 128)) ||
+      !is_2d(*Bs, cdiv(N, 128), cdiv(K, 128)) || code < B200_BF16 || code > B200_F32)
+    Py_RETURN_NONE;
+  Tensor out = empty_on(dev, {M, N}, dtype_of_code(code));
+  void* st = stream_of(dev);
+  const size_t need = abi.gemm_ws(M, N, K);
+  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
+  const int rc = abi.gemm(A->data_ptr(), As->data_ptr<float>(), As->stride(0), As->stride(1), B->data_ptr(),
+                          Bs->data_ptr<float>(), out.data_ptr(), (int)code, M, N, K, need ? buf.data_ptr() : nullptr, need, st);
+  if (rc) return fail(rc, "w8a8_block_fp8_matmul");
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// matmul_ue8m0(A, B, As, Bs, out_dtype_code): both scales packed exponent words, row index contiguous
+PyObject* matmul_ue8m0(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 5) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor *A = plain(args[0], dev, kFp8), *B = plain(args[1], dev, kFp8);
+  const Tensor *As = plain(args[2], dev), *Bs = plain(args[3], dev);
+  const long code = PyLong_AsLong(args[4]);
+  if (!A || !B || !As || !Bs || A->dim() != 2 || B->dim() != 2 || As->scalar_type() != at::kInt || Bs->scalar_type() != at::kInt)
+    Py_RETURN_NONE;
+  const int64_t M = A->size(0), K = A->size(1), N = B->size(0), words = cdiv(K, 512);
+  auto mn_major = [&](const Tensor& s, int64_t rows) {
+    return s.dim() == 2 && s.size(0) == rows && s.size(1) >= words && (s.stride(0) == 1 || rows == 1) &&
+           (s.size(1) == 1 || s.stride(1) >= rows);
+  };
+  if (M == 0 || N == 0 || K == 0 || K % 16 || N % 8 || B->size(1) != K || !mn_major(*As, M) || code < B200_BF16 || code > B200_F32)
+    Py_RETURN_NONE;
+  const int rows_per_word = mn_major(*Bs, N) ? 1 : mn_major(*Bs, cdiv(N, 128)) ? 128 : 0;
+  if (!rows_per_word) Py_RETURN_NONE;
+  auto pitch = [](const Tensor& s) { return s.size(1) > 1 ? s.stride(1) : s.size(0); };
+  Tensor out = empty_on(dev, {M, N}, dtype_of_code(code));
+  const int rc = abi.gemm_ue8m0(A->data_ptr(), As->data_ptr<int>(), pitch(*As), B->data_ptr(), Bs->data_ptr<int>(), pitch(*Bs),
+                                rows_per_word, out.data_ptr(), (int)code, M, N, K, stream_of(dev));
+  if (rc) return fail(rc, "w8a8_block_fp8_matmul (UE8M0)");
+  return THPVariable_Wrap(std::move(out));
+  END_HANDLE_TH_ERRORS
+}
+
+// experts(hidden, w1, w2, topk_weights, topk_ids, w1_scale, w2_scale, inplace, no_combine, weight_on_input, scale)
+PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 11) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor* x = plain(args[0], dev);
+  const Tensor *w1 = plain(args[1], dev, kFp8), *w2 = plain(args[2], dev, kFp8);
+  const Tensor *tw = plain(args[3], dev, at::kFloat), *ti = plain(args[4], dev, at::kInt);
+  const Tensor *s1 = plain(args[5], dev, at::kFloat), *s2 = plain(args[6], dev, at::kFloat);
+  const bool inplace = args[7] == Py_True, no_combine = args[8] == Py_True, on_input = args[9] == Py_True;
+  const double scale = args[10] == Py_None ? 1.0 : PyFloat_AsDouble(args[10]);
+  if (PyErr_Occurred()) PyErr_Clear();
+  else if (x && w1 && w2 && tw && ti && s1 && s2 && x->dim() == 2 && x->is_contiguous() && w1->dim() == 3 && w2->dim() == 3 &&
+           ti->dim() == 2) {
+    const int code = dtype_code(x->scalar_type());
+    const int64_t T = x->size(0), H = x->size(1), E = w1->size(0), I = w1->size(1) / 2, k = ti->size(1);
+    auto is_3d = [](const Tensor& t, int64_t a, int64_t b, int64_t c) {
+      return t.dim() == 3 && t.size(0) == a && t.size(1) == b && t.size(2) == c;
+    };
+    if ((code == B200_BF16 || code == B200_F16) && T > 0 && k > 0 && ti->size(0) == T && is_2d(*tw, T, k) &&
+        w1->size(2) == H && is_3d(*w2, E, H, I) && is_3d(*s1, E, cdiv(2 * I, 128), cdiv(H, 128)) &&
+        is_3d(*s2, E, cdiv(H, 128), cdiv(I, 128)) && !(inplace && no_combine) && (!on_input || k == 1)) {
+      Tensor out = inplace      ? *x
+                   : no_combine ? empty_on(dev, {T, k, H}, x->scalar_type())
+                                : empty_on(dev, {T, H}, x->scalar_type());
+      void* st = stream_of(dev);
+      const size_t need = abi.experts_ws(T, (int)k, (int)E, H, I);
+      const Tensor buf = workspace(dev, st, need);
+      const int rc = abi.experts(x->data_ptr(), nullptr, code, w1->data_ptr(), w2->data_ptr(), s1->data_ptr<float>(),
+                                 s2->data_ptr<float>(), tw->data_ptr<float>(), ti->data_ptr<int>(), out.data_ptr(), T, (int)k,
+                                 (int)E, H, I, no_combine, on_input, (float)scale, buf.data_ptr(), need, st);
+      if (rc) return fail(rc, "fused_experts");
+      return THPVariable_Wrap(std::move(out));
+    }
+  }
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
+// route(logits, bias or None, topk, scoring, groups, topk_group, group_score, renormalize, scale) -> (weights, ids)
+PyObject* route(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 9) Py_RETURN_NONE;
+  const int dev = c10::cuda::current_device();
+  const Tensor* x = plain(args[0], dev);
+  const bool biased = args[1] != Py_None;
+  const Tensor* bias = biased ? plain(args[1], dev, at::kFloat) : nullptr;
+  long v[5];
+  for (int i = 0; i < 5; ++i) v[i] = args[2 + i] == Py_None ? 0 : PyLong_AsLong(args[2 + i]);
+  const bool renormalize = args[7] == Py_True;
+  const double scale = PyFloat_AsDouble(args[8]);
+  if (PyErr_Occurred() || !x || x->dim() != 2 || !x->is_contiguous() || v[0] <= 0 || x->size(0) == 0 ||
+      dtype_code(x->scalar_type()) < 0 || (biased && (!bias || bias->numel() != x->size(1)))) {
+    PyErr_Clear();
+    Py_RETURN_NONE;
+  }
+  const int64_t T = x->size(0);
+  Tensor w = empty_on(dev, {T, v[0]}, at::kFloat), ids = empty_on(dev, {T, v[0]}, at::kInt);
+  const int rc = abi.route(x->data_ptr(), dtype_code(x->scalar_type()), bias ? bias->data_ptr<float>() : nullptr, T,
+                           (int)x->size(1), (int)v[0], (int)v[1], (int)v[2], (int)v[3], (int)v[4], renormalize, (float)scale,
+                           nullptr, w.data_ptr<float>(), ids.data_ptr<int>(), stream_of(dev));
+  if (rc) return fail(rc, "route_topk");
+  return pair(std::move(w), std::move(ids));
+  END_HANDLE_TH_ERRORS
+}
+
+// scratch(device, bytes): the current stream's scratch buffer as a uint8 tensor of at least that size
+PyObject* scratch_tensor(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "scratch(device, bytes)");
+  const long dev = PyLong_AsLong(args[0]);
+  const size_t bytes = PyLong_AsSize_t(args[1]);
+  if (PyErr_Occurred()) return nullptr;
+  return THPVariable_Wrap(workspace((int)dev, stream_of((int)dev), bytes));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* tickets(PyObject*, PyObject* arg) {
+  HANDLE_TH_ERRORS
+  const long dev = PyLong_AsLong(arg);
+  if (PyErr_Occurred()) return nullptr;
+  return PyLong_FromVoidPtr(tickets_of((int)dev, stream_of((int)dev)));
+  END_HANDLE_TH_ERRORS
+}
+
+// bind(path of the C-ABI library)
+PyObject* bind(PyObject*, PyObject* arg) {
+  const char* path = PyUnicode_AsUTF8(arg);
+  if (!path) return nullptr;
+  void* lib = dlopen(path, RTLD_NOW | RTLD_LOCAL);
+  if (!lib) return PyErr_Format(PyExc_ImportError, "%s", dlerror());
+  bool ok = true;
+  auto get = [&](auto& fn, const char* name) {
+    fn = reinterpret_cast<std::decay_t<decltype(fn)>>(dlsym(lib, name));
+    ok = ok && fn != nullptr;
+  };
+  get(abi.status_string, "b200_status_string");
+  get(abi.last_error_detail, "b200_last_error_detail");
+  get(abi.get_tuning, "b200_get_tuning");
+  get(abi.quant, "b200_per_token_group_quant_fp8");
+  get(abi.quant_ue8m0, "b200_per_token_group_quant_fp8_ue8m0");
+  get(abi.gemm_ws, "b200_w8a8_block_fp8_gemm_workspace_bytes");
+  get(abi.gemm, "b200_w8a8_block_fp8_gemm");
+  get(abi.gemm_ue8m0, "b200_w8a8_block_fp8_gemm_ue8m0");
+  get(abi.decode_ws, "b200_w8a8_block_fp8_linear_decode_workspace_bytes");
+  get(abi.decode, "b200_w8a8_block_fp8_linear_decode");
+  get(abi.experts_ws, "b200_fused_experts_fp8_workspace_bytes");
+  get(abi.experts, "b200_fused_experts_fp8");
+  get(abi.route, "b200_route_topk");
+  if (!ok) return PyErr_Format(PyExc_ImportError, "%s lacks a symbol of its header", path);
+  Py_RETURN_NONE;
+}
+
+#define FAST(fn) reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(fn)), METH_FASTCALL
+PyMethodDef methods[] = {
+    {"bind", bind, METH_O, nullptr},          {"linear", FAST(linear), nullptr},
+    {"quant", FAST(quant), nullptr},          {"matmul", FAST(matmul), nullptr},
+    {"matmul_ue8m0", FAST(matmul_ue8m0), nullptr}, {"experts", FAST(experts), nullptr},
+    {"route", FAST(route), nullptr},          {"scratch", FAST(scratch_tensor), nullptr},
+    {"tickets", tickets, METH_O, nullptr},    {nullptr, nullptr, 0, nullptr}};
+PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the block-FP8 operators.", -1, methods,
+                      nullptr, nullptr, nullptr, nullptr};
+
+}  // namespace
+
+PyMODINIT_FUNC PyInit__host() { return PyModule_Create(&module); }

@@ -317,11 +317,7 @@ inline int launch_decode_linear(const void* W, DecodeLinearParams p, cudaStream_
   if (rc) return rc;
   auto k = block_fp8_linear_decode_kernel<InT, OutT>;
   const size_t smem = DecodeLinearCfg::kSmemBytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.n_tiles * p.k_splits));
   cfg.blockDim = dim3(DecodeLinearCfg::kThreads);
@@ -333,7 +329,7 @@ inline int launch_decode_linear(const void* W, DecodeLinearParams p, cudaStream_
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, tw, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, tw, p);
   if (e != cudaSuccess) {
     set_error_detail("block_fp8_linear_decode_kernel: %s", cudaGetErrorString(e));
     return B200_E_LAUNCH;

@@ -436,11 +436,7 @@ inline int launch_moe_decode(const void* W, int64_t w_rows, const MoeDecodeParam
   if (rc) return rc;
   auto k = moe_decode_gemm_kernel<NT, STAGE, InT>;
   const size_t smem = MoeDecodeCfg<NT>::kSmemBytes;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) {
-    set_error_detail("cudaFuncSetAttribute(smem=%zu): %s", smem, cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
+  if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(p.n_tiles * p.k_splits), (unsigned)max_active);
   cfg.blockDim = dim3(MoeDecodeCfg<NT>::kThreads);
@@ -451,7 +447,7 @@ inline int launch_moe_decode(const void* W, int64_t w_rows, const MoeDecodeParam
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  e = cudaLaunchKernelEx(&cfg, k, tw, p);
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, tw, p);
   if (e != cudaSuccess) {
     set_error_detail("moe_decode_gemm_kernel: %s", cudaGetErrorString(e));
     return B200_E_LAUNCH;

@@ -96,6 +96,12 @@ def per_token_group_quant_fp8(
     ``x`` is ``[E, T_pad, 2K]`` and only the first ``masked_m[e]`` rows of expert ``e`` are
     processed.
     """
+    if not fuse_silu_and_mul and masked_m is None and (not scale_ue8m0 or eps == 1e-10):
+        N.load()
+        pair = N.host.quant(x, group_size, column_major_scales, scale_tma_aligned, scale_ue8m0,
+                            quant_formula_for(x.dtype, eps), eps)
+        if pair is not None:
+            return pair
     assert x.shape[-1] % group_size == 0, "the last dimension of `x` cannot be divisible by `group_size`"
     assert x.is_contiguous(), "`x` is not contiguous"
     N.require_cuda(x)
@@ -185,31 +191,18 @@ def prepare_block_fp8_matmul_inputs(
     return M, Nn, K, C
 
 
-_workspaces = {}
-_retired = []  # superseded buffers that a captured CUDA graph may still address
-_capture_seen = False
-
-
 def _workspace(device, nbytes: int) -> Optional[torch.Tensor]:
-    """Grow-only per-(device, stream) scratch buffer for the kernels that need one.
+    """Grow-only per-(device, stream) scratch buffer for the kernels that need one, kept by the native host
+    path (``csrc/host_ext.cpp``), which uses the same buffer.
 
     A CUDA graph bakes the buffer's address into its kernel nodes. Once any call has been made during a
     stream capture, a buffer that has to grow is therefore kept alive (never returned to the allocator)
     instead of being dropped, so replays of an earlier capture keep writing into memory nobody else owns.
     ``reserve_workspace`` sizes the buffer up front."""
-    global _capture_seen
     if nbytes == 0:
         return None
-    key = (device.index, N.current_stream(device))
-    buf = _workspaces.get(key)
-    capturing = torch.cuda.is_current_stream_capturing()
-    _capture_seen = _capture_seen or capturing
-    if buf is None or buf.numel() < nbytes:
-        if buf is not None and _capture_seen:
-            _retired.append(buf)
-        buf = torch.empty(max(nbytes, 0 if buf is None else buf.numel() * 3 // 2), dtype=torch.uint8, device=device)
-        _workspaces[key] = buf
-    return buf
+    N.load()
+    return N.host.scratch(device.index, nbytes)
 
 
 def reserve_workspace(max_bytes: int, device=None) -> None:
@@ -276,6 +269,17 @@ def w8a8_block_fp8_matmul(
     FP8 E4M3, contiguous; ``As [.., ceil(K/128)]`` fp32 with any strides (row- or
     column-major); ``Bs [ceil(N/128), ceil(K/128)]`` fp32. Only ``block_size == [128, 128]``.
     """
+    if list(block_size) == [128, 128]:
+        N.load()
+        code = N.DTYPE_CODE.get(output_dtype, -1)
+        if As.dtype == torch.float32:
+            C = N.host.matmul(A, B, As, Bs, code)
+        elif A.shape[0] >= UE8M0_MIN_M and N.get_tuning("gemm_ue8m0") != 0:
+            C = N.host.matmul_ue8m0(A, B, As, Bs, code)
+        else:
+            C = None
+        if C is not None:
+            return C
     if As.dtype == torch.int32 and Bs.dtype == torch.int32:
         C = _matmul_ue8m0(A, B, As, Bs, block_size, output_dtype)
         if C is not None:
@@ -327,6 +331,13 @@ def w8a8_block_fp8_linear(
     (fp8_utils.py:814-834). Scales are produced column-major so the GEMM reads one
     contiguous run of 128 row-scales per K block."""
     assert input_scale is None
+    if list(block_size) == [128, 128] and _QUANT_FORMULA == 0:
+        N.load()
+        output = N.host.linear(input, weight, weight_scale, DECODE_FUSED_MAX_M)
+        if output is not None:
+            if bias is not None:
+                output += bias
+            return output.to(dtype=input.dtype)
     input_2d = input.view(-1, input.shape[-1])
     output_shape = [*input.shape[:-1], weight.shape[0]]
     output = _linear_decode_fused(input_2d, weight, block_size, weight_scale)
@@ -338,7 +349,6 @@ def w8a8_block_fp8_linear(
     return output.to(dtype=input_2d.dtype).view(*output_shape)
 
 
-_tickets = {}
 # Rows up to which the one-launch kernel is taken. Measured on B200 (us, one launch / quantiser + GEMM + split-K sum,
 # weights rotated so that they come from HBM): 6144x4096 8.8/11.4 at M=1, 12.7/12.1 at M=4, 26.8/12.9 at M=16;
 # 4096x4096 6.7/10.8, 9.0/11.0, 16.9/11.6: the in-kernel quantisers pace the weight stream once many rows are live.
@@ -365,15 +375,11 @@ def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weig
     out = torch.empty(M, Nn, dtype=x.dtype, device=x.device)
     with N.on_device(x):
         stream = N.current_stream()
-        key = (x.device.index, stream)
-        tickets = _tickets.get(key)
-        if tickets is None:  # zero once; every call leaves them zero
-            tickets = _tickets[key] = torch.zeros(4096, dtype=torch.int32, device=x.device)
         ws_bytes = lib.b200_w8a8_block_fp8_linear_decode_workspace_bytes(M, Nn, K)
         ws = _workspace(x.device, ws_bytes)
         st = lib.b200_w8a8_block_fp8_linear_decode(
             N.ptr(x), N.DTYPE_CODE[x.dtype], N.ptr(weight), N.ptr(weight_scale), N.ptr(out), M, Nn, K, 1e-10,
-            N.ptr(ws), ws_bytes, N.ptr(tickets), stream,
+            N.ptr(ws), ws_bytes, N.host.tickets(x.device.index), stream,
         )
     N.check(st, "w8a8_block_fp8_linear (decode)")
     return out

@@ -75,6 +75,12 @@ def fused_experts_impl(
     ``hidden_states_scale`` (extension used by the expert-parallel all-to-all path): when given,
     ``hidden_states`` is already FP8 E4M3 ``[T, H]`` with row-major fp32 1x128 scales
     ``[T, H/128]`` and ``output_dtype`` names the result dtype."""
+    if hidden_states_scale is None and out is None and not skip_unrouted_rows:
+        N.load()
+        result = N.host.experts(hidden_states, w1, w2, topk_weights, topk_ids, w1_scale, w2_scale, inplace, no_combine,
+                                apply_router_weight_on_input, routed_scaling_factor)
+        if result is not None:
+            return result
     assert hidden_states.shape[1] == w1.shape[2], "Hidden size mismatch"
     assert topk_weights.shape == topk_ids.shape, "topk shape mismatch"
     assert hidden_states.is_contiguous(), "Hidden_states must be contiguous"

@@ -34,6 +34,12 @@ def _route(
     topk_weights: Optional[torch.Tensor] = None,
     topk_ids: Optional[torch.Tensor] = None,
 ) -> Tuple[torch.Tensor, torch.Tensor]:
+    if num_token_non_padded is None and topk_weights is None and topk_ids is None:
+        N.load()
+        pair = N.host.route(gating_output, correction_bias, topk, scoring, num_expert_group, topk_group, group_score,
+                            bool(renormalize), float(output_scale))
+        if pair is not None:
+            return pair
     assert gating_output.dim() == 2, "gating_output must be [num_tokens, num_experts]"
     N.require_cuda(gating_output)
     assert gating_output.dtype in (torch.float32, torch.bfloat16, torch.float16), "unsupported logits dtype"
