@@ -13,7 +13,7 @@
 #include <stdlib.h>
 
 #include "gemm_host.cuh"
-#include "moe_decode.cuh"
+#include "gemm_stream.cuh"
 
 namespace b200 {
 
@@ -29,9 +29,9 @@ template <typename T>
 __global__ void __launch_bounds__(256) moe_gather_quant_kernel(
     const T* __restrict__ hidden, const int32_t* __restrict__ sorted_ids, const int32_t* __restrict__ expert_ids,
     const int32_t* __restrict__ num_post_pad, uint8_t* __restrict__ q, float* __restrict__ s, int chunks_per_row,
-    int64_t H, int numel, int topk, int64_t cap, int zero_pads) {
+    int64_t H, int numel, int topk, int64_t cap, int zero_pads, int block_m) {
   const int64_t slot0 = (int64_t)blockIdx.x * kGatherRows;
-  if (slot0 >= *num_post_pad || expert_ids[slot0 / kMoeBlockM] < 0) return;  // uniform per block
+  if (slot0 >= *num_post_pad || expert_ids[slot0 / block_m] < 0) return;  // uniform per block
   const int chunk = blockIdx.y * blockDim.x + threadIdx.x;
   const bool active = chunk < chunks_per_row;  // whole 8-lane groups are in or out (H % 128 == 0)
   int flat[kGatherRows];
@@ -93,9 +93,9 @@ __global__ void __launch_bounds__(256) moe_gather_quant_kernel(
 __global__ void __launch_bounds__(256) moe_gather_fp8_kernel(
     const uint8_t* __restrict__ hidden_q, const float* __restrict__ hidden_s, const int32_t* __restrict__ sorted_ids,
     const int32_t* __restrict__ expert_ids, const int32_t* __restrict__ num_post_pad, uint8_t* __restrict__ q,
-    float* __restrict__ s, int chunks_per_row, int64_t H, int numel, int topk, int64_t cap, int zero_pads) {
+    float* __restrict__ s, int chunks_per_row, int64_t H, int numel, int topk, int64_t cap, int zero_pads, int block_m) {
   const int64_t slot0 = (int64_t)blockIdx.x * kGatherRows;
-  if (slot0 >= *num_post_pad || expert_ids[slot0 / kMoeBlockM] < 0) return;  // uniform per block
+  if (slot0 >= *num_post_pad || expert_ids[slot0 / block_m] < 0) return;  // uniform per block
   const int chunk = blockIdx.y * blockDim.x + threadIdx.x;
   if (chunk >= chunks_per_row) return;
   int flat[kGatherRows];
@@ -233,38 +233,36 @@ static int moe_down_k_splits(int64_t numel, int E, int64_t H, int64_t I, int sms
 }
 
 struct MoeWorkspace {
-  int64_t cap;  // rows of the expert-sorted layout (multiple of 128)
+  int block_m;  // rows per expert block of the sorted layout
+  int64_t cap;  // rows of the expert-sorted layout (multiple of block_m)
   int64_t cap_blocks;
   int down_splits;  // > 1: the down GEMM writes fp32 split-K partials instead of 16-bit rows
-  bool decode;      // few-token path: swapped-operand kernels, no align / gather pass
-  int decode_nt;    // its token tile (16, 32 or 64)
-  int decode_splits;  // K splits of its down stage
-  size_t off_act;   // its fp32 activation rows [numel][I] between the two stages
   bool quant_first;  // quantise the T input rows once, then gather FP8 rows (instead of quantising every pair)
   size_t off_sorted, off_expert, off_npp, off_cumsum, off_align, off_aq1, off_as1, off_aq2, off_as2, off_c3, off_xq, off_xs, total;
 };
 
-// K splits of the few-token down stage: about two work items (routed expert x 128-row weight tile x split)
-// per SM, at least as many as the scale table of one CTA requires.
-static int moe_decode_down_splits(int64_t numel, int E, int64_t H, int64_t I, int sms) {
-  const int64_t active = numel < E ? numel : E;
-  const int64_t items = active * (H / 128);
-  const int64_t num_kb = I / 128;
-  int64_t s = (2 * (int64_t)sms) / (items > 0 ? items : 1);
-  if (s > num_kb / 4) s = num_kb / 4;
-  const int64_t need = cdiv(num_kb, 64);
-  if (s < need) s = need;
-  if (s < 1) s = 1;
-  if (s > 16) s = 16 > need ? 16 : need;
-  return (int)s;
+// Rows per expert block of the sorted layout, and with it the kernel: 16 / 32 / 64 for the weight-streaming kernel,
+// 128 for the tile kernel. An expert's weights are read once per block of its rows, so the block should hold the
+// rows of most experts; a wider one costs promotion work for columns of padding.
+static int moe_block_rows(int64_t numel, int E) {
+  const long knob = tuning().moe_decode;
+  if (knob == 0) return kMoeBlockM;
+  if (knob == 16 || knob == 32 || knob == 64) return (int)knob;
+  const int64_t reached = numel < E ? numel : E;
+  const int64_t avg = numel / reached;
+  if (avg <= 8) return 16;
+  if (avg <= 20) return 32;
+  if (avg <= 48 || knob == 1) return 64;
+  return kMoeBlockM;
 }
 
-static MoeWorkspace moe_workspace_layout(int64_t T, int topk, int E, int64_t H, int64_t I) {
+static MoeWorkspace moe_workspace_layout(int64_t T, int topk, int E, int64_t H, int64_t I, bool tile_only) {
   MoeWorkspace w = {};
   const int64_t numel = T * topk;
-  int64_t max_pad = numel < E + 1 ? numel * kMoeBlockM : numel + (int64_t)(E + 1) * (kMoeBlockM - 1);
-  w.cap = cdiv(max_pad, kMoeBlockM) * kMoeBlockM;
-  w.cap_blocks = w.cap / kMoeBlockM;
+  w.block_m = tile_only ? kMoeBlockM : moe_block_rows(numel, E);
+  const int64_t max_pad = numel < E + 1 ? numel * w.block_m : numel + (int64_t)(E + 1) * (w.block_m - 1);
+  w.cap = cdiv(max_pad, w.block_m) * w.block_m;
+  w.cap_blocks = w.cap / w.block_m;
   size_t o = 0;
   auto take = [&](size_t bytes) { size_t at = o; o = align_up(o + bytes, 256); return at; };
   w.off_sorted = take((size_t)w.cap * 4);
@@ -283,69 +281,23 @@ static MoeWorkspace moe_workspace_layout(int64_t T, int topk, int E, int64_t H, 
   w.quant_first = topk >= 3;
   w.off_xq = take(w.quant_first ? (size_t)T * H : 0);
   w.off_xs = take(w.quant_first ? (size_t)T * (H / 128) * 4 : 0);
-  // a handful of tokens: the swapped-operand path (its buffers are taken in addition, so that the
-  // tuning knob can switch paths on the same workspace)
-  w.decode = T <= 64 && numel <= kDecodeMaxIds && E <= kDecodeMaxExperts && H <= 64 * 128 && H % 128 == 0 && I % 128 == 0;
-  w.decode_nt = T <= 16 ? 16 : (T <= 32 ? 32 : 64);
-  w.decode_splits = w.decode ? moe_decode_down_splits(numel, E, H, I, 148) : 1;
-  w.off_act = take(w.decode ? (size_t)numel * I * 4 : 0);
-  if (w.decode) {
-    const size_t need = (size_t)w.decode_splits * numel * H * 4;
-    const size_t have = w.down_splits > 1 ? (size_t)w.down_splits * numel * H * 4 : (size_t)numel * H * 2;
-    if (need > have) {  // the partials of the decode path share the c3 region: grow it
-      w.off_c3 = take(need);
-    }
-  }
   w.total = o;
   return w;
 }
 
-// Few-token path (see moe_decode.cuh): gate_up -> fp32 activation rows -> down -> slot / split sum.
-template <typename T>
-static int run_fused_experts_decode(const void* hidden, const float* hidden_scale, const void* w1, const void* w2,
-                                    const float* w1_scale, const float* w2_scale, const float* topk_weights,
-                                    const int32_t* topk_ids, void* out, int64_t T_tokens, int topk, int E, int64_t H,
-                                    int64_t I, int combine_mode, int weight_on_input, float routed_scale, uint8_t* ws,
-                                    const MoeWorkspace& L, cudaStream_t st) {
-  const int no_combine = combine_mode == B200_COMBINE_NONE;
-  const int skip_unrouted = combine_mode == B200_COMBINE_SUM_SKIP_UNROUTED;
-  const int64_t numel = T_tokens * topk;
-  const int max_active = (int)(numel < E ? numel : E);
-  MoeDecodeParams p = {};
-  p.topk_ids = topk_ids; p.topk_weights = topk_weights; p.numel = (int)numel; p.topk = topk; p.E = E;
-  p.act = reinterpret_cast<float*>(ws + L.off_act);
-  p.partial = reinterpret_cast<float*>(ws + L.off_c3);
-  p.status = device_status_word();
-  if (!p.status) {
-    set_error_detail("cannot resolve the device status word");
-    return B200_E_LAUNCH;
-  }
-  // gate_up: K = H, 64 gate + 64 up rows per tile
-  p.x = hidden_scale ? nullptr : hidden;
-  p.x_q = hidden_scale ? static_cast<const uint8_t*>(hidden) : nullptr;
-  p.x_s = hidden_scale;
-  p.Bs = w1_scale; p.K = (int)H; p.num_kb = (int)(H / 128); p.n_out = (int)I; p.n_tiles = (int)(I / 64);
-  p.k_splits = 1; p.kb_per_split = p.num_kb; p.weight_on_input = weight_on_input; p.apply_weight = 0;
-  int rc;
-#define B200_MOE_DECODE(STAGE, W, ROWS)                                                             \
-  (L.decode_nt == 16   ? launch_moe_decode<16, STAGE, T>(W, ROWS, p, max_active, st)                \
-   : L.decode_nt == 32 ? launch_moe_decode<32, STAGE, T>(W, ROWS, p, max_active, st)                \
-                       : launch_moe_decode<64, STAGE, T>(W, ROWS, p, max_active, st))
-  if ((rc = B200_MOE_DECODE(1, w1, (int64_t)E * 2 * I))) return rc;
-  // down: K = I, 128 rows of w2 per tile, K split
-  p.x = nullptr; p.x_q = nullptr; p.x_s = nullptr;
-  p.Bs = w2_scale; p.K = (int)I; p.num_kb = (int)(I / 128); p.n_out = (int)H; p.n_tiles = (int)(H / 128);
-  p.kb_per_split = (int)cdiv(p.num_kb, L.decode_splits);
-  p.k_splits = (int)cdiv(p.num_kb, p.kb_per_split);
-  p.weight_on_input = 0; p.apply_weight = weight_on_input ? 0 : 1;
-  if ((rc = B200_MOE_DECODE(2, w2, (int64_t)E * H))) return rc;
-#undef B200_MOE_DECODE
-  const int64_t rows = no_combine ? numel : T_tokens;
-  const int64_t total = rows * (H / 8);
-  moe_sum_reduce_splits_kernel<T><<<(unsigned)cdiv(total, 256), 256, 0, st>>>(
-      p.partial, topk_ids, static_cast<T*>(out), rows, no_combine ? 1 : topk, p.k_splits, numel * H, E, H,
-      no_combine ? 1.0f : routed_scale, skip_unrouted);
-  return check_launch("moe_sum_reduce_splits");
+// The two grouped GEMMs over token blocks of NT rows (see gemm_stream.cuh).
+template <int NT, typename T>
+static int run_stream_gemms(const uint8_t* aq1, const float* as1, uint8_t* aq2, float* as2, const void* w1, const void* w2,
+                            const float* w1_scale, const float* w2_scale, const float* topk_weights, int weight_on_input,
+                            T* rows, int E, int64_t H, int64_t I, int64_t cap, StreamParams p, cudaStream_t st) {
+  p.as_ld = cap;
+  p.As = as1; p.Bs = w1_scale; p.n_out = (int)I; p.q_out = aq2; p.q_scales = as2; p.q_ld = cap;
+  p.topk_weights = weight_on_input ? topk_weights : nullptr;
+  int rc = launch_stream<NT, STREAM_GATE_UP, T>(w1, (int64_t)E * 2 * I, aq1, cap, H, p, st);
+  if (rc) return rc;
+  p.As = as2; p.Bs = w2_scale; p.n_out = (int)H; p.C = rows;
+  p.topk_weights = weight_on_input ? nullptr : topk_weights;
+  return launch_stream<NT, STREAM_DOWN, T>(w2, (int64_t)E * H, aq2, cap, I, p, st);
 }
 
 // Destinations of the (token, slot) rows when they leave for several buffers (expert-parallel combine by push).
@@ -364,7 +316,8 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   if (scatter != nullptr) combine_mode = B200_COMBINE_NONE;  // rows leave per (token, slot); the receiver sums
   const int no_combine = combine_mode == B200_COMBINE_NONE;
   const int skip_unrouted = combine_mode == B200_COMBINE_SUM_SKIP_UNROUTED;
-  const MoeWorkspace L = moe_workspace_layout(T_tokens, topk, E, H, I);
+  // rows that leave for several buffers are sent by the tile kernel's epilogue
+  const MoeWorkspace L = moe_workspace_layout(T_tokens, topk, E, H, I, scatter != nullptr);
   const int64_t numel = T_tokens * topk;
   int32_t* sorted = reinterpret_cast<int32_t*>(ws + L.off_sorted);
   int32_t* expert_ids = reinterpret_cast<int32_t*>(ws + L.off_expert);
@@ -374,19 +327,14 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   float* as1 = reinterpret_cast<float*>(ws + L.off_as1);
   uint8_t* aq2 = ws + L.off_aq2;
   float* as2 = reinterpret_cast<float*>(ws + L.off_as2);
-  // Opt-in (knob moe_decode = 1): measured slower than the tile path below at every token count tried (the
-  // in-kernel row fetches sit behind the saturated weight stream in L2 and pace the pipeline, and more work
-  // items than resident CTAs run in waves), so the tile path stays the default.
-  if (L.decode && tuning().moe_decode == 1 && scatter == nullptr)
-    return run_fused_experts_decode<T>(hidden, hidden_scale, w1, w2, w1_scale, w2_scale, topk_weights, topk_ids, out, T_tokens,
-                                       topk, E, H, I, combine_mode, weight_on_input, routed_scale, ws, L, st);
   int down_splits = L.down_splits;
   if (tuning().moe_down_splitk == 0) down_splits = 1;  // knob: keep the 16-bit single-pass path
-  if (scatter != nullptr) down_splits = 1;             // rows go straight to their receivers in 16 bits
+  const bool stream = L.block_m != kMoeBlockM;
+  if (scatter != nullptr || stream) down_splits = 1;   // rows go straight to their receivers in 16 bits
   const bool split = down_splits > 1;
   T* c3 = no_combine && !split ? static_cast<T*>(out) : reinterpret_cast<T*>(ws + L.off_c3);
 
-  int rc = b200_moe_align_block_size(topk_ids, B200_I32, numel, E + 1, kMoeBlockM, sorted, L.cap, expert_ids,
+  int rc = b200_moe_align_block_size(topk_ids, B200_I32, numel, E + 1, L.block_m, sorted, L.cap, expert_ids,
                                      L.cap_blocks, npp, cumsum, 1, ws + L.off_align,
                                      b200_moe_align_workspace_bytes(numel, E + 1), st);
   if (rc) return rc;
@@ -417,11 +365,28 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
     if (tuning().moe_zero_pads >= 0) zero_pads = (int)tuning().moe_zero_pads;
     if (hs != nullptr)
       moe_gather_fp8_kernel<<<grid, threads, 0, st>>>(hq, hs, sorted, expert_ids, npp, aq1, as1, cpr, H, (int)numel, topk,
-                                                     L.cap, zero_pads);
+                                                     L.cap, zero_pads, L.block_m);
     else
       moe_gather_quant_kernel<T><<<grid, threads, 0, st>>>(static_cast<const T*>(hidden), sorted, expert_ids, npp, aq1,
-                                                          as1, cpr, H, (int)numel, topk, L.cap, zero_pads);
+                                                          as1, cpr, H, (int)numel, topk, L.cap, zero_pads, L.block_m);
     if ((rc = check_launch("moe_gather"))) return rc;
+  }
+  if (stream) {
+    StreamParams sp = {};
+    sp.expert_ids = expert_ids; sp.num_post_pad = npp; sp.sorted_ids = sorted; sp.numel = (int)numel;
+    // every reached expert has at most one partly filled block
+    const int64_t bound = (numel < E ? numel : E) + numel / L.block_m;
+    sp.max_blocks = (int)(bound < L.cap_blocks ? bound : L.cap_blocks);
+#define B200_STREAM(NT)                                                                                                    \
+  run_stream_gemms<NT, T>(aq1, as1, aq2, as2, w1, w2, w1_scale, w2_scale, topk_weights, weight_on_input, c3, E, H, I, \
+                          L.cap, sp, st)
+    rc = L.block_m == 16 ? B200_STREAM(16) : L.block_m == 32 ? B200_STREAM(32) : B200_STREAM(64);
+#undef B200_STREAM
+    if (rc) return rc;
+    if (no_combine) return B200_OK;
+    moe_sum_reduce_kernel<T><<<(unsigned)T_tokens, 256, 0, st>>>(c3, topk_ids, static_cast<T*>(out), topk, E, H,
+                                                                  routed_scale, skip_unrouted, nullptr);
+    return check_launch("moe_sum_reduce");
   }
   const int force_bn = tuning().gemm_bn == 128 || tuning().gemm_bn == 256 ? (int)tuning().gemm_bn : 0;
   // expected live row tiles: every pair once, plus up to one partial tile per expert
@@ -564,7 +529,8 @@ extern "C" int b200_masked_experts_fp8(const void* hidden_q, const float* hidden
 
 extern "C" size_t b200_fused_experts_fp8_workspace_bytes(int64_t T, int topk, int E, int64_t H, int64_t I) {
   if (T <= 0 || topk <= 0 || E <= 0 || H <= 0 || I <= 0) return 0;
-  return b200::moe_workspace_layout(T, topk, E, H, I).total;
+  // the layout with 128-row blocks is the larger one, and either may be used with this size
+  return b200::moe_workspace_layout(T, topk, E, H, I, true).total;
 }
 
 extern "C" int b200_fused_experts_fp8(const void* hidden, const float* hidden_scale, int h_dtype, const void* w1,
