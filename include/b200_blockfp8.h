@@ -62,7 +62,7 @@ int b200_read_device_status(int* out, void* stream);
  * "gemm_skinny_max_m", "gemm_splitk" (> 0 forces the K split; size the workspace after setting
  * it), "gemm_2cta" (0 / 1), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
  * fp32-scale kernels), "linear_decode_fused" (0 = never the one-launch decode linear), "moe_decode"
- * (1 = few-token swapped-operand MoE kernels; default off), "moe_down_splitk" (0 = never),
+ * (0 = never the weight-streaming MoE kernels, 1 = always, 16 / 32 / 64 = always with that row block), "moe_down_splitk" (0 = never),
  * "moe_zero_pads" (0 / 1), "peer_wait_ms" (limit of a device-side wait for another GPU, 100 .. 60000).
  * No counterpart in the reference (its Triton launchers read tuned JSON configs instead,
  * python/sglang/srt/layers/moe/fused_moe_triton/fused_moe_triton_config.py). Not thread-safe
@@ -152,6 +152,20 @@ int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B,
                                       void* out, int64_t M, int64_t N, int64_t K, float eps,
                                       void* workspace, size_t workspace_bytes, void* tickets,
                                       void* stream);
+
+/* ---------------------------------------------------------------------------------------
+ * w8a8_block_fp8_linear: quantise + GEMM of one linear layer in one call, any M
+ * replaces: python/sglang/srt/layers/quantization/fp8_utils.py:814-834 (the same composition)
+ * out = the result of b200_per_token_group_quant_fp8 (group 128) followed by b200_w8a8_block_fp8_gemm,
+ * with the kernels chained as programmatic dependents (up to 4 rows: the one-launch kernel above).
+ * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out, tickets as above. The weights B may
+ * be fetched before earlier kernels of the stream have finished if those signal their dependents early
+ * (kernels of this library do; its quantisers called on their own do not).
+ * workspace: b200_w8a8_block_fp8_linear_workspace_bytes(M,N,K) bytes, 256-byte aligned. */
+size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out,
+                               int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes,
+                               void* tickets, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * moe_align_block_size

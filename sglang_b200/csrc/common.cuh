@@ -55,7 +55,7 @@ struct Tuning {
   long gemm_2cta = -1;          // 0: never, 1: CTA-pair kernel whenever legal
   long gemm_ue8m0 = -1;          // 0: packed power-of-two scales never take the block-scaled MMA kernel
   long linear_decode_fused = -1; // 0: callers keep quantiser + GEMM as separate launches at decode sizes
-  long moe_decode = -1;         // 1: fused_experts takes the few-token (swapped-operand) path for T <= 64
+  long moe_decode = -1;         // 0 / 1: never / always the weight-streaming experts; 16, 32, 64: with that row block
   long moe_down_splitk = -1;    // 0: the down GEMM never splits K
   long moe_zero_pads = -1;      // 0 / 1: whether the gather pass zeroes pad rows
   long peer_wait_ms = -1;       // limit of a device-side wait for another GPU
@@ -71,6 +71,41 @@ inline unsigned long long peer_wait_ns() {
   if (ms > 60000) ms = 60000;
   return (unsigned long long)ms * 1000000ull;
 }
+
+
+// Launch as a programmatic dependent of the kernel before it in the stream: the grid may be set up while that kernel
+// drains. The kernel executes griddepcontrol.wait before it touches global memory that an earlier kernel may use.
+// cluster > 1: thread-block clusters of that many blocks along x.
+template <typename... P, typename... A>
+inline int launch_dependent(void (*k)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t st, unsigned cluster,
+                            const char* what, A&&... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, k, P(args)...);
+  if (e != cudaSuccess) {
+    set_error_detail("%s: %s", what, cudaGetErrorString(e));
+    return B200_E_LAUNCH;
+  }
+  return check_launch(what);
+}
+__device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// Quantiser of a linear layer (quant.cu): 16-bit x [M, K] -> FP8 rows + column-major scales, launched so that it overlaps
+// the kernels on either side. Only for scratch operands: the GEMM that follows may fetch its WEIGHTS before this grid's
+// predecessors have finished, so those must not have been written by a kernel that triggers its dependents early.
+int quant_for_linear(const void* x, int x_dtype, void* q, float* s, int64_t M, int64_t K, cudaStream_t st);
 
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }

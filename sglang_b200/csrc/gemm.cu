@@ -22,7 +22,8 @@ __global__ void __launch_bounds__(256) splitk_reduce_kernel(const float* __restr
   const int64_t i = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8;
   // launched with programmatic stream serialisation: this grid may start while the GEMM that
   // writes the partials is still draining; everything above is index arithmetic only
-  asm volatile("griddepcontrol.wait;" ::: "memory");
+  grid_launch_dependents();
+  grid_dependency_wait();
   if (i >= mn) return;
   float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   for (int s = 0; s < splits; ++s) {
@@ -205,6 +206,48 @@ extern "C" int b200_w8a8_block_fp8_gemm_fanout(const void* A, const float* As, i
   for (int d = 0; d < n_dest; ++d) fan.dest[d] = dest[d];
   return gemm_impl(A, As, as_stride_m, as_stride_k, B, Bs, nullptr, c_dtype, M, N, K, workspace, workspace_bytes, stream,
                    fan);
+}
+
+// Quantised activations of a linear layer: FP8 rows, then column-major scales, in front of the GEMM's own workspace.
+namespace b200 {
+constexpr int64_t kDecodeLinearMaxM = 4;  // rows up to which the one-launch kernel (linear_decode.cuh) is the faster one
+static size_t linear_q_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * K), 256); }
+static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * (K / 128)) * 4, 256); }
+static bool linear_one_launch(int64_t M, int64_t N) {
+  return M <= kDecodeLinearMaxM && N <= 4096 * 128 && tuning().linear_decode_fused != 0;
+}
+}  // namespace b200
+
+extern "C" size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  using namespace b200;
+  if (M <= 0 || N <= 0 || K <= 0) return 0;
+  if (linear_one_launch(M, N)) return b200_w8a8_block_fp8_linear_decode_workspace_bytes(M, N, K);
+  return linear_q_bytes(M, K) + linear_s_bytes(M, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
+}
+
+extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out, int64_t M,
+                                          int64_t N, int64_t K, void* workspace, size_t workspace_bytes, void* tickets,
+                                          void* stream) {
+  using namespace b200;
+  B200_CHECK_ARG(M >= 0 && N >= 0 && K > 0, "linear: bad shape");
+  if (M == 0 || N == 0) return B200_OK;
+  B200_UNSUPPORTED(x_dtype != B200_BF16 && x_dtype != B200_F16, "linear: 16-bit activations only (dtype code %d)", x_dtype);
+  B200_UNSUPPORTED(K % 128 != 0, "linear: K=%lld must be a multiple of 128", (long long)K);
+  B200_CHECK_ARG(x && B && Bs && out && tickets, "linear: null pointer");
+  B200_CHECK_ARG(((uintptr_t)x & 15) == 0, "linear: x must be 16-byte aligned");
+  const size_t need = b200_w8a8_block_fp8_linear_workspace_bytes(M, N, K);
+  if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0)) {
+    set_error_detail("linear: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
+    return B200_E_WORKSPACE;
+  }
+  if (linear_one_launch(M, N))
+    return b200_w8a8_block_fp8_linear_decode(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, workspace, workspace_bytes, tickets, stream);
+  uint8_t* q = static_cast<uint8_t*>(workspace);
+  float* s = reinterpret_cast<float*>(q + linear_q_bytes(M, K));
+  uint8_t* rest = reinterpret_cast<uint8_t*>(s) + linear_s_bytes(M, K);
+  int rc = quant_for_linear(x, x_dtype, q, s, M, K, static_cast<cudaStream_t>(stream));
+  if (rc) return rc;
+  return gemm_impl(q, s, 1, M, B, Bs, out, x_dtype, M, N, K, rest, need - (size_t)(rest - q), stream, FanOut{});
 }
 
 extern "C" size_t b200_w8a8_block_fp8_linear_decode_workspace_bytes(int64_t M, int64_t N, int64_t K) {

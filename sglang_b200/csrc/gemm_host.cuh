@@ -174,6 +174,8 @@ inline int launch_gemm_inst(const CUtensorMap& ta, const CUtensorMap& tb, const 
   auto k = block_fp8_gemm_kernel<BN, MODE, OutT, FAN>;
   const size_t smem = GemmLayout<BN, MODE, OutT>::kSmemBytes;
   if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
+  if (MODE == GEMM_DENSE)
+    return launch_dependent(k, dim3((unsigned)grid), GemmCfg<BN>::kThreads, smem, st, 1, "block_fp8_gemm_kernel", ta, tb, tc, p);
   k<<<grid, GemmCfg<BN>::kThreads, smem, st>>>(ta, tb, tc, p);
   return check_launch("block_fp8_gemm_kernel");
 }

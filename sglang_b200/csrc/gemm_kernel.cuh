@@ -295,6 +295,10 @@ block_fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  if (MODE == GEMM_DENSE) {  // launched as a programmatic dependent of the quantiser (or of whatever came before)
+    grid_launch_dependents();
+    grid_dependency_wait();
+  }
 
   // live problem size (grouped: decided on the device by the align kernel)
   int m_tiles = p.m_tiles;

@@ -11,6 +11,8 @@
 // instead (one item per cluster) and the partial sums go to the first CTA through distributed shared memory.
 //   warps 0-3  promotion of the first 128 rows (lane = weight row, columns = tokens), warps 4-7 of the second
 //   warp  8    TMA producer          warp 9  MMA issuer
+//   warps 10, 11  scale tables, ids and router weights of the next item into the other of two table buffers: loaded
+//              by the promotion warps at the start of an item they stopped the weight stream for the L2 round trips
 #pragma once
 
 #include "gemm_host.cuh"
@@ -41,20 +43,22 @@ struct StreamParams {
 
 template <int NT>
 struct StreamCfg {
-  static constexpr int kThreads = 320;
+  static constexpr int kThreads = 384;
   static constexpr int kStageW = 256 * kBK, kStageX = NT * kBK, kStage = kStageW + kStageX;
   static constexpr int kAccBufs = 4;  // the tensor core runs this many K blocks ahead of the promotion warps
   static constexpr int kTmemCols = kAccBufs * 2 * NT;
-  // behind the ring: barriers, exchange area (the other half's gate / up values), partial row amax, ids and weights
-  // of the rows, then the scale table [kb][NT] and the weight-block scales [2][kb], sized by the K blocks of one CTA
-  static constexpr int kExch = NT * 128 * 4, kPart = 4 * NT * 4, kRows = NT * 8;
-  static constexpr int kFixed = 256 + kExch + kPart + kRows + 1024;
+  // behind the ring: barriers, exchange area (the other half's gate / up values), partial row amax, then two buffers
+  // of [ids of the rows][their router weights][scale table [kb][NT]][weight-block scales [2][kb]], sized by the K
+  // blocks of one CTA
+  static constexpr int kExch = NT * 128 * 4, kPart = 4 * NT * 4;
+  static constexpr int kFixed = 256 + kExch + kPart + 1024;
   static constexpr int kMaxStages = 8, kSmemLimit = 232448;
+  __host__ __device__ static constexpr int table_bytes(int table_kb) { return 2 * NT * 4 + table_kb * NT * 4 + (table_kb * 8 + 15) / 16 * 16; }
   static int stages_for(int table_kb) {
-    const int s = (kSmemLimit - kFixed - table_kb * (NT + 2) * 4) / kStage;
+    const int s = (kSmemLimit - kFixed - 2 * table_bytes(table_kb)) / kStage;
     return s < kMaxStages ? s : kMaxStages;
   }
-  static size_t smem_for(int stages, int table_kb) { return (size_t)stages * kStage + kFixed + (size_t)table_kb * (NT + 2) * 4; }
+  static size_t smem_for(int stages, int table_kb) { return (size_t)stages * kStage + kFixed + 2 * (size_t)table_bytes(table_kb); }
 };
 
 namespace ptx {
@@ -102,17 +106,21 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem_al + (size_t)S * Cfg::kStage);
   float* exch = reinterpret_cast<float*>(bars + 32);   // [NT][128]
   float* part = exch + NT * 128;                       // [4][NT]
-  float* row_w = part + 4 * NT;                        // [NT] router weights
-  int* row_id = reinterpret_cast<int*>(row_w + NT);    // [NT] flat ids
-  float* table = reinterpret_cast<float*>(row_id + NT);  // [kb][NT] row scales
-  float* bs_tab = table + p.table_kb * NT;             // [2][kb] weight-block scales
+  uint8_t* tables = reinterpret_cast<uint8_t*>(part + 4 * NT);
+  const int table_bytes = Cfg::table_bytes(p.table_kb);
+  auto row_id_of = [&](int buf) { return reinterpret_cast<int*>(tables + buf * table_bytes); };           // [NT] flat ids
+  auto row_w_of = [&](int buf) { return reinterpret_cast<float*>(tables + buf * table_bytes) + NT; };     // [NT] weights
+  auto table_of = [&](int buf) { return reinterpret_cast<float*>(tables + buf * table_bytes) + 2 * NT; };  // [kb][NT]
+  auto bs_tab_of = [&](int buf) { return table_of(buf) + p.table_kb * NT; };                               // [2][kb]
   const uint32_t bar0 = ptx::smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (8 + s); };
   auto tfull_bar = [&](int b) { return bar0 + 8u * (16 + b); };
   auto tempty_bar = [&](int b) { return bar0 + 8u * (16 + NB + b); };
-  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 16 + 2 * NB);
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 16 + 2 * NB + 1);
+  auto tab_full_bar = [&](int b) { return bar0 + 8u * (16 + 2 * NB + b); };
+  auto tab_empty_bar = [&](int b) { return bar0 + 8u * (18 + 2 * NB + b); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 20 + 2 * NB);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 20 + 2 * NB + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kProducerWarp = 8, kMmaWarp = 9;
@@ -129,6 +137,10 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       ptx::mbar_init(tfull_bar(b), 1);
       ptx::mbar_init(tempty_bar(b), 8);
     }
+    for (int b = 0; b < 2; ++b) {
+      ptx::mbar_init(tab_full_bar(b), 2);
+      ptx::mbar_init(tab_empty_bar(b), 8);
+    }
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
@@ -144,6 +156,16 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Everything read below, and what the epilogue overwrites, belongs to the kernels before. The down GEMM's schedule
+  // was written two kernels ago (gate_up has waited for it before it let this grid start), so its producer can fetch
+  // the first weight tiles while gate_up still runs; only the activations have to be waited for.
+  if (STAGE == STREAM_GATE_UP) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+  } else {
+    grid_launch_dependents();
+    if (warp != kProducerWarp) grid_dependency_wait();
+  }
 
   const int blocks = min(p.max_blocks, *p.num_post_pad / NT);
   const int total = blocks * p.n_tiles;
@@ -163,11 +185,13 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
 
   float acc[NT];
   bool sum_ok = false;
-  int my_block = -1, my_nt = 0;  // item whose sums acc holds
+  int my_block = -1, my_nt = 0, my_buf = 0;  // item whose sums acc holds
 
   // Work after the K loop of one item, by the eight promotion warps (256 threads, named barriers 1..3)
   const int half = warp >> 2, r = threadIdx.x & 127;
   auto epilogue = [&]() {
+    const float* row_w = row_w_of(my_buf);
+    const int* row_id = row_id_of(my_buf);
     const int row0 = my_block * NT;
     if constexpr (STAGE == STREAM_GATE_UP) {
       if (p.topk_weights != nullptr) {  // router weight on the fp32 product, before the activation
@@ -215,13 +239,28 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     if (ptx::elect_one()) {
       int s = 0;
       uint32_t phase = 1;
-      bool ok = true;
+      bool ok = true, waited = STAGE == STREAM_GATE_UP;
       for (int item = item0; item < total && ok; item += step) {
         const int blk = item / p.n_tiles, nt = item - blk * p.n_tiles;
         const int e = p.expert_ids[blk];
         if (e < 0) continue;
         const int ra = weight_row(e, nt, 0), rb = weight_row(e, nt, 1);
-        for (int kb = kb0; kb < kb1; ++kb) {
+        int kb = kb0;
+        if (!waited) {  // first item: the ring is empty, fill it with weights, then wait, then the token tiles
+          const int n = min(S, nkb);
+          for (int i = 0; i < n; ++i) {
+            ptx::mbar_expect_tx(full_bar(i), Cfg::kStage);
+            ptx::tma_load_2d(sW + i * Cfg::kStageW, &tmap_w, (kb0 + i) * kBK, ra, full_bar(i));
+            ptx::tma_load_2d(sW + i * Cfg::kStageW + 128 * kBK, &tmap_w, (kb0 + i) * kBK, rb, full_bar(i));
+          }
+          grid_dependency_wait();
+          waited = true;
+          for (int i = 0; i < n; ++i) ptx::tma_load_2d(sX + i * Cfg::kStageX, &tmap_x, (kb0 + i) * kBK, blk * NT, full_bar(i));
+          kb = kb0 + n;
+          s = n % S;
+          if (n == S) phase ^= 1;
+        }
+        for (; kb < kb1; ++kb) {
           ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
           if (!ok) break;
           ptx::mbar_expect_tx(full_bar(s), Cfg::kStage);
@@ -262,36 +301,56 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
       }
     }
     __syncwarp();
-  } else {
-    const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half * NT;
-    uint32_t it = 0;
-    bool ok = true;
-    for (int item = item0; item < total && ok; item += step) {
+  } else if (warp > kMmaWarp) {
+    const int tid = threadIdx.x - (kMmaWarp + 1) * 32;  // 0..63
+    uint32_t n_item = 0;
+    for (int item = item0; item < total; item += step) {
       const int blk = item / p.n_tiles, nt = item - blk * p.n_tiles;
       const int e = p.expert_ids[blk];
       if (e < 0) continue;
-      named_bar_sync(1, 256);  // every warp is done with the tables of the previous item
-      for (int i = threadIdx.x; i < nkb * NT; i += 256)
-        table[i] = __ldg(p.As + (int64_t)(kb0 + i / NT) * p.as_ld + blk * NT + i % NT);
-      for (int i = threadIdx.x; i < 2 * nkb; i += 256) {
+      const int tb = n_item & 1;
+      if (!ptx::mbar_wait(tab_empty_bar(tb), ((n_item >> 1) & 1) ^ 1, abort_flag)) break;
+      float4* table = reinterpret_cast<float4*>(table_of(tb));
+      constexpr int V = NT / 4;  // 16-byte vectors per K block: as_ld and the block's first row are multiples of 16
+      const float* as = p.As + (int64_t)kb0 * p.as_ld + blk * NT;
+#pragma unroll 8
+      for (int i = tid; i < nkb * V; i += 64)
+        table[i] = __ldg(reinterpret_cast<const float4*>(as + (int64_t)(i / V) * p.as_ld) + i % V);
+      float* bs_tab = bs_tab_of(tb);
+#pragma unroll 4
+      for (int i = tid; i < 2 * nkb; i += 64) {
         const int h = i >= nkb, kb = i - h * nkb;
         bs_tab[h * p.table_kb + kb] = __ldg(p.Bs + (int64_t)scale_row(e, nt, h) * p.num_kb + kb0 + kb);
       }
-      if (threadIdx.x < NT) {
-        const int flat = p.sorted_ids[blk * NT + threadIdx.x];
-        row_id[threadIdx.x] = flat;
-        row_w[threadIdx.x] = p.topk_weights == nullptr ? 1.f : flat < p.numel ? __ldg(p.topk_weights + flat) : 0.f;
+      if (tid < NT) {
+        const int flat = p.sorted_ids[blk * NT + tid];
+        row_id_of(tb)[tid] = flat;
+        row_w_of(tb)[tid] = p.topk_weights == nullptr ? 1.f : flat < p.numel ? __ldg(p.topk_weights + flat) : 0.f;
       }
-      named_bar_sync(1, 256);
-      my_block = blk, my_nt = nt;
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(tab_full_bar(tb));
+      ++n_item;
+    }
+    __syncwarp();
+  } else {
+    const uint32_t lane_base = tmem_base + ((uint32_t)((warp & 3) * 32) << 16) + half * NT;
+    uint32_t it = 0, n_item = 0;
+    bool ok = true;
+    for (int item = item0; item < total && ok; item += step) {
+      const int blk = item / p.n_tiles, nt = item - blk * p.n_tiles;
+      if (p.expert_ids[blk] < 0) continue;
+      const int tb = n_item & 1;
+      ok = ptx::mbar_wait(tab_full_bar(tb), (n_item >> 1) & 1, abort_flag);
+      my_block = blk, my_nt = nt, my_buf = tb;
+      const float *table = table_of(tb), *bs_tab = bs_tab_of(tb) + half * p.table_kb;
 #pragma unroll
       for (int t = 0; t < NT; ++t) acc[t] = 0.f;
-      for (int j = 0; j < nkb; ++j, ++it) {
+      for (int j = 0; j < nkb && ok; ++j, ++it) {
         const int b = it % NB;
         ok = ptx::mbar_wait(tfull_bar(b), (it / NB) & 1, abort_flag);
         if (!ok) break;
         ptx::tc_fence_after();
-        const float bs = bs_tab[half * p.table_kb + j];
+        const float bs = bs_tab[j];
         const float4* sc = reinterpret_cast<const float4*>(table + j * NT);
         constexpr int CH = NT < 32 ? NT : 32;
 #pragma unroll
@@ -319,10 +378,13 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
           }
         }
       }
+      ++n_item;
       if (csize > 1) break;  // one item per cluster: finished below
       // a warp whose wait gave up must not leave the others alone at the barriers of the epilogue
       if (named_bar_any(1, 256, !ok)) break;
       epilogue();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(tab_empty_bar(tb));
     }
     if (csize > 1) sum_ok = !named_bar_any(1, 256, !ok);
   }
@@ -400,23 +462,9 @@ inline int launch_stream(const void* W, int64_t w_rows, const void* X, int64_t x
   if (rc) return rc;
   auto k = stream_gemm_kernel<NT, STAGE, OutT>;
   if (int rc_smem = allow_smem(k, Cfg::kSmemLimit, "stream_gemm_kernel")) return rc_smem;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(csize > 1 ? items * csize : items < sms ? items : sms));
-  cfg.blockDim = dim3(Cfg::kThreads);
-  cfg.dynamicSmemBytes = Cfg::smem_for(p.stages, p.table_kb);
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = csize;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = csize > 1 ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, tw, tx, p);
-  if (e != cudaSuccess) {
-    set_error_detail("stream_gemm_kernel: %s", cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
-  return check_launch("stream_gemm_kernel");
+  const int64_t grid = csize > 1 ? items * csize : items < sms ? items : sms;
+  return launch_dependent(k, dim3((unsigned)grid), Cfg::kThreads, Cfg::smem_for(p.stages, p.table_kb), st, csize,
+                          "stream_gemm_kernel", tw, tx, p);
 }
 
 }  // namespace b200

@@ -29,14 +29,13 @@ using at::Tensor;
 struct Abi {
   decltype(&b200_status_string) status_string;
   decltype(&b200_last_error_detail) last_error_detail;
-  decltype(&b200_get_tuning) get_tuning;
   decltype(&b200_per_token_group_quant_fp8) quant;
   decltype(&b200_per_token_group_quant_fp8_ue8m0) quant_ue8m0;
   decltype(&b200_w8a8_block_fp8_gemm_workspace_bytes) gemm_ws;
   decltype(&b200_w8a8_block_fp8_gemm) gemm;
   decltype(&b200_w8a8_block_fp8_gemm_ue8m0) gemm_ue8m0;
-  decltype(&b200_w8a8_block_fp8_linear_decode_workspace_bytes) decode_ws;
-  decltype(&b200_w8a8_block_fp8_linear_decode) decode;
+  decltype(&b200_w8a8_block_fp8_linear_workspace_bytes) linear_ws;
+  decltype(&b200_w8a8_block_fp8_linear) linear;
   decltype(&b200_fused_experts_fp8_workspace_bytes) experts_ws;
   decltype(&b200_fused_experts_fp8) experts;
   decltype(&b200_route_topk) route;
@@ -113,27 +112,18 @@ at::ScalarType dtype_of_code(long code) {
   return code == B200_BF16 ? at::kBFloat16 : code == B200_F16 ? at::kHalf : at::kFloat;
 }
 int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
-size_t align256(size_t n) { return (n + 255) & ~(size_t)255; }
 void* stream_of(int device) { return c10::cuda::getCurrentCUDAStream((c10::DeviceIndex)device).stream(); }
-bool knob_off(const char* name) {
-  long v = -1;
-  abi.get_tuning(name, &v);
-  return v == 0;
-}
 constexpr auto kFp8 = at::kFloat8_e4m3fn;
-// Activation bytes up to which the quantised copy lives in the scratch buffer (no tensor to allocate); larger
-// copies are worth a block of the caching allocator, which other work can use in between.
-constexpr size_t kScratchActivation = 8u << 20;
+constexpr size_t kKeptScratch = 32u << 20;
 
-// linear(x, weight, weight_scale, decode_max_rows): quantise per 1x128 group, block-FP8 GEMM, result of x's type.
+// linear(x, weight, weight_scale): quantise per 1x128 group, block-FP8 GEMM, result of x's type.
 PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 4) Py_RETURN_NONE;
+  if (nargs != 3) Py_RETURN_NONE;
   const int dev = c10::cuda::current_device();
   const Tensor* x = plain(args[0], dev);
   const Tensor* w = plain(args[1], dev, kFp8);
   const Tensor* ws = plain(args[2], dev, at::kFloat);
-  const long decode_rows = PyLong_AsLong(args[3]);
   if (!x || !w || !ws || x->dim() < 1 || w->dim() != 2 || !x->is_contiguous()) Py_RETURN_NONE;
   const auto type = x->scalar_type();
   const int code = dtype_code(type);
@@ -145,34 +135,12 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   shape.back() = N;
   Tensor out = empty_on(dev, shape, type);
   void* st = stream_of(dev);
-  if (M <= decode_rows && N <= 4096 * 128 && !knob_off("linear_decode_fused")) {
-    const size_t need = abi.decode_ws(M, N, K);
-    const Tensor scratch_buf = need ? workspace(dev, st, need) : Tensor();
-    const int rc = abi.decode(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K, 1e-10f,
-                              need ? scratch_buf.data_ptr() : nullptr, need, tickets_of(dev, st), st);
-    if (rc) return fail(rc, "w8a8_block_fp8_linear (decode)");
-    return THPVariable_Wrap(std::move(out));
-  }
-  const size_t qb = align256((size_t)(M * K)), sb = align256((size_t)(M * (K / 128)) * 4), gb = abi.gemm_ws(M, N, K);
-  const bool inside = qb <= kScratchActivation;
-  const size_t need = gb + (inside ? qb + sb : 0);
-  Tensor q_own, s_own;
-  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
-  uint8_t* base = need ? static_cast<uint8_t*>(buf.data_ptr()) : nullptr;
-  uint8_t* q = base;
-  float* s = reinterpret_cast<float*>(base + qb);
-  uint8_t* gws = inside ? base + qb + sb : base;
-  if (!inside) {
-    q_own = empty_on(dev, {M, K}, kFp8);
-    s_own = empty_on(dev, {K / 128, M}, at::kFloat);
-    q = static_cast<uint8_t*>(q_own.data_ptr());
-    s = s_own.data_ptr<float>();
-  }
-  // scales column-major: the GEMM reads one contiguous run of row scales per K block
-  int rc = abi.quant(x->data_ptr(), code, q, s, M, K, 128, 1, M, 1e-10f, B200_QUANT_DIV_CORRECTED, st);
-  if (rc) return fail(rc, "per_token_group_quant_fp8");
-  rc = abi.gemm(q, s, 1, M, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), code, M, N, K, gb ? gws : nullptr, gb, st);
-  if (rc) return fail(rc, "w8a8_block_fp8_matmul");
+  const size_t need = abi.linear_ws(M, N, K);
+  // a large scratch (long prefill) is worth a block of the caching allocator, which other work can use in between
+  const Tensor buf = need == 0 ? Tensor() : need <= kKeptScratch ? workspace(dev, st, need) : empty_on(dev, {(int64_t)need}, at::kByte);
+  const int rc = abi.linear(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K,
+                            need ? buf.data_ptr() : nullptr, need, tickets_of(dev, st), st);
+  if (rc) return fail(rc, "w8a8_block_fp8_linear");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
 }
@@ -369,14 +337,13 @@ PyObject* bind(PyObject*, PyObject* arg) {
   };
   get(abi.status_string, "b200_status_string");
   get(abi.last_error_detail, "b200_last_error_detail");
-  get(abi.get_tuning, "b200_get_tuning");
   get(abi.quant, "b200_per_token_group_quant_fp8");
   get(abi.quant_ue8m0, "b200_per_token_group_quant_fp8_ue8m0");
   get(abi.gemm_ws, "b200_w8a8_block_fp8_gemm_workspace_bytes");
   get(abi.gemm, "b200_w8a8_block_fp8_gemm");
   get(abi.gemm_ue8m0, "b200_w8a8_block_fp8_gemm_ue8m0");
-  get(abi.decode_ws, "b200_w8a8_block_fp8_linear_decode_workspace_bytes");
-  get(abi.decode, "b200_w8a8_block_fp8_linear_decode");
+  get(abi.linear_ws, "b200_w8a8_block_fp8_linear_workspace_bytes");
+  get(abi.linear, "b200_w8a8_block_fp8_linear");
   get(abi.experts_ws, "b200_fused_experts_fp8_workspace_bytes");
   get(abi.experts, "b200_fused_experts_fp8");
   get(abi.route, "b200_route_topk");

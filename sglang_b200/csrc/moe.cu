@@ -10,6 +10,7 @@
 //   5 sum_reduce       fp32 sum over the top-k slots -> out                     (HBM bound)
 // Scales of the two intermediate activations are stored column-major ([K/128][rows]) so a
 // GEMM promotion warp reads 32 consecutive floats per K block.
+#include <math.h>
 #include <stdlib.h>
 
 #include "gemm_host.cuh"
@@ -118,6 +119,91 @@ __global__ void __launch_bounds__(256) moe_gather_fp8_kernel(
   }
 }
 
+// A few pairs (the weight-streaming path): align, quantise and gather in ONE launch, one block per (token, slot)
+// pair. The position of a pair in the expert-sorted layout is the padded size of the lower experts' runs plus its
+// rank among the pairs of its expert: two sums over a histogram and one over the ids, cheap enough for every block
+// to redo (numel <= 1024) instead of passing them through memory between three kernels. Same layout as
+// moe_align_block_size, without the runs of ids that are not on this rank. One token of 256 experts: 3 kernels, 9.5 us
+// plus two launch gaps -> one of 5 us.
+constexpr int kPrepMaxPairs = 1024;
+template <typename T>
+__global__ void __launch_bounds__(256) moe_prep_kernel(const T* __restrict__ hidden, const uint8_t* __restrict__ hidden_q,
+                                                       const float* __restrict__ hidden_s, const int32_t* __restrict__ topk_ids,
+                                                       int32_t* __restrict__ sorted, int32_t* __restrict__ expert_ids,
+                                                       int32_t* __restrict__ npp, uint8_t* __restrict__ q,
+                                                       float* __restrict__ s, int64_t H, int E, int numel, int topk, int block_m,
+                                                       int64_t cap) {
+  __shared__ int cnt[1024];
+  __shared__ int part[3][8];
+  const int tid = threadIdx.x, i = blockIdx.x;
+  for (int b = tid; b < E; b += 256) cnt[b] = 0;
+  grid_dependency_wait();
+  grid_launch_dependents();
+  __syncthreads();
+  const int mine = __ldg(topk_ids + i);
+  const bool valid = mine >= 0 && mine < E;
+  if (!valid && i != 0) return;
+  int rank = 0;
+  for (int j = tid; j < numel; j += 256) {
+    const int e = __ldg(topk_ids + j);
+    if (e >= 0 && e < E) {
+      atomicAdd(&cnt[e], 1);
+      rank += (e == mine && j < i) ? 1 : 0;
+    }
+  }
+  __syncthreads();
+  int before = 0, total = 0;
+  for (int b = tid; b < E; b += 256) {
+    const int padded = (cnt[b] + block_m - 1) / block_m * block_m;
+    total += padded;
+    before += b < mine ? padded : 0;
+  }
+  rank = __reduce_add_sync(0xffffffffu, rank);
+  before = __reduce_add_sync(0xffffffffu, before);
+  total = __reduce_add_sync(0xffffffffu, total);
+  if ((tid & 31) == 0) part[0][tid >> 5] = rank, part[1][tid >> 5] = before, part[2][tid >> 5] = total;
+  __syncthreads();
+  rank = before = total = 0;
+#pragma unroll
+  for (int w = 0; w < 8; ++w) rank += part[0][w], before += part[1][w], total += part[2][w];
+  if (i == 0 && tid == 0) *npp = total;
+  if (!valid) return;
+  const int pos = before + rank, run = cnt[mine];
+  if (tid == 0) {
+    sorted[pos] = i;
+    if (rank % block_m == 0) expert_ids[pos / block_m] = mine;
+  }
+  if (rank == run - 1)  // the last pair of an expert marks the pad rows behind it
+    for (int k = run + tid; k < (run + block_m - 1) / block_m * block_m; k += 256) sorted[before + k] = numel;
+  const int64_t tok = i / topk;
+  for (int c0 = tid & ~31; c0 < H / 16; c0 += 256) {  // whole warps; 8 consecutive lanes share a 128-group
+    const int chunk = c0 + (tid & 31);
+    const bool active = chunk < H / 16;
+    uint4 out;
+    float scale;
+    if (hidden_q != nullptr) {
+      out = active ? ld_nc_16(hidden_q + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
+      scale = active && (chunk & 7) == 0 ? __ldg(hidden_s + tok * (H / 128) + chunk / 8) : 0.f;
+    } else {
+      uint4 raw[2];
+      raw[0] = active ? ld_nc_16(hidden + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
+      raw[1] = active ? ld_nc_16(hidden + tok * H + chunk * 16 + 8) : make_uint4(0, 0, 0, 0);
+      const T* v = reinterpret_cast<const T*>(raw);
+      float f[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) f[k] = to_f32<T>(v[k]);
+      float amax = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(f[k]));
+      amax = fmaxf(group_max<8>(amax), 1e-10f);
+      scale = quant16(f, amax, B200_QUANT_DIV_CORRECTED, out);  // the stand-alone quantiser's bytes and scales
+    }
+    if (!active) continue;
+    *reinterpret_cast<uint4*>(q + (int64_t)pos * H + chunk * 16) = out;
+    if ((chunk & 7) == 0) s[(int64_t)(chunk / 8) * cap + pos] = scale;
+  }
+}
+
 // out[t, :] = scale * sum_j y[t*topk + j, :] over the slots whose expert id is valid. One block per token: the
 // valid slots are listed once in shared memory, so a row none of whose slots is valid (most rows of an
 // expert-parallel receive area) costs one read of its ids, and there is no per-thread division. Four row loads
@@ -130,10 +216,11 @@ __global__ void __launch_bounds__(256, 6) moe_sum_reduce_kernel(const T* __restr
   __shared__ int s_slot[kSumReduceMaxSlots];
   __shared__ int s_n;
   const int64_t t = blockIdx.x;
+  grid_dependency_wait();
   if (poison_status != nullptr && *reinterpret_cast<const volatile int*>(poison_status) != 0) {
     // the rows were to be written by other GPUs and the handshake before this kernel gave up: NaNs, not stale rows
     const uint4 nan16 = make_uint4(0xffffffffu, 0xffffffffu, 0xffffffffu, 0xffffffffu);  // NaN in bf16 and fp16
-    for (int64_t c = threadIdx.x * 8; c < H; c += blockDim.x * 8) *reinterpret_cast<uint4*>(out + t * H + c) = nan16;
+    for (int64_t c = (blockIdx.y * blockDim.x + threadIdx.x) * 8; c < H; c += (int64_t)gridDim.y * blockDim.x * 8) *reinterpret_cast<uint4*>(out + t * H + c) = nan16;
     return;
   }
   if (threadIdx.x < 32) {  // warp 0 compacts the valid slots, ascending (topk <= 64: two rounds of 32)
@@ -153,7 +240,7 @@ __global__ void __launch_bounds__(256, 6) moe_sum_reduce_kernel(const T* __restr
   if (n == 0 && skip_unrouted) return;  // a row no local expert serves: nobody reads it
   const int vec_per_row = (int)(H / 8);
   const T* base = y + t * topk * H;
-  for (int v = threadIdx.x; v < vec_per_row; v += blockDim.x) {
+  for (int v = blockIdx.y * blockDim.x + threadIdx.x; v < vec_per_row; v += gridDim.y * blockDim.x) {
     float acc[8];
 #pragma unroll
     for (int i = 0; i < 8; ++i) acc[i] = 0.f;
@@ -243,16 +330,20 @@ struct MoeWorkspace {
 
 // Rows per expert block of the sorted layout, and with it the kernel: 16 / 32 / 64 for the weight-streaming kernel,
 // 128 for the tile kernel. An expert's weights are read once per block of its rows, so the block should hold the
-// rows of most experts; a wider one costs promotion work for columns of padding.
+// rows of a busy expert; a wider one only adds columns of padding. With evenly loaded experts a busy one has about
+// avg + 2 sqrt(avg) rows; with few experts the router skews more and the hottest ones set the time: twice the
+// average. Layer times in us for blocks of 16 / 32 / 64 / 128 rows: 256 experts (7168 x 2048) at 8 rows on average
+// 1807 / 1795 / 1944 / 2202, 16: 2178 / 1825 / 1958 / 2169, 32: 2854 / 2160 / 1968 / 2172, 64: 4044 / 2978 / 2736 /
+// 2257; 8 skewed experts (4096 x 14336) at 4: 207 / 216 / 237 / 240, 8: 269 / 241 / 266 / 270, 32: 422 / 346 / 356 / 292.
 static int moe_block_rows(int64_t numel, int E) {
   const long knob = tuning().moe_decode;
   if (knob == 0) return kMoeBlockM;
   if (knob == 16 || knob == 32 || knob == 64) return (int)knob;
-  const int64_t reached = numel < E ? numel : E;
-  const int64_t avg = numel / reached;
-  if (avg <= 8) return 16;
-  if (avg <= 20) return 32;
-  if (avg <= 48 || knob == 1) return 64;
+  const double avg = (double)numel / (double)(numel < E ? numel : E);
+  const double busy = (E <= 32 ? 2.0 : 1.0) * avg + 2.0 * sqrt(avg);
+  if (busy <= 16) return 16;
+  if (busy <= 32) return 32;
+  if (busy <= 64 || knob == 1) return 64;
   return kMoeBlockM;
 }
 
@@ -334,10 +425,14 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   const bool split = down_splits > 1;
   T* c3 = no_combine && !split ? static_cast<T*>(out) : reinterpret_cast<T*>(ws + L.off_c3);
 
-  int rc = b200_moe_align_block_size(topk_ids, B200_I32, numel, E + 1, L.block_m, sorted, L.cap, expert_ids,
-                                     L.cap_blocks, npp, cumsum, 1, ws + L.off_align,
-                                     b200_moe_align_workspace_bytes(numel, E + 1), st);
-  if (rc) return rc;
+  int rc = B200_OK;
+  const bool one_launch = stream && numel <= kPrepMaxPairs && E <= 1024;
+  if (!one_launch) {
+    rc = b200_moe_align_block_size(topk_ids, B200_I32, numel, E + 1, L.block_m, sorted, L.cap, expert_ids,
+                                       L.cap_blocks, npp, cumsum, 1, ws + L.off_align,
+                                       b200_moe_align_workspace_bytes(numel, E + 1), st);
+    if (rc) return rc;
+  }
   if (no_combine && !split && scatter == nullptr) {
     // rows of slots whose expert is not on this rank are never written by GEMM 2
     cudaError_t e = cudaMemsetAsync(out, 0, (size_t)numel * H * sizeof(T), st);
@@ -346,7 +441,13 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
       return B200_E_LAUNCH;
     }
   }
-  {
+  if (one_launch) {
+    rc = launch_dependent(moe_prep_kernel<T>, dim3((unsigned)numel), 256, 0, st, 1, "moe_prep_kernel",
+                          hidden_scale ? nullptr : static_cast<const T*>(hidden),
+                          hidden_scale ? static_cast<const uint8_t*>(hidden) : nullptr, hidden_scale, topk_ids, sorted,
+                          expert_ids, npp, aq1, as1, H, E, (int)numel, topk, L.block_m, L.cap);
+    if (rc) return rc;
+  } else {
     const uint8_t* hq = static_cast<const uint8_t*>(hidden);
     const float* hs = hidden_scale;
     if (hs == nullptr && L.quant_first) {
@@ -384,9 +485,10 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
 #undef B200_STREAM
     if (rc) return rc;
     if (no_combine) return B200_OK;
-    moe_sum_reduce_kernel<T><<<(unsigned)T_tokens, 256, 0, st>>>(c3, topk_ids, static_cast<T*>(out), topk, E, H,
-                                                                  routed_scale, skip_unrouted, nullptr);
-    return check_launch("moe_sum_reduce");
+    // a few tokens: several blocks per token, one 16-byte vector per thread
+    const unsigned cols = T_tokens <= 512 ? (unsigned)cdiv(H / 8, 256) : 1u;
+    return launch_dependent(moe_sum_reduce_kernel<T>, dim3((unsigned)T_tokens, cols), 256, 0, st, 1, "moe_sum_reduce", c3,
+                            topk_ids, static_cast<T*>(out), topk, E, H, routed_scale, skip_unrouted, nullptr);
   }
   const int force_bn = tuning().gemm_bn == 128 || tuning().gemm_bn == 256 ? (int)tuning().gemm_bn : 0;
   // expected live row tiles: every pair once, plus up to one partial tile per expert

@@ -11,12 +11,14 @@ template <typename T, int LPG, int FORMULA>
 __global__ void __launch_bounds__(256) quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ q,
                                                           float* __restrict__ s, int64_t total_chunks,
                                                           int chunks_per_row, int64_t s_stride_m,
-                                                          int64_t s_stride_g, float eps) {
+                                                          int64_t s_stride_g, float eps, int early) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = c < total_chunks;  // whole lane-groups are active or not (total % LPG == 0)
-  // a GEMM launched as programmatic dependent may set itself up now; it waits for this grid's
-  // completion before it reads the bytes and scales written here
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  // A GEMM launched as programmatic dependent may set itself up (and fetch weights) now; it waits for this grid's
+  // completion before it reads the bytes and scales written here. Not for the stand-alone quantiser, whose output
+  // may itself be the next GEMM's weights.
+  if (early) grid_launch_dependents();
+  grid_dependency_wait();  // x, and the readers of the buffers overwritten below
   float f[16];
   if (active) {
     Vec16<T>::load(x + c * 16, f);
@@ -55,7 +57,7 @@ static int launch_quant(const void* x, void* q, float* s, int64_t M, int64_t K, 
 #define B200_Q_LAUNCH_F(LPG, F)                                                                            \
   quant_group_kernel<T, LPG, F><<<(unsigned)blocks, threads, 0, st>>>(static_cast<const T*>(x),            \
                                                                       static_cast<uint8_t*>(q), s, total, \
-                                                                      cpr, ssm, ssg, eps)
+                                                                      cpr, ssm, ssg, eps, 0)
 #define B200_Q_LAUNCH(LPG)                                        \
   switch (formula) {                                              \
     case B200_QUANT_RECIP: B200_Q_LAUNCH_F(LPG, B200_QUANT_RECIP); break; \
@@ -77,6 +79,19 @@ static int launch_quant(const void* x, void* q, float* s, int64_t M, int64_t K, 
 #undef B200_Q_LAUNCH
 #undef B200_Q_LAUNCH_F
   return check_launch("per_token_group_quant_fp8");
+}
+
+template <typename T>
+static int launch_quant_for_linear(const void* x, void* q, float* s, int64_t M, int64_t K, cudaStream_t st) {
+  const int64_t total = M * (K / 16);
+  return launch_dependent(quant_group_kernel<T, 8, B200_QUANT_DIV_CORRECTED>, dim3((unsigned)cdiv(total, 256)), 256, 0, st, 1,
+                          "per_token_group_quant_fp8", static_cast<const T*>(x), static_cast<uint8_t*>(q), s, total,
+                          (int)(K / 16), 1, M, 1e-10f, 1);
+}
+
+int quant_for_linear(const void* x, int x_dtype, void* q, float* s, int64_t M, int64_t K, cudaStream_t st) {
+  return x_dtype == B200_BF16 ? launch_quant_for_linear<__nv_bfloat16>(x, q, s, M, K, st)
+                              : launch_quant_for_linear<__half>(x, q, s, M, K, st);
 }
 
 // Power-of-two ("UE8M0") scales, packed for MN-major consumers: the scale of (row t, group g) is

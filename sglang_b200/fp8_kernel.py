@@ -333,7 +333,7 @@ def w8a8_block_fp8_linear(
     assert input_scale is None
     if list(block_size) == [128, 128] and _QUANT_FORMULA == 0:
         N.load()
-        output = N.host.linear(input, weight, weight_scale, DECODE_FUSED_MAX_M)
+        output = N.host.linear(input, weight, weight_scale)
         if output is not None:
             if bias is not None:
                 output += bias
