@@ -60,7 +60,7 @@ int b200_read_device_status(int* out, void* stream);
  * Product calls never read the environment; a knob left at -1 is decided automatically.
  * Names: "gemm_bn" (128 / 256), "gemm_skinny" (0 = never the decode kernel),
  * "gemm_skinny_max_m", "gemm_splitk" (> 0 forces the K split; size the workspace after setting
- * it), "gemm_2cta" (0 / 1), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
+ * it), "gemm_2cta" (0 = never CTA pairs, 1 = always, 128 / 192 / 256 = always with that tile width), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
  * fp32-scale kernels), "linear_decode_fused" (0 = never the one-launch decode linear), "moe_decode"
  * (0 = never the weight-streaming MoE kernels, 1 = always, 16 / 32 / 64 = always with that row block), "moe_down_splitk" (0 = never),
  * "moe_zero_pads" (0 / 1), "peer_wait_ms" (limit of a device-side wait for another GPU, 100 .. 60000).
@@ -131,6 +131,17 @@ int b200_w8a8_block_fp8_gemm(const void* A, const float* As, int64_t as_stride_m
 int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
                                    const int32_t* sfb, int64_t sfb_ld, int sfb_rows_per_word, void* C,
                                    int c_dtype, int64_t M, int64_t N, int64_t K, void* stream);
+
+/* ---------------------------------------------------------------------------------------
+ * w8a8_block_fp8_matmul with packed power-of-two scales, any M: the block-scaled kernel above or, where that is the
+ * faster way (a few rows, or tiles that leave SMs idle), the scales unpacked on the GPU (exact) and the fp32-scale
+ * kernels. Same arguments and limits as b200_w8a8_block_fp8_gemm_ue8m0; workspace: the given number of bytes
+ * (0 when the block-scaled kernel is taken), 256-byte aligned. */
+size_t b200_w8a8_block_fp8_gemm_packed_workspace_bytes(int64_t M, int64_t N, int64_t K);
+int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
+                                    const int32_t* sfb, int64_t sfb_ld, int sfb_rows_per_word, void* C,
+                                    int c_dtype, int64_t M, int64_t N, int64_t K, void* workspace,
+                                    size_t workspace_bytes, void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * w8a8_block_fp8_linear at decode size: quantise + GEMM + split-K sum in ONE launch

@@ -1,7 +1,7 @@
 // w8a8_block_fp8_matmul: dense block-FP8 GEMM entry point (tcgen05 / TMEM / TMA kernel in
 // gemm_kernel.cuh).
 #include "gemm_host.cuh"
-#include "gemm_2cta.cuh"
+#include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
 #include "linear_decode.cuh"
 #include "gemm_ue8m0.cuh"
@@ -68,16 +68,60 @@ static int launch_reduce(const float* partial, void* C, int64_t mn, int splits, 
 }  // namespace b200
 
 namespace b200 {
-constexpr int64_t kSkinnyMaxM = 64;  // rows up to which the swapped-operand decode kernel is used
-constexpr bool kPairedByDefault = false;  // CTA-pair kernel for large dense problems
+constexpr int64_t kSkinnyMaxM = 64;       // rows up to which the swapped-operand decode kernel is always used
+constexpr int64_t kSkinnyPlanMaxM = 256;  // ... and up to which it is considered
+struct GemmPlan {
+  int splits;   // K splits (fp32 partials + a reduction pass when > 1)
+  int pair_bn;  // 0: single-CTA 128 x 256 tiles, else CTA pairs with 256 x pair_bn tiles
+  bool skinny;  // swapped-operand decode kernel
+  double us;    // modelled time (0: not modelled, decode sizes)
+};
+
+// Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up
+// (4.5 us), then whole waves of tiles: microseconds per 128-K block of a tile and 0.8 us for its epilogue; K splits add a
+// reduction pass (2 us and their fp32 partials, written and read at about 4 TB/s); nothing is faster than reading the
+// weights (6.2 TB/s). The decode kernel re-reads the weights for every 32 rows at the L2's 10.5 TB/s. The constants are
+// fits to measurements at 10 weight shapes (1280..28672 x 1024..14336) and 8 row counts (72..1027), where the plan is
+// within 10 % of the best configuration; what they decide is mostly wave counts, e.g. 203 x 6144 x 4096: single 22.3 us,
+// pair 256 wide 19.5, pair 128 wide 15.8; 1027 x 8192 x 3584: single 35.3, pair 44.3 and up.
+static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair) {
+  const Tuning& tune = tuning();
+  const int64_t num_kb = cdiv(K, 128);
+  const int64_t skinny_max = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
+  const bool skinny_ok = may_pair && tune.gemm_skinny != 0;
+  if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, 0.0};
+  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : (int)tune.gemm_2cta, false, 0.0};
+  GemmPlan best = {1, 0, false, 1e30};
+  const double stream_us = (double)N * (double)K / 6.2e6;
+  auto consider = [&](int bm, int bn, int slots, double us_per_kb, int pair_bn) {
+    const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
+    for (int s = 1; s <= 8 && (s == 1 || num_kb >= 4 * s); ++s) {
+      const double waves = (double)cdiv(tiles * s, slots);
+      double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + 0.8);
+      if (work < stream_us) work = stream_us;
+      const double us = 4.5 + work + (s > 1 ? 2.0 + 8.0 * s * (double)M * (double)N / 4e6 : 0.0);
+      if (us < best.us) best = {s, pair_bn, false, us};
+      if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
+    }
+  };
+  consider(128, N > 128 ? 256 : 128, sms, 0.54, 0);
+  if (may_pair && tune.gemm_2cta != 0 && N >= 256) {
+    consider(256, 256, sms / 2, 0.47, 256);
+    consider(256, 192, sms / 2, 0.44, 192);
+    consider(256, 128, sms / 2, 0.34, 128);
+  }
+  const double skinny_us = 4.5 + (double)cdiv(M, 32) * (double)N * (double)K / 10.5e6;
+  if (skinny_ok && tune.gemm_skinny_max_m < 0 && M <= kSkinnyPlanMaxM && skinny_us < best.us)
+    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, skinny_us};
+  return best;
+}
 }
 
 extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  // sized for the largest split any SM count <= 148 picks (or the tuning knobs force)
+  // sized for the split that 148 SMs pick (or the tuning knobs force)
   const b200::Tuning& tune = b200::tuning();
-  int s = M <= b200::kSkinnyMaxM ? b200::skinny_k_splits(M, N, K, b200::skinny_token_tile(M), 148)
-                                 : b200::choose_k_splits(M, N, K, 148);
+  int s = b200::plan_gemm(M, N, K, 148, tune.gemm_bn < 0).splits;
   if (tune.gemm_splitk > s) s = (int)tune.gemm_splitk;
   if (tune.gemm_skinny_max_m >= 0 && s < 16) s = 16;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
@@ -111,9 +155,9 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
   B200_CHECK_ARG(c_dtype == B200_BF16 || c_dtype == B200_F16 || c_dtype == B200_F32, "gemm: unknown output dtype code %d",
                  c_dtype);
   const int sms = sm_count() < 148 ? sm_count() : 148;
-  const int64_t skinny_max_m = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
-  const bool skinny = M <= skinny_max_m && force_bn == 0 && tune.gemm_skinny != 0;
-  int splits = skinny ? skinny_k_splits(M, N, K, skinny_token_tile(M), sms) : choose_k_splits(M, N, K, sms);
+  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0);
+  const bool skinny = plan.skinny;
+  int splits = plan.splits;
   if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
   if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
   if (skinny) {
@@ -140,8 +184,9 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
+  const int bn = plan.pair_bn;
   if (splits > 1) {
-    // decode-sized problem: fp32 partials per K split in the workspace, then one reduction pass
+    // few tiles: fp32 partials per K split in the workspace, then one reduction pass
     const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15) != 0) {
       set_error_detail("gemm: split-K needs a 16-byte aligned workspace of %zu bytes (got %zu)", need, workspace_bytes);
@@ -150,30 +195,23 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     p.C = workspace;
     p.split_stride = M * N;
     p.n_dest = 0;  // the partials stay local; the reduction pass fans the sum out
-    int rc = launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, 0, splits);
+    int rc = bn ? launch_gemm_pair<float>(bn, A, B, p, splits, st)
+                : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, 0, splits);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
     if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
     if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
-  // Large dense problems with 16-bit output: CTA pairs (each CTA loads half of the B tile)
-  {
-    const int mode2 = (int)tune.gemm_2cta;  // 0 = never, 1 = whenever legal
-    const bool legal = c_dtype != B200_F32 && force_bn == 0 && N >= 256 && fan.n == 0;
-    const bool want = mode2 == 1 || (mode2 != 0 && kPairedByDefault && M >= 1024 && cdiv(M, 256) * cdiv(N, 256) >= 64);
-    if (legal && want) {
-      if (c_dtype == B200_BF16) return launch_gemm_2cta<__nv_bfloat16>(A, B, p, st);
-      return launch_gemm_2cta<__half>(A, B, p, st);
-    }
+  if (bn && fan.n == 0) {
+    if (c_dtype == B200_BF16) return launch_gemm_pair<__nv_bfloat16>(bn, A, B, p, 1, st);
+    if (c_dtype == B200_F16) return launch_gemm_pair<__half>(bn, A, B, p, 1, st);
+    return launch_gemm_pair<float>(bn, A, B, p, 1, st);
   }
   switch (c_dtype) {
     case B200_BF16: return launch_gemm<GEMM_DENSE, __nv_bfloat16>(A, B, N, p, force_bn, st);
     case B200_F16: return launch_gemm<GEMM_DENSE, __half>(A, B, N, p, force_bn, st);
-    case B200_F32: return launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st);
-    default:
-      set_error_detail("gemm: unknown output dtype code %d", c_dtype);
-      return B200_E_BAD_ARG;
+    default: return launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st);
   }
 }
 }  // namespace b200
@@ -189,7 +227,7 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_fanout_workspace_bytes(int64_t M, int
   if (M <= 0 || N <= 0 || K <= 0) return 0;
   const size_t plain = b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
   // the decode kernel always goes through an fp32 partial when its result is fanned out
-  const size_t one = M <= b200::kSkinnyMaxM ? (size_t)M * (size_t)N * sizeof(float) : 0;
+  const size_t one = M <= b200::kSkinnyPlanMaxM ? (size_t)M * (size_t)N * sizeof(float) : 0;
   return plain > one ? plain : one;
 }
 
@@ -322,4 +360,76 @@ extern "C" int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa,
       set_error_detail("gemm_ue8m0: unknown output dtype code %d", c_dtype);
       return B200_E_BAD_ARG;
   }
+}
+
+// ---------------------------------------------------------------- packed power-of-two scales, any M
+namespace b200 {
+// Packed exponent words -> the fp32 scales of the promotion kernels (exact): As column-major [num_kb][M], Bs
+// [n_blocks][num_kb]. One thread per word of four K blocks.
+__global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __restrict__ sfa, int64_t sfa_ld,
+                                                            const int32_t* __restrict__ sfb, int64_t sfb_ld, int sfb_step,
+                                                            float* __restrict__ as, float* __restrict__ bs, int M, int n_blocks,
+                                                            int num_kb) {
+  grid_launch_dependents();
+  grid_dependency_wait();
+  const int words = (num_kb + 3) / 4;
+  const int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < (int64_t)M * words) {
+    const int w = (int)(i / M), m = (int)(i - (int64_t)w * M);
+    const uint32_t e = (uint32_t)__ldg(sfa + w * sfa_ld + m);
+    for (int k = 0; k < 4 && 4 * w + k < num_kb; ++k) as[(int64_t)(4 * w + k) * M + m] = __uint_as_float((e >> (8 * k) & 0xffu) << 23);
+  } else if (i - (int64_t)M * words < (int64_t)n_blocks * words) {
+    const int j = (int)(i - (int64_t)M * words), w = j / n_blocks, n = j - w * n_blocks;
+    const uint32_t e = (uint32_t)__ldg(sfb + w * sfb_ld + (int64_t)n * sfb_step);
+    for (int k = 0; k < 4 && 4 * w + k < num_kb; ++k) bs[(int64_t)n * num_kb + 4 * w + k] = __uint_as_float((e >> (8 * k) & 0xffu) << 23);
+  }
+}
+
+// Whether the block-scaled kernel (tiles of 128 x 224, scales applied by the tensor core, no K split) beats the
+// promotion kernels on unpacked scales: below 65 rows the weight stream decides, then wave counts (see plan_gemm; a
+// 128-K block of a 128 x 224 tile takes 0.41 us, unpacking 2 us).
+static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
+  if (M <= kSkinnyMaxM) return false;
+  const double waves = (double)cdiv(cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN), sms);
+  return 4.5 + waves * ((double)cdiv(K, 128) * 0.41 + 0.3) <= plan_gemm(M, N, K, sms, true).us + 2.0;
+}
+static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
+static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }
+}  // namespace b200
+
+extern "C" size_t b200_w8a8_block_fp8_gemm_packed_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  using namespace b200;
+  if (M <= 0 || N <= 0 || K <= 0 || block_scaled_wins(M, N, K, 148)) return 0;
+  return packed_as_bytes(M, K) + packed_bs_bytes(N, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
+}
+
+extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
+                                               const int32_t* sfb, int64_t sfb_ld, int sfb_rows_per_word, void* C, int c_dtype,
+                                               int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes,
+                                               void* stream) {
+  using namespace b200;
+  B200_CHECK_ARG(M >= 0 && N >= 0 && K > 0, "gemm_packed: bad shape");
+  if (M == 0 || N == 0) return B200_OK;
+  const size_t need = b200_w8a8_block_fp8_gemm_packed_workspace_bytes(M, N, K);
+  if (need == 0)
+    return b200_w8a8_block_fp8_gemm_ue8m0(A, sfa, sfa_ld, B, sfb, sfb_ld, sfb_rows_per_word, C, c_dtype, M, N, K, stream);
+  B200_CHECK_ARG(sfa && sfb, "gemm_packed: null pointer");
+  B200_CHECK_ARG(sfb_rows_per_word == 1 || sfb_rows_per_word == 128, "gemm_packed: one scale word per row or per 128 rows of B");
+  B200_CHECK_ARG(sfa_ld >= M && sfb_ld >= cdiv(N, sfb_rows_per_word), "gemm_packed: scale row pitch shorter than the rows");
+  B200_UNSUPPORTED(M > 0x7fffff00LL || N > 0x7fffff00LL || K > 0x7fffff00LL, "gemm_packed: dimension too large");
+  if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0) {
+    set_error_detail("gemm_packed: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
+    return B200_E_WORKSPACE;
+  }
+  float* as = static_cast<float*>(workspace);
+  uint8_t* bs = static_cast<uint8_t*>(workspace) + packed_as_bytes(M, K);
+  uint8_t* rest = bs + packed_bs_bytes(N, K);
+  const int n_blocks = (int)cdiv(N, 128), num_kb = (int)cdiv(K, 128);
+  const int64_t total = (M + n_blocks) * cdiv(num_kb, 4);
+  int rc = launch_dependent(unpack_scales_kernel, dim3((unsigned)cdiv(total, 256)), 256, 0, static_cast<cudaStream_t>(stream), 1,
+                            "unpack_scales_kernel", sfa, sfa_ld, sfb, sfb_ld, 128 / sfb_rows_per_word, as,
+                            reinterpret_cast<float*>(bs), (int)M, n_blocks, num_kb);
+  if (rc) return rc;
+  return gemm_impl(A, as, 1, M, B, reinterpret_cast<const float*>(bs), C, c_dtype, M, N, K, rest,
+                   need - (size_t)(rest - static_cast<uint8_t*>(workspace)), stream, FanOut{});
 }

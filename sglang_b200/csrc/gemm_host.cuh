@@ -9,18 +9,6 @@
 
 namespace b200 {
 
-// Split-K factor for the dense GEMM: when the 128 x 256 tiles alone would leave most SMs idle
-// (a few hundred rows), split K so that about one work item per SM streams the weights.
-inline int choose_k_splits(int64_t M, int64_t N, int64_t K, int sms) {
-  const int64_t tiles = cdiv(M, 128) * cdiv(N, N > 128 ? 256 : 128);
-  const int64_t num_kb = cdiv(K, 128);
-  if (tiles * 4 >= (int64_t)sms * 3 || num_kb < 8) return 1;
-  int64_t s = sms / tiles;
-  if (s > num_kb / 4) s = num_kb / 4;
-  if (s > 8) s = 8;
-  return s < 1 ? 1 : (int)s;
-}
-
 // cuTensorMapEncodeTiled, resolved through the runtime so the library needs no -lcuda.
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*,
                                   const cuuint64_t*, const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave,
@@ -88,26 +76,28 @@ inline int make_tmap_u8(CUtensorMap* m, const void* base, uint64_t rows, uint64_
 }
 
 // Output tensor [S, rows, cols] (S = K splits, 1 otherwise) of `elem_bytes`-wide elements, stored
-// through boxes of [32 rows x 128 bytes] with the 128-byte swizzle.
+// through boxes of [32 rows x 128 bytes] with the 128-byte swizzle, or (box_cols > 0) of [32 rows x box_cols], without
+// a swizzle when those are not 128 bytes.
 inline int make_tmap_out(CUtensorMap* m, const void* base, uint64_t splits, uint64_t rows, uint64_t cols,
-                         int elem_bytes, bool is_bf16, const char* what) {
+                         int elem_bytes, bool is_bf16, const char* what, int box_cols = 0) {
   // kept per thread like the operand maps above: the allocator hands the same few output buffers out again
   struct Key {
     const void* base;
     uint64_t splits, rows, cols;
-    int elem_bytes, is_bf16;
+    int elem_bytes, is_bf16, box_cols;
     bool operator==(const Key& o) const {
       return base == o.base && splits == o.splits && rows == o.rows && cols == o.cols && elem_bytes == o.elem_bytes &&
-             is_bf16 == o.is_bf16;
+             is_bf16 == o.is_bf16 && box_cols == o.box_cols;
     }
   };
   struct Hash {
     size_t operator()(const Key& k) const {
-      return (size_t)((uintptr_t)k.base * 0x9E3779B97F4A7C15ull) ^ (size_t)(k.rows * 31 + k.cols * 131 + k.splits);
+      return (size_t)((uintptr_t)k.base * 0x9E3779B97F4A7C15ull) ^ (size_t)(k.rows * 31 + k.cols * 131 + k.splits + k.box_cols * 7);
     }
   };
   static thread_local std::unordered_map<Key, CUtensorMap, Hash> cache;
-  const Key key{base, splits, rows, cols, elem_bytes, (int)is_bf16};
+  if (box_cols == 0) box_cols = 128 / elem_bytes;
+  const Key key{base, splits, rows, cols, elem_bytes, (int)is_bf16, box_cols};
   auto hit = cache.find(key);
   if (hit != cache.end()) {
     *m = hit->second;
@@ -124,10 +114,11 @@ inline int make_tmap_out(CUtensorMap* m, const void* base, uint64_t splits, uint
                                                    : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
   cuuint64_t dims[3] = {cols, rows, splits};
   cuuint64_t strides[2] = {cols * (uint64_t)elem_bytes, rows * cols * (uint64_t)elem_bytes};
-  cuuint32_t box[3] = {(cuuint32_t)(128 / elem_bytes), 32, 1};
+  cuuint32_t box[3] = {(cuuint32_t)box_cols, 32, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = enc(m, dt, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+                   box_cols * elem_bytes == 128 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+                   CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) {
     set_error_detail("cuTensorMapEncodeTiled(%s: splits=%llu rows=%llu cols=%llu elem=%d) failed with CUresult %d", what,
                      (unsigned long long)splits, (unsigned long long)rows, (unsigned long long)cols, elem_bytes, (int)r);

@@ -1,0 +1,448 @@
+// Dense block-FP8 GEMM on CTA pairs (tcgen05 cta_group::2): two CTAs of a cluster compute one 256 x 256 output tile.
+// Each CTA loads its own 128 rows of A and HALF of the B tile (128 of its 256 rows); the tensor cores of the pair read
+// both halves. Per 128-K block a CTA then moves 32 KB into shared memory and its tensor core reads 32 KB back, which
+// fits the 512 clocks its MMAs take at 128 B/clk; the single-CTA tile (48 KB each way) does not.
+//
+// The fp32 scales change every 128 of K, so every K block is pulled out of TMEM, scaled and added in registers.
+// Roles per CTA (640 threads):
+//   warps 0-15   promotion: warp w owns TMEM lanes 32 (w % 4).. and columns 64 (w / 4)..; 64 accumulators per thread.
+//                Four warps per SM sub-partition: the TMEM round trip of one hides behind the FMAs of the others.
+//   warp  16     TMA producer (no multicast: every load has one destination CTA)
+//   warp  17     MMA issuer (leader CTA only)
+//   warps 18-19  scale loaders: products As[row] * Bs[128-column block] of four K blocks at a time into a
+//                shared-memory ring, so a promotion thread reads one float per K block
+// Cross-CTA protocol (rank 0 = leader):
+//   full[s]   (leader's)  2 arrivals (one expect_tx per producer) + the bytes of both CTAs' TMA loads
+//   empty[s]  (each CTA)  arrival of promotion warp 0 once it saw the MMAs of the stage complete
+//   tfull[b]  (each CTA)  arrival from the leader's tcgen05.commit
+//   tempty[b] (leader's)  32 arrivals: the promotion warps of both CTAs
+#pragma once
+
+#include "gemm_host.cuh"
+
+namespace b200 {
+
+namespace ptx {
+__device__ __forceinline__ uint32_t cluster_ctarank() {
+  uint32_t r;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+  return r;
+}
+// shared::cluster address of the same shared-memory offset in CTA `rank` of the cluster
+__device__ __forceinline__ uint32_t mapa(uint32_t addr, uint32_t rank) {
+  uint32_t out;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
+  return out;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+}
+__device__ __forceinline__ void mbar_expect_tx_cluster(uint32_t cluster_addr, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.relaxed.cluster.shared::cluster.b64 _, [%0], %1;" ::"r"(cluster_addr), "r"(bytes)
+               : "memory");
+}
+// tiled load whose completion bytes are counted on a barrier of the CTA pair's leader
+__device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap* m, int c0, int c1, uint32_t leader_bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];"
+      ::"r"(dst), "l"(m), "r"(c0), "r"(c1), "r"(leader_bar)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_alloc_pair(uint32_t smem_slot, uint32_t ncols) {
+  asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_slot), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void tmem_relinquish_pair() {
+  asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
+  asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+__device__ __forceinline__ void mma_f8_pair(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc,
+                                            uint32_t accumulate) {
+  asm volatile(
+      "{\n\t"
+      ".reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::2.kind::f8f6f4 [%0], %1, %2, %3, p;\n\t"
+      "}" ::"r"(tmem_d),
+      "l"(desc_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+// one commit that arrives on the barrier at the same shared-memory offset in every CTA of `mask`
+// (tcgen05.commit is the one multicast form used anywhere in this library; no data is moved)
+__device__ __forceinline__ void mma_commit_pair_multicast(uint32_t bar, uint16_t mask) {
+  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(bar),
+               "h"(mask)
+               : "memory");
+}
+// a += b * s on two packed floats
+__device__ __forceinline__ void ffma2(uint64_t& a, uint32_t b0, uint32_t b1, uint64_t s) {
+  uint64_t b;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(b0), "r"(b1));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(b), "l"(s));
+}
+}  // namespace ptx
+
+// BN: columns of the pair's tile, 256 / 192 / 128. The wide tile does the most work per byte moved and per TMEM round
+// trip; the narrow ones are for problems of a few waves, whose last wave they fill better.
+template <int BN>
+struct Pair {
+  static constexpr int kStageA = kBM * kBK;       // this CTA's 128 rows of A
+  static constexpr int kStageB = (BN / 2) * kBK;  // this CTA's half of the B tile
+  static constexpr int kStages = BN == 256 ? 4 : 5;
+  static constexpr int kAccBufs = BN == 128 ? 4 : 2, kAccStride = BN == 128 ? 128 : 256;  // TMEM accumulator buffers
+  static constexpr int kPromWarps = 16, kProducerWarp = 16, kMmaWarp = 17, kScaleWarp = 18;
+  static constexpr int kCols = BN / 4, kChunks = kCols / 16;  // columns of one promotion warp, in 16-column chunks
+  static constexpr int kThreads = 640;
+  // 20 warps start with 96 registers each (5 per sub-partition); 4 x 104 + 64 = 5 x 96
+  static constexpr int kRegsPromotion = 104, kRegsOther = 64;
+  static constexpr int kBoxBytes = 32 * kCols * 2;             // a warp's 32 rows of 16-bit output
+  static constexpr int kStagingBytes = 16 * 32 * 128;          // at most 128 bytes per row
+  static constexpr int kBlocks = BN == 192 ? 3 : BN / 128;     // 128-column scale blocks a tile touches
+  static constexpr int kScaleSlots = 3, kScaleSlotBytes = 4 * kBlocks * 128 * 4;  // four K blocks x blocks x rows
+  static constexpr int kTmemCols = 512;
+  static constexpr size_t kSmemBytes =
+      (size_t)kStages * (kStageA + kStageB) + kStagingBytes + kScaleSlots * kScaleSlotBytes + 1024 + 256;
+};
+
+// OutT: 16-bit output [M, N], or fp32 (C + split * split_stride: partial sums of a K split, or an fp32 result)
+template <int BN, typename OutT>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair<BN>::kThreads, 1)
+block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+                           const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
+  using Pair = b200::Pair<BN>;
+  constexpr int S = Pair::kStages, NB = Pair::kAccBufs, SQ = Pair::kScaleSlots;
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint8_t* smem_al = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
+  const uint32_t sA = smem_base;
+  const uint32_t sB = smem_base + S * Pair::kStageA;
+  const uint32_t staging = smem_base + S * (Pair::kStageA + Pair::kStageB);
+  float* scales = reinterpret_cast<float*>(smem_al + (size_t)S * (Pair::kStageA + Pair::kStageB) + Pair::kStagingBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scales) + SQ * Pair::kScaleSlotBytes);
+  const uint32_t bar0 = ptx::smem_u32(bars);
+  auto full_bar = [&](int s) { return bar0 + 8u * s; };
+  auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };
+  auto tfull_bar = [&](int b) { return bar0 + 8u * (2 * S + b); };
+  auto tempty_bar = [&](int b) { return bar0 + 8u * (2 * S + NB + b); };
+  auto sfull_bar = [&](int q) { return bar0 + 8u * (2 * S + 2 * NB + q); };
+  auto sempty_bar = [&](int q) { return bar0 + 8u * (2 * S + 2 * NB + SQ + q); };
+  volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * S + 2 * NB + 2 * SQ);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * S + 2 * NB + 2 * SQ + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t rank = ptx::cluster_ctarank();
+  const bool leader = rank == 0;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < S; ++s) {
+      ptx::mbar_init(full_bar(s), 2);
+      ptx::mbar_init(empty_bar(s), 1);
+    }
+    for (int b = 0; b < NB; ++b) {
+      ptx::mbar_init(tfull_bar(b), 1);
+      ptx::mbar_init(tempty_bar(b), 2 * Pair::kPromWarps);
+    }
+    for (int q = 0; q < SQ; ++q) {
+      ptx::mbar_init(sfull_bar(q), 2);
+      ptx::mbar_init(sempty_bar(q), Pair::kPromWarps);
+    }
+    *abort_flag = 0;
+    ptx::fence_mbar_init();
+  }
+  if (warp == Pair::kMmaWarp) {
+    ptx::tmem_alloc_pair(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), Pair::kTmemCols);
+    ptx::tmem_relinquish_pair();
+  }
+  if (warp == Pair::kProducerWarp && lane == 0) {
+    ptx::prefetch_tensormap(&tmap_a);
+    ptx::prefetch_tensormap(&tmap_b);
+    ptx::prefetch_tensormap(&tmap_c);
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();  // the peer's barriers are initialised before anything signals them
+  ptx::tc_fence_after();
+  const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+  grid_dependency_wait();
+
+  const int S_k = p.k_splits;
+  const int total_items = p.m_tiles * p.n_tiles * S_k;
+  const int num_kb = p.num_kb;
+  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  struct Item {
+    int mt, nt, ks, kb0, kb1;
+  };
+  auto item_of = [&](int item) {
+    Item c;
+    const int t = fast_div(item, p.k_splits_div);
+    c.ks = item - t * S_k;
+    c.kb0 = c.ks * p.kb_per_split;
+    c.kb1 = min(num_kb, c.kb0 + p.kb_per_split);
+    tile_coords(t, p.m_tiles, p.n_tiles, p.group_m, p.per_group_div, c.mt, c.nt);
+    return c;
+  };
+
+  if (warp >= Pair::kPromWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair::kRegsOther));
+    if (warp == Pair::kProducerWarp) {
+      if (ptx::elect_one()) {  // -------------------------------------------------- TMA producer (both CTAs)
+        int s = 0;
+        uint32_t phase = 1;
+        bool ok = true;
+        for (int item = pair; item < total_items && ok; item += npairs) {
+          const Item c = item_of(item);
+          const int a_row = c.mt * 2 * kBM + (int)rank * kBM, b_row = c.nt * BN + (int)rank * (BN / 2);
+          for (int kb = c.kb0; kb < c.kb1; ++kb) {
+            ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
+            if (!ok) break;
+            const uint32_t lf = ptx::mapa(full_bar(s), 0);
+            ptx::mbar_expect_tx_cluster(lf, Pair::kStageA + Pair::kStageB);
+            ptx::tma_load_2d_pair(sA + s * Pair::kStageA, &tmap_a, kb * kBK, a_row, lf);
+            ptx::tma_load_2d_pair(sB + s * Pair::kStageB, &tmap_b, kb * kBK, b_row, lf);
+            if (++s == S) s = 0, phase ^= 1;
+          }
+        }
+      }
+      __syncwarp();
+    } else if (warp == Pair::kMmaWarp) {
+      if (leader && ptx::elect_one()) {  // ------------------------------------------ MMA issuer (leader only)
+        constexpr uint32_t idesc = ptx::idesc_e4m3_f32(2 * kBM, BN);
+        int s = 0;
+        uint32_t phase = 0, it = 0;
+        bool ok = true;
+        for (int item = pair; item < total_items && ok; item += npairs) {
+          const Item c = item_of(item);
+          for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
+            const int b = it % NB;
+            ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
+                 ptx::mbar_wait(full_bar(s), phase, abort_flag);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t da = ptx::smem_desc_sw128(sA + s * Pair::kStageA);
+            const uint64_t db = ptx::smem_desc_sw128(sB + s * Pair::kStageB);
+            const uint32_t d = tmem_base + b * Pair::kAccStride;
+#pragma unroll
+            for (int k = 0; k < kBK / 32; ++k) ptx::mma_f8_pair(d, da + 2 * k, db + 2 * k, idesc, k > 0);
+            ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
+            if (++s == S) s = 0, phase ^= 1;
+          }
+        }
+      }
+      __syncwarp();
+    } else {  // ------------------------------------------------------------------ scale loaders (both CTAs)
+      const int tid = threadIdx.x - Pair::kScaleWarp * 32;  // 0..63: rows tid and tid + 64
+      int q = 0;
+      uint32_t phase = 1;
+      bool ok = true;
+      for (int item = pair; item < total_items && ok; item += npairs) {
+        const Item c = item_of(item);
+        const int row = c.mt * 2 * kBM + (int)rank * kBM + tid;
+        const float* as0 = p.As + (int64_t)min(row, p.M - 1) * p.as_sm;
+        const float* as1 = p.As + (int64_t)min(row + 64, p.M - 1) * p.as_sm;
+        const int blk0 = c.nt * BN / 128;  // first scale block of the tile
+        for (int kbase = c.kb0; kbase < c.kb1; kbase += 4) {
+          float a[4][2], b[4][Pair::kBlocks];
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const int kb = min(kbase + j, c.kb1 - 1);
+            a[j][0] = __ldg(as0 + (int64_t)kb * p.as_sk);
+            a[j][1] = __ldg(as1 + (int64_t)kb * p.as_sk);
+#pragma unroll
+            for (int n = 0; n < Pair::kBlocks; ++n)
+              b[j][n] = __ldg(p.Bs + (int64_t)min(blk0 + n, p.n_blocks - 1) * num_kb + kb);
+          }
+          ok = ptx::mbar_wait(sempty_bar(q), phase, abort_flag);
+          if (!ok) break;
+          float* dst = scales + q * (Pair::kScaleSlotBytes / 4) + tid;
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+#pragma unroll
+            for (int n = 0; n < Pair::kBlocks; ++n) {
+              dst[(j * Pair::kBlocks + n) * 128] = a[j][0] * b[j][n];
+              dst[(j * Pair::kBlocks + n) * 128 + 64] = a[j][1] * b[j][n];
+            }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(sfull_bar(q));
+          if (++q == SQ) q = 0, phase ^= 1;
+        }
+      }
+      __syncwarp();
+    }
+  } else {
+    // -------------------------------------------------------------------- promotion warps (both CTAs)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Pair::kRegsPromotion));
+    const int quarter = warp & 3, colq = warp >> 2;
+    constexpr int kCols = Pair::kCols, CH = Pair::kChunks;
+    const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + colq * kCols;
+    const uint32_t wstage = staging + warp * Pair::kBoxBytes;
+    const uint32_t my_scales = ptx::smem_u32(scales) + (quarter * 32 + lane) * 4;
+    const uint32_t leader_tempty = ptx::mapa(tempty_bar(0), 0);
+    uint32_t it = 0;
+    int s = 0, q = 0;
+    uint32_t sphase = 0;
+    bool ok = true;
+    for (int item = pair; item < total_items && ok; item += npairs) {
+      const Item c = item_of(item);
+      // byte offset of the scale block of every 16-column chunk of this warp (a 192-wide tile starts inside a block)
+      uint32_t blk_off[CH];
+#pragma unroll
+      for (int h = 0; h < CH; ++h)
+        blk_off[h] = (BN == 192 ? (c.nt * BN + colq * kCols + 16 * h) / 128 - c.nt * BN / 128 : colq * kCols / 128) * 512;
+      uint64_t acc[kCols / 2];
+#pragma unroll
+      for (int j = 0; j < kCols / 2; ++j) acc[j] = 0;
+      for (int kbase = c.kb0; kbase < c.kb1 && ok; kbase += 4) {
+        ok = ptx::mbar_wait(sfull_bar(q), sphase, abort_flag);
+        const int n = min(4, c.kb1 - kbase);
+        for (int j = 0; j < n && ok; ++j, ++it) {
+          const int b = it % NB;
+          uint64_t sc[CH];  // {scale, scale} of every chunk; one value where the tile is aligned to the blocks
+#pragma unroll
+          for (int h = 0; h < CH; ++h) {
+            if (BN == 192 || h == 0) {
+              float v;
+              asm volatile("ld.shared.f32 %0, [%1];"
+                           : "=f"(v)
+                           : "r"(my_scales + q * Pair::kScaleSlotBytes + j * Pair::kBlocks * 512 + blk_off[h])
+                           : "memory");
+              asm("mov.b64 %0, {%1, %1};" : "=l"(sc[h]) : "f"(v));
+            } else {
+              sc[h] = sc[0];
+            }
+          }
+          ok = ptx::mbar_wait(tfull_bar(b), (it / NB) & 1, abort_flag);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          const uint32_t ta = lane_base + b * Pair::kAccStride;
+          uint32_t v[32];
+          ptx::tmem_ld32(ta, v);
+          if (warp == 0 && lane == 0) ptx::mbar_arrive(empty_bar(s));  // the MMAs of this stage have read it
+          if (++s == S) s = 0;
+          ptx::tmem_ld_wait(v);
+          if (kCols > 32) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) ptx::ffma2(acc[i], v[2 * i], v[2 * i + 1], sc[i / 8]);
+            if (kCols == 64) {
+              ptx::tmem_ld32(ta + 32, v);
+              ptx::tmem_ld_wait(v);
+            } else {
+              ptx::tmem_ld16(ta + 32, v);
+              ptx::tmem_ld_wait16(v);
+            }
+          }
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster(leader_tempty + 8 * b);
+          constexpr int base = kCols > 32 ? 16 : 0;
+#pragma unroll
+          for (int i = 0; i < kCols / 2 - base; ++i) ptx::ffma2(acc[base + i], v[2 * i], v[2 * i + 1], sc[(base + i) / 8]);
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(sempty_bar(q));
+        if (++q == SQ) q = 0, sphase ^= 1;
+      }
+      if (!ok) break;
+
+      // ------------------------------------------------------------------------ tile epilogue
+      const int row0 = c.mt * 2 * kBM + (int)rank * kBM + quarter * 32, col0 = c.nt * BN + colq * kCols;
+      if constexpr (sizeof(OutT) == 2) {
+        if (lane == 0) ptx::tma_store_wait_read();  // the last tile's box has left the staging area
+        __syncwarp();
+#pragma unroll
+        for (int ch = 0; ch < kCols / 8; ++ch) {
+          float t[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) t[i] = __uint_as_float((uint32_t)(acc[(ch * 8 + i) / 2] >> (32 * (i & 1))));
+          const uint4 v = pack8<OutT>(t);
+          // a 64-column box is stored with the TMA 128-byte swizzle; narrower ones row by row
+          const uint32_t addr = wstage + lane * kCols * 2 + ((kCols == 64 ? ch ^ (lane & 7) : ch) << 4);
+          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w)
+                       : "memory");
+        }
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) {
+          if (col0 < p.N && row0 < p.M) ptx::tma_store_3d(&tmap_c, wstage, col0, row0, 0);
+          ptx::tma_store_commit();
+        }
+      } else {
+        if (row0 + lane < p.M) {
+          OutT* dst = static_cast<OutT*>(p.C) + c.ks * p.split_stride + (int64_t)(row0 + lane) * p.ldc + col0;
+#pragma unroll
+          for (int ch = 0; ch < kCols / 8; ++ch) {
+            float t[8];
+#pragma unroll
+            for (int i = 0; i < 8; ++i) t[i] = __uint_as_float((uint32_t)(acc[(ch * 8 + i) / 2] >> (32 * (i & 1))));
+            if (col0 + ch * 8 < p.N) store8<OutT>(dst + ch * 8, t);
+          }
+        }
+      }
+    }
+    if (sizeof(OutT) == 2 && lane == 0) ptx::tma_store_wait_all();
+  }
+
+  // ---------------------------------------------------------------------- teardown
+  if (*abort_flag) {
+    const unsigned long long t0 = ptx::globaltimer_ns();
+    while (ptx::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
+  }
+  ptx::tc_fence_before();
+  __syncthreads();
+  ptx::cluster_sync();  // neither CTA leaves while the other may still signal its barriers or use its smem
+  if (threadIdx.x == 0 && *abort_flag) atomicCAS(p.status, 0, 1);
+  if (warp == Pair::kMmaWarp) {
+    ptx::tc_fence_after();
+    ptx::tmem_dealloc_pair(tmem_base, Pair::kTmemCols);
+  }
+}
+
+// p.M/N/K/As/Bs/C/ldc (and split_stride) filled by the caller.
+template <int BN, typename OutT>
+inline int launch_gemm_pair(const void* A, const void* B, GemmParams p, int k_splits, cudaStream_t st) {
+  p.num_kb = (int)cdiv(p.K, kBK);
+  p.n_blocks = (int)cdiv(p.N, 128);
+  p.n_tiles = (int)cdiv(p.N, BN);
+  p.m_tiles = (int)cdiv(p.M, 2 * kBM);
+  p.group_m = 8;  // 8 pair tiles = 2048 rows swept per column tile
+  p.k_splits = k_splits;
+  p.kb_per_split = (int)cdiv(p.num_kb, k_splits);
+  p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);
+  p.k_splits_div = make_fastdiv(p.k_splits);
+  p.status = device_status_word();
+  if (!p.status) {
+    set_error_detail("cannot resolve the device status word");
+    return B200_E_LAUNCH;
+  }
+  const int64_t items = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
+  if (items == 0) return B200_OK;
+  const int max_pairs = sm_count() / 2;
+  const int pairs = (int)(items < max_pairs ? items : max_pairs);
+  CUtensorMap ta, tb, tc;
+  int rc = make_tmap_u8(&ta, A, (uint64_t)p.M, (uint64_t)p.K, kBM, "A");
+  if (rc) return rc;
+  rc = make_tmap_u8(&tb, B, (uint64_t)p.N, (uint64_t)p.K, BN / 2, "B (half tile)");
+  if (rc) return rc;
+  tc = ta;
+  if (sizeof(OutT) == 2) {
+    rc = make_tmap_out(&tc, p.C, 1, (uint64_t)p.M, (uint64_t)p.N, 2, std::is_same<OutT, __nv_bfloat16>::value, "C", BN / 4);
+    if (rc) return rc;
+  }
+  auto k = block_fp8_gemm_pair_kernel<BN, OutT>;
+  if (int rc_smem = allow_smem(k, Pair<BN>::kSmemBytes, "block_fp8_gemm_pair_kernel")) return rc_smem;
+  return launch_dependent(k, dim3((unsigned)(2 * pairs)), Pair<BN>::kThreads, Pair<BN>::kSmemBytes, st, 1,
+                          "block_fp8_gemm_pair_kernel", ta, tb, tc, p);
+}
+template <typename OutT>
+inline int launch_gemm_pair(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, cudaStream_t st) {
+  if (bn == 128) return launch_gemm_pair<128, OutT>(A, B, p, k_splits, st);
+  if (bn == 192) return launch_gemm_pair<192, OutT>(A, B, p, k_splits, st);
+  return launch_gemm_pair<256, OutT>(A, B, p, k_splits, st);
+}
+
+}  // namespace b200

@@ -29,11 +29,13 @@ using at::Tensor;
 struct Abi {
   decltype(&b200_status_string) status_string;
   decltype(&b200_last_error_detail) last_error_detail;
+  decltype(&b200_get_tuning) get_tuning;
   decltype(&b200_per_token_group_quant_fp8) quant;
   decltype(&b200_per_token_group_quant_fp8_ue8m0) quant_ue8m0;
   decltype(&b200_w8a8_block_fp8_gemm_workspace_bytes) gemm_ws;
   decltype(&b200_w8a8_block_fp8_gemm) gemm;
-  decltype(&b200_w8a8_block_fp8_gemm_ue8m0) gemm_ue8m0;
+  decltype(&b200_w8a8_block_fp8_gemm_packed_workspace_bytes) packed_ws;
+  decltype(&b200_w8a8_block_fp8_gemm_packed) packed;
   decltype(&b200_w8a8_block_fp8_linear_workspace_bytes) linear_ws;
   decltype(&b200_w8a8_block_fp8_linear) linear;
   decltype(&b200_fused_experts_fp8_workspace_bytes) experts_ws;
@@ -215,7 +217,9 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
 // matmul_ue8m0(A, B, As, Bs, out_dtype_code): both scales packed exponent words, row index contiguous
 PyObject* matmul_ue8m0(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   HANDLE_TH_ERRORS
-  if (nargs != 5) Py_RETURN_NONE;
+  long knob = -1;
+  abi.get_tuning("gemm_ue8m0", &knob);
+  if (nargs != 5 || knob == 0) Py_RETURN_NONE;
   const int dev = c10::cuda::current_device();
   const Tensor *A = plain(args[0], dev, kFp8), *B = plain(args[1], dev, kFp8);
   const Tensor *As = plain(args[2], dev), *Bs = plain(args[3], dev);
@@ -233,8 +237,11 @@ PyObject* matmul_ue8m0(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (!rows_per_word) Py_RETURN_NONE;
   auto pitch = [](const Tensor& s) { return s.size(1) > 1 ? s.stride(1) : s.size(0); };
   Tensor out = empty_on(dev, {M, N}, dtype_of_code(code));
-  const int rc = abi.gemm_ue8m0(A->data_ptr(), As->data_ptr<int>(), pitch(*As), B->data_ptr(), Bs->data_ptr<int>(), pitch(*Bs),
-                                rows_per_word, out.data_ptr(), (int)code, M, N, K, stream_of(dev));
+  void* st = stream_of(dev);
+  const size_t need = abi.packed_ws(M, N, K);
+  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
+  const int rc = abi.packed(A->data_ptr(), As->data_ptr<int>(), pitch(*As), B->data_ptr(), Bs->data_ptr<int>(), pitch(*Bs),
+                            rows_per_word, out.data_ptr(), (int)code, M, N, K, need ? buf.data_ptr() : nullptr, need, st);
   if (rc) return fail(rc, "w8a8_block_fp8_matmul (UE8M0)");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -337,11 +344,13 @@ PyObject* bind(PyObject*, PyObject* arg) {
   };
   get(abi.status_string, "b200_status_string");
   get(abi.last_error_detail, "b200_last_error_detail");
+  get(abi.get_tuning, "b200_get_tuning");
   get(abi.quant, "b200_per_token_group_quant_fp8");
   get(abi.quant_ue8m0, "b200_per_token_group_quant_fp8_ue8m0");
   get(abi.gemm_ws, "b200_w8a8_block_fp8_gemm_workspace_bytes");
   get(abi.gemm, "b200_w8a8_block_fp8_gemm");
-  get(abi.gemm_ue8m0, "b200_w8a8_block_fp8_gemm_ue8m0");
+  get(abi.packed_ws, "b200_w8a8_block_fp8_gemm_packed_workspace_bytes");
+  get(abi.packed, "b200_w8a8_block_fp8_gemm_packed");
   get(abi.linear_ws, "b200_w8a8_block_fp8_linear_workspace_bytes");
   get(abi.linear, "b200_w8a8_block_fp8_linear");
   get(abi.experts_ws, "b200_fused_experts_fp8_workspace_bytes");

@@ -288,3 +288,16 @@ def test_cta_pair_kernel(M, N, K):
     with tuning(gemm_2cta=1):
         _case(M, N, K, 500 + M)
         _case(M, N, K, 501 + M, out_dtype=torch.float16, col_major=True)
+
+
+@pytest.mark.parametrize("bn", [128, 192, 256])
+@pytest.mark.parametrize("splitk", [1, 3])
+@pytest.mark.parametrize("M,N,K", [(1, 256, 128), (203, 392, 640), (256, 768, 1152), (515, 1032, 1424)])
+def test_cta_pair_widths(M, N, K, bn, splitk):
+    """Every tile width of the CTA-pair kernel (a 192-wide tile starts inside a scale block), with and without a K
+    split (an uneven one included), at ragged rows, columns and K."""
+    from sglang_b200._native import tuning
+
+    with tuning(gemm_2cta=bn, gemm_skinny=0, gemm_splitk=splitk):
+        for dt in (torch.bfloat16, torch.float32):
+            _case(M, N, K, 900 + M, out_dtype=dt, col_major=True)
