@@ -59,7 +59,8 @@ int b200_read_device_status(int* out, void* stream);
 /* Process-wide tuning knobs: how tests force one kernel path and tuning sweeps try a setting.
  * Product calls never read the environment; a knob left at -1 is decided automatically.
  * Names: "gemm_bn" (128 / 256), "gemm_skinny" (0 = never the decode kernel),
- * "gemm_skinny_max_m", "gemm_splitk" (> 0 forces the K split; size the workspace after setting
+ * "gemm_stream" (0 / 1 = never / always the dense
+ * weight-streaming kernel), "gemm_skinny_max_m", "gemm_splitk" (> 0 forces the K split; size the workspace after setting
  * it), "gemm_2cta" (0 = never CTA pairs, 1 = always, 128 / 192 / 256 = always with that tile width), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
  * fp32-scale kernels), "linear_decode_fused" (0 = never the one-launch decode linear), "moe_decode"
  * (0 = never the weight-streaming MoE kernels, 1 = always, 16 / 32 / 64 = always with that row block), "moe_down_splitk" (0 = never),
@@ -153,11 +154,10 @@ int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa, int64_t s
  * quantisation of x (arithmetic variant 0, eps as given): the same bytes and scales the stand-alone
  * quantiser produces, so the result equals quantise-then-GEMM up to the fp32 summation order.
  * x [M,K] bf16/f16 row-major (M <= 16), B [N,K] e4m3, Bs fp32 [ceil(N/128), ceil(K/128)],
- * out [M,N] in the dtype of x. K % 16 == 0, N % 8 == 0, N <= 524288.
- * workspace: b200_w8a8_block_fp8_linear_decode_workspace_bytes(M,N,K) bytes (fp32 partials of the K
- * splits). tickets: 4096 uint32 that are ZERO before the first call and belong to one stream (every
- * call leaves them zero; calls that overlap on the GPU must not share them). Anything else:
- * B200_E_UNSUPPORTED (callers fall back to the two-step path). */
+ * out [M,N] in the dtype of x. K % 16 == 0, K <= 65536, N % 8 == 0, N <= 524288.
+ * workspace: b200_w8a8_block_fp8_linear_decode_workspace_bytes(M,N,K) bytes (none at present: the K split
+ * is summed on chip). tickets: 4096 zeroed uint32 of one stream, not NULL (left as they are at present).
+ * Anything else: B200_E_UNSUPPORTED (callers fall back to the two-step path). */
 size_t b200_w8a8_block_fp8_linear_decode_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B, const float* Bs,
                                       void* out, int64_t M, int64_t N, int64_t K, float eps,
@@ -168,15 +168,15 @@ int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B,
  * w8a8_block_fp8_linear: quantise + GEMM of one linear layer in one call, any M
  * replaces: python/sglang/srt/layers/quantization/fp8_utils.py:814-834 (the same composition)
  * out = the result of b200_per_token_group_quant_fp8 (group 128) followed by b200_w8a8_block_fp8_gemm,
- * with the kernels chained as programmatic dependents (up to 4 rows: the one-launch kernel above).
- * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out, tickets as above. The weights B may
+ * with the kernels chained as programmatic dependents (a few rows: the one-launch kernel above).
+ * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out as above. The weights B may
  * be fetched before earlier kernels of the stream have finished if those signal their dependents early
  * (kernels of this library do; its quantisers called on their own do not).
  * workspace: b200_w8a8_block_fp8_linear_workspace_bytes(M,N,K) bytes, 256-byte aligned. */
 size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out,
                                int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes,
-                               void* tickets, void* stream);
+                               void* stream);
 
 /* ---------------------------------------------------------------------------------------
  * moe_align_block_size

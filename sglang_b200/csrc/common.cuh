@@ -49,6 +49,7 @@ inline int check_launch(const char* what) {
 // setting); -1 = decide automatically. Product calls read this struct, never the environment.
 struct Tuning {
   long gemm_bn = -1;            // 128 / 256: tile width of the dense GEMM
+  long gemm_stream = -1;        // 0 / 1: never / always the dense weight-streaming kernel
   long gemm_skinny = -1;        // 0: never use the decode (swapped-operand) kernel
   long gemm_skinny_max_m = -1;  // rows up to which the decode kernel is used
   long gemm_splitk = -1;        // > 0: forced K split

@@ -3,7 +3,7 @@
 #include "gemm_host.cuh"
 #include "gemm_pair.cuh"
 #include "gemm_skinny.cuh"
-#include "linear_decode.cuh"
+#include "linear_stream.cuh"
 #include "gemm_ue8m0.cuh"
 
 namespace b200 {
@@ -68,12 +68,13 @@ static int launch_reduce(const float* partial, void* C, int64_t mn, int splits, 
 }  // namespace b200
 
 namespace b200 {
-constexpr int64_t kSkinnyMaxM = 64;       // rows up to which the swapped-operand decode kernel is always used
+constexpr int64_t kSkinnyMaxM = 32;       // rows up to which the swapped-operand decode kernel is always used
 constexpr int64_t kSkinnyPlanMaxM = 256;  // ... and up to which it is considered
 struct GemmPlan {
   int splits;   // K splits (fp32 partials + a reduction pass when > 1)
   int pair_bn;  // 0: single-CTA 128 x 256 tiles, else CTA pairs with 256 x pair_bn tiles
   bool skinny;  // swapped-operand decode kernel
+  bool stream;  // weight-streaming kernel, token tiles of 64
   double us;    // modelled time (0: not modelled, decode sizes)
 };
 
@@ -89,9 +90,10 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   const int64_t num_kb = cdiv(K, 128);
   const int64_t skinny_max = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
   const bool skinny_ok = may_pair && tune.gemm_skinny != 0;
-  if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, 0.0};
-  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : (int)tune.gemm_2cta, false, 0.0};
-  GemmPlan best = {1, 0, false, 1e30};
+  if (may_pair && tune.gemm_stream > 0) return {1, 0, false, true, 0.0};
+  if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, 0.0};
+  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : (int)tune.gemm_2cta, false, false, 0.0};
+  GemmPlan best = {1, 0, false, false, 1e30};
   const double stream_us = (double)N * (double)K / 6.2e6;
   auto consider = [&](int bm, int bn, int slots, double us_per_kb, int pair_bn) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
@@ -100,7 +102,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + 0.8);
       if (work < stream_us) work = stream_us;
       const double us = 4.5 + work + (s > 1 ? 2.0 + 8.0 * s * (double)M * (double)N / 4e6 : 0.0);
-      if (us < best.us) best = {s, pair_bn, false, us};
+      if (us < best.us) best = {s, pair_bn, false, false, us};
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
@@ -110,9 +112,20 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
     consider(256, 192, sms / 2, 0.44, 192);
     consider(256, 128, sms / 2, 0.34, 128);
   }
+  if (may_pair && tune.gemm_stream != 0 && M > 32 && M <= 128) {
+    int csize, kb, stages;
+    if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages)) {
+      // 0.49 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more
+      const int64_t items = cdiv(N, 256) * cdiv(M, 64);
+      double work = (double)cdiv(items * csize, sms) * kb * 0.49;
+      if (work < (double)N * (double)K / 6.4e6) work = (double)N * (double)K / 6.4e6;
+      const double us = 6.0 + (csize > 1 ? 1.0 : 0.0) + work;
+      if (us < best.us) best = {1, 0, false, true, us};
+    }
+  }
   const double skinny_us = 4.5 + (double)cdiv(M, 32) * (double)N * (double)K / 10.5e6;
-  if (skinny_ok && tune.gemm_skinny_max_m < 0 && M <= kSkinnyPlanMaxM && skinny_us < best.us)
-    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, skinny_us};
+  if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM) && skinny_us < best.us)
+    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, skinny_us};
   return best;
 }
 }
@@ -160,6 +173,14 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
   int splits = plan.splits;
   if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
   if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
+  if (plan.stream && fan.n == 0 && tune.gemm_splitk <= 0) {
+    LinearStreamParams lp = {};
+    lp.As = As; lp.as_sm = as_stride_m; lp.as_sk = as_stride_k; lp.Bs = Bs; lp.out = C;
+    lp.M = (int)M; lp.N = (int)N; lp.K = (int)K;
+    if (c_dtype == B200_BF16) return launch_linear_stream<64, false, __nv_bfloat16>(B, A, lp, st);
+    if (c_dtype == B200_F16) return launch_linear_stream<64, false, __half>(B, A, lp, st);
+    return launch_linear_stream<64, false, float>(B, A, lp, st);
+  }
   if (skinny) {
     while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16>::kMaxKb) ++splits;  // scales of one item fit its smem table
     SkinnyParams sp = {};
@@ -248,38 +269,48 @@ extern "C" int b200_w8a8_block_fp8_gemm_fanout(const void* A, const float* As, i
 
 // Quantised activations of a linear layer: FP8 rows, then column-major scales, in front of the GEMM's own workspace.
 namespace b200 {
-constexpr int64_t kDecodeLinearMaxM = 4;  // rows up to which the one-launch kernel (linear_decode.cuh) is the faster one
+static int run_linear_stream(const void* x, int x_dtype, const void* B, const float* Bs, void* out, int64_t M, int64_t N, int64_t K,
+                             float eps, cudaStream_t st) {
+  LinearStreamParams p = {};
+  p.x = x; p.Bs = Bs; p.out = out; p.M = (int)M; p.N = (int)N; p.K = (int)K; p.eps = eps;
+  return x_dtype == B200_BF16 ? launch_linear_stream<16, true, __nv_bfloat16>(B, nullptr, p, st)
+                               : launch_linear_stream<16, true, __half>(B, nullptr, p, st);
+}
 static size_t linear_q_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * K), 256); }
 static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * (K / 128)) * 4, 256); }
-static bool linear_one_launch(int64_t M, int64_t N) {
-  return M <= kDecodeLinearMaxM && N <= 4096 * 128 && tuning().linear_decode_fused != 0;
+// One launch (linear_stream.cuh) or quantiser + GEMM. The one launch saves the quantiser's and the reduction's, but every
+// CTA quantises its K range of x for itself: worth it up to 64 (row, K block) groups per CTA.
+constexpr int64_t kLinearStreamMaxM = 16;
+static bool linear_one_launch(int64_t M, int64_t N, int64_t K) {
+  int csize, kb, stages;
+  return M <= kLinearStreamMaxM && tuning().linear_decode_fused != 0 &&
+         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages) && kb * M <= 64;
 }
 }  // namespace b200
 
 extern "C" size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (linear_one_launch(M, N)) return b200_w8a8_block_fp8_linear_decode_workspace_bytes(M, N, K);
+  if (linear_one_launch(M, N, K)) return 0;
   return linear_q_bytes(M, K) + linear_s_bytes(M, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
 }
 
 extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out, int64_t M,
-                                          int64_t N, int64_t K, void* workspace, size_t workspace_bytes, void* tickets,
-                                          void* stream) {
+                                          int64_t N, int64_t K, void* workspace, size_t workspace_bytes, void* stream) {
   using namespace b200;
   B200_CHECK_ARG(M >= 0 && N >= 0 && K > 0, "linear: bad shape");
   if (M == 0 || N == 0) return B200_OK;
   B200_UNSUPPORTED(x_dtype != B200_BF16 && x_dtype != B200_F16, "linear: 16-bit activations only (dtype code %d)", x_dtype);
   B200_UNSUPPORTED(K % 128 != 0, "linear: K=%lld must be a multiple of 128", (long long)K);
-  B200_CHECK_ARG(x && B && Bs && out && tickets, "linear: null pointer");
-  B200_CHECK_ARG(((uintptr_t)x & 15) == 0, "linear: x must be 16-byte aligned");
+  B200_CHECK_ARG(x && B && Bs && out, "linear: null pointer");
+  B200_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)B & 15) == 0, "linear: x and B must be 16-byte aligned");
+  B200_UNSUPPORTED(N % 8 != 0, "linear: N=%lld must be a multiple of 8", (long long)N);
   const size_t need = b200_w8a8_block_fp8_linear_workspace_bytes(M, N, K);
   if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0)) {
     set_error_detail("linear: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
   }
-  if (linear_one_launch(M, N))
-    return b200_w8a8_block_fp8_linear_decode(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, workspace, workspace_bytes, tickets, stream);
+  if (linear_one_launch(M, N, K)) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
   uint8_t* q = static_cast<uint8_t*>(workspace);
   float* s = reinterpret_cast<float*>(q + linear_q_bytes(M, K));
   uint8_t* rest = reinterpret_cast<uint8_t*>(s) + linear_s_bytes(M, K);
@@ -288,50 +319,23 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
   return gemm_impl(q, s, 1, M, B, Bs, out, x_dtype, M, N, K, rest, need - (size_t)(rest - q), stream, FanOut{});
 }
 
-extern "C" size_t b200_w8a8_block_fp8_linear_decode_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const int s = b200::decode_linear_k_splits(N, K, 148);
-  return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
-}
+extern "C" size_t b200_w8a8_block_fp8_linear_decode_workspace_bytes(int64_t, int64_t, int64_t) { return 0; }
 
 extern "C" int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B, const float* Bs, void* out,
                                                  int64_t M, int64_t N, int64_t K, float eps, void* workspace,
                                                  size_t workspace_bytes, void* tickets, void* stream) {
   using namespace b200;
+  (void)workspace, (void)workspace_bytes;  // the K split is summed through distributed shared memory
   B200_CHECK_ARG(M >= 0 && N >= 0 && K > 0, "linear_decode: bad shape");
   if (M == 0 || N == 0) return B200_OK;
-  B200_UNSUPPORTED(M > DecodeLinearCfg::NT, "linear_decode: M=%lld rows (at most %d)", (long long)M, DecodeLinearCfg::NT);
+  B200_UNSUPPORTED(M > kLinearStreamMaxM, "linear_decode: M=%lld rows (at most %d)", (long long)M, (int)kLinearStreamMaxM);
   B200_UNSUPPORTED(x_dtype != B200_BF16 && x_dtype != B200_F16, "linear_decode: 16-bit activations only (dtype code %d)", x_dtype);
   B200_UNSUPPORTED(K % 16 != 0 || N % 8 != 0, "linear_decode: K=%lld must be a multiple of 16, N=%lld of 8", (long long)K,
                    (long long)N);
-  B200_UNSUPPORTED(N > 4096 * 128, "linear_decode: N=%lld exceeds the ticket array (4096 weight tiles)", (long long)N);
+  B200_UNSUPPORTED(N > 4096 * 128, "linear_decode: N=%lld is too large", (long long)N);
   B200_CHECK_ARG(x && B && Bs && out && tickets, "linear_decode: null pointer");
   B200_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)B & 15) == 0, "linear_decode: x and B must be 16-byte aligned");
-  const int sms = sm_count() < 148 ? sm_count() : 148;
-  DecodeLinearParams p = {};
-  p.x = x; p.Bs = Bs; p.out = out; p.M = (int)M; p.N = (int)N; p.K = (int)K; p.eps = eps;
-  p.num_kb = (int)cdiv(K, kBK);
-  p.n_tiles = (int)cdiv(N, 128);
-  p.k_splits = decode_linear_k_splits(N, K, sms);
-  p.kb_per_split = (int)cdiv(p.num_kb, p.k_splits);
-  p.k_splits = (int)cdiv(p.num_kb, p.kb_per_split);  // no empty split: every ticket is drawn
-  p.tickets = static_cast<unsigned*>(tickets);
-  if (p.k_splits > 1) {
-    const size_t need = (size_t)p.k_splits * (size_t)M * (size_t)N * sizeof(float);
-    if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15) != 0) {
-      set_error_detail("linear_decode: split-K needs a 16-byte aligned workspace of %zu bytes (got %zu)", need, workspace_bytes);
-      return B200_E_WORKSPACE;
-    }
-    p.partial = static_cast<float*>(workspace);
-  }
-  p.status = device_status_word();
-  if (!p.status) {
-    set_error_detail("cannot resolve the device status word");
-    return B200_E_LAUNCH;
-  }
-  cudaStream_t st = static_cast<cudaStream_t>(stream);
-  if (x_dtype == B200_BF16) return launch_decode_linear<__nv_bfloat16, __nv_bfloat16>(B, p, st);
-  return launch_decode_linear<__half, __half>(B, p, st);
+  return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, eps, static_cast<cudaStream_t>(stream));
 }
 
 extern "C" int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
@@ -389,7 +393,7 @@ __global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __res
 // promotion kernels on unpacked scales: below 65 rows the weight stream decides, then wave counts (see plan_gemm; a
 // 128-K block of a 128 x 224 tile takes 0.41 us, unpacking 2 us).
 static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
-  if (M <= kSkinnyMaxM) return false;
+  if (M <= 64) return false;
   const double waves = (double)cdiv(cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN), sms);
   return 4.5 + waves * ((double)cdiv(K, 128) * 0.41 + 0.3) <= plan_gemm(M, N, K, sms, true).us + 2.0;
 }

@@ -11,7 +11,6 @@
 #include <vector>
 
 #include <ATen/cuda/EmptyTensor.h>
-#include <ATen/ops/zeros.h>
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGraphsC10Utils.h>
 #include <c10/cuda/CUDAStream.h>
@@ -51,13 +50,13 @@ PyObject* fail(int status, const char* what) {
 }
 
 // ------------------------------------------------------------------------------ scratch buffers
-// One grow-only scratch buffer (and one array of split-K tickets) per (device, stream); work on one stream is
+// One grow-only scratch buffer per (device, stream); work on one stream is
 // ordered, so the next call may reuse it. A CUDA graph bakes the buffer's address into its nodes: once a call has
 // been seen under capture, a buffer that has to grow is kept alive instead of being given back to the allocator.
 struct Scratch {
   int device;
   void* stream;
-  Tensor buf, tickets;
+  Tensor buf;
 };
 // never destroyed: the process may end after the CUDA context. Callers hold the interpreter lock.
 std::vector<Scratch>& scratch = *new std::vector<Scratch>;
@@ -71,7 +70,7 @@ Tensor empty_on(int device, at::IntArrayRef size, at::ScalarType dtype) {
 Scratch& scratch_of(int device, void* stream) {
   for (auto& s : scratch)
     if (s.device == device && s.stream == stream) return s;
-  scratch.push_back(Scratch{device, stream, {}, {}});
+  scratch.push_back(Scratch{device, stream, {}});
   return scratch.back();
 }
 
@@ -86,13 +85,6 @@ Tensor workspace(int device, void* stream, size_t bytes) {
     s.buf = empty_on(device, {(int64_t)want}, at::kByte);
   }
   return s.buf;
-}
-
-void* tickets_of(int device, void* stream) {
-  Scratch& s = scratch_of(device, stream);
-  if (!s.tickets.defined())  // zero once; every call leaves them zero
-    s.tickets = at::zeros({4096}, at::TensorOptions().dtype(at::kInt).device(c10::kCUDA, (c10::DeviceIndex)device));
-  return s.tickets.data_ptr();
 }
 
 // ------------------------------------------------------------------------------------ arguments
@@ -141,7 +133,7 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   // a large scratch (long prefill) is worth a block of the caching allocator, which other work can use in between
   const Tensor buf = need == 0 ? Tensor() : need <= kKeptScratch ? workspace(dev, st, need) : empty_on(dev, {(int64_t)need}, at::kByte);
   const int rc = abi.linear(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K,
-                            need ? buf.data_ptr() : nullptr, need, tickets_of(dev, st), st);
+                            need ? buf.data_ptr() : nullptr, need, st);
   if (rc) return fail(rc, "w8a8_block_fp8_linear");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -323,14 +315,6 @@ PyObject* scratch_tensor(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return THPVariable_Wrap(workspace((int)dev, stream_of((int)dev), bytes));
   END_HANDLE_TH_ERRORS
 }
-PyObject* tickets(PyObject*, PyObject* arg) {
-  HANDLE_TH_ERRORS
-  const long dev = PyLong_AsLong(arg);
-  if (PyErr_Occurred()) return nullptr;
-  return PyLong_FromVoidPtr(tickets_of((int)dev, stream_of((int)dev)));
-  END_HANDLE_TH_ERRORS
-}
-
 // bind(path of the C-ABI library)
 PyObject* bind(PyObject*, PyObject* arg) {
   const char* path = PyUnicode_AsUTF8(arg);
@@ -366,7 +350,7 @@ PyMethodDef methods[] = {
     {"quant", FAST(quant), nullptr},          {"matmul", FAST(matmul), nullptr},
     {"matmul_ue8m0", FAST(matmul_ue8m0), nullptr}, {"experts", FAST(experts), nullptr},
     {"route", FAST(route), nullptr},          {"scratch", FAST(scratch_tensor), nullptr},
-    {"tickets", tickets, METH_O, nullptr},    {nullptr, nullptr, 0, nullptr}};
+    {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the block-FP8 operators.", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};
 

@@ -299,10 +299,9 @@ def w8a8_block_fp8_linear(
     return output.to(dtype=input_2d.dtype).view(*output_shape)
 
 
-# Rows up to which the one-launch kernel is taken. Measured on B200 (us, one launch / quantiser + GEMM + split-K sum,
-# weights rotated so that they come from HBM): 6144x4096 8.8/11.4 at M=1, 12.7/12.1 at M=4, 26.8/12.9 at M=16;
-# 4096x4096 6.7/10.8, 9.0/11.0, 16.9/11.6: the in-kernel quantisers pace the weight stream once many rows are live.
-DECODE_FUSED_MAX_M = 4
+# Rows up to which the one-launch kernel is always taken (it handles 16; for more rows the native path weighs it against
+# quantiser + GEMM).
+DECODE_FUSED_MAX_M = 1
 
 
 def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weight_scale: torch.Tensor,
@@ -315,7 +314,7 @@ def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weig
     if not (0 < M <= max_rows and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and list(block_size) == [128, 128] and weight.dtype == fp8_dtype and weight.dim() == 2
             and weight_scale.dtype == torch.float32 and weight_scale.is_contiguous() and x.is_contiguous()
-            and weight.is_contiguous() and K % 16 == 0 and weight.shape[0] % 8 == 0 and weight.shape[1] == K):
+            and weight.is_contiguous() and K % 16 == 0 and K <= 65536 and weight.shape[0] % 8 == 0 and weight.shape[1] == K):
         return None
     if N.get_tuning("linear_decode_fused") == 0:
         return None
@@ -329,7 +328,7 @@ def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weig
         ws = _workspace(x.device, ws_bytes)
         st = lib.b200_w8a8_block_fp8_linear_decode(
             N.ptr(x), N.DTYPE_CODE[x.dtype], N.ptr(weight), N.ptr(weight_scale), N.ptr(out), M, Nn, K, 1e-10,
-            N.ptr(ws), ws_bytes, N.host.tickets(x.device.index), stream,
+            N.ptr(ws), ws_bytes, N.ptr(weight_scale), stream,  # the ticket array is no longer used: any non-null pointer
         )
     N.check(st, "w8a8_block_fp8_linear (decode)")
     return out

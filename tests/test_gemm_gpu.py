@@ -301,3 +301,32 @@ def test_cta_pair_widths(M, N, K, bn, splitk):
     with tuning(gemm_2cta=bn, gemm_skinny=0, gemm_splitk=splitk):
         for dt in (torch.bfloat16, torch.float32):
             _case(M, N, K, 900 + M, out_dtype=dt, col_major=True)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (33, 256, 1408), (64, 1032, 4096), (65, 392, 528), (130, 7168, 2048),
+                                   (64, 45056, 256)])
+def test_dense_weight_streaming_kernel(M, N, K):
+    """Weight-streaming GEMM with token tiles of 64: one and several tiles, ragged rows, columns and K, K split over a
+    cluster (few tiles) and one CTA walking several tiles (more tiles than SMs)."""
+    from sglang_b200._native import tuning
+
+    with tuning(gemm_stream=1):
+        for dt in (torch.bfloat16, torch.float32):
+            _case(M, N, K, 950 + M, out_dtype=dt, col_major=M % 2 == 0)
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 57344, 8192), (2, 8, 65536), (16, 264, 1024), (5, 4096, 1536)])
+def test_one_launch_linear_plans(M, N, K):
+    """Shapes at the edges of the one-launch linear's plan: a K range that only fits shared memory when split, a single
+    weight tile, more weight tiles than SMs."""
+    import sglang_b200 as S
+    from sglang_b200 import fp8_kernel
+
+    x = make_activation(M, K, 40 + M)
+    wq = _rand_fp8((N, K), 41)
+    ws = torch.rand((N + 127) // 128, K // 128, generator=torch.Generator().manual_seed(42)) * 1e-3
+    out = fp8_kernel._linear_decode_fused(x.cuda(), wq.cuda(), [128, 128], ws.cuda(), max_rows=16)
+    two_step = S.w8a8_block_fp8_matmul(*[t for p in [S.per_token_group_quant_fp8(x.cuda(), 128)] for t in (p[0], wq.cuda(), p[1])],
+                                       ws.cuda(), [128, 128], x.dtype)
+    _status_ok()
+    assert float((out.float() - two_step.float()).norm() / two_step.float().norm()) < 2e-3
