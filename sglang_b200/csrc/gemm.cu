@@ -5,6 +5,7 @@
 #include "gemm_skinny.cuh"
 #include "linear_stream.cuh"
 #include "gemm_ue8m0.cuh"
+#include "gemm_ue8m0_pair.cuh"
 
 namespace b200 {
 
@@ -338,6 +339,16 @@ extern "C" int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, con
   return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, eps, static_cast<cudaStream_t>(stream));
 }
 
+namespace b200 {
+// Modelled time of the block-scaled kernels (see plan_gemm): a 128-K block takes about 0.36 us for a CTA's 128 x 224 tile
+// and for a pair's 256 x 240 one, so the pair does twice the work per SM clock where whole waves allow it (3000 x 4096 x
+// 14336: 2759 against 2244 TFLOP/s; 1027 x 7168 x 8192, three waves instead of two: 1849 against 2288).
+static double block_scaled_us(int64_t M, int64_t N, int64_t K, int sms, bool pair) {
+  const int64_t tiles = pair ? cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN) : cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN);
+  return 4.5 + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * 0.36 + 0.3) * (pair ? 0.97 : 1.0);
+}
+}  // namespace b200
+
 extern "C" int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
                                               const int32_t* sfb, int64_t sfb_ld, int sfb_rows_per_word, void* C,
                                               int c_dtype, int64_t M, int64_t N, int64_t K, void* stream) {
@@ -356,6 +367,16 @@ extern "C" int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa,
   p.sfa = sfa; p.sfb = sfb; p.sfa_ld = sfa_ld; p.sfb_ld = sfb_ld; p.sfb_rows_per_word = sfb_rows_per_word;
   p.C = C; p.M = (int)M; p.N = (int)N; p.K = (int)K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
+  const long knob = tuning().gemm_ue8m0;
+  const bool pair = knob == 2 || (knob != 1 && block_scaled_us(M, N, K, sm_count(), true) <= block_scaled_us(M, N, K, sm_count(), false));
+  if (pair) {
+    switch (c_dtype) {
+      case B200_BF16: return launch_gemm_ue8m0_pair<__nv_bfloat16>(A, B, p, st);
+      case B200_F16: return launch_gemm_ue8m0_pair<__half>(A, B, p, st);
+      case B200_F32: return launch_gemm_ue8m0_pair<float>(A, B, p, st);
+      default: break;
+    }
+  }
   switch (c_dtype) {
     case B200_BF16: return launch_gemm_ue8m0<__nv_bfloat16>(A, B, p, st);
     case B200_F16: return launch_gemm_ue8m0<__half>(A, B, p, st);
@@ -389,13 +410,13 @@ __global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __res
   }
 }
 
-// Whether the block-scaled kernel (tiles of 128 x 224, scales applied by the tensor core, no K split) beats the
-// promotion kernels on unpacked scales: below 65 rows the weight stream decides, then wave counts (see plan_gemm; a
-// 128-K block of a 128 x 224 tile takes 0.41 us, unpacking 2 us).
+// Whether the block-scaled kernels (scales applied by the tensor core, no K split) beat the promotion kernels on unpacked
+// scales: below 65 rows the weight stream decides, then wave counts (unpacking takes 2 us).
 static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
+  if (tuning().gemm_ue8m0 > 0) return true;
   if (M <= 64) return false;
-  const double waves = (double)cdiv(cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN), sms);
-  return 4.5 + waves * ((double)cdiv(K, 128) * 0.41 + 0.3) <= plan_gemm(M, N, K, sms, true).us + 2.0;
+  const double one = block_scaled_us(M, N, K, sms, false), two = block_scaled_us(M, N, K, sms, true);
+  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true).us + 2.0;
 }
 static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
 static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }

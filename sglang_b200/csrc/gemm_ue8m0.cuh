@@ -20,7 +20,7 @@
 //   warps 0-7  epilogue: tcgen05.ld of the finished accumulator, convert, 16-byte row stores
 //   warp  8    TMA producer (A 128 x 128 B, B 224 x 128 B per stage, 128-byte swizzle, no multicast)
 //   warp  9    MMA issuer (and the scale copies smem -> TMEM)
-//   warp  10   scale loader: packed words -> transposed atoms in a 4-slot shared-memory ring
+//   warps 10, 11  scale loaders: packed words -> transposed atoms in a 4-slot shared-memory ring
 #pragma once
 
 #include "gemm_host.cuh"
@@ -160,43 +160,53 @@ block_fp8_gemm_ue8m0_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
       }
     }
     __syncwarp();
-  } else if (warp == Cfg::kSfWarp) {
+  } else if (warp >= Cfg::kSfWarp) {
     // ------------------------------------------------------------------ scale loader
     // Atom layout expected by the 32x128b.warpx4 copy: row r of a 128-row atom at byte (r % 32) * 16 + (r / 32) * 4.
-    // Lane l therefore holds rows l, 32 + l, 64 + l, 96 + l and writes one 16-byte vector.
+    // Lane l therefore holds rows l, 32 + l, 64 + l, 96 + l and writes one 16-byte vector. Two warps take turns, each
+    // with the words of its next group in flight while it stores this one: with one warp and no prefetch the L2 round
+    // trip of every group paced the tensor core (a CTA pair waited 548 of 943 clocks per K block for scales).
     constexpr int32_t kOne = 0x7F7F7F7F;  // exponent 127 = 2^0 for rows past the edge (their data is zero-filled)
-    uint32_t gi = 0;
-    bool ok = true;
-    for (int t = blockIdx.x; t < total_tiles && ok; t += gridDim.x) {
+    int t = blockIdx.x, g = warp - Cfg::kSfWarp;
+    auto advance = [&](int by) {
+      for (g += by; g >= groups; g -= groups) t += gridDim.x;
+    };
+    int32_t wa[4], wb[8];
+    auto fetch = [&]() {
       int mt, nt;
       tile_coords(t, p.m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
       const int m0 = mt * kBM, n0 = nt * BN;
-      for (int g = 0; g < groups; ++g, ++gi) {
-        const int slot = gi % SFS;
-        int32_t wa[4], wb[8];
-        const int32_t* ga = p.sfa + (int64_t)g * p.sfa_ld;
-        const int32_t* gb = p.sfb + (int64_t)g * p.sfb_ld;
+      const int32_t* ga = p.sfa + (int64_t)g * p.sfa_ld;
+      const int32_t* gb = p.sfb + (int64_t)g * p.sfb_ld;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int r = m0 + 32 * j + lane;
-          wa[j] = r < p.M ? __ldg(ga + r) : kOne;
-        }
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const int r = n0 + 32 * j + lane;
-          wb[j] = (j < BN / 32 && r < p.N) ? __ldg(gb + r / p.sfb_rows_per_word) : kOne;
-        }
-        ok = ptx::mbar_wait(sf_empty_bar(slot), ((gi / SFS) & 1) ^ 1, abort_flag);
-        if (!ok) break;
-        uint8_t* dst = sSF_ptr + (size_t)slot * Cfg::kSfSlotBytes + lane * 16;
-        *reinterpret_cast<int4*>(dst) = make_int4(wa[0], wa[1], wa[2], wa[3]);
-        *reinterpret_cast<int4*>(dst + 512) = make_int4(wb[0], wb[1], wb[2], wb[3]);
-        *reinterpret_cast<int4*>(dst + 1024) = make_int4(wb[4], wb[5], wb[6], wb[7]);
-        ptx::fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's copy
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(sf_full_bar(slot));
+      for (int j = 0; j < 4; ++j) {
+        const int r = m0 + 32 * j + lane;
+        wa[j] = r < p.M ? __ldg(ga + r) : kOne;
       }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const int r = n0 + 32 * j + lane;
+        wb[j] = (j < BN / 32 && r < p.N) ? __ldg(gb + (p.sfb_rows_per_word == 1 ? r : r / 128)) : kOne;
+      }
+    };
+    advance(0);
+    if (t < total_tiles) fetch();
+    for (uint32_t gi = warp - Cfg::kSfWarp; t < total_tiles; gi += 2) {
+      const int slot = gi % SFS;
+      const int4 va = make_int4(wa[0], wa[1], wa[2], wa[3]), vb = make_int4(wb[0], wb[1], wb[2], wb[3]),
+                 vc = make_int4(wb[4], wb[5], wb[6], wb[7]);
+      if (!ptx::mbar_wait(sf_empty_bar(slot), ((gi / SFS) & 1) ^ 1, abort_flag)) break;
+      uint8_t* dst = sSF_ptr + (size_t)slot * Cfg::kSfSlotBytes + lane * 16;
+      *reinterpret_cast<int4*>(dst) = va;
+      *reinterpret_cast<int4*>(dst + 512) = vb;
+      *reinterpret_cast<int4*>(dst + 1024) = vc;
+      advance(2);
+      if (t < total_tiles) fetch();  // in flight across the fence, the arrival and the next wait
+      ptx::fence_proxy_async_smem();  // generic-proxy writes -> visible to the tensor core's copy
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(sf_full_bar(slot));
     }
+    __syncwarp();
   } else if (warp == Cfg::kMmaWarp) {
     if (ptx::elect_one()) {
       // ------------------------------------------------------------------- MMA issuer

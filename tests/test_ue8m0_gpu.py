@@ -157,3 +157,20 @@ def test_block_scaled_kernel_shapes(M, N, K, out_dtype):
     out2 = S.w8a8_block_fp8_matmul(xq, wq.cuda(), xs_packed, per_block, [128, 128], out_dtype)
     _status_ok()
     assert torch.equal(out2, out)
+
+
+@pytest.mark.parametrize("knob", [1, 2])
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (257, 240, 512), (300, 1000, 640), (129, 248, 2048), (2100, 2048, 1152)])
+def test_block_scaled_single_and_pair_tiles(M, N, K, knob):
+    """The single-CTA (128 x 224) and CTA-pair (256 x 240) block-scaled kernels forced at edges of their tiles: few rows,
+    ragged columns, one scale group per tile, several tiles per CTA."""
+    import sglang_b200 as S
+    from sglang_b200 import weight_quant as W
+    from sglang_b200._native import tuning
+
+    xq, xs_packed, wq, ws, osf, ref = _ue8m0_case(M, N, K, 31 + M + N)
+    for packed in (W.transform_scale_ue8m0(ws, mn=N).cuda(), W.pack_ue8m0_mn_major(ws).cuda()):
+        with tuning(gemm_ue8m0=knob):
+            out = S.w8a8_block_fp8_matmul(xq, wq.cuda(), xs_packed, packed, [128, 128], torch.float32)
+        _status_ok()
+        assert O.rel_frobenius(out.cpu(), ref) < 1e-4
