@@ -112,7 +112,7 @@ template <typename IdT>
 __global__ void __launch_bounds__(kAlignThreads) align_single_kernel(
     const IdT* __restrict__ ids, int64_t numel, int B, int block_size, int32_t* __restrict__ sorted,
     int64_t max_pad, int32_t* __restrict__ expert_ids, int64_t max_blocks, int32_t* __restrict__ num_post_pad,
-    int32_t* __restrict__ cumsum) {
+    int32_t* __restrict__ cumsum, int32_t* __restrict__ inverse) {
   extern __shared__ int smem[];
   int* warp_cnt = smem;                   // [32][B]
   int* cnt = warp_cnt + kAlignWarps * B;  // [B]
@@ -129,6 +129,9 @@ __global__ void __launch_bounds__(kAlignThreads) align_single_kernel(
   if (bucket >= 0) {
     const int64_t pos = (int64_t)start[bucket] + warp_cnt[(tid >> 5) * B + bucket] + rank;
     if (pos < max_pad) sorted[pos] = tid;  // always true when max_pad follows the reference's sizing
+    if (inverse) inverse[tid] = bucket > 0 ? (int32_t)pos : -1;
+  } else if (inverse && tid < numel) {
+    inverse[tid] = -1;
   }
 }
 
@@ -203,7 +206,8 @@ __global__ void __launch_bounds__(kAlignThreads) align_scan_kernel(int32_t* __re
 template <typename IdT>
 __global__ void __launch_bounds__(kAlignThreads) align_scatter_kernel(const IdT* __restrict__ ids, int64_t numel, int B,
                                                                       const int32_t* __restrict__ chunk_base,
-                                                                      int32_t* __restrict__ sorted, int64_t max_pad) {
+                                                                      int32_t* __restrict__ sorted, int64_t max_pad,
+                                                                      int32_t* __restrict__ inverse) {
   extern __shared__ int smem[];
   int* warp_cnt = smem;                   // [32][B]
   int* cnt = warp_cnt + kAlignWarps * B;  // [B] (unused result)
@@ -214,20 +218,23 @@ __global__ void __launch_bounds__(kAlignThreads) align_scatter_kernel(const IdT*
   if (bucket >= 0) {
     const int64_t pos = (int64_t)chunk_base[(int64_t)blockIdx.x * B + bucket] + warp_cnt[(tid >> 5) * B + bucket] + rank;
     if (pos < max_pad) sorted[pos] = (int32_t)i;
+    if (inverse) inverse[i] = bucket > 0 ? (int32_t)pos : -1;
+  } else if (inverse && i < numel) {
+    inverse[i] = -1;
   }
 }
 
 template <typename IdT>
 static int launch_align(const void* ids_, int64_t numel, int B, int block_size, int32_t* sorted, int64_t max_pad,
                         int32_t* expert_ids, int64_t max_blocks, int32_t* num_post_pad, int32_t* cumsum, void* ws,
-                        cudaStream_t st) {
+                        cudaStream_t st, int32_t* inverse = nullptr) {
   const IdT* ids = static_cast<const IdT*>(ids_);
   const size_t rank_smem = (size_t)(kAlignWarps * B + 2 * B + 1) * sizeof(int);
   if (numel <= kAlignThreads) {
     auto k = align_single_kernel<IdT>;
     if (rank_smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rank_smem);
     k<<<1, kAlignThreads, rank_smem, st>>>(ids, numel, B, block_size, sorted, max_pad, expert_ids, max_blocks,
-                                           num_post_pad, cumsum);
+                                           num_post_pad, cumsum, inverse);
     return check_launch("moe_align_block_size (single block)");
   }
   const int chunks = (int)cdiv(numel, kAlignThreads);
@@ -240,8 +247,15 @@ static int launch_align(const void* ids_, int64_t numel, int B, int block_size, 
                                                                                expert_ids, max_blocks, num_post_pad, cumsum);
   auto k = align_scatter_kernel<IdT>;
   if (rank_smem > 48 * 1024) cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rank_smem);
-  k<<<chunks, kAlignThreads, rank_smem, st>>>(ids, numel, B, chunk_hist, sorted, max_pad);
+  k<<<chunks, kAlignThreads, rank_smem, st>>>(ids, numel, B, chunk_hist, sorted, max_pad, inverse);
   return check_launch("moe_align_block_size");
+}
+
+int align_with_inverse(const int32_t* ids, int64_t numel, int num_buckets, int block_size, int32_t* sorted, int64_t max_pad,
+                       int32_t* expert_ids, int64_t max_blocks, int32_t* num_post_pad, int32_t* cumsum, int32_t* inverse,
+                       void* ws, cudaStream_t st) {
+  return launch_align<int32_t>(ids, numel, num_buckets, block_size, sorted, max_pad, expert_ids, max_blocks, num_post_pad,
+                               cumsum, ws, st, inverse);
 }
 
 // ---------------------------------------------------------------- allocation-free variant

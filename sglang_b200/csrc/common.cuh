@@ -108,6 +108,12 @@ __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddep
 // predecessors have finished, so those must not have been written by a kernel that triggers its dependents early.
 int quant_for_linear(const void* x, int x_dtype, void* q, float* s, int64_t M, int64_t K, cudaStream_t st);
 
+// moe_align_block_size of int32 ids (align.cu) that also writes every id's position in the sorted layout, -1 for ids that
+// are not in [0, num_buckets - 1). ws: b200_moe_align_workspace_bytes.
+int align_with_inverse(const int32_t* ids, int64_t numel, int num_buckets, int block_size, int32_t* sorted, int64_t max_pad,
+                       int32_t* expert_ids, int64_t max_blocks, int32_t* num_post_pad, int32_t* cumsum, int32_t* inverse,
+                       void* ws, cudaStream_t st);
+
 inline int64_t cdiv(int64_t a, int64_t b) { return (a + b - 1) / b; }
 inline size_t align_up(size_t x, size_t a) { return (x + a - 1) / a * a; }
 

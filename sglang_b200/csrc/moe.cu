@@ -1,9 +1,9 @@
 // fused_experts(use_fp8_w8a8=True, block_shape=[128,128]) for sm_100a.
 //
 // Launch sequence (all on the caller's stream, no host sync):
-//   1 align            token->expert buckets padded to 128 rows                 (align.cu)
-//   2 gather_quant     hidden rows -> expert-sorted FP8 rows + 1x128 scales     (HBM bound;
-//                      top-k >= 3: rows quantised once per token, then FP8 rows gathered)
+//   1 align            token->expert buckets padded to 16 .. 128 rows           (align.cu)
+//   2 scatter_quant    hidden rows -> expert-sorted FP8 rows + 1x128 scales     (HBM bound)
+//     (up to 1024 pairs of the weight-streaming path: 1 and 2 in one launch)
 //   3 grouped GEMM 1   sorted rows x w1[expert]^T; the epilogue applies silu(gate)*up in fp32
 //                      and re-quantises to FP8 + 1x128 scales from the accumulators (tcgen05)
 //   4 grouped GEMM 2   x w2[expert]^T, * router weight, scattered to (token, slot)
@@ -20,102 +20,76 @@ namespace b200 {
 
 constexpr int kMoeBlockM = 128;
 
-// One thread = 16 consecutive elements of kGatherRows consecutive sorted rows (8 lanes share a
-// 128-group). blockIdx.x = group of rows, blockIdx.y = 256-chunk segment of the row. The row
-// indices and then the row data of all kGatherRows rows are requested before any is used, so
-// the dependent index -> data round trips overlap instead of adding up per row.
-constexpr int kGatherRows = 4;  // divides the 128-row expert blocks
-
+// Token rows -> expert-sorted FP8 rows + scales: one block per token quantises (or reads) its row once and writes it to
+// the positions of all of its pairs, so a 16-bit row is read once instead of once per pair (or quantised, written and
+// read back). Blocks past the tokens zero pad rows. HBM-bound by the sorted rows written: 16384 tokens of 7168 to 8 experts
+// each, quantiser + gather 465 us, this kernel 250.
+// 8 consecutive lanes share a 128-group; a thread holds 16 consecutive elements.
+constexpr int kPadSlots = 32;     // sorted slots a pad block looks at
+constexpr int kRowScales = 1024;  // groups of a row whose scales are written together
 template <typename T>
-__global__ void __launch_bounds__(256) moe_gather_quant_kernel(
-    const T* __restrict__ hidden, const int32_t* __restrict__ sorted_ids, const int32_t* __restrict__ expert_ids,
-    const int32_t* __restrict__ num_post_pad, uint8_t* __restrict__ q, float* __restrict__ s, int chunks_per_row,
-    int64_t H, int numel, int topk, int64_t cap, int zero_pads, int block_m) {
-  const int64_t slot0 = (int64_t)blockIdx.x * kGatherRows;
-  if (slot0 >= *num_post_pad || expert_ids[slot0 / block_m] < 0) return;  // uniform per block
-  const int chunk = blockIdx.y * blockDim.x + threadIdx.x;
-  const bool active = chunk < chunks_per_row;  // whole 8-lane groups are in or out (H % 128 == 0)
-  int flat[kGatherRows];
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) flat[r] = __ldg(sorted_ids + slot0 + r);
-  constexpr int kRegs = 16 * (int)sizeof(T) / 16;  // 16-byte registers per 16 elements
-  uint4 raw[kGatherRows][kRegs];
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) {
-    const bool real = active && flat[r] < numel;
-    const T* src = hidden + (int64_t)(real ? flat[r] / topk : 0) * H + chunk * 16;
-#pragma unroll
-    for (int i = 0; i < kRegs; ++i) raw[r][i] = real ? ld_nc_16(src + i * (16 / (int)sizeof(T))) : make_uint4(0, 0, 0, 0);
-  }
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) {
-    float f[16];
-    const T* e = reinterpret_cast<const T*>(raw[r]);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) f[i] = to_f32<T>(e[i]);
-    float amax = 0.f;
-#pragma unroll
-    for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
-    amax = fmaxf(group_max<8>(amax), 1e-10f);
-    // scale = amax / 448 and q = x / scale as the reference's quantiser computes them. The quotient
-    // is formed as x * (1 / scale) plus one residual correction (rem = x - q * scale, exact in an
-    // FMA): two FMAs per element instead of an IEEE division sequence. For 16-bit inputs the
-    // FP8 bytes equal those of the division on every (x, amax) pair (the quantiser's tests
-    // enumerate them all). A plain
-    // reciprocal multiply is not enough for 16-bit inputs: when amax has a short mantissa many
-    // quotients sit exactly on an FP8 tie and would be broken the other way.
-    const float scale = __fdiv_rn(amax, 448.0f);
-    const float inv = __fdiv_rn(1.0f, scale);
-#pragma unroll
-    for (int i = 0; i < 16; ++i) {
-      const float q0 = f[i] * inv;
-      f[i] = copysignf(fmaf(fmaf(-q0, scale, f[i]), inv, q0), f[i]);  // -0 stays -0, as with x / scale
+__global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
+    const T* __restrict__ hidden, const uint8_t* __restrict__ hidden_q, const float* __restrict__ hidden_s,
+    const int32_t* __restrict__ position, const int32_t* __restrict__ sorted_ids, const int32_t* __restrict__ num_post_pad,
+    uint8_t* __restrict__ q, float* __restrict__ s, int64_t T_tokens, int64_t H, int numel, int topk, int64_t s_row, int64_t s_group) {
+  if (blockIdx.x >= T_tokens) {
+    // Pad rows: a GEMM output row depends on its own A row only and rows computed from pad slots are never scattered,
+    // so their content is free. Zeros keep the tensor cores' power draw down when tiles are mostly real rows; with a few
+    // tokens per expert writing them would dominate this kernel, and the launch leaves these blocks out.
+    const int64_t slot0 = ((int64_t)blockIdx.x - T_tokens) * kPadSlots;
+    const int live = (int)min((int64_t)kPadSlots, *num_post_pad - slot0);
+    for (int r = 0; r < live; ++r) {
+      if (__ldg(sorted_ids + slot0 + r) < numel) continue;  // the same for every thread
+      for (int chunk = threadIdx.x; chunk < H / 16; chunk += blockDim.x) {
+        *reinterpret_cast<uint4*>(q + (slot0 + r) * H + chunk * 16) = make_uint4(0, 0, 0, 0);
+        if ((chunk & 7) == 0) s[(slot0 + r) * s_row + (chunk / 8) * s_group] = 0.f;
+      }
     }
+    return;
+  }
+  __shared__ int pos[64];        // topk <= kSumReduceMaxSlots
+  __shared__ float row_s[kRowScales];
+  const int64_t tok = blockIdx.x;
+  for (int j = threadIdx.x; j < topk; j += blockDim.x) pos[j] = __ldg(position + tok * topk + j);
+  __syncthreads();
+  const int groups = (int)(H / 128);
+  for (int c0 = threadIdx.x & ~31; c0 < H / 16; c0 += blockDim.x) {  // whole warps
+    const int chunk = c0 + (threadIdx.x & 31);
+    const bool active = chunk < H / 16;
     uint4 out;
-    out.x = pack4_e4m3(f[0], f[1], f[2], f[3]);
-    out.y = pack4_e4m3(f[4], f[5], f[6], f[7]);
-    out.z = pack4_e4m3(f[8], f[9], f[10], f[11]);
-    out.w = pack4_e4m3(f[12], f[13], f[14], f[15]);
-    // Pad rows: a GEMM output row depends on its own A row only and rows computed from pad slots
-    // are never scattered, so their content is free. Zeros keep the tensor cores' power draw
-    // down when tiles are mostly real rows; with a few tokens per expert (tiles that are mostly
-    // padding, weight streaming bound) writing them would dominate this kernel, so they are skipped.
-    if (active && (zero_pads || flat[r] < numel)) {
-      *reinterpret_cast<uint4*>(q + (slot0 + r) * H + chunk * 16) = out;
-      if ((threadIdx.x & 7) == 0) s[(int64_t)(chunk / 8) * cap + slot0 + r] = scale;
+    float scale;
+    if (hidden_q != nullptr) {
+      out = active ? ld_nc_16(hidden_q + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
+      scale = active && (chunk & 7) == 0 ? __ldg(hidden_s + tok * (H / 128) + chunk / 8) : 0.f;
+    } else {
+      uint4 raw[2];
+      raw[0] = active ? ld_nc_16(hidden + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
+      raw[1] = active ? ld_nc_16(hidden + tok * H + chunk * 16 + 8) : make_uint4(0, 0, 0, 0);
+      const T* v = reinterpret_cast<const T*>(raw);
+      float f[16];
+#pragma unroll
+      for (int k = 0; k < 16; ++k) f[k] = to_f32<T>(v[k]);
+      float amax = 0.f;
+#pragma unroll
+      for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(f[k]));
+      amax = fmaxf(group_max<8>(amax), 1e-10f);
+      scale = quant16(f, amax, B200_QUANT_DIV_CORRECTED, out);  // the stand-alone quantiser's bytes and scales
+    }
+    if (!active) continue;
+    if ((chunk & 7) == 0 && chunk / 8 < kRowScales) row_s[chunk / 8] = scale;
+    for (int j = 0; j < topk; ++j) {
+      const int64_t p = pos[j];
+      if (p < 0) continue;  // an expert on another rank
+      *reinterpret_cast<uint4*>(q + p * H + chunk * 16) = out;
+      if ((chunk & 7) == 0 && chunk / 8 >= kRowScales) s[p * s_row + (chunk / 8) * s_group] = scale;
     }
   }
-}
-
-// Pre-quantised input (rows quantised once per token by the step before, or FP8 rows + 1x128
-// scales delivered by the expert-parallel dispatch): plain gather of bytes and scales into the
-// expert-sorted layout. One thread = 16 bytes of kGatherRows consecutive sorted rows; indices,
-// then data, of all rows are requested before any is stored.
-__global__ void __launch_bounds__(256) moe_gather_fp8_kernel(
-    const uint8_t* __restrict__ hidden_q, const float* __restrict__ hidden_s, const int32_t* __restrict__ sorted_ids,
-    const int32_t* __restrict__ expert_ids, const int32_t* __restrict__ num_post_pad, uint8_t* __restrict__ q,
-    float* __restrict__ s, int chunks_per_row, int64_t H, int numel, int topk, int64_t cap, int zero_pads, int block_m) {
-  const int64_t slot0 = (int64_t)blockIdx.x * kGatherRows;
-  if (slot0 >= *num_post_pad || expert_ids[slot0 / block_m] < 0) return;  // uniform per block
-  const int chunk = blockIdx.y * blockDim.x + threadIdx.x;
-  if (chunk >= chunks_per_row) return;
-  int flat[kGatherRows];
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) flat[r] = __ldg(sorted_ids + slot0 + r);
-  uint4 v[kGatherRows];
-  float sc[kGatherRows];
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) {
-    const bool real = flat[r] < numel;
-    const int64_t tok = real ? flat[r] / topk : 0;
-    v[r] = real ? ld_nc_16(hidden_q + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
-    sc[r] = real && (chunk & 7) == 0 ? __ldg(hidden_s + tok * (H / 128) + chunk / 8) : 0.f;
-  }
-#pragma unroll
-  for (int r = 0; r < kGatherRows; ++r) {
-    if (!zero_pads && flat[r] >= numel) continue;  // see moe_gather_quant_kernel
-    *reinterpret_cast<uint4*>(q + (slot0 + r) * H + chunk * 16) = v[r];
-    if ((chunk & 7) == 0) s[(int64_t)(chunk / 8) * cap + slot0 + r] = sc[r];
+  __syncthreads();
+  const int kept = min(groups, kRowScales);
+  for (int i = threadIdx.x; i < topk * kept; i += blockDim.x) {  // consecutive threads -> consecutive groups of one row
+    const int j = i / kept, g = i - j * kept;
+    const int64_t p = pos[j];
+    if (p >= 0) s[p * s_row + g * s_group] = row_s[g];
   }
 }
 
@@ -324,8 +298,7 @@ struct MoeWorkspace {
   int64_t cap;  // rows of the expert-sorted layout (multiple of block_m)
   int64_t cap_blocks;
   int down_splits;  // > 1: the down GEMM writes fp32 split-K partials instead of 16-bit rows
-  bool quant_first;  // quantise the T input rows once, then gather FP8 rows (instead of quantising every pair)
-  size_t off_sorted, off_expert, off_npp, off_cumsum, off_align, off_aq1, off_as1, off_aq2, off_as2, off_c3, off_xq, off_xs, total;
+  size_t off_sorted, off_expert, off_npp, off_cumsum, off_align, off_aq1, off_as1, off_aq2, off_as2, off_c3, off_pos, total;
 };
 
 // Rows per expert block of the sorted layout, and with it the kernel: 16 / 32 / 64 for the weight-streaming kernel,
@@ -367,11 +340,7 @@ static MoeWorkspace moe_workspace_layout(int64_t T, int topk, int E, int64_t H, 
   w.off_as2 = take((size_t)w.cap * (I / 128) * 4);
   w.down_splits = moe_down_k_splits(numel, E, H, I, sm_count());
   w.off_c3 = take(w.down_splits > 1 ? (size_t)w.down_splits * numel * H * 4 : (size_t)numel * H * 2);
-  // Each token's row is used by topk pairs: from three slots up, quantising it once and moving
-  // FP8 bytes moves fewer bytes than re-reading the 16-bit row per pair.
-  w.quant_first = topk >= 3;
-  w.off_xq = take(w.quant_first ? (size_t)T * H : 0);
-  w.off_xs = take(w.quant_first ? (size_t)T * (H / 128) * 4 : 0);
+  w.off_pos = take((size_t)numel * 4);
   w.total = o;
   return w;
 }
@@ -421,6 +390,9 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   int down_splits = L.down_splits;
   if (tuning().moe_down_splitk == 0) down_splits = 1;  // knob: keep the 16-bit single-pass path
   const bool stream = L.block_m != kMoeBlockM;
+  // Layout of the sorted rows' scales: [H/128][cap] is what the GEMMs read fastest (a warp's 32 rows are one run), but
+  // with several pairs per token the scatter then writes many single floats (16384 tokens to 8 experts: 70 us)
+  const bool scales_by_row = !stream && topk >= 4;
   if (scatter != nullptr || stream) down_splits = 1;   // rows go straight to their receivers in 16 bits
   const bool split = down_splits > 1;
   T* c3 = no_combine && !split ? static_cast<T*>(out) : reinterpret_cast<T*>(ws + L.off_c3);
@@ -428,9 +400,8 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   int rc = B200_OK;
   const bool one_launch = stream && numel <= kPrepMaxPairs && E <= 1024;
   if (!one_launch) {
-    rc = b200_moe_align_block_size(topk_ids, B200_I32, numel, E + 1, L.block_m, sorted, L.cap, expert_ids,
-                                       L.cap_blocks, npp, cumsum, 1, ws + L.off_align,
-                                       b200_moe_align_workspace_bytes(numel, E + 1), st);
+    rc = align_with_inverse(topk_ids, numel, E + 1, L.block_m, sorted, L.cap, expert_ids, L.cap_blocks, npp, cumsum,
+                            reinterpret_cast<int32_t*>(ws + L.off_pos), ws + L.off_align, st);
     if (rc) return rc;
   }
   if (no_combine && !split && scatter == nullptr) {
@@ -448,29 +419,16 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
                           expert_ids, npp, aq1, as1, H, E, (int)numel, topk, L.block_m, L.cap);
     if (rc) return rc;
   } else {
-    const uint8_t* hq = static_cast<const uint8_t*>(hidden);
-    const float* hs = hidden_scale;
-    if (hs == nullptr && L.quant_first) {
-      uint8_t* xq = ws + L.off_xq;
-      float* xs = reinterpret_cast<float*>(ws + L.off_xs);
-      rc = b200_per_token_group_quant_fp8(hidden, std::is_same<T, __half>::value ? B200_F16 : B200_BF16, xq, xs, T_tokens,
-                                          H, 128, H / 128, 1, 1e-10f, B200_QUANT_DIV_CORRECTED, st);  // 16-bit input: same bits as the division
-      if (rc) return rc;
-      hq = xq;
-      hs = xs;
-    }
-    const int cpr = (int)(H / 16);
-    const int threads = cpr < 256 ? (cpr + 31) / 32 * 32 : 256;  // whole warps; cpr is a multiple of 8
-    dim3 grid((unsigned)(L.cap / kGatherRows), (unsigned)cdiv(cpr, threads));
-    int zero_pads = numel >= (int64_t)E * 32;  // on average a quarter of a tile per expert or more
-    if (tuning().moe_zero_pads >= 0) zero_pads = (int)tuning().moe_zero_pads;
-    if (hs != nullptr)
-      moe_gather_fp8_kernel<<<grid, threads, 0, st>>>(hq, hs, sorted, expert_ids, npp, aq1, as1, cpr, H, (int)numel, topk,
-                                                     L.cap, zero_pads, L.block_m);
-    else
-      moe_gather_quant_kernel<T><<<grid, threads, 0, st>>>(static_cast<const T*>(hidden), sorted, expert_ids, npp, aq1,
-                                                          as1, cpr, H, (int)numel, topk, L.cap, zero_pads, L.block_m);
-    if ((rc = check_launch("moe_gather"))) return rc;
+    // zero pad rows where on average a quarter of a tile per expert or more is real
+    bool zero_pads = numel >= (int64_t)E * 32;
+    if (tuning().moe_zero_pads >= 0) zero_pads = tuning().moe_zero_pads != 0;
+    const int64_t blocks = T_tokens + (zero_pads ? cdiv(L.cap, kPadSlots) : 0);
+    const int threads = H / 16 < 512 ? (int)cdiv(H / 16, 32) * 32 : 512;
+    moe_scatter_quant_kernel<T><<<(unsigned)blocks, threads, 0, st>>>(
+        hidden_scale ? nullptr : static_cast<const T*>(hidden), hidden_scale ? static_cast<const uint8_t*>(hidden) : nullptr,
+        hidden_scale, reinterpret_cast<const int32_t*>(ws + L.off_pos), sorted, npp, aq1, as1, T_tokens, H, (int)numel, topk,
+        scales_by_row ? H / 128 : 1, scales_by_row ? 1 : L.cap);
+    if ((rc = check_launch("moe_scatter_quant_kernel"))) return rc;
   }
   if (stream) {
     StreamParams sp = {};
@@ -497,12 +455,12 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   p.expert_ids = expert_ids; p.num_post_pad = npp; p.sorted_ids = sorted; p.numel = (int)numel;
   p.M = (int)L.cap;
   // GEMM 1: [cap, H] x w1[E, 2I, H]^T -> silu(gate)*up -> FP8 [cap, I] + column-major scales
-  p.As = as1; p.as_sm = 1; p.as_sk = L.cap; p.Bs = w1_scale; p.C = nullptr; p.ldc = 0;
+  p.As = as1; p.as_sm = scales_by_row ? H / 128 : 1; p.as_sk = scales_by_row ? 1 : L.cap; p.Bs = w1_scale; p.C = nullptr; p.ldc = 0;
   p.N = (int)I; p.K = (int)H; p.topk_weights = weight_on_input ? topk_weights : nullptr;
   p.q_out = aq2; p.q_scales = as2; p.q_scale_ld = L.cap;
   if ((rc = launch_gemm<GEMM_GROUPED_SILU_QUANT, T>(aq1, w1, (int64_t)E * 2 * I, p, 256, st, tiles_hint))) return rc;
   // GEMM 2: [cap, I] x w2[E, H, I]^T -> rows scattered to (token, slot), times the router weight
-  p.As = as2; p.as_sk = L.cap; p.Bs = w2_scale; p.C = c3; p.ldc = H; p.N = (int)H; p.K = (int)I;
+  p.As = as2; p.as_sm = 1; p.as_sk = L.cap; p.Bs = w2_scale; p.C = c3; p.ldc = H; p.N = (int)H; p.K = (int)I;
   p.topk_weights = weight_on_input ? nullptr : topk_weights;
   if (scatter != nullptr) {
     p.C = nullptr;
