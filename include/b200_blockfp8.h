@@ -61,7 +61,8 @@ int b200_read_device_status(int* out, void* stream);
  * Names: "gemm_bn" (128 / 256), "gemm_skinny" (0 = never the decode kernel),
  * "gemm_stream" (0 / 1 = never / always the dense
  * weight-streaming kernel), "gemm_skinny_max_m", "gemm_splitk" (> 0 forces the K split; size the workspace after setting
- * it), "gemm_2cta" (0 = never CTA pairs, 1 = always, 128 / 192 / 256 = always with that tile width), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
+ * it), "gemm_2cta" (0 = never the 16-warp kernel, 1 / 2 = always, on CTA pairs / single CTAs,
+ * 128 / 192 / 256 = always on pairs with that tile width), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the
  * fp32-scale kernels, 1 / 2 = always the single-CTA / CTA-pair block-scaled kernel), "linear_decode_fused" (0 = never the one-launch decode linear), "moe_decode"
  * (0 = never the weight-streaming MoE kernels, 1 = always, 16 / 32 / 64 = always with that row block), "moe_down_splitk" (0 = never),
  * "moe_zero_pads" (0 / 1), "peer_wait_ms" (limit of a device-side wait for another GPU, 100 .. 60000).

@@ -93,7 +93,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   const bool skinny_ok = may_pair && tune.gemm_skinny != 0;
   if (may_pair && tune.gemm_stream > 0) return {1, 0, false, true, 0.0};
   if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, 0.0};
-  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : (int)tune.gemm_2cta, false, false, 0.0};
+  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : tune.gemm_2cta == 2 ? 0 : (int)tune.gemm_2cta, false, false, 0.0};
   GemmPlan best = {1, 0, false, false, 1e30};
   const double stream_us = (double)N * (double)K / 6.2e6;
   auto consider = [&](int bm, int bn, int slots, double us_per_kb, int pair_bn) {
@@ -107,7 +107,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
-  consider(128, N > 128 ? 256 : 128, sms, 0.54, 0);
+  consider(128, N > 128 ? 256 : 128, sms, 0.51, 0);
   if (may_pair && tune.gemm_2cta != 0 && N >= 256) {
     consider(256, 256, sms / 2, 0.47, 256);
     consider(256, 192, sms / 2, 0.44, 192);
@@ -207,6 +207,8 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
   const int bn = plan.pair_bn;
+  // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
+  const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
   if (splits > 1) {
     // few tiles: fp32 partials per K split in the workspace, then one reduction pass
     const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
@@ -217,18 +219,18 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     p.C = workspace;
     p.split_stride = M * N;
     p.n_dest = 0;  // the partials stay local; the reduction pass fans the sum out
-    int rc = bn ? launch_gemm_pair<float>(bn, A, B, p, splits, st)
-                : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, 0, splits);
+    int rc = wide ? launch_gemm_wide<float>(bn, A, B, p, splits, st)
+                  : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, 0, splits);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
     if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
     if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
-  if (bn && fan.n == 0) {
-    if (c_dtype == B200_BF16) return launch_gemm_pair<__nv_bfloat16>(bn, A, B, p, 1, st);
-    if (c_dtype == B200_F16) return launch_gemm_pair<__half>(bn, A, B, p, 1, st);
-    return launch_gemm_pair<float>(bn, A, B, p, 1, st);
+  if (wide && fan.n == 0) {
+    if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, 1, st);
+    if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, 1, st);
+    return launch_gemm_wide<float>(bn, A, B, p, 1, st);
   }
   switch (c_dtype) {
     case B200_BF16: return launch_gemm<GEMM_DENSE, __nv_bfloat16>(A, B, N, p, force_bn, st);

@@ -1,4 +1,5 @@
-// Dense block-FP8 GEMM on CTA pairs (tcgen05 cta_group::2): two CTAs of a cluster compute one 256 x 256 output tile.
+// Dense block-FP8 GEMM with 16 promotion warps, on CTA pairs (tcgen05 cta_group::2) or single CTAs. Two CTAs of a cluster
+// compute one 256 x 256 output tile.
 // Each CTA loads its own 128 rows of A and HALF of the B tile (128 of its 256 rows); the tensor cores of the pair read
 // both halves. Per 128-K block a CTA then moves 32 KB into shared memory and its tensor core reads 32 KB back, which
 // fits the 512 clocks its MMAs take at 128 B/clk; the single-CTA tile (48 KB each way) does not.
@@ -79,6 +80,22 @@ __device__ __forceinline__ void mma_commit_pair_multicast(uint32_t bar, uint16_t
                "h"(mask)
                : "memory");
 }
+// The forms that differ between a CTA on its own and a pair
+template <int CTAS>
+__device__ __forceinline__ void wide_mma(uint32_t d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t acc) {
+  if constexpr (CTAS == 2) mma_f8_pair(d, da, db, idesc, acc);
+  else mma_f8(d, da, db, idesc, acc);
+}
+template <int CTAS>
+__device__ __forceinline__ void wide_load(uint32_t dst, const CUtensorMap* m, int c0, int c1, uint32_t leader_bar) {
+  if constexpr (CTAS == 2) tma_load_2d_pair(dst, m, c0, c1, leader_bar);
+  else tma_load_2d(dst, m, c0, c1, leader_bar);
+}
+template <int CTAS>
+__device__ __forceinline__ void wide_sync() {
+  __syncthreads();
+  if constexpr (CTAS == 2) cluster_sync();
+}
 // a += b * s on two packed floats
 __device__ __forceinline__ void ffma2(uint64_t& a, uint32_t b0, uint32_t b1, uint64_t s) {
   uint64_t b;
@@ -87,13 +104,14 @@ __device__ __forceinline__ void ffma2(uint64_t& a, uint32_t b0, uint32_t b1, uin
 }
 }  // namespace ptx
 
+// CTAS = 1: a CTA's own 128 x 256 tile (problems whose rows or waves a pair's 256 rows would waste). CTAS = 2:
 // BN: columns of the pair's tile, 256 / 192 / 128. The wide tile does the most work per byte moved and per TMEM round
 // trip; the narrow ones are for problems of a few waves, whose last wave they fill better.
-template <int BN>
-struct Pair {
+template <int CTAS, int BN>
+struct Wide {
   static constexpr int kStageA = kBM * kBK;       // this CTA's 128 rows of A
-  static constexpr int kStageB = (BN / 2) * kBK;  // this CTA's half of the B tile
-  static constexpr int kStages = BN == 256 ? 4 : 5;
+  static constexpr int kStageB = (BN / CTAS) * kBK;  // this CTA's share of the B tile
+  static constexpr int kStages = CTAS == 1 ? 3 : BN == 256 ? 4 : 5;
   static constexpr int kAccBufs = BN == 128 ? 4 : 2, kAccStride = BN == 128 ? 128 : 256;  // TMEM accumulator buffers
   static constexpr int kPromWarps = 16, kProducerWarp = 16, kMmaWarp = 17, kScaleWarp = 18;
   static constexpr int kCols = BN / 4, kChunks = kCols / 16;  // columns of one promotion warp, in 16-column chunks
@@ -103,27 +121,27 @@ struct Pair {
   static constexpr int kBoxBytes = 32 * kCols * 2;             // a warp's 32 rows of 16-bit output
   static constexpr int kStagingBytes = 16 * 32 * 128;          // at most 128 bytes per row
   static constexpr int kBlocks = BN == 192 ? 3 : BN / 128;     // 128-column scale blocks a tile touches
-  static constexpr int kScaleSlots = 3, kScaleSlotBytes = 4 * kBlocks * 128 * 4;  // four K blocks x blocks x rows
+  static constexpr int kScaleSlots = CTAS == 1 ? 2 : 3, kScaleSlotBytes = 4 * kBlocks * 128 * 4;  // four K blocks x blocks x rows
   static constexpr int kTmemCols = 512;
   static constexpr size_t kSmemBytes =
       (size_t)kStages * (kStageA + kStageB) + kStagingBytes + kScaleSlots * kScaleSlotBytes + 1024 + 256;
 };
 
 // OutT: 16-bit output [M, N], or fp32 (C + split * split_stride: partial sums of a K split, or an fp32 result)
-template <int BN, typename OutT>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(Pair<BN>::kThreads, 1)
-block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
+template <int CTAS, int BN, typename OutT>
+__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(Wide<CTAS, BN>::kThreads, 1)
+block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                            const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
-  using Pair = b200::Pair<BN>;
-  constexpr int S = Pair::kStages, NB = Pair::kAccBufs, SQ = Pair::kScaleSlots;
+  using Cfg = Wide<CTAS, BN>;
+  constexpr int S = Cfg::kStages, NB = Cfg::kAccBufs, SQ = Cfg::kScaleSlots, kRows = CTAS * kBM;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
   uint8_t* smem_al = smem_raw + (smem_base - ptx::smem_u32(smem_raw));
   const uint32_t sA = smem_base;
-  const uint32_t sB = smem_base + S * Pair::kStageA;
-  const uint32_t staging = smem_base + S * (Pair::kStageA + Pair::kStageB);
-  float* scales = reinterpret_cast<float*>(smem_al + (size_t)S * (Pair::kStageA + Pair::kStageB) + Pair::kStagingBytes);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scales) + SQ * Pair::kScaleSlotBytes);
+  const uint32_t sB = smem_base + S * Cfg::kStageA;
+  const uint32_t staging = smem_base + S * (Cfg::kStageA + Cfg::kStageB);
+  float* scales = reinterpret_cast<float*>(smem_al + (size_t)S * (Cfg::kStageA + Cfg::kStageB) + Cfg::kStagingBytes);
+  uint64_t* bars = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(scales) + SQ * Cfg::kScaleSlotBytes);
   const uint32_t bar0 = ptx::smem_u32(bars);
   auto full_bar = [&](int s) { return bar0 + 8u * s; };
   auto empty_bar = [&](int s) { return bar0 + 8u * (S + s); };
@@ -135,37 +153,42 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * S + 2 * NB + 2 * SQ + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t rank = ptx::cluster_ctarank();
+  const uint32_t rank = CTAS == 2 ? ptx::cluster_ctarank() : 0;
   const bool leader = rank == 0;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      ptx::mbar_init(full_bar(s), 2);
+      ptx::mbar_init(full_bar(s), CTAS);
       ptx::mbar_init(empty_bar(s), 1);
     }
     for (int b = 0; b < NB; ++b) {
       ptx::mbar_init(tfull_bar(b), 1);
-      ptx::mbar_init(tempty_bar(b), 2 * Pair::kPromWarps);
+      ptx::mbar_init(tempty_bar(b), CTAS * Cfg::kPromWarps);
     }
     for (int q = 0; q < SQ; ++q) {
       ptx::mbar_init(sfull_bar(q), 2);
-      ptx::mbar_init(sempty_bar(q), Pair::kPromWarps);
+      ptx::mbar_init(sempty_bar(q), Cfg::kPromWarps);
     }
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
-  if (warp == Pair::kMmaWarp) {
-    ptx::tmem_alloc_pair(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), Pair::kTmemCols);
-    ptx::tmem_relinquish_pair();
+  if (warp == Cfg::kMmaWarp) {
+    const uint32_t slot = ptx::smem_u32(const_cast<uint32_t*>(tmem_slot));
+    if constexpr (CTAS == 2) {
+      ptx::tmem_alloc_pair(slot, Cfg::kTmemCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(slot, Cfg::kTmemCols);
+      ptx::tmem_relinquish();
+    }
   }
-  if (warp == Pair::kProducerWarp && lane == 0) {
+  if (warp == Cfg::kProducerWarp && lane == 0) {
     ptx::prefetch_tensormap(&tmap_a);
     ptx::prefetch_tensormap(&tmap_b);
     ptx::prefetch_tensormap(&tmap_c);
   }
   ptx::tc_fence_before();
-  __syncthreads();
-  ptx::cluster_sync();  // the peer's barriers are initialised before anything signals them
+  ptx::wide_sync<CTAS>();  // the peer's barriers are initialised before anything signals them
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   grid_launch_dependents();
@@ -174,7 +197,7 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
   const int S_k = p.k_splits;
   const int total_items = p.m_tiles * p.n_tiles * S_k;
   const int num_kb = p.num_kb;
-  const int pair = blockIdx.x >> 1, npairs = gridDim.x >> 1;
+  const int pair = blockIdx.x / CTAS, npairs = gridDim.x / CTAS;
   struct Item {
     int mt, nt, ks, kb0, kb1;
   };
@@ -188,31 +211,36 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     return c;
   };
 
-  if (warp >= Pair::kPromWarps) {
-    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Pair::kRegsOther));
-    if (warp == Pair::kProducerWarp) {
+  if (warp >= Cfg::kPromWarps) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsOther));
+    if (warp == Cfg::kProducerWarp) {
       if (ptx::elect_one()) {  // -------------------------------------------------- TMA producer (both CTAs)
         int s = 0;
         uint32_t phase = 1;
         bool ok = true;
         for (int item = pair; item < total_items && ok; item += npairs) {
           const Item c = item_of(item);
-          const int a_row = c.mt * 2 * kBM + (int)rank * kBM, b_row = c.nt * BN + (int)rank * (BN / 2);
+          const int a_row = c.mt * kRows + (int)rank * kBM, b_row = c.nt * BN + (int)rank * (BN / CTAS);
           for (int kb = c.kb0; kb < c.kb1; ++kb) {
             ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
             if (!ok) break;
-            const uint32_t lf = ptx::mapa(full_bar(s), 0);
-            ptx::mbar_expect_tx_cluster(lf, Pair::kStageA + Pair::kStageB);
-            ptx::tma_load_2d_pair(sA + s * Pair::kStageA, &tmap_a, kb * kBK, a_row, lf);
-            ptx::tma_load_2d_pair(sB + s * Pair::kStageB, &tmap_b, kb * kBK, b_row, lf);
+            uint32_t lf = full_bar(s);
+            if constexpr (CTAS == 2) {
+              lf = ptx::mapa(lf, 0);
+              ptx::mbar_expect_tx_cluster(lf, Cfg::kStageA + Cfg::kStageB);
+            } else {
+              ptx::mbar_expect_tx(lf, Cfg::kStageA + Cfg::kStageB);
+            }
+            ptx::wide_load<CTAS>(sA + s * Cfg::kStageA, &tmap_a, kb * kBK, a_row, lf);
+            ptx::wide_load<CTAS>(sB + s * Cfg::kStageB, &tmap_b, kb * kBK, b_row, lf);
             if (++s == S) s = 0, phase ^= 1;
           }
         }
       }
       __syncwarp();
-    } else if (warp == Pair::kMmaWarp) {
+    } else if (warp == Cfg::kMmaWarp) {
       if (leader && ptx::elect_one()) {  // ------------------------------------------ MMA issuer (leader only)
-        constexpr uint32_t idesc = ptx::idesc_e4m3_f32(2 * kBM, BN);
+        constexpr uint32_t idesc = ptx::idesc_e4m3_f32(kRows, BN);
         int s = 0;
         uint32_t phase = 0, it = 0;
         bool ok = true;
@@ -224,48 +252,49 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
                  ptx::mbar_wait(full_bar(s), phase, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after();
-            const uint64_t da = ptx::smem_desc_sw128(sA + s * Pair::kStageA);
-            const uint64_t db = ptx::smem_desc_sw128(sB + s * Pair::kStageB);
-            const uint32_t d = tmem_base + b * Pair::kAccStride;
+            const uint64_t da = ptx::smem_desc_sw128(sA + s * Cfg::kStageA);
+            const uint64_t db = ptx::smem_desc_sw128(sB + s * Cfg::kStageB);
+            const uint32_t d = tmem_base + b * Cfg::kAccStride;
 #pragma unroll
-            for (int k = 0; k < kBK / 32; ++k) ptx::mma_f8_pair(d, da + 2 * k, db + 2 * k, idesc, k > 0);
-            ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
+            for (int k = 0; k < kBK / 32; ++k) ptx::wide_mma<CTAS>(d, da + 2 * k, db + 2 * k, idesc, k > 0);
+            if constexpr (CTAS == 2) ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
+            else ptx::mma_commit(tfull_bar(b));
             if (++s == S) s = 0, phase ^= 1;
           }
         }
       }
       __syncwarp();
     } else {  // ------------------------------------------------------------------ scale loaders (both CTAs)
-      const int tid = threadIdx.x - Pair::kScaleWarp * 32;  // 0..63: rows tid and tid + 64
+      const int tid = threadIdx.x - Cfg::kScaleWarp * 32;  // 0..63: rows tid and tid + 64
       int q = 0;
       uint32_t phase = 1;
       bool ok = true;
       for (int item = pair; item < total_items && ok; item += npairs) {
         const Item c = item_of(item);
-        const int row = c.mt * 2 * kBM + (int)rank * kBM + tid;
+        const int row = c.mt * kRows + (int)rank * kBM + tid;
         const float* as0 = p.As + (int64_t)min(row, p.M - 1) * p.as_sm;
         const float* as1 = p.As + (int64_t)min(row + 64, p.M - 1) * p.as_sm;
         const int blk0 = c.nt * BN / 128;  // first scale block of the tile
         for (int kbase = c.kb0; kbase < c.kb1; kbase += 4) {
-          float a[4][2], b[4][Pair::kBlocks];
+          float a[4][2], b[4][Cfg::kBlocks];
 #pragma unroll
           for (int j = 0; j < 4; ++j) {
             const int kb = min(kbase + j, c.kb1 - 1);
             a[j][0] = __ldg(as0 + (int64_t)kb * p.as_sk);
             a[j][1] = __ldg(as1 + (int64_t)kb * p.as_sk);
 #pragma unroll
-            for (int n = 0; n < Pair::kBlocks; ++n)
+            for (int n = 0; n < Cfg::kBlocks; ++n)
               b[j][n] = __ldg(p.Bs + (int64_t)min(blk0 + n, p.n_blocks - 1) * num_kb + kb);
           }
           ok = ptx::mbar_wait(sempty_bar(q), phase, abort_flag);
           if (!ok) break;
-          float* dst = scales + q * (Pair::kScaleSlotBytes / 4) + tid;
+          float* dst = scales + q * (Cfg::kScaleSlotBytes / 4) + tid;
 #pragma unroll
           for (int j = 0; j < 4; ++j)
 #pragma unroll
-            for (int n = 0; n < Pair::kBlocks; ++n) {
-              dst[(j * Pair::kBlocks + n) * 128] = a[j][0] * b[j][n];
-              dst[(j * Pair::kBlocks + n) * 128 + 64] = a[j][1] * b[j][n];
+            for (int n = 0; n < Cfg::kBlocks; ++n) {
+              dst[(j * Cfg::kBlocks + n) * 128] = a[j][0] * b[j][n];
+              dst[(j * Cfg::kBlocks + n) * 128 + 64] = a[j][1] * b[j][n];
             }
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(sfull_bar(q));
@@ -276,13 +305,13 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     }
   } else {
     // -------------------------------------------------------------------- promotion warps (both CTAs)
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Pair::kRegsPromotion));
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(Cfg::kRegsPromotion));
     const int quarter = warp & 3, colq = warp >> 2;
-    constexpr int kCols = Pair::kCols, CH = Pair::kChunks;
+    constexpr int kCols = Cfg::kCols, CH = Cfg::kChunks;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + colq * kCols;
-    const uint32_t wstage = staging + warp * Pair::kBoxBytes;
+    const uint32_t wstage = staging + warp * Cfg::kBoxBytes;
     const uint32_t my_scales = ptx::smem_u32(scales) + (quarter * 32 + lane) * 4;
-    const uint32_t leader_tempty = ptx::mapa(tempty_bar(0), 0);
+    const uint32_t leader_tempty = CTAS == 2 ? ptx::mapa(tempty_bar(0), 0) : tempty_bar(0);
     uint32_t it = 0;
     int s = 0, q = 0;
     uint32_t sphase = 0;
@@ -309,7 +338,7 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
               float v;
               asm volatile("ld.shared.f32 %0, [%1];"
                            : "=f"(v)
-                           : "r"(my_scales + q * Pair::kScaleSlotBytes + j * Pair::kBlocks * 512 + blk_off[h])
+                           : "r"(my_scales + q * Cfg::kScaleSlotBytes + j * Cfg::kBlocks * 512 + blk_off[h])
                            : "memory");
               asm("mov.b64 %0, {%1, %1};" : "=l"(sc[h]) : "f"(v));
             } else {
@@ -319,7 +348,7 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
           ok = ptx::mbar_wait(tfull_bar(b), (it / NB) & 1, abort_flag);
           if (!ok) break;
           ptx::tc_fence_after();
-          const uint32_t ta = lane_base + b * Pair::kAccStride;
+          const uint32_t ta = lane_base + b * Cfg::kAccStride;
           uint32_t v[32];
           ptx::tmem_ld32(ta, v);
           if (warp == 0 && lane == 0) ptx::mbar_arrive(empty_bar(s));  // the MMAs of this stage have read it
@@ -338,7 +367,10 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
           }
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive_cluster(leader_tempty + 8 * b);
+          if (lane == 0) {
+            if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(leader_tempty + 8 * b);
+            else ptx::mbar_arrive(leader_tempty + 8 * b);
+          }
           constexpr int base = kCols > 32 ? 16 : 0;
 #pragma unroll
           for (int i = 0; i < kCols / 2 - base; ++i) ptx::ffma2(acc[base + i], v[2 * i], v[2 * i + 1], sc[(base + i) / 8]);
@@ -350,7 +382,7 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
       if (!ok) break;
 
       // ------------------------------------------------------------------------ tile epilogue
-      const int row0 = c.mt * 2 * kBM + (int)rank * kBM + quarter * 32, col0 = c.nt * BN + colq * kCols;
+      const int row0 = c.mt * kRows + (int)rank * kBM + quarter * 32, col0 = c.nt * BN + colq * kCols;
       if constexpr (sizeof(OutT) == 2) {
         if (lane == 0) ptx::tma_store_wait_read();  // the last tile's box has left the staging area
         __syncwarp();
@@ -393,23 +425,23 @@ block_fp8_gemm_pair_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     while (ptx::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
   }
   ptx::tc_fence_before();
-  __syncthreads();
-  ptx::cluster_sync();  // neither CTA leaves while the other may still signal its barriers or use its smem
+  ptx::wide_sync<CTAS>();  // neither CTA leaves while the other may still signal its barriers or use its smem
   if (threadIdx.x == 0 && *abort_flag) atomicCAS(p.status, 0, 1);
-  if (warp == Pair::kMmaWarp) {
+  if (warp == Cfg::kMmaWarp) {
     ptx::tc_fence_after();
-    ptx::tmem_dealloc_pair(tmem_base, Pair::kTmemCols);
+    if constexpr (CTAS == 2) ptx::tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+    else ptx::tmem_dealloc(tmem_base, Cfg::kTmemCols);
   }
 }
 
 // p.M/N/K/As/Bs/C/ldc (and split_stride) filled by the caller.
-template <int BN, typename OutT>
-inline int launch_gemm_pair(const void* A, const void* B, GemmParams p, int k_splits, cudaStream_t st) {
+template <int CTAS, int BN, typename OutT>
+inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_splits, cudaStream_t st) {
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_blocks = (int)cdiv(p.N, 128);
   p.n_tiles = (int)cdiv(p.N, BN);
-  p.m_tiles = (int)cdiv(p.M, 2 * kBM);
-  p.group_m = 8;  // 8 pair tiles = 2048 rows swept per column tile
+  p.m_tiles = (int)cdiv(p.M, CTAS * kBM);
+  p.group_m = 16 / CTAS;  // 2048 rows swept per column tile
   p.k_splits = k_splits;
   p.kb_per_split = (int)cdiv(p.num_kb, k_splits);
   p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);
@@ -421,28 +453,30 @@ inline int launch_gemm_pair(const void* A, const void* B, GemmParams p, int k_sp
   }
   const int64_t items = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
   if (items == 0) return B200_OK;
-  const int max_pairs = sm_count() / 2;
-  const int pairs = (int)(items < max_pairs ? items : max_pairs);
+  const int slots = sm_count() / CTAS;
+  const int units = (int)(items < slots ? items : slots);
   CUtensorMap ta, tb, tc;
   int rc = make_tmap_u8(&ta, A, (uint64_t)p.M, (uint64_t)p.K, kBM, "A");
   if (rc) return rc;
-  rc = make_tmap_u8(&tb, B, (uint64_t)p.N, (uint64_t)p.K, BN / 2, "B (half tile)");
+  rc = make_tmap_u8(&tb, B, (uint64_t)p.N, (uint64_t)p.K, BN / CTAS, "B");
   if (rc) return rc;
   tc = ta;
   if (sizeof(OutT) == 2) {
     rc = make_tmap_out(&tc, p.C, 1, (uint64_t)p.M, (uint64_t)p.N, 2, std::is_same<OutT, __nv_bfloat16>::value, "C", BN / 4);
     if (rc) return rc;
   }
-  auto k = block_fp8_gemm_pair_kernel<BN, OutT>;
-  if (int rc_smem = allow_smem(k, Pair<BN>::kSmemBytes, "block_fp8_gemm_pair_kernel")) return rc_smem;
-  return launch_dependent(k, dim3((unsigned)(2 * pairs)), Pair<BN>::kThreads, Pair<BN>::kSmemBytes, st, 1,
-                          "block_fp8_gemm_pair_kernel", ta, tb, tc, p);
+  auto k = block_fp8_gemm_wide_kernel<CTAS, BN, OutT>;
+  if (int rc_smem = allow_smem(k, Wide<CTAS, BN>::kSmemBytes, "block_fp8_gemm_wide_kernel")) return rc_smem;
+  return launch_dependent(k, dim3((unsigned)(CTAS * units)), Wide<CTAS, BN>::kThreads, Wide<CTAS, BN>::kSmemBytes, st, 1,
+                          "block_fp8_gemm_wide_kernel", ta, tb, tc, p);
 }
+// bn: columns of a pair's tile, or 0: single CTAs
 template <typename OutT>
-inline int launch_gemm_pair(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, cudaStream_t st) {
-  if (bn == 128) return launch_gemm_pair<128, OutT>(A, B, p, k_splits, st);
-  if (bn == 192) return launch_gemm_pair<192, OutT>(A, B, p, k_splits, st);
-  return launch_gemm_pair<256, OutT>(A, B, p, k_splits, st);
+inline int launch_gemm_wide(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, cudaStream_t st) {
+  if (bn == 0) return launch_gemm_wide<1, 256, OutT>(A, B, p, k_splits, st);
+  if (bn == 128) return launch_gemm_wide<2, 128, OutT>(A, B, p, k_splits, st);
+  if (bn == 192) return launch_gemm_wide<2, 192, OutT>(A, B, p, k_splits, st);
+  return launch_gemm_wide<2, 256, OutT>(A, B, p, k_splits, st);
 }
 
 }  // namespace b200

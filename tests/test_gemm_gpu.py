@@ -290,7 +290,7 @@ def test_cta_pair_kernel(M, N, K):
         _case(M, N, K, 501 + M, out_dtype=torch.float16, col_major=True)
 
 
-@pytest.mark.parametrize("bn", [128, 192, 256])
+@pytest.mark.parametrize("bn", [2, 128, 192, 256])  # 2: single CTAs
 @pytest.mark.parametrize("splitk", [1, 3])
 @pytest.mark.parametrize("M,N,K", [(1, 256, 128), (203, 392, 640), (256, 768, 1152), (515, 1032, 1424)])
 def test_cta_pair_widths(M, N, K, bn, splitk):
