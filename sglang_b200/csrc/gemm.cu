@@ -114,8 +114,8 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
     consider(256, 128, sms / 2, 0.34, 128);
   }
   if (may_pair && tune.gemm_stream != 0 && M > 32 && M <= 128) {
-    int csize, kb, stages;
-    if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages)) {
+    int csize, kb, stages, own;
+    if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own)) {
       // 0.49 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more
       const int64_t items = cdiv(N, 256) * cdiv(M, 64);
       double work = (double)cdiv(items * csize, sms) * kb * 0.49;
@@ -187,11 +187,15 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     SkinnyParams sp = {};
     sp.As = As; sp.as_sm = as_stride_m; sp.as_sk = as_stride_k; sp.Bs = Bs;
     sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
-    if (splits == 1 && fan.n == 0) {
+    // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
+    const int nt = skinny_token_tile(M);
+    const int cluster = splits > 1 && tune.gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
+    if (cluster > 1) splits = cluster;
+    if (fan.n == 0 && (splits == 1 || cluster > 1)) {
       sp.C = C;
-      if (c_dtype == B200_BF16) return launch_skinny<__nv_bfloat16>(A, B, sp, 1, st);
-      if (c_dtype == B200_F16) return launch_skinny<__half>(A, B, sp, 1, st);
-      return launch_skinny<float>(A, B, sp, 1, st);
+      if (c_dtype == B200_BF16) return launch_skinny<__nv_bfloat16>(A, B, sp, splits, splits > 1, st);
+      if (c_dtype == B200_F16) return launch_skinny<__half>(A, B, sp, splits, splits > 1, st);
+      return launch_skinny<float>(A, B, sp, splits, splits > 1, st);
     }
     const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
     if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15) != 0) {
@@ -199,7 +203,7 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
       return B200_E_WORKSPACE;
     }
     sp.C = workspace;
-    int rc = launch_skinny<float>(A, B, sp, splits, st);
+    int rc = launch_skinny<float>(A, B, sp, splits, false, st);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
     if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
@@ -285,9 +289,9 @@ static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M 
 // CTA quantises its K range of x for itself: worth it up to 64 (row, K block) groups per CTA.
 constexpr int64_t kLinearStreamMaxM = 16;
 static bool linear_one_launch(int64_t M, int64_t N, int64_t K) {
-  int csize, kb, stages;
+  int csize, kb, stages, own;
   return M <= kLinearStreamMaxM && tuning().linear_decode_fused != 0 &&
-         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages) && kb * M <= 64;
+         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages, own) && kb * M <= 64;
 }
 }  // namespace b200
 

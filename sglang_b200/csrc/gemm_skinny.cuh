@@ -6,10 +6,11 @@
 // accumulators instead of 128, so the per-K-block TMEM -> register promotion that bounds the
 // large-tile kernel at small M shrinks 4-8x and the kernel streams the weights at HBM rate.
 // Work item = (128-row weight tile, token tile, K split); one CTA per item, two CTAs per SM.
-// K splits write fp32 partials that splitk_reduce_kernel sums.
+// K splits form a thread-block cluster (up to 8) who exchange their sums through distributed shared
+// memory; a fan-out, and K too long for 8 splits, write fp32 partials that splitk_reduce_kernel sums.
 #pragma once
 
-#include "gemm_host.cuh"
+#include "gemm_stream.cuh"
 
 namespace b200 {
 
@@ -20,6 +21,7 @@ struct SkinnyParams {
   void* C;          // OutT [M, N], or fp32 partials [splits][M, N]
   int M, N, K, num_kb;
   int n_tiles, t_tiles, k_splits, kb_per_split;
+  int cluster;  // the K splits of an item are one cluster
   int* status;
 };
 
@@ -34,8 +36,11 @@ struct SkinnyCfg {
   static constexpr int kAccBufs = 4;
   static constexpr int kTmemCols = kAccBufs * NT;
   static constexpr int kMaxKb = 64;          // K blocks one CTA may own (scales staged in smem)
+  // sums exchanged within a cluster of K splits, [split][rows of this CTA][128]; with 32 tokens two CTAs per SM leave no
+  // room for them and they go to the ring once it is idle
+  static constexpr int kSumBytes = NT == 16 ? 21 * 512 : 0;
   static constexpr size_t kSmemBytes =
-      (size_t)kStages * (kStageW + kStageX) + (size_t)kMaxKb * NT * 4 + 1024 + 256;
+      (size_t)kStages * (kStageW + kStageX) + (size_t)kMaxKb * NT * 4 + kSumBytes + 1024 + 256;
 };
 
 template <int NT, typename OutT>
@@ -95,6 +100,8 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // "I have started", waited for before another CTA's shared memory is written at the very end
+  if (p.cluster) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   // every CTA of this grid is running: a dependent grid (the split-K reduction) may be set up now;
   // it waits for this grid's completion before it reads anything
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
@@ -115,6 +122,8 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     asm volatile("bar.sync 1, 128;" ::: "memory");
   }
 
+  float acc[NT];
+  bool ok_sum = false;
   if (warp == kProducerWarp) {
     if (ptx::elect_one()) {
       bool ok = true;
@@ -164,7 +173,6 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     // promotion warps: lane = weight row, columns = tokens
     const int n = n0 + warp * 32 + lane;
     const uint32_t lane_base = tmem_base + ((uint32_t)(warp * 32) << 16);
-    float acc[NT];
 #pragma unroll
     for (int t = 0; t < NT; ++t) acc[t] = 0.f;
     bool ok = true;
@@ -195,11 +203,40 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         acc[4 * j + 3] = fmaf(__uint_as_float(v[4 * j + 3]), s4.w, acc[4 * j + 3]);
       }
     }
-    if (ok && n < p.N) {
+    ok_sum = ok;
+    if (!p.cluster && ok && n < p.N) {
       OutT* out = static_cast<OutT*>(p.C) + (int64_t)ks * p.M * p.N + n;
 #pragma unroll
       for (int t = 0; t < NT; ++t)
         if (m0 + t < p.M) out[(int64_t)(m0 + t) * p.N] = from_f32<OutT>(acc[t]);  // 32 lanes -> 32 consecutive n
+    }
+  }
+
+  if (p.cluster) {
+    __syncwarp();
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    if (Cfg::kSumBytes == 0) ptx::cluster_barrier();  // every ring is idle
+    // every split adds up its share of the rows: row t belongs to split t / per
+    const int rows = min(NT, p.M - m0), r = threadIdx.x & 127, per = (rows + p.k_splits - 1) / p.k_splits;
+    const uint32_t sums_off = Cfg::kSumBytes ? (uint32_t)(reinterpret_cast<uint8_t*>(bars + 32) - smem_al) : 0u;
+    if (warp < 4) {
+      int owner = 0, j = 0;
+#pragma unroll
+      for (int t = 0; t < NT; ++t) {
+        if (t < rows) ptx::st_cluster_f32(ptx::stream_mapa(smem_base + sums_off, owner) + ((ks * per + j) * 128 + r) * 4, acc[t]);
+        if (++j == per) j = 0, ++owner;
+      }
+    }
+    __syncwarp();
+    ptx::cluster_barrier();
+    if (warp < 4 && ok_sum && n0 + r < p.N) {
+      const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + r;
+      OutT* out = static_cast<OutT*>(p.C) + n0 + r;
+      for (int j = 0; j < per && ks * per + j < rows; ++j) {
+        float sum = 0.f;
+        for (int c = 0; c < p.k_splits; ++c) sum += src[(c * per + j) * 128];  // split order: the same sum on every run
+        out[(int64_t)(m0 + ks * per + j) * p.N] = from_f32<OutT>(sum);
+      }
     }
   }
 
@@ -232,41 +269,41 @@ inline int skinny_k_splits(int64_t M, int64_t N, int64_t K, int nt, int sms) {
 
 inline int skinny_token_tile(int64_t M) { return M <= 16 ? 16 : 32; }
 
+// K splits as one cluster, no empty one; 1: through memory. Clusters of up to 4 fit the chip's SM groups anywhere, of up to 6 or
+// 8 where few items leave most of the chip free, and none may have to wait for a second wave: 96 items in clusters of 3 fill
+// 288 of the 296 slots, not all of them usable (50 x 6144 x 4096: 18.4 us against 11.5). With 32 tokens the exchange needs the
+// idle ring and only pays from three splits on. 16 x 4096 x 4096: 10.0 -> 7.3 us, 16 x 1280 x 8192: 9.0 -> 6.5,
+// 32 x 1536 x 4096: 9.4 -> 6.8.
+inline int skinny_cluster(int64_t items, int64_t K, int nt, int want) {
+  const int64_t num_kb = cdiv(K, 128);
+  const int cap = items * 8 <= 96 ? 8 : items * 6 <= 128 ? 6 : 4;
+  int c = want < cap ? want : cap;
+  c = (int)cdiv(num_kb, cdiv(num_kb, c));
+  if (cdiv(num_kb, c) > 64 || items * c > 264 || (nt > 16 && c < 3)) return 1;
+  return c;
+}
+
 template <int NT, typename OutT>
 inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, cudaStream_t st) {
   auto k = block_fp8_gemm_skinny_kernel<NT, OutT>;
   const size_t smem = SkinnyCfg<NT>::kSmemBytes;
   if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
-  const int grid = p.n_tiles * p.t_tiles * p.k_splits;
   // programmatic dependent of the kernel before it (normally the activation quantiser, which
   // signals launch_dependents at once): set-up and the first weight loads overlap its tail
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)grid);
-  cfg.blockDim = dim3(SkinnyCfg<NT>::kThreads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, k, tw, tx, p);
-  if (e != cudaSuccess) {
-    set_error_detail("block_fp8_gemm_skinny_kernel: %s", cudaGetErrorString(e));
-    return B200_E_LAUNCH;
-  }
-  return check_launch("block_fp8_gemm_skinny_kernel");
+  return launch_dependent(k, dim3((unsigned)(p.n_tiles * p.t_tiles * p.k_splits)), SkinnyCfg<NT>::kThreads, smem, st,
+                          p.cluster ? p.k_splits : 1, "block_fp8_gemm_skinny_kernel", tw, tx, p);
 }
 
-// out: OutT [M, N] when splits == 1, else fp32 partials [splits][M, N].
+// out: OutT [M, N] when splits == 1 or they are a cluster, else fp32 partials [splits][M, N].
 template <typename OutT>
-inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int splits, cudaStream_t st) {
+inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int splits, bool cluster, cudaStream_t st) {
   const int nt = skinny_token_tile(p.M);
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_tiles = (int)cdiv(p.N, 128);
   p.t_tiles = (int)cdiv(p.M, nt);
   p.k_splits = splits;
   p.kb_per_split = (int)cdiv(p.num_kb, splits);
+  p.cluster = cluster;
   p.status = device_status_word();
   if (!p.status) {
     set_error_detail("cannot resolve the device status word");

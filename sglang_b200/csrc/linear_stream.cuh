@@ -1,10 +1,9 @@
 // Dense block-FP8 GEMM for few rows, bound by reading the weights:
 //     out[m, n] = sum_kb (X[m, kb] . W[n, kb]) * xs[m, kb] * Bs[n / 128, kb]
 // Operands are swapped as in gemm_stream.cuh: a CTA owns 256 weight rows (two UMMA tiles of 128), NT = 16 / 32 / 64 tokens
-// are the UMMA N dimension. K is split over a thread-block cluster of up to 4 CTAs so that about every SM streams
-// weights, and the partial sums go to the cluster's first CTA through distributed shared memory: no fp32 partials in
-// memory and no reduction launch. (Clusters of 8 take 19.6 us for 1 x 4096 x 14336 where clusters of 4 take 13.7: fewer
-// of them find room in the chip's SM groups.) The first weight tiles are requested before the kernels ahead in the
+// are the UMMA N dimension. K is split over a thread-block cluster of up to 8 CTAs so that about every SM streams
+// weights, and the partial sums are exchanged through distributed shared memory: no fp32 partials in memory and no
+// reduction launch. The first weight tiles are requested before the kernels ahead in the
 // stream have finished.
 //   QUANT = true: X is the 16-bit input of a linear layer of a few rows (NT = 16); every CTA quantises its K range once,
 //       up front (same bytes and scales as the stand-alone quantiser), and keeps it in shared memory for all of its
@@ -27,6 +26,7 @@ struct LinearStreamParams {
   void* out;        // OutT [M, N]
   int M, N, K, num_kb, kb_per_rank;
   int n_tiles, t_tiles, stages;
+  int own_sums;  // a cluster's sums have a place outside the ring
   float eps;
   int* status;
 };
@@ -100,6 +100,8 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // "I have started", waited for before another CTA's shared memory is written at the very end
+  if (csize > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   // after the TMEM allocation: a dependent grid's CTA that got its columns first, and then waits for this grid, would
   // otherwise hold them for ever
   grid_launch_dependents();
@@ -294,23 +296,31 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 
   if (csize > 1) {
     __syncwarp();
-    ptx::cluster_barrier();  // the first CTA's ring is idle: the other ranks' sums go there, [rank - 1][token][row]
-    const int rows = min(NT, p.M - item0 % p.t_tiles * NT);
-    if (warp < 8 && rank > 0) {
-      const uint32_t dst = ptx::stream_mapa(smem_base, 0) + (((rank - 1) * rows) * 256 + half * 128 + r) * 4;
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+    // every rank adds up its share of the tokens (token t belongs to rank t / per): [rank][token][row], behind the tables, or
+    // in the ring, which is idle once every rank is here
+    if (!p.own_sums) ptx::cluster_barrier();
+    const uint32_t sums_off = p.own_sums ? (uint32_t)(reinterpret_cast<uint8_t*>(bs_tab + 2 * cap) - smem_al + 15) & ~15u : 0u;
+    const int nt = item0 / p.t_tiles, m0 = (item0 - nt * p.t_tiles) * NT;
+    const int rows = min(NT, p.M - m0), per = (rows + (int)csize - 1) / (int)csize, n = half * 128 + r;
+    if (warp < 8) {
+      int owner = 0, j = 0;
 #pragma unroll
-      for (int t = 0; t < NT; ++t)
-        if (t < rows) ptx::st_cluster_f32(dst + t * 1024, acc[t]);
+      for (int t = 0; t < NT; ++t) {
+        if (t < rows) ptx::st_cluster_f32(ptx::stream_mapa(smem_base + sums_off, owner) + (((int)rank * per + j) * 256 + n) * 4, acc[t]);
+        if (++j == per) j = 0, ++owner;
+      }
     }
     __syncwarp();
     ptx::cluster_barrier();
-    if (warp < 8 && rank == 0 && sum_ok) {
-      const float* src = reinterpret_cast<const float*>(smem_al) + half * 128 + r;
-      for (int c = 1; c < (int)csize; ++c)  // rank order: the same sum on every run
-#pragma unroll
-        for (int t = 0; t < NT; ++t)
-          if (t < rows) acc[t] += src[((c - 1) * rows + t) * 256];
-      store(item0);
+    if (warp < 8 && sum_ok && nt * 256 + n < p.N) {
+      const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + n;
+      T* out = static_cast<T*>(p.out) + nt * 256 + n;
+      for (int j = 0; j < per && (int)rank * per + j < rows; ++j) {
+        float sum = 0.f;
+        for (int c = 0; c < (int)csize; ++c) sum += src[(c * per + j) * 256];  // rank order: the same sum on every run
+        out[(int64_t)(m0 + (int)rank * per + j) * p.N] = from_f32<T>(sum);
+      }
     }
   }
 
@@ -327,15 +337,19 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   }
 }
 
+inline int64_t linear_sum_bytes(int64_t csize, int64_t rows) { return csize * cdiv(rows, csize) * 1024 + 16; }
+
 // Cluster size and ring depth; false when nothing fits.
 template <int NT, bool QUANT>
-inline bool plan_linear_stream(int64_t M, int64_t N, int64_t K, int sms, int& csize, int& kb_per_rank, int& stages) {
+inline bool plan_linear_stream(int64_t M, int64_t N, int64_t K, int sms, int& csize, int& kb_per_rank, int& stages, int& own_sums) {
   using Cfg = LinearStreamCfg<NT, QUANT>;
   const int64_t items = cdiv(N, 256) * cdiv(M, NT), num_kb = cdiv(K, kBK), rows = M < NT ? M : NT;
   // as many ranks per item as bring items x ranks up to the SM count, two K blocks each at least; where a rank could not
   // hold its K range, or the ring not the other ranks' sums, the nearest cluster size that fits
   int64_t want = sms / items;
-  if (want > 4) want = 4;
+  // Clusters of up to 8 where they leave a quarter of the chip free; up to 4 otherwise, which fit its SM groups (16 tiles,
+  // 1 x 4096 x 14336: 19.7 us with clusters of 8, 13.9 with 4; 3 tiles, 1 x 768 x 4096: 5.6 and 6.6)
+  if (want > 4) want = items * 8 * 4 <= (int64_t)sms * 3 + 12 ? 8 : 4;
   if (want > num_kb / 2) want = num_kb / 2;
   if (want < 1) want = 1;
   for (int i = 0; i < 16; ++i) {
@@ -348,8 +362,14 @@ inline bool plan_linear_stream(int64_t M, int64_t N, int64_t K, int sms, int& cs
     int64_t s = Cfg::kMinCtas == 2 ? (Cfg::kHalfSm - tail) / Cfg::kStage : 0;
     if (s < 3) s = (Cfg::kSmemLimit - tail) / Cfg::kStage;
     stages = (int)(s < Cfg::kMaxStages ? s : Cfg::kMaxStages);
-    // the other ranks' sums (1 KB per row each) land in the ring
-    if (stages >= 2 && (csize - 1) * rows * 1024 <= (int64_t)stages * Cfg::kStage) return true;
+    // the ranks' sums (1 KB per row) get a place of their own where three stages remain, else they land in the ring, one more
+    // barrier later
+    const int64_t sums = linear_sum_bytes(csize, rows);
+    const bool half = Cfg::kMinCtas == 2 && (int64_t)stages * Cfg::kStage + tail <= Cfg::kHalfSm;
+    const int64_t left = ((half ? Cfg::kHalfSm : Cfg::kSmemLimit) - tail - sums) / Cfg::kStage;
+    own_sums = csize > 1 && left >= 3;
+    if (own_sums) stages = (int)(left < Cfg::kMaxStages ? left : Cfg::kMaxStages);
+    if (own_sums || (stages >= 2 && (csize == 1 || sums <= (int64_t)stages * Cfg::kStage))) return true;
   }
   return false;
 }
@@ -363,7 +383,7 @@ inline int launch_linear_stream(const void* W, const void* X, LinearStreamParams
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_tiles = (int)cdiv(p.N, 256);
   p.t_tiles = (int)cdiv(p.M, NT);
-  if (!plan_linear_stream<NT, QUANT>(p.M, p.N, p.K, sms, csize, p.kb_per_rank, p.stages)) {
+  if (!plan_linear_stream<NT, QUANT>(p.M, p.N, p.K, sms, csize, p.kb_per_rank, p.stages, p.own_sums)) {
     set_error_detail("linear_stream: K=%d does not fit shared memory", p.K);
     return B200_E_UNSUPPORTED;
   }
@@ -381,7 +401,7 @@ inline int launch_linear_stream(const void* W, const void* X, LinearStreamParams
   if (int rc_smem = allow_smem(k, Cfg::kSmemLimit, "linear_stream_kernel")) return rc_smem;
   const int64_t items = (int64_t)p.n_tiles * p.t_tiles;
   const int64_t clusters = csize > 1 ? items : (items < sms ? items : sms);
-  return launch_dependent(k, dim3((unsigned)(clusters * csize)), Cfg::kThreads, Cfg::smem_for(p.stages, p.kb_per_rank), st,
+  return launch_dependent(k, dim3((unsigned)(clusters * csize)), Cfg::kThreads, Cfg::smem_for(p.stages, p.kb_per_rank) + (p.own_sums ? (size_t)linear_sum_bytes(csize, p.M < NT ? p.M : NT) : 0), st,
                           csize, "linear_stream_kernel", tw, tx, p);
 }
 

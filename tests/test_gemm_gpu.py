@@ -330,3 +330,11 @@ def test_one_launch_linear_plans(M, N, K):
                                        ws.cuda(), [128, 128], x.dtype)
     _status_ok()
     assert float((out.float() - two_step.float()).norm() / two_step.float().norm()) < 2e-3
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 128, 512), (5, 392, 1280), (16, 768, 4096), (17, 256, 1152), (32, 1280, 8192), (50, 520, 2064)])
+def test_decode_kernel_cluster_sums(M, N, K):
+    """K splits of the decode kernel summed within a cluster: cluster sizes 2 to 8, rows that do not divide by them, ragged
+    columns and K, one and two token tiles."""
+    for dt in (torch.bfloat16, torch.float32):
+        _case(M, N, K, 970 + M, out_dtype=dt, col_major=M % 2 == 0)
