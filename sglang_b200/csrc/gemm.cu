@@ -81,7 +81,7 @@ struct GemmPlan {
 
 // Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up
 // (4.5 us), then whole waves of tiles: microseconds per 128-K block of a tile and 0.8 us for its epilogue; K splits add a
-// reduction pass (2 us and their fp32 partials, written and read at about 4 TB/s); nothing is faster than reading the
+// reduction pass (0.5 us and their fp32 partials, written and read at about 2 TB/s); nothing is faster than reading the
 // weights (6.2 TB/s). The decode kernel re-reads the weights for every 32 rows at the L2's 10.5 TB/s. The constants are
 // fits to measurements at 10 weight shapes (1280..28672 x 1024..14336) and 8 row counts (72..1027), where the plan is
 // within 10 % of the best configuration; what they decide is mostly wave counts, e.g. 203 x 6144 x 4096: single 22.3 us,
@@ -102,7 +102,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       const double waves = (double)cdiv(tiles * s, slots);
       double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + 0.8);
       if (work < stream_us) work = stream_us;
-      const double us = 4.5 + work + (s > 1 ? 2.0 + 8.0 * s * (double)M * (double)N / 4e6 : 0.0);
+      const double us = 4.5 + work + (s > 1 ? 0.5 + 16.0 * s * (double)M * (double)N / 4e6 : 0.0);
       if (us < best.us) best = {s, pair_bn, false, false, us};
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }

@@ -190,6 +190,7 @@ __global__ void __launch_bounds__(256, 6) moe_sum_reduce_kernel(const T* __restr
   __shared__ int s_slot[kSumReduceMaxSlots];
   __shared__ int s_n;
   const int64_t t = blockIdx.x;
+  grid_launch_dependents();
   grid_dependency_wait();
   if (poison_status != nullptr && *reinterpret_cast<const volatile int*>(poison_status) != 0) {
     // the rows were to be written by other GPUs and the handshake before this kernel gave up: NaNs, not stale rows

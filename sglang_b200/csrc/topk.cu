@@ -54,6 +54,8 @@ template <typename T, int VMAX>
 __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
   const int lane = threadIdx.x & 31;
   const int64_t tok = (int64_t)blockIdx.x * 4 + (threadIdx.x >> 5);
+  grid_launch_dependents();  // the kernels that follow may be set up; they wait for this grid
+  grid_dependency_wait();
   if (tok >= p.T) return;
   const unsigned full = 0xffffffffu;
   const int vpl = p.vpl, E = p.E;
@@ -205,16 +207,18 @@ __global__ void __launch_bounds__(128) route_topk_kernel(const RouteParams p) {
   }
 }
 
+template <typename T, int VMAX>
+static int launch_route_inst(const RouteParams& p, cudaStream_t st) {
+  return launch_dependent(route_topk_kernel<T, VMAX>, dim3((unsigned)cdiv(p.T, 4)), 128, 0, st, 1, "route_topk_kernel", p);
+}
 template <typename T>
 static int launch_route(const RouteParams& p, cudaStream_t st) {
-  const unsigned grid = (unsigned)cdiv(p.T, 4);
-  if (p.vpl <= 1) route_topk_kernel<T, 1><<<grid, 128, 0, st>>>(p);
-  else if (p.vpl <= 2) route_topk_kernel<T, 2><<<grid, 128, 0, st>>>(p);
-  else if (p.vpl <= 4) route_topk_kernel<T, 4><<<grid, 128, 0, st>>>(p);
-  else if (p.vpl <= 8) route_topk_kernel<T, 8><<<grid, 128, 0, st>>>(p);
-  else if (p.vpl <= 16) route_topk_kernel<T, 16><<<grid, 128, 0, st>>>(p);
-  else route_topk_kernel<T, 32><<<grid, 128, 0, st>>>(p);
-  return check_launch("route_topk_kernel");
+  if (p.vpl <= 1) return launch_route_inst<T, 1>(p, st);
+  if (p.vpl <= 2) return launch_route_inst<T, 2>(p, st);
+  if (p.vpl <= 4) return launch_route_inst<T, 4>(p, st);
+  if (p.vpl <= 8) return launch_route_inst<T, 8>(p, st);
+  if (p.vpl <= 16) return launch_route_inst<T, 16>(p, st);
+  return launch_route_inst<T, 32>(p, st);
 }
 
 static int launch_route_dtype(const RouteParams& p, int logits_dtype, void* stream) {
