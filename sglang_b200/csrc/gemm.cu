@@ -286,12 +286,15 @@ static int run_linear_stream(const void* x, int x_dtype, const void* B, const fl
 static size_t linear_q_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * K), 256); }
 static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * (K / 128)) * 4, 256); }
 // One launch (linear_stream.cuh) or quantiser + GEMM. The one launch saves the quantiser's and the reduction's, but every
-// CTA quantises its K range of x for itself: worth it up to 64 (row, K block) groups per CTA.
+// CTA quantises its K range of x for itself. On the GPU the two are level within a few tenths of a microsecond up to 32 (row,
+// K block) groups per CTA (1 x 1536 x 4096: 4.7 us against 5.2, 1 x 4096 x 1792: 5.3 against 4.9) and the second wins beyond
+// (16 x 768 x 4096: 6.6 against 5.2) and for larger weights (1 x 8192 x 3584: 8.3 against 7.2); with small weights the GPU
+// finishes before the host, which pays 4.7 us for one launch and 7 for two.
 constexpr int64_t kLinearStreamMaxM = 16;
 static bool linear_one_launch(int64_t M, int64_t N, int64_t K) {
   int csize, kb, stages, own;
   return M <= kLinearStreamMaxM && tuning().linear_decode_fused != 0 &&
-         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages, own) && kb * M <= 64;
+         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages, own) && kb * M <= 32 && N * K < (16 << 20);
 }
 }  // namespace b200
 

@@ -290,7 +290,7 @@ def w8a8_block_fp8_linear(
             return output.to(dtype=input.dtype)
     input_2d = input.view(-1, input.shape[-1])
     output_shape = [*input.shape[:-1], weight.shape[0]]
-    output = _linear_decode_fused(input_2d, weight, block_size, weight_scale)
+    output = _linear_decode_fused(input_2d, weight, block_size, weight_scale, max_rows=4)
     if output is None:
         q_input, x_scale = per_token_group_quant_fp8(input_2d, block_size[1], column_major_scales=True)
         output = w8a8_block_fp8_matmul(q_input, weight, x_scale, weight_scale, block_size, output_dtype=input_2d.dtype)
@@ -299,14 +299,14 @@ def w8a8_block_fp8_linear(
     return output.to(dtype=input_2d.dtype).view(*output_shape)
 
 
-# Rows up to which the one-launch kernel is always taken (it handles 16; for more rows the native path weighs it against
-# quantiser + GEMM).
-DECODE_FUSED_MAX_M = 1
+# Rows up to which every call takes the one-launch kernel: none, the native path weighs it against quantiser + GEMM by
+# size. (It takes up to 16 rows, and for up to 4 any K that is a multiple of 16.)
+DECODE_FUSED_MAX_M = 0
 
 
 def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weight_scale: torch.Tensor,
                          max_rows: int = DECODE_FUSED_MAX_M):
-    """A few rows (the kernel takes up to 16, this wrapper sends it up to ``DECODE_FUSED_MAX_M``) of 16-bit
+    """A few rows (the kernel takes up to 16, the wrapper sends it up to ``max_rows``) of 16-bit
     activations: quantiser, GEMM and split-K sum as ONE launch (every CTA
     quantises the slice of ``x`` it needs; same bytes and scales as ``per_token_group_quant_fp8``). Returns
     None when the shapes or dtypes are outside that kernel, and the caller takes the two-step path."""

@@ -338,3 +338,20 @@ def test_decode_kernel_cluster_sums(M, N, K):
     columns and K, one and two token tiles."""
     for dt in (torch.bfloat16, torch.float32):
         _case(M, N, K, 970 + M, out_dtype=dt, col_major=M % 2 == 0)
+
+
+def test_linear_of_a_few_rows_takes_any_k():
+    """Up to four rows the linear takes a K that is no multiple of the 128-group (the last group is shorter)."""
+    import sglang_b200 as S
+
+    M, N, K = 3, 264, 400
+    x, wq = make_activation(M, K, 60), _rand_fp8((N, K), 61)
+    ws = torch.rand(3, 4, generator=torch.Generator().manual_seed(62)) * 1e-3
+    pad = torch.zeros(M, 512, dtype=x.dtype)
+    pad[:, :K] = x
+    wpad = torch.zeros(N, 512).to(torch.float8_e4m3fn)
+    wpad[:, :K] = wq
+    ref = O.w8a8_block_fp8_linear(pad, wpad, ws, output_dtype=torch.float32)
+    out = S.w8a8_block_fp8_linear(x.cuda(), wq.cuda(), [128, 128], ws.cuda())
+    _status_ok()
+    assert O.rel_frobenius(out.float().cpu(), ref) < TOL
