@@ -47,11 +47,12 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
     }
     return;
   }
-  __shared__ int pos[64];        // topk <= kSumReduceMaxSlots
+  __shared__ int pos[64];
   __shared__ float row_s[kRowScales];
   const int64_t tok = blockIdx.x;
-  for (int j = threadIdx.x; j < topk; j += blockDim.x) pos[j] = __ldg(position + tok * topk + j);
+  for (int j = threadIdx.x; j < min(topk, 64); j += blockDim.x) pos[j] = __ldg(position + tok * topk + j);
   __syncthreads();
+  auto position_of = [&](int j) { return j < 64 ? pos[j] : __ldg(position + tok * topk + j); };
   const int groups = (int)(H / 128);
   for (int c0 = threadIdx.x & ~31; c0 < H / 16; c0 += blockDim.x) {  // whole warps
     const int chunk = c0 + (threadIdx.x & 31);
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
     if (!active) continue;
     if ((chunk & 7) == 0 && chunk / 8 < kRowScales) row_s[chunk / 8] = scale;
     for (int j = 0; j < topk; ++j) {
-      const int64_t p = pos[j];
+      const int64_t p = position_of(j);
       if (p < 0) continue;  // an expert on another rank
       *reinterpret_cast<uint4*>(q + p * H + chunk * 16) = out;
       if ((chunk & 7) == 0 && chunk / 8 >= kRowScales) s[p * s_row + (chunk / 8) * s_group] = scale;
@@ -88,7 +89,7 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
   const int kept = min(groups, kRowScales);
   for (int i = threadIdx.x; i < topk * kept; i += blockDim.x) {  // consecutive threads -> consecutive groups of one row
     const int j = i / kept, g = i - j * kept;
-    const int64_t p = pos[j];
+    const int64_t p = position_of(j);
     if (p >= 0) s[p * s_row + g * s_group] = row_s[g];
   }
 }
