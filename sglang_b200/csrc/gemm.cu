@@ -142,6 +142,35 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N,
 }
 
 namespace b200 {
+// The decode kernel (gemm_skinny.cuh) with its K split; sp holds the scales.
+static int run_skinny(const void* A, const void* B, SkinnyParams sp, int splits, void* C, int c_dtype, int64_t M, int64_t N,
+                      int64_t K, void* workspace, size_t workspace_bytes, cudaStream_t st, const FanOut& fan) {
+  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16>::kMaxKb) ++splits;  // scales of one item fit its smem table
+  sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
+  // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
+  const int nt = skinny_token_tile(M);
+  const int cluster = splits > 1 && tuning().gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
+  if (cluster > 1) splits = cluster;
+  if (fan.n == 0 && (splits == 1 || cluster > 1)) {
+    sp.C = C;
+    if (c_dtype == B200_BF16) return launch_skinny<__nv_bfloat16>(A, B, sp, splits, splits > 1, st);
+    if (c_dtype == B200_F16) return launch_skinny<__half>(A, B, sp, splits, splits > 1, st);
+    return launch_skinny<float>(A, B, sp, splits, splits > 1, st);
+  }
+  const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
+  if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15) != 0) {
+    set_error_detail("gemm: split-K needs a 16-byte aligned workspace of %zu bytes (got %zu)", need, workspace_bytes);
+    return B200_E_WORKSPACE;
+  }
+  sp.C = workspace;
+  int rc = launch_skinny<float>(A, B, sp, splits, false, st);
+  if (rc) return rc;
+  const float* part = static_cast<const float*>(workspace);
+  if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
+  if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
+  return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
+}
+
 static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_t as_stride_k, const void* B,
                      const float* Bs, void* C, int c_dtype, int64_t M, int64_t N, int64_t K, void* workspace,
                      size_t workspace_bytes, void* stream, const FanOut& fan) {
@@ -183,32 +212,9 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     return launch_linear_stream<64, false, float>(B, A, lp, st);
   }
   if (skinny) {
-    while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16>::kMaxKb) ++splits;  // scales of one item fit its smem table
     SkinnyParams sp = {};
     sp.As = As; sp.as_sm = as_stride_m; sp.as_sk = as_stride_k; sp.Bs = Bs;
-    sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
-    // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
-    const int nt = skinny_token_tile(M);
-    const int cluster = splits > 1 && tune.gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
-    if (cluster > 1) splits = cluster;
-    if (fan.n == 0 && (splits == 1 || cluster > 1)) {
-      sp.C = C;
-      if (c_dtype == B200_BF16) return launch_skinny<__nv_bfloat16>(A, B, sp, splits, splits > 1, st);
-      if (c_dtype == B200_F16) return launch_skinny<__half>(A, B, sp, splits, splits > 1, st);
-      return launch_skinny<float>(A, B, sp, splits, splits > 1, st);
-    }
-    const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
-    if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 15) != 0) {
-      set_error_detail("gemm: split-K needs a 16-byte aligned workspace of %zu bytes (got %zu)", need, workspace_bytes);
-      return B200_E_WORKSPACE;
-    }
-    sp.C = workspace;
-    int rc = launch_skinny<float>(A, B, sp, splits, false, st);
-    if (rc) return rc;
-    const float* part = static_cast<const float*>(workspace);
-    if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
-    if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
-    return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
+    return run_skinny(A, B, sp, splits, C, c_dtype, M, N, K, workspace, workspace_bytes, st, fan);
   }
   const int bn = plan.pair_bn;
   // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
@@ -454,6 +460,16 @@ extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa
   if (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0) {
     set_error_detail("gemm_packed: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
+  }
+  const GemmPlan plan = plan_gemm(M, N, K, sm_count() < 148 ? sm_count() : 148, tuning().gemm_bn < 0);
+  if (plan.skinny && tuning().gemm_splitk <= 0) {  // a few rows: the decode kernel reads the packed words itself
+    B200_CHECK_ARG(A && B && C && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B & 15) == 0 && ((uintptr_t)C & 15) == 0,
+                   "gemm_packed: A, B and C must be 16-byte aligned");
+    B200_CHECK_ARG(c_dtype == B200_BF16 || c_dtype == B200_F16 || c_dtype == B200_F32, "gemm_packed: unknown output dtype code %d", c_dtype);
+    B200_UNSUPPORTED(K % 16 != 0 || N % 8 != 0, "gemm_packed: K=%lld must be a multiple of 16, N=%lld of 8", (long long)K, (long long)N);
+    SkinnyParams sp = {};
+    sp.sfa = sfa; sp.sfb = sfb; sp.sfa_ld = sfa_ld; sp.sfb_ld = sfb_ld; sp.sfb_step = 128 / sfb_rows_per_word;
+    return run_skinny(A, B, sp, plan.splits, C, c_dtype, M, N, K, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), FanOut{});
   }
   float* as = static_cast<float*>(workspace);
   uint8_t* bs = static_cast<uint8_t*>(workspace) + packed_as_bytes(M, K);

@@ -18,6 +18,11 @@ struct SkinnyParams {
   const float* As;  // As[m*as_sm + kb*as_sk]
   int64_t as_sm, as_sk;
   const float* Bs;  // [ceil(N/128)][num_kb]
+  // packed power-of-two scales instead (As null): word (kb / 4) * ld + row holds the exponents of four K blocks; sfb_step rows
+  // of words per 128 weight rows
+  const int32_t *sfa, *sfb;
+  int64_t sfa_ld, sfb_ld;
+  int sfb_step;
   void* C;          // OutT [M, N], or fp32 partials [splits][M, N]
   int M, N, K, num_kb;
   int n_tiles, t_tiles, k_splits, kb_per_split;
@@ -117,7 +122,17 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     for (int i = threadIdx.x; i < (kb1 - kb0) * NT; i += 128) {
       const int kb = kb0 + i / NT, t = i % NT;
       const int m = m0 + t;
-      scales[i] = m < p.M ? __ldg(p.As + (int64_t)m * p.as_sm + (int64_t)kb * p.as_sk) * __ldg(bs_row + kb) : 0.f;
+      float s = 0.f;
+      if (m < p.M) {
+        if (p.As != nullptr) {
+          s = __ldg(p.As + (int64_t)m * p.as_sm + (int64_t)kb * p.as_sk) * __ldg(bs_row + kb);
+        } else {  // exponent byte -> power of two
+          const uint32_t a = (uint32_t)__ldg(p.sfa + (kb >> 2) * p.sfa_ld + m) >> (8 * (kb & 3));
+          const uint32_t b = (uint32_t)__ldg(p.sfb + (kb >> 2) * p.sfb_ld + (int64_t)nt * p.sfb_step) >> (8 * (kb & 3));
+          s = __uint_as_float((a & 0xffu) << 23) * __uint_as_float((b & 0xffu) << 23);
+        }
+      }
+      scales[i] = s;
     }
     asm volatile("bar.sync 1, 128;" ::: "memory");
   }

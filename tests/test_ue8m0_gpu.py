@@ -174,3 +174,18 @@ def test_block_scaled_single_and_pair_tiles(M, N, K, knob):
             out = S.w8a8_block_fp8_matmul(xq, wq.cuda(), xs_packed, packed, [128, 128], torch.float32)
         _status_ok()
         assert O.rel_frobenius(out.cpu(), ref) < 1e-4
+
+
+@pytest.mark.parametrize("M,N,K", [(1, 8, 128), (7, 768, 4096), (32, 1032, 640), (50, 512, 2048), (64, 256, 8192)])
+def test_packed_scales_of_a_few_rows(M, N, K):
+    """Few rows: the decode kernel reads the packed words itself; equal to the same kernel on the unpacked scales."""
+    import sglang_b200 as S
+    from sglang_b200 import weight_quant as W
+
+    xq, xs_packed, wq, ws, osf, ref = _ue8m0_case(M, N, K, 71 + M + N)
+    for packed in (W.transform_scale_ue8m0(ws, mn=N).cuda(), W.pack_ue8m0_mn_major(ws).cuda()):
+        for dt in (torch.bfloat16, torch.float32):
+            out = S.w8a8_block_fp8_matmul(xq, wq.cuda(), xs_packed, packed, [128, 128], dt)
+            _status_ok()
+            assert O.rel_frobenius(out.float().cpu(), ref) < (1e-4 if dt == torch.float32 else 5e-3)
+            assert torch.equal(out, S.w8a8_block_fp8_matmul(xq, wq.cuda(), osf.cuda(), ws.cuda(), [128, 128], dt))
