@@ -136,6 +136,8 @@ block_fp8_gemm_ue8m0_kernel(const __grid_constant__ CUtensorMap tmap_a, const __
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  grid_launch_dependents();
+  grid_dependency_wait();
 
   const int total_tiles = p.m_tiles * p.n_tiles;
   const int num_kb = p.num_kb;
@@ -323,8 +325,7 @@ inline int launch_gemm_ue8m0(const void* A, const void* B, Ue8m0Params p, cudaSt
   if (rc) return rc;
   auto k = block_fp8_gemm_ue8m0_kernel<OutT>;
   if (int rc_smem = allow_smem(k, Ue8m0Cfg::kSmemBytes, "GEMM kernel")) return rc_smem;
-  k<<<grid, Ue8m0Cfg::kThreads, Ue8m0Cfg::kSmemBytes, st>>>(ta, tb, p);
-  return check_launch("block_fp8_gemm_ue8m0_kernel");
+  return launch_dependent(k, dim3((unsigned)grid), Ue8m0Cfg::kThreads, Ue8m0Cfg::kSmemBytes, st, 1, "block_fp8_gemm_ue8m0_kernel", ta, tb, p);
 }
 
 }  // namespace b200

@@ -54,31 +54,29 @@ static int launch_quant(const void* x, void* q, float* s, int64_t M, int64_t K, 
     return B200_E_UNSUPPORTED;
   }
   const int cpr = (int)(K / 16);
-#define B200_Q_LAUNCH_F(LPG, F)                                                                            \
-  quant_group_kernel<T, LPG, F><<<(unsigned)blocks, threads, 0, st>>>(static_cast<const T*>(x),            \
-                                                                      static_cast<uint8_t*>(q), s, total, \
-                                                                      cpr, ssm, ssg, eps, 0)
-#define B200_Q_LAUNCH(LPG)                                        \
-  switch (formula) {                                              \
-    case B200_QUANT_RECIP: B200_Q_LAUNCH_F(LPG, B200_QUANT_RECIP); break; \
-    case B200_QUANT_V2: B200_Q_LAUNCH_F(LPG, B200_QUANT_V2); break;       \
-    case B200_QUANT_DIV_CORRECTED: B200_Q_LAUNCH_F(LPG, B200_QUANT_DIV_CORRECTED); break; \
-    default: B200_Q_LAUNCH_F(LPG, B200_QUANT_DIV); break;         \
+#define B200_Q_LAUNCH_F(LPG, F)                                                                                            \
+  return launch_dependent(quant_group_kernel<T, LPG, F>, dim3((unsigned)blocks), threads, 0, st, 1, "per_token_group_quant_fp8", \
+                          static_cast<const T*>(x), static_cast<uint8_t*>(q), s, total, cpr, ssm, ssg, eps, 0)
+#define B200_Q_LAUNCH(LPG)                                                        \
+  switch (formula) {                                                              \
+    case B200_QUANT_RECIP: B200_Q_LAUNCH_F(LPG, B200_QUANT_RECIP);                \
+    case B200_QUANT_V2: B200_Q_LAUNCH_F(LPG, B200_QUANT_V2);                      \
+    case B200_QUANT_DIV_CORRECTED: B200_Q_LAUNCH_F(LPG, B200_QUANT_DIV_CORRECTED); \
+    default: B200_Q_LAUNCH_F(LPG, B200_QUANT_DIV);                                \
   }
   switch (group) {
-    case 16: B200_Q_LAUNCH(1); break;
-    case 32: B200_Q_LAUNCH(2); break;
-    case 64: B200_Q_LAUNCH(4); break;
-    case 128: B200_Q_LAUNCH(8); break;
-    case 256: B200_Q_LAUNCH(16); break;
-    case 512: B200_Q_LAUNCH(32); break;
+    case 16: B200_Q_LAUNCH(1);
+    case 32: B200_Q_LAUNCH(2);
+    case 64: B200_Q_LAUNCH(4);
+    case 128: B200_Q_LAUNCH(8);
+    case 256: B200_Q_LAUNCH(16);
+    case 512: B200_Q_LAUNCH(32);
     default:
       set_error_detail("quant: group size %d not in {16,32,64,128,256,512}", group);
       return B200_E_UNSUPPORTED;
   }
 #undef B200_Q_LAUNCH
 #undef B200_Q_LAUNCH_F
-  return check_launch("per_token_group_quant_fp8");
 }
 
 template <typename T>
@@ -107,6 +105,7 @@ __global__ void __launch_bounds__(256) quant_group_ue8m0_kernel(const T* __restr
                                                                 int chunks_per_row, int64_t aligned_mn,
                                                                 const int32_t* __restrict__ masked_m,
                                                                 int64_t rows_per_expert) {
+  grid_dependency_wait();  // x, and the readers of the buffers overwritten below
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   bool active = c < total_chunks;
   const int64_t row = active ? c / chunks_per_row : 0;
@@ -167,28 +166,24 @@ static int launch_quant_ue8m0(const void* x, void* q, void* s, int64_t M, int64_
     return B200_E_UNSUPPORTED;
   }
   const int cpr = (int)(K / 16);
-#define B200_QU_LAUNCH(LPG)                                                                                          \
-  do {                                                                                                               \
-    if (silu)                                                                                                        \
-      quant_group_ue8m0_kernel<T, LPG, true><<<(unsigned)blocks, 256, 0, st>>>(                                      \
-          static_cast<const T*>(x), static_cast<uint8_t*>(q), static_cast<uint8_t*>(s), total, cpr, aligned_mn,     \
-          masked_m, rows_per_expert);                                                                                \
-    else                                                                                                             \
-      quant_group_ue8m0_kernel<T, LPG, false><<<(unsigned)blocks, 256, 0, st>>>(                                     \
-          static_cast<const T*>(x), static_cast<uint8_t*>(q), static_cast<uint8_t*>(s), total, cpr, aligned_mn,     \
-          masked_m, rows_per_expert);                                                                                \
-  } while (0)
+#define B200_QU_LAUNCH_S(LPG, SILU)                                                                                        \
+  return launch_dependent(quant_group_ue8m0_kernel<T, LPG, SILU>, dim3((unsigned)blocks), 256, 0, st, 1,                   \
+                          "per_token_group_quant_fp8_ue8m0", static_cast<const T*>(x), static_cast<uint8_t*>(q),           \
+                          static_cast<uint8_t*>(s), total, cpr, aligned_mn, masked_m, rows_per_expert)
+#define B200_QU_LAUNCH(LPG)           \
+  if (silu) B200_QU_LAUNCH_S(LPG, true); \
+  B200_QU_LAUNCH_S(LPG, false)
   switch (group) {
-    case 16: B200_QU_LAUNCH(1); break;
-    case 32: B200_QU_LAUNCH(2); break;
-    case 64: B200_QU_LAUNCH(4); break;
-    case 128: B200_QU_LAUNCH(8); break;
+    case 16: B200_QU_LAUNCH(1);
+    case 32: B200_QU_LAUNCH(2);
+    case 64: B200_QU_LAUNCH(4);
+    case 128: B200_QU_LAUNCH(8);
     default:
       set_error_detail("quant (UE8M0): group size %d not in {16,32,64,128}", group);
       return B200_E_UNSUPPORTED;
   }
 #undef B200_QU_LAUNCH
-  return check_launch("per_token_group_quant_fp8_ue8m0");
+#undef B200_QU_LAUNCH_S
 }
 
 }  // namespace b200
