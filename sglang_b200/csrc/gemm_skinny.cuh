@@ -247,10 +247,18 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     if (warp < 4 && ok_sum && n0 + r < p.N) {
       const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + r;
       OutT* out = static_cast<OutT*>(p.C) + n0 + r;
-      for (int j = 0; j < per && ks * per + j < rows; ++j) {
-        float sum = 0.f;
-        for (int c = 0; c < p.k_splits; ++c) sum += src[(c * per + j) * 128];  // split order: the same sum on every run
-        out[(int64_t)(m0 + ks * per + j) * p.N] = from_f32<OutT>(sum);
+      const int t0 = ks * per, n_mine = min(per, rows - t0);
+      constexpr int U = 4;  // rows in flight
+      for (int j = 0; j < n_mine; j += U) {
+        float sum[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) sum[u] = 0.f;
+        for (int c = 0; c < p.k_splits; ++c)  // split order: the same sum on every run
+#pragma unroll
+          for (int u = 0; u < U; ++u) sum[u] += src[(c * per + min(j + u, n_mine - 1)) * 128];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (j + u < n_mine) out[(int64_t)(m0 + t0 + j + u) * p.N] = from_f32<OutT>(sum[u]);
       }
     }
   }

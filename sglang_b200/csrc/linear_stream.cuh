@@ -316,10 +316,18 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if (warp < 8 && sum_ok && nt * 256 + n < p.N) {
       const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + n;
       T* out = static_cast<T*>(p.out) + nt * 256 + n;
-      for (int j = 0; j < per && (int)rank * per + j < rows; ++j) {
-        float sum = 0.f;
-        for (int c = 0; c < (int)csize; ++c) sum += src[(c * per + j) * 256];  // rank order: the same sum on every run
-        out[(int64_t)(m0 + (int)rank * per + j) * p.N] = from_f32<T>(sum);
+      const int t0 = (int)rank * per, n_mine = min(per, rows - t0);
+      constexpr int U = NT == 16 ? 2 : 8;  // rows in flight
+      for (int j = 0; j < n_mine; j += U) {
+        float sum[U];
+#pragma unroll
+        for (int u = 0; u < U; ++u) sum[u] = 0.f;
+        for (int c = 0; c < (int)csize; ++c)  // rank order: the same sum on every run
+#pragma unroll
+          for (int u = 0; u < U; ++u) sum[u] += src[(c * per + min(j + u, n_mine - 1)) * 256];
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+          if (j + u < n_mine) out[(int64_t)(m0 + t0 + j + u) * p.N] = from_f32<T>(sum[u]);
       }
     }
   }
@@ -362,12 +370,12 @@ inline bool plan_linear_stream(int64_t M, int64_t N, int64_t K, int sms, int& cs
     int64_t s = Cfg::kMinCtas == 2 ? (Cfg::kHalfSm - tail) / Cfg::kStage : 0;
     if (s < 3) s = (Cfg::kSmemLimit - tail) / Cfg::kStage;
     stages = (int)(s < Cfg::kMaxStages ? s : Cfg::kMaxStages);
-    // the ranks' sums (1 KB per row) get a place of their own where three stages remain, else they land in the ring, one more
-    // barrier later
+    // the ranks' sums (1 KB per row) get a place of their own where that costs the ring no stage it needs (64 KB of 64-token sums took two of
+    // five: 61 rows, four projections of a rank of four 76 -> 79.5 us), else they land in the ring, one more barrier later
     const int64_t sums = linear_sum_bytes(csize, rows);
     const bool half = Cfg::kMinCtas == 2 && (int64_t)stages * Cfg::kStage + tail <= Cfg::kHalfSm;
     const int64_t left = ((half ? Cfg::kHalfSm : Cfg::kSmemLimit) - tail - sums) / Cfg::kStage;
-    own_sums = csize > 1 && left >= 3;
+    own_sums = csize > 1 && (left >= 5 || left >= (stages < Cfg::kMaxStages ? stages : Cfg::kMaxStages));
     if (own_sums) stages = (int)(left < Cfg::kMaxStages ? left : Cfg::kMaxStages);
     if (own_sums || (stages >= 2 && (csize == 1 || sums <= (int64_t)stages * Cfg::kStage))) return true;
   }

@@ -37,9 +37,11 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
     // so their content is free. Zeros keep the tensor cores' power draw down when tiles are mostly real rows; with a few
     // tokens per expert writing them would dominate this kernel, and the launch leaves these blocks out.
     const int64_t slot0 = ((int64_t)blockIdx.x - T_tokens) * kPadSlots;
-    const int live = (int)min((int64_t)kPadSlots, *num_post_pad - slot0);
-    for (int r = 0; r < live; ++r) {
-      if (__ldg(sorted_ids + slot0 + r) < numel) continue;  // the same for every thread
+    // every warp looks at the slots at once (kPadSlots == 32) and then only at the pads among them
+    const int64_t slot = slot0 + (threadIdx.x & 31);
+    unsigned pads = __ballot_sync(0xffffffffu, slot < *num_post_pad && __ldg(sorted_ids + slot) >= numel);
+    for (; pads; pads &= pads - 1) {
+      const int r = __ffs(pads) - 1;
       for (int chunk = threadIdx.x; chunk < H / 16; chunk += blockDim.x) {
         *reinterpret_cast<uint4*>(q + (slot0 + r) * H + chunk * 16) = make_uint4(0, 0, 0, 0);
         if ((chunk & 7) == 0) s[(slot0 + r) * s_row + (chunk / 8) * s_group] = 0.f;
