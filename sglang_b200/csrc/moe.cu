@@ -437,8 +437,10 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   if (stream) {
     StreamParams sp = {};
     sp.expert_ids = expert_ids; sp.num_post_pad = npp; sp.sorted_ids = sorted; sp.numel = (int)numel;
-    // every reached expert has at most one partly filled block
-    const int64_t bound = (numel < E ? numel : E) + numel / L.block_m;
+    // Every bucket that has rows has at most one partly filled block. The separate align lays out the pairs of other ranks
+    // (id -1) as a bucket of its own, in front of the experts'; moe_prep_kernel leaves them out.
+    const int64_t buckets = one_launch ? E : E + 1;
+    const int64_t bound = (numel < buckets ? numel : buckets) + numel / L.block_m;
     sp.max_blocks = (int)(bound < L.cap_blocks ? bound : L.cap_blocks);
 #define B200_STREAM(NT)                                                                                                    \
   run_stream_gemms<NT, T>(aq1, as1, aq2, as2, w1, w2, w1_scale, w2_scale, topk_weights, weight_on_input, c3, E, H, I, \

@@ -192,6 +192,40 @@ def test_expert_parallel_minus_one_ids_sum_to_full_result():
     assert none.abs().max().item() == 0
 
 
+@pytest.mark.parametrize("block,T,E,topk", [(16, 263, 8, 4), (32, 262, 20, 4), (64, 275, 40, 6)])
+def test_streaming_experts_behind_a_run_of_remote_ids(block, T, E, topk):
+    """More than 1024 pairs, all but one pair per local expert on other ranks (-1): the run of remote ids has a partly
+    filled block of its own in front of the experts', so there are E + ceil(remote / block) blocks, more than
+    E + pairs // block. The scratch is filled with NaN bytes first: a row that no kernel wrote shows."""
+    from sglang_b200._native import tuning
+    from sglang_b200.fp8_kernel import _workspace
+
+    H, I, numel = 256, 128, T * topk
+    remote = numel - E
+    assert numel > 1024 and E + -(-remote // block) > E + numel // block
+    g = torch.Generator().manual_seed(700 + block)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    w1, w2, w1_s, w2_s = _weights(E, I, H, 70 + block)
+    tw = torch.rand(T, topk, generator=g) + 0.1
+    ti = torch.full((numel,), -1, dtype=torch.int32)
+    ti[torch.randperm(numel, generator=g)[:E]] = torch.arange(E, dtype=torch.int32)
+    ti = ti.view(T, topk)
+    ref = O.fused_experts_fp8(x, w1, w2, w1_s, w2_s, tw, ti, [128, 128])
+    scratch = _workspace(torch.device("cuda", torch.cuda.current_device()), 1 << 24)
+    with tuning(moe_decode=block):
+        scratch.fill_(255)
+        out = _run(x, w1, w2, w1_s, w2_s, tw, ti).float().cpu()
+        scratch.fill_(255)
+        nc = _run(x, w1, w2, w1_s, w2_s, tw, ti, no_combine=True).float().cpu()
+    for e in range(E):  # every expert's only pair
+        t, j = (ti == e).nonzero()[0].tolist()
+        assert O.rel_frobenius(out[t], ref[t]) < TOL, e
+        assert float(nc[t, j].abs().max()) > 0, e
+    assert O.rel_frobenius(out, ref) < TOL
+    assert O.rel_frobenius(nc.sum(1), ref) < TOL
+    assert float(nc[ti < 0].abs().max()) == 0
+
+
 def test_flags_inplace_no_combine_scaling_weight_on_input():
     import sglang_b200 as S
 
