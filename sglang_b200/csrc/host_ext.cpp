@@ -6,8 +6,14 @@
 // Every function here handles the regular case only and returns None for anything else (another layout, dtype or
 // device, a tensor subclass, an unsupported shape): the Python wrapper then takes its general path, which also
 // raises the errors. Nothing is kept from one call to the next except the scratch buffers below.
+//
+// The interpreter lock is given back while a function allocates and launches: a launch waits when the stream's queue is
+// full, for as long as the work ahead of it takes, and that work may include a host callback that needs the lock.
 #include <dlfcn.h>
 
+#include <atomic>
+#include <list>
+#include <mutex>
 #include <vector>
 
 #include <ATen/cuda/EmptyTensor.h>
@@ -49,43 +55,70 @@ PyObject* fail(int status, const char* what) {
   return PyErr_Format(type, "%s: %s: %s", what, abi.status_string(status), abi.last_error_detail());
 }
 
+// Other Python threads run while one of these is alive: no Python object is touched in its scope.
+struct WithoutInterpreterLock {
+  PyThreadState* state = PyEval_SaveThread();
+  WithoutInterpreterLock() = default;
+  WithoutInterpreterLock(const WithoutInterpreterLock&) = delete;
+  ~WithoutInterpreterLock() { PyEval_RestoreThread(state); }
+};
+
 // ------------------------------------------------------------------------------ scratch buffers
-// One grow-only scratch buffer per (device, stream); work on one stream is
-// ordered, so the next call may reuse it. A CUDA graph bakes the buffer's address into its nodes: once a call has
-// been seen under capture, a buffer that has to grow is kept alive instead of being given back to the allocator.
+// One grow-only scratch buffer per (device, stream); work on one stream is ordered, so the next call may reuse it.
+// Threads may share a stream: a call keeps the buffer's lock until its last kernel is launched, so that another call's
+// kernels cannot come between them. The lock is only ever waited for without the interpreter lock.
+// A CUDA graph bakes the buffer's address into its nodes: once a call has been seen under capture, a buffer that has to
+// grow is kept alive instead of being given back to the allocator.
 struct Scratch {
   int device;
   void* stream;
+  std::mutex busy;  // guards the members below
   Tensor buf;
+  std::vector<Tensor> retired;
 };
-// never destroyed: the process may end after the CUDA context. Callers hold the interpreter lock.
-std::vector<Scratch>& scratch = *new std::vector<Scratch>;
-std::vector<Tensor>& retired = *new std::vector<Tensor>;
-bool capture_seen = false;
+// never destroyed: the process may end after the CUDA context
+std::mutex& scratch_list_lock = *new std::mutex;
+std::list<Scratch>& scratch = *new std::list<Scratch>;
+std::atomic<bool> capture_seen{false};
 
 Tensor empty_on(int device, at::IntArrayRef size, at::ScalarType dtype) {
   return Tensor(at::detail::empty_cuda(size, dtype, c10::Device(c10::kCUDA, (c10::DeviceIndex)device), std::nullopt));
 }
 
 Scratch& scratch_of(int device, void* stream) {
+  std::lock_guard<std::mutex> guard(scratch_list_lock);
   for (auto& s : scratch)
     if (s.device == device && s.stream == stream) return s;
-  scratch.push_back(Scratch{device, stream, {}});
-  return scratch.back();
+  Scratch& s = scratch.emplace_back();  // a list: the references of other threads stay valid
+  s.device = device;
+  s.stream = stream;
+  return s;
 }
 
-Tensor workspace(int device, void* stream, size_t bytes) {
-  Scratch& s = scratch_of(device, stream);
+// At least `bytes` bytes; s.busy is held.
+void grow(Scratch& s, size_t bytes) {
   if (c10::cuda::currentStreamCaptureStatusMayInitCtx() != c10::cuda::CaptureStatus::None) capture_seen = true;
   const size_t have = s.buf.defined() ? (size_t)s.buf.numel() : 0;
-  if (have < bytes) {
-    if (have && capture_seen) retired.push_back(s.buf);
-    const size_t want = bytes > have + have / 2 ? bytes : have + have / 2;
-    s.buf = Tensor();  // back to the allocator first: the larger block may take its place
-    s.buf = empty_on(device, {(int64_t)want}, at::kByte);
-  }
-  return s.buf;
+  if (have >= bytes) return;
+  if (have && capture_seen) s.retired.push_back(s.buf);
+  const size_t want = bytes > have + have / 2 ? bytes : have + have / 2;
+  s.buf = Tensor();  // back to the allocator first: the larger block may take its place
+  s.buf = empty_on(s.device, {(int64_t)want}, at::kByte);
 }
+
+// A stream's scratch for the kernels of one call: nothing when no bytes are needed.
+struct Lease {
+  std::unique_lock<std::mutex> lock;
+  void* ptr = nullptr;
+  Lease() = default;
+  Lease(int device, void* stream, size_t bytes) {
+    if (bytes == 0) return;
+    Scratch& s = scratch_of(device, stream);
+    lock = std::unique_lock<std::mutex>(s.busy);
+    grow(s, bytes);
+    ptr = s.buf.data_ptr();
+  }
+};
 
 // ------------------------------------------------------------------------------------ arguments
 // A plain CUDA tensor on the current device, or null.
@@ -127,13 +160,20 @@ PyObject* linear(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (M == 0 || !is_2d(*ws, cdiv(N, 128), K / 128)) Py_RETURN_NONE;
   c10::SmallVector<int64_t, 4> shape(x->sizes().begin(), x->sizes().end());
   shape.back() = N;
-  Tensor out = empty_on(dev, shape, type);
-  void* st = stream_of(dev);
-  const size_t need = abi.linear_ws(M, N, K);
-  // a large scratch (long prefill) is worth a block of the caching allocator, which other work can use in between
-  const Tensor buf = need == 0 ? Tensor() : need <= kKeptScratch ? workspace(dev, st, need) : empty_on(dev, {(int64_t)need}, at::kByte);
-  const int rc = abi.linear(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K,
-                            need ? buf.data_ptr() : nullptr, need, st);
+  Tensor out;
+  int rc;
+  {
+    WithoutInterpreterLock unlocked;
+    out = empty_on(dev, shape, type);
+    void* st = stream_of(dev);
+    const size_t need = abi.linear_ws(M, N, K);
+    // a large scratch (long prefill) is worth a block of the caching allocator, which other work can use in between
+    const bool kept = need <= kKeptScratch;
+    const Lease lease = kept ? Lease(dev, st, need) : Lease();
+    const Tensor own = kept ? Tensor() : empty_on(dev, {(int64_t)need}, at::kByte);
+    rc = abi.linear(x->data_ptr(), code, w->data_ptr(), ws->data_ptr<float>(), out.data_ptr(), M, N, K,
+                    kept ? lease.ptr : own.data_ptr(), need, st);
+  }
   if (rc) return fail(rc, "w8a8_block_fp8_linear");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -172,18 +212,27 @@ PyObject* quant(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int64_t M = x->size(0), K = x->size(1);
   if (code < 0 || M == 0 || K == 0 || K % group || (ue8m0 && !(col && aligned))) Py_RETURN_NONE;
   const int64_t groups = K / group, padded = cdiv(M, 4) * 4;
-  Tensor q = empty_on(dev, {M, K}, kFp8);
-  void* st = stream_of(dev);
+  Tensor q, s;
+  int rc;
   if (ue8m0) {  // four exponent bytes per word, row index contiguous, rows padded to 4
-    Tensor s = empty_on(dev, {cdiv(groups, 4), padded}, at::kInt);
-    const int rc = abi.quant_ue8m0(x->data_ptr(), code, q.data_ptr(), s.data_ptr(), M, K, (int)group, padded, 0, nullptr, 1, st);
+    {
+      WithoutInterpreterLock unlocked;
+      q = empty_on(dev, {M, K}, kFp8);
+      s = empty_on(dev, {cdiv(groups, 4), padded}, at::kInt);
+      rc = abi.quant_ue8m0(x->data_ptr(), code, q.data_ptr(), s.data_ptr(), M, K, (int)group, padded, 0, nullptr, 1,
+                           stream_of(dev));
+    }
     if (rc) return fail(rc, "per_token_group_quant_fp8 (UE8M0)");
     return pair(std::move(q), row_contiguous(s, M, cdiv(groups, 4), padded));
   }
   const int64_t ld = aligned ? padded : M;
-  Tensor s = col ? empty_on(dev, {groups, ld}, at::kFloat) : empty_on(dev, {M, groups}, at::kFloat);
-  const int rc = abi.quant(x->data_ptr(), code, q.data_ptr(), s.data_ptr<float>(), M, K, (int)group, col ? 1 : groups,
-                           col ? ld : 1, (float)eps, (int)formula, st);
+  {
+    WithoutInterpreterLock unlocked;
+    q = empty_on(dev, {M, K}, kFp8);
+    s = col ? empty_on(dev, {groups, ld}, at::kFloat) : empty_on(dev, {M, groups}, at::kFloat);
+    rc = abi.quant(x->data_ptr(), code, q.data_ptr(), s.data_ptr<float>(), M, K, (int)group, col ? 1 : groups, col ? ld : 1,
+                   (float)eps, (int)formula, stream_of(dev));
+  }
   if (rc) return fail(rc, "per_token_group_quant_fp8");
   return pair(std::move(q), col ? row_contiguous(s, M, groups, ld) : s);
   END_HANDLE_TH_ERRORS
@@ -202,12 +251,17 @@ PyObject* matmul(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   if (M == 0 || N == 0 || K == 0 || B->size(1) != K || !is_2d(*As, M, cdiv(K, 128)) ||
       !is_2d(*Bs, cdiv(N, 128), cdiv(K, 128)) || code < B200_BF16 || code > B200_F32)
     Py_RETURN_NONE;
-  Tensor out = empty_on(dev, {M, N}, dtype_of_code(code));
-  void* st = stream_of(dev);
-  const size_t need = abi.gemm_ws(M, N, K);
-  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
-  const int rc = abi.gemm(A->data_ptr(), As->data_ptr<float>(), As->stride(0), As->stride(1), B->data_ptr(),
-                          Bs->data_ptr<float>(), out.data_ptr(), (int)code, M, N, K, need ? buf.data_ptr() : nullptr, need, st);
+  Tensor out;
+  int rc;
+  {
+    WithoutInterpreterLock unlocked;
+    out = empty_on(dev, {M, N}, dtype_of_code(code));
+    void* st = stream_of(dev);
+    const size_t need = abi.gemm_ws(M, N, K);
+    const Lease lease(dev, st, need);
+    rc = abi.gemm(A->data_ptr(), As->data_ptr<float>(), As->stride(0), As->stride(1), B->data_ptr(), Bs->data_ptr<float>(),
+                  out.data_ptr(), (int)code, M, N, K, lease.ptr, need, st);
+  }
   if (rc) return fail(rc, "w8a8_block_fp8_matmul");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -235,12 +289,17 @@ PyObject* matmul_ue8m0(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const int rows_per_word = mn_major(*Bs, N) ? 1 : mn_major(*Bs, cdiv(N, 128)) ? 128 : 0;
   if (!rows_per_word) Py_RETURN_NONE;
   auto pitch = [](const Tensor& s) { return s.size(1) > 1 ? s.stride(1) : s.size(0); };
-  Tensor out = empty_on(dev, {M, N}, dtype_of_code(code));
-  void* st = stream_of(dev);
-  const size_t need = abi.packed_ws(M, N, K);
-  const Tensor buf = need ? workspace(dev, st, need) : Tensor();
-  const int rc = abi.packed(A->data_ptr(), As->data_ptr<int>(), pitch(*As), B->data_ptr(), Bs->data_ptr<int>(), pitch(*Bs),
-                            rows_per_word, out.data_ptr(), (int)code, M, N, K, need ? buf.data_ptr() : nullptr, need, st);
+  Tensor out;
+  int rc;
+  {
+    WithoutInterpreterLock unlocked;
+    out = empty_on(dev, {M, N}, dtype_of_code(code));
+    void* st = stream_of(dev);
+    const size_t need = abi.packed_ws(M, N, K);
+    const Lease lease(dev, st, need);
+    rc = abi.packed(A->data_ptr(), As->data_ptr<int>(), pitch(*As), B->data_ptr(), Bs->data_ptr<int>(), pitch(*Bs),
+                    rows_per_word, out.data_ptr(), (int)code, M, N, K, lease.ptr, need, st);
+  }
   if (rc) return fail(rc, "w8a8_block_fp8_matmul (UE8M0)");
   return THPVariable_Wrap(std::move(out));
   END_HANDLE_TH_ERRORS
@@ -268,15 +327,19 @@ PyObject* experts(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     if ((code == B200_BF16 || code == B200_F16) && T > 0 && k > 0 && ti->size(0) == T && is_2d(*tw, T, k) &&
         w1->size(2) == H && is_3d(*w2, E, H, I) && is_3d(*s1, E, cdiv(2 * I, 128), cdiv(H, 128)) &&
         is_3d(*s2, E, cdiv(H, 128), cdiv(I, 128)) && !(inplace && no_combine) && (!on_input || k == 1)) {
-      Tensor out = inplace      ? *x
-                   : no_combine ? empty_on(dev, {T, k, H}, x->scalar_type())
-                                : empty_on(dev, {T, H}, x->scalar_type());
-      void* st = stream_of(dev);
-      const size_t need = abi.experts_ws(T, (int)k, (int)E, H, I);
-      const Tensor buf = workspace(dev, st, need);
-      const int rc = abi.experts(x->data_ptr(), nullptr, code, w1->data_ptr(), w2->data_ptr(), s1->data_ptr<float>(),
-                                 s2->data_ptr<float>(), tw->data_ptr<float>(), ti->data_ptr<int>(), out.data_ptr(), T, (int)k,
-                                 (int)E, H, I, no_combine, on_input, (float)scale, buf.data_ptr(), need, st);
+      Tensor out;
+      if (inplace) out = *x;
+      int rc;
+      {
+        WithoutInterpreterLock unlocked;
+        if (!inplace) out = no_combine ? empty_on(dev, {T, k, H}, x->scalar_type()) : empty_on(dev, {T, H}, x->scalar_type());
+        void* st = stream_of(dev);
+        const size_t need = abi.experts_ws(T, (int)k, (int)E, H, I);
+        const Lease lease(dev, st, need);
+        rc = abi.experts(x->data_ptr(), nullptr, code, w1->data_ptr(), w2->data_ptr(), s1->data_ptr<float>(),
+                         s2->data_ptr<float>(), tw->data_ptr<float>(), ti->data_ptr<int>(), out.data_ptr(), T, (int)k, (int)E, H,
+                         I, no_combine, on_input, (float)scale, lease.ptr, need, st);
+      }
       if (rc) return fail(rc, "fused_experts");
       return THPVariable_Wrap(std::move(out));
     }
@@ -303,10 +366,16 @@ PyObject* route(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
     Py_RETURN_NONE;
   }
   const int64_t T = x->size(0);
-  Tensor w = empty_on(dev, {T, v[0]}, at::kFloat), ids = empty_on(dev, {T, v[0]}, at::kInt);
-  const int rc = abi.route(x->data_ptr(), dtype_code(x->scalar_type()), bias ? bias->data_ptr<float>() : nullptr, T,
-                           (int)x->size(1), (int)v[0], (int)v[1], (int)v[2], (int)v[3], (int)v[4], renormalize, (float)scale,
-                           nullptr, w.data_ptr<float>(), ids.data_ptr<int>(), stream_of(dev));
+  Tensor w, ids;
+  int rc;
+  {
+    WithoutInterpreterLock unlocked;
+    w = empty_on(dev, {T, v[0]}, at::kFloat);
+    ids = empty_on(dev, {T, v[0]}, at::kInt);
+    rc = abi.route(x->data_ptr(), dtype_code(x->scalar_type()), bias ? bias->data_ptr<float>() : nullptr, T, (int)x->size(1),
+                   (int)v[0], (int)v[1], (int)v[2], (int)v[3], (int)v[4], renormalize, (float)scale, nullptr,
+                   w.data_ptr<float>(), ids.data_ptr<int>(), stream_of(dev));
+  }
   if (rc) return fail(rc, "route_topk");
   return pair(std::move(w), std::move(ids));
   END_HANDLE_TH_ERRORS
@@ -319,7 +388,15 @@ PyObject* scratch_tensor(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   const long dev = PyLong_AsLong(args[0]);
   const size_t bytes = PyLong_AsSize_t(args[1]);
   if (PyErr_Occurred()) return nullptr;
-  return THPVariable_Wrap(workspace((int)dev, stream_of((int)dev), bytes));
+  Tensor buf;
+  {
+    WithoutInterpreterLock unlocked;
+    Scratch& s = scratch_of((int)dev, stream_of((int)dev));
+    std::lock_guard<std::mutex> guard(s.busy);
+    grow(s, bytes);
+    buf = s.buf;
+  }
+  return THPVariable_Wrap(std::move(buf));
   END_HANDLE_TH_ERRORS
 }
 // bind(path of the C-ABI library)
