@@ -399,6 +399,35 @@ PyObject* scratch_tensor(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
   return THPVariable_Wrap(std::move(buf));
   END_HANDLE_TH_ERRORS
 }
+
+// acquire(device, bytes): the same, kept from every other call that uses this scratch until release(device)
+PyObject* acquire(PyObject*, PyObject* const* args, Py_ssize_t nargs) {
+  HANDLE_TH_ERRORS
+  if (nargs != 2) return PyErr_Format(PyExc_TypeError, "acquire(device, bytes)");
+  const long dev = PyLong_AsLong(args[0]);
+  const size_t bytes = PyLong_AsSize_t(args[1]);
+  if (PyErr_Occurred()) return nullptr;
+  Tensor buf;
+  {
+    WithoutInterpreterLock unlocked;
+    Scratch& s = scratch_of((int)dev, stream_of((int)dev));
+    std::unique_lock<std::mutex> lock(s.busy);
+    grow(s, bytes);
+    buf = s.buf;
+    lock.release();  // stays locked
+  }
+  return THPVariable_Wrap(std::move(buf));
+  END_HANDLE_TH_ERRORS
+}
+PyObject* release(PyObject*, PyObject* arg) {
+  HANDLE_TH_ERRORS
+  const long dev = PyLong_AsLong(arg);
+  if (PyErr_Occurred()) return nullptr;
+  scratch_of((int)dev, stream_of((int)dev)).busy.unlock();
+  Py_RETURN_NONE;
+  END_HANDLE_TH_ERRORS
+}
+
 // bind(path of the C-ABI library)
 PyObject* bind(PyObject*, PyObject* arg) {
   const char* path = PyUnicode_AsUTF8(arg);
@@ -434,6 +463,7 @@ PyMethodDef methods[] = {
     {"quant", FAST(quant), nullptr},          {"matmul", FAST(matmul), nullptr},
     {"matmul_ue8m0", FAST(matmul_ue8m0), nullptr}, {"experts", FAST(experts), nullptr},
     {"route", FAST(route), nullptr},          {"scratch", FAST(scratch_tensor), nullptr},
+    {"acquire", FAST(acquire), nullptr},      {"release", release, METH_O, nullptr},
     {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_host", "Native host path of the block-FP8 operators.", -1, methods,
                       nullptr, nullptr, nullptr, nullptr};

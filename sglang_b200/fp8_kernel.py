@@ -198,11 +198,33 @@ def _workspace(device, nbytes: int) -> Optional[torch.Tensor]:
     A CUDA graph bakes the buffer's address into its kernel nodes. Once any call has been made during a
     stream capture, a buffer that has to grow is therefore kept alive (never returned to the allocator)
     instead of being dropped, so replays of an earlier capture keep writing into memory nobody else owns.
-    ``reserve_workspace`` sizes the buffer up front."""
+    ``reserve_workspace`` sizes the buffer up front. Launches that use the buffer go inside ``scratch``."""
     if nbytes == 0:
         return None
     N.load()
     return N.host.scratch(device.index, nbytes)
+
+
+class scratch:
+    """``with scratch(device, nbytes) as ws:`` lends the stream's scratch buffer (``None`` for no bytes) to the launches
+    inside. Threads may share a stream: until the block ends, no other call launches kernels that use the buffer, so
+    nothing but launches belongs in it."""
+
+    __slots__ = ("device", "nbytes")
+
+    def __init__(self, device, nbytes: int):
+        self.device, self.nbytes = device.index, nbytes
+
+    def __enter__(self) -> Optional[torch.Tensor]:
+        if self.nbytes == 0:
+            return None
+        N.load()
+        return N.host.acquire(self.device, self.nbytes)
+
+    def __exit__(self, *a):
+        if self.nbytes:
+            N.host.release(self.device)
+        return False
 
 
 def reserve_workspace(max_bytes: int, device=None) -> None:
@@ -258,8 +280,7 @@ def w8a8_block_fp8_matmul(
     Bs = Bs.float().contiguous() if (Bs.dtype != torch.float32 or not Bs.is_contiguous()) else Bs
     lib = N.load()
     ws_bytes = lib.b200_w8a8_block_fp8_gemm_workspace_bytes(M, Nn, K)
-    with N.on_device(A):
-        ws = _workspace(A.device, ws_bytes)
+    with N.on_device(A), scratch(A.device, ws_bytes) as ws:
         st = lib.b200_w8a8_block_fp8_gemm(
             N.ptr(A), N.ptr(As2), As2.stride(0), As2.stride(1), N.ptr(B), N.ptr(Bs), N.ptr(C),
             N.DTYPE_CODE[output_dtype], M, Nn, K, N.ptr(ws), ws_bytes, N.current_stream(),
@@ -323,12 +344,11 @@ def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weig
     lib = N.load()
     out = torch.empty(M, Nn, dtype=x.dtype, device=x.device)
     with N.on_device(x):
-        stream = N.current_stream()
         ws_bytes = lib.b200_w8a8_block_fp8_linear_decode_workspace_bytes(M, Nn, K)
-        ws = _workspace(x.device, ws_bytes)
-        st = lib.b200_w8a8_block_fp8_linear_decode(
-            N.ptr(x), N.DTYPE_CODE[x.dtype], N.ptr(weight), N.ptr(weight_scale), N.ptr(out), M, Nn, K, 1e-10,
-            N.ptr(ws), ws_bytes, N.ptr(weight_scale), stream,  # the ticket array is no longer used: any non-null pointer
-        )
+        with scratch(x.device, ws_bytes) as ws:
+            st = lib.b200_w8a8_block_fp8_linear_decode(
+                N.ptr(x), N.DTYPE_CODE[x.dtype], N.ptr(weight), N.ptr(weight_scale), N.ptr(out), M, Nn, K, 1e-10, N.ptr(ws),
+                ws_bytes, N.ptr(weight_scale), N.current_stream(),  # the ticket array is no longer used: any non-null pointer
+            )
     N.check(st, "w8a8_block_fp8_linear (decode)")
     return out

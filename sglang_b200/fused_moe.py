@@ -13,7 +13,7 @@ from typing import List, NamedTuple, Optional
 import torch
 
 from . import _native as N
-from .fp8_kernel import _workspace, fp8_dtype
+from .fp8_kernel import fp8_dtype, scratch
 
 
 class StandardTopKOutput(NamedTuple):
@@ -126,8 +126,7 @@ def fused_experts_impl(
         return out
     lib = N.load()
     ws_bytes = lib.b200_fused_experts_fp8_workspace_bytes(T, topk, E, H, I)
-    with N.on_device(hidden_states):
-        ws = _workspace(hidden_states.device, ws_bytes)
+    with N.on_device(hidden_states), scratch(hidden_states.device, ws_bytes) as ws:
         st = lib.b200_fused_experts_fp8(
             N.ptr(hidden_states), N.ptr(hidden_states_scale), N.DTYPE_CODE[out_dtype], N.ptr(w1), N.ptr(w2), N.ptr(w1_scale),
             N.ptr(w2_scale), N.ptr(topk_weights), N.ptr(topk_ids), N.ptr(out), T, topk, E, H, I,
@@ -168,8 +167,7 @@ def fused_experts_scatter(
         return
     lib = N.load()
     ws_bytes = lib.b200_fused_experts_fp8_workspace_bytes(T, topk, E, H, I)
-    with N.on_device(rows_q):
-        ws = _workspace(rows_q.device, ws_bytes)
+    with N.on_device(rows_q), scratch(rows_q.device, ws_bytes) as ws:
         st = lib.b200_fused_experts_fp8_scatter(
             N.ptr(rows_q), N.ptr(rows_scale), N.DTYPE_CODE[output_dtype], N.ptr(w1), N.ptr(w2), N.ptr(w1_scale),
             N.ptr(w2_scale), N.ptr(topk_weights), N.ptr(topk_ids), dest_ptrs, len(dest_ptrs), rows_per_dest, T, topk, E, H, I,
@@ -282,8 +280,7 @@ def masked_fused_experts(
     out = torch.empty((E, T_pad, H), dtype=output_dtype, device=hidden_states.device)
     lib = N.load()
     ws_bytes = lib.b200_masked_experts_fp8_workspace_bytes(E, T_pad, H, I)
-    with N.on_device(hidden_states):
-        ws = _workspace(hidden_states.device, ws_bytes)
+    with N.on_device(hidden_states), scratch(hidden_states.device, ws_bytes) as ws:
         st = lib.b200_masked_experts_fp8(
             N.ptr(hidden_states), N.ptr(hs), N.ptr(w13_weight), N.ptr(w2_weight), N.ptr(w13_scale), N.ptr(w2_scale),
             N.ptr(mm), N.ptr(out), N.DTYPE_CODE[output_dtype], E, T_pad, H, I, N.ptr(ws), ws_bytes, N.current_stream(),

@@ -10,7 +10,7 @@ from typing import Tuple
 import torch
 
 from . import _native as N
-from .fp8_kernel import _workspace
+from .fp8_kernel import scratch
 
 
 def cdiv(a: int, b: int) -> int:
@@ -40,8 +40,7 @@ def sgl_moe_align_block_size(
     lib = N.load()
     numel = topk_ids.numel()
     ws_bytes = lib.b200_moe_align_workspace_bytes(numel, num_experts)
-    with N.on_device(topk_ids):
-        ws = _workspace(topk_ids.device, ws_bytes)
+    with N.on_device(topk_ids), scratch(topk_ids.device, ws_bytes) as ws:
         st = lib.b200_moe_align_block_size(
             N.ptr(topk_ids), N.DTYPE_CODE[topk_ids.dtype], numel, num_experts, block_size,
             N.ptr(sorted_token_ids), sorted_token_ids.numel(), N.ptr(experts_ids), experts_ids.numel(),

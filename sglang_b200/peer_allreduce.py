@@ -31,7 +31,7 @@ import torch
 import torch.distributed as dist
 
 from . import _native as N
-from .fp8_kernel import _workspace, fp8_dtype, per_token_group_quant_fp8
+from .fp8_kernel import fp8_dtype, per_token_group_quant_fp8, scratch
 
 MAX_RANKS = 8
 
@@ -136,11 +136,11 @@ class PeerAllReduce:
             return out, res_out
         with N.on_device(x_q):
             stream = N.current_stream()
-            ws = _workspace(x_q.device, ws_bytes)
-            st = lib.b200_w8a8_block_fp8_gemm_fanout(
-                N.ptr(x_q), N.ptr(xs), xs.stride(0), xs.stride(1), N.ptr(weight), N.ptr(wsc), dests, self.world,
-                int(self.two_shot), code, m, n, k, N.ptr(ws), ws_bytes, stream,
-            )
+            with scratch(x_q.device, ws_bytes) as ws:
+                st = lib.b200_w8a8_block_fp8_gemm_fanout(
+                    N.ptr(x_q), N.ptr(xs), xs.stride(0), xs.stride(1), N.ptr(weight), N.ptr(wsc), dests, self.world,
+                    int(self.two_shot), code, m, n, k, N.ptr(ws), ws_bytes, stream,
+                )
             N.check(st, "w8a8_block_fp8_gemm_fanout")
             st = lib.b200_allreduce_finish(
                 self._slot_ptr(self.rank, parity, 0), self.slot_elems, outs, code, m, n, self.world, self.rank, int(self.two_shot),
