@@ -6,6 +6,10 @@
  *    library borrows it for the duration of the call, allocates nothing, never
  *    synchronises and never creates a stream. Work is enqueued on `stream` (a
  *    cudaStream_t passed as void*).
+ *  - Stream order holds for every operand, weights included: kernels may start before the
+ *    work ahead of them in the stream has finished, but until then they read nothing (they
+ *    prefetch weights into L2). A kernel, copy or event wait that precedes a call may write
+ *    any of its operands.
  *  - Every entry point returns 0 on success or a negative B200_E_* code; nothing throws.
  *    b200_status_string() turns a code into text, b200_last_error_detail() gives the
  *    detail of the most recent failure on the calling thread.
@@ -170,9 +174,7 @@ int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B,
  * replaces: python/sglang/srt/layers/quantization/fp8_utils.py:814-834 (the same composition)
  * out = the result of b200_per_token_group_quant_fp8 (group 128) followed by b200_w8a8_block_fp8_gemm,
  * with the kernels chained as programmatic dependents (a few rows: the one-launch kernel above).
- * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out as above. The weights B may
- * be fetched before earlier kernels of the stream have finished if those signal their dependents early
- * (kernels of this library do; its quantisers called on their own do not).
+ * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out as above.
  * workspace: b200_w8a8_block_fp8_linear_workspace_bytes(M,N,K) bytes, 256-byte aligned. */
 size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out,

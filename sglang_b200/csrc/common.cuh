@@ -104,8 +104,7 @@ __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepco
 __device__ __forceinline__ void grid_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 // Quantiser of a linear layer (quant.cu): 16-bit x [M, K] -> FP8 rows + column-major scales, launched so that it overlaps
-// the kernels on either side. Only for scratch operands: the GEMM that follows may fetch its WEIGHTS before this grid's
-// predecessors have finished, so those must not have been written by a kernel that triggers its dependents early.
+// the kernels on either side.
 int quant_for_linear(const void* x, int x_dtype, void* q, float* s, int64_t M, int64_t K, cudaStream_t st);
 
 // moe_align_block_size of int32 ids (align.cu) that also writes every id's position in the sorted layout, -1 for ids that
@@ -143,6 +142,17 @@ __device__ __forceinline__ uint4 ld_nc_16(const void* p) {
                : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
                : "l"(p));
   return v;
+}
+
+// The first n 128-byte K blocks of a weight row into L2. Nothing is read, so a kernel launched as a programmatic dependent
+// may ask for its weights while an earlier kernel still writes them: the write goes to the same L2 line.
+// Depth, in K blocks per CTA of the dense kernels: beyond what fits the gap before the wait ends, the requests hold up the
+// loads behind them. Four projections of 6144..28672 x 4096..14336, 1 / 16 rows: 3 blocks 52.7 / 55.6 us, 4 53.0 / 55.7,
+// 5 53.5 / 56.0, 10 55.3 / 57.7, none 58.5 / 58.7; the same boxes by cp.async.bulk.prefetch.tensor, which queue in front of
+// the loads, 5 blocks 59.5 / 59.7; loads into the ring before the wait, which nothing orders behind a writer, 53.2 / 56.6.
+constexpr int kPrefetchKb = 3;
+__device__ __forceinline__ void prefetch_weight_row(const uint8_t* row, int n) {
+  for (int i = 0; i < n; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + i * 128) : "memory");
 }
 
 // Four consecutive floats from shared memory, read at this point of the program (never cached in

@@ -26,6 +26,7 @@ struct SkinnyParams {
   void* C;          // OutT [M, N], or fp32 partials [splits][M, N]
   int M, N, K, num_kb;
   int n_tiles, t_tiles, k_splits, kb_per_split;
+  const uint8_t* w;  // the weights [N, K]
   int cluster;  // the K splits of an item are one cluster
   int* status;
 };
@@ -109,15 +110,15 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   if (p.cluster) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
   // every CTA of this grid is running: a dependent grid (the split-K reduction) may be set up now;
   // it waits for this grid's completion before it reads anything
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  // The producer and the MMA issuer start at once; meanwhile the promotion warps stage
-  // As[m, kb] * Bs[n0/128, kb] for this item's tokens and K blocks in shared memory (their own
-  // 128-thread barrier: only they read the table), so the first weight tiles are already in
-  // flight while the scales are fetched.
+  grid_launch_dependents();
+  // This grid is launched as a programmatic dependent: every operand, and at the end the output buffer, belongs to the
+  // kernels before it in the stream, which may still run. The weight stream starts all the same, as a prefetch into L2
+  // by the promotion warps, who have nothing else to do (a row each); after the wait they stage As[m, kb] * Bs[n0/128, kb]
+  // for this item's tokens and K blocks in shared memory (their own 128-thread barrier: only they read the table).
   if (warp < 4) {
-    // the activation scales (and, at the end, the output buffer) belong to the kernels before this
-    // one in the stream: this grid is launched as their programmatic dependent, so wait for them here
-    asm volatile("griddepcontrol.wait;" ::: "memory");
+    if (n0 + (int)threadIdx.x < p.N)
+      prefetch_weight_row(p.w + (int64_t)(n0 + threadIdx.x) * p.K + kb0 * kBK, min(kPrefetchKb, kb1 - kb0));
+    grid_dependency_wait();
     const float* bs_row = p.Bs + (int64_t)nt * p.num_kb;
     for (int i = threadIdx.x; i < (kb1 - kb0) * NT; i += 128) {
       const int kb = kb0 + i / NT, t = i % NT;
@@ -142,18 +143,9 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   if (warp == kProducerWarp) {
     if (ptx::elect_one()) {
       bool ok = true;
-      // Prologue: the weights do not depend on the previous kernel, the quantised activations do.
-      // The weight tiles of the first stages are requested before waiting for that kernel, so the
-      // weight stream starts while it is still finishing.
-      const int npro = min(S, kb1 - kb0);
-      for (int i = 0; i < npro; ++i) {
-        ptx::mbar_expect_tx(full_bar(i), Cfg::kStageW + Cfg::kStageX);
-        ptx::tma_load_2d(sW + i * Cfg::kStageW, &tmap_w, (kb0 + i) * kBK, n0, full_bar(i));
-      }
-      asm volatile("griddepcontrol.wait;" ::: "memory");
-      for (int i = 0; i < npro; ++i) ptx::tma_load_2d(sX + i * Cfg::kStageX, &tmap_x, (kb0 + i) * kBK, m0, full_bar(i));
-      uint32_t it = npro;
-      for (int kb = kb0 + npro; kb < kb1 && ok; ++kb, ++it) {
+      grid_dependency_wait();
+      uint32_t it = 0;
+      for (int kb = kb0; kb < kb1 && ok; ++kb, ++it) {
         const int s = it % S;
         ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
         if (!ok) break;
@@ -312,7 +304,7 @@ inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, cons
   const size_t smem = SkinnyCfg<NT>::kSmemBytes;
   if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   // programmatic dependent of the kernel before it (normally the activation quantiser, which
-  // signals launch_dependents at once): set-up and the first weight loads overlap its tail
+  // signals launch_dependents at once): set-up and the first weight prefetches overlap its tail
   return launch_dependent(k, dim3((unsigned)(p.n_tiles * p.t_tiles * p.k_splits)), SkinnyCfg<NT>::kThreads, smem, st,
                           p.cluster ? p.k_splits : 1, "block_fp8_gemm_skinny_kernel", tw, tx, p);
 }
@@ -327,6 +319,7 @@ inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int split
   p.k_splits = splits;
   p.kb_per_split = (int)cdiv(p.num_kb, splits);
   p.cluster = cluster;
+  p.w = static_cast<const uint8_t*>(W);
   p.status = device_status_word();
   if (!p.status) {
     set_error_detail("cannot resolve the device status word");

@@ -32,7 +32,8 @@ struct StreamParams {
   const int32_t* num_post_pad;  // [1] live rows (a multiple of NT)
   const int32_t* sorted_ids;    // [rows] flat (token * topk + slot), >= numel = pad
   const float* topk_weights;    // router weight per flat index, or null
-  int numel, max_blocks;
+  int numel, max_blocks, experts;
+  const uint8_t* w;  // the stacked weights, rows of num_kb * 128 bytes
   void* C;  // down: OutT [numel][n_out]
   uint8_t* q_out;   // gate_up: FP8 [rows][n_out] and its scales q_scales[(n / 128) * q_ld + row]
   float* q_scales;
@@ -156,19 +157,6 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
-  // Everything read below, and what the epilogue overwrites, belongs to the kernels before. The down GEMM's schedule
-  // was written two kernels ago (gate_up has waited for it before it let this grid start), so its producer can fetch
-  // the first weight tiles while gate_up still runs; only the activations have to be waited for.
-  if (STAGE == STREAM_GATE_UP) {
-    grid_dependency_wait();
-    grid_launch_dependents();
-  } else {
-    grid_launch_dependents();
-    if (warp != kProducerWarp) grid_dependency_wait();
-  }
-
-  const int blocks = min(p.max_blocks, *p.num_post_pad / NT);
-  const int total = blocks * p.n_tiles;
   const int item0 = csize == 1 ? blockIdx.x : blockIdx.x / csize;
   const int step = csize == 1 ? gridDim.x : gridDim.x / csize;
   const int kb0 = (int)rank * p.kb_per_rank, kb1 = min(p.num_kb, kb0 + p.kb_per_rank);
@@ -182,6 +170,28 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     return STAGE == STREAM_GATE_UP ? e * 2 * row_blocks + h * row_blocks + nt
                                    : e * row_blocks + min(nt * 2 + h, row_blocks - 1);
   };
+
+  // Everything read below, and what the epilogue overwrites, belongs to the kernels before. The down GEMM's schedule was
+  // written two kernels ago (gate_up lets this grid start after its own wait for it): while gate_up still runs, the
+  // promotion warps ask for the first weight tiles, a row each. That is a prefetch into L2 and the id that picks the rows is
+  // only a hint: nothing read before the wait is used after it.
+  if (STAGE == STREAM_GATE_UP) {
+    grid_dependency_wait();
+    grid_launch_dependents();
+  } else {
+    grid_launch_dependents();
+    if (warp < 8) {
+      const int blk = item0 / p.n_tiles, nt = item0 - blk * p.n_tiles;
+      int live, e;
+      asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(live) : "l"(p.num_post_pad) : "memory");
+      asm volatile("ld.relaxed.gpu.global.s32 %0, [%1];" : "=r"(e) : "l"(p.expert_ids + blk) : "memory");
+      if (blk * NT < live && e >= 0 && e < p.experts && nt * 256 + (int)threadIdx.x < p.n_out)
+        prefetch_weight_row(p.w + ((int64_t)weight_row(e, nt, 0) + threadIdx.x) * p.num_kb * kBK + kb0 * kBK, min(S, nkb));
+    }
+    grid_dependency_wait();
+  }
+  const int blocks = min(p.max_blocks, *p.num_post_pad / NT);
+  const int total = blocks * p.n_tiles;
 
   float acc[NT];
   bool sum_ok = false;
@@ -239,28 +249,13 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
     if (ptx::elect_one()) {
       int s = 0;
       uint32_t phase = 1;
-      bool ok = true, waited = STAGE == STREAM_GATE_UP;
+      bool ok = true;
       for (int item = item0; item < total && ok; item += step) {
         const int blk = item / p.n_tiles, nt = item - blk * p.n_tiles;
         const int e = p.expert_ids[blk];
         if (e < 0) continue;
         const int ra = weight_row(e, nt, 0), rb = weight_row(e, nt, 1);
-        int kb = kb0;
-        if (!waited) {  // first item: the ring is empty, fill it with weights, then wait, then the token tiles
-          const int n = min(S, nkb);
-          for (int i = 0; i < n; ++i) {
-            ptx::mbar_expect_tx(full_bar(i), Cfg::kStage);
-            ptx::tma_load_2d(sW + i * Cfg::kStageW, &tmap_w, (kb0 + i) * kBK, ra, full_bar(i));
-            ptx::tma_load_2d(sW + i * Cfg::kStageW + 128 * kBK, &tmap_w, (kb0 + i) * kBK, rb, full_bar(i));
-          }
-          grid_dependency_wait();
-          waited = true;
-          for (int i = 0; i < n; ++i) ptx::tma_load_2d(sX + i * Cfg::kStageX, &tmap_x, (kb0 + i) * kBK, blk * NT, full_bar(i));
-          kb = kb0 + n;
-          s = n % S;
-          if (n == S) phase ^= 1;
-        }
-        for (; kb < kb1; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
           if (!ok) break;
           ptx::mbar_expect_tx(full_bar(s), Cfg::kStage);
@@ -455,6 +450,7 @@ inline int launch_stream(const void* W, int64_t w_rows, const void* X, int64_t x
     set_error_detail("cannot resolve the device status word");
     return B200_E_LAUNCH;
   }
+  p.w = static_cast<const uint8_t*>(W);
   CUtensorMap tw, tx;
   int rc = make_tmap_u8(&tw, W, (uint64_t)w_rows, (uint64_t)K, 128, "W");
   if (rc) return rc;

@@ -3,8 +3,8 @@
 // Operands are swapped as in gemm_stream.cuh: a CTA owns 256 weight rows (two UMMA tiles of 128), NT = 16 / 32 / 64 tokens
 // are the UMMA N dimension. K is split over a thread-block cluster of up to 8 CTAs so that about every SM streams
 // weights, and the partial sums are exchanged through distributed shared memory: no fp32 partials in memory and no
-// reduction launch. The first weight tiles are requested before the kernels ahead in the
-// stream have finished.
+// reduction launch. The first weight tiles are on their way into L2 before the kernels
+// ahead in the stream have finished.
 //   QUANT = true: X is the 16-bit input of a linear layer of a few rows (NT = 16); every CTA quantises its K range once,
 //       up front (same bytes and scales as the stand-alone quantiser), and keeps it in shared memory for all of its
 //       weight tiles: quantiser, GEMM and sum in ONE launch.
@@ -26,6 +26,7 @@ struct LinearStreamParams {
   void* out;        // OutT [M, N]
   int M, N, K, num_kb, kb_per_rank;
   int n_tiles, t_tiles, stages;
+  const uint8_t* w;  // the weights [N, K]
   int own_sums;  // a cluster's sums have a place outside the ring
   float eps;
   int* status;
@@ -130,29 +131,16 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     if (ptx::elect_one()) {
       int s = 0;
       uint32_t phase = 1;
-      bool ok = true, waited = QUANT;
+      bool ok = true;
+      grid_dependency_wait();
       for (int item = item0; item < items && ok; item += step) {
         const int nt = item / p.t_tiles, m0 = (item - nt * p.t_tiles) * NT;
-        auto load_w = [&](int st, int kb) {
-          ptx::mbar_expect_tx(full_bar(st), Cfg::kStage);
-          ptx::tma_load_2d(sW + st * Cfg::kStageW, &tmap_w, kb * kBK, nt * 256, full_bar(st));
-          ptx::tma_load_2d(sW + st * Cfg::kStageW + 128 * kBK, &tmap_w, kb * kBK, nt * 256 + 128, full_bar(st));
-        };
-        int kb = kb0;
-        if (!waited) {  // fill the empty ring with weights, then wait for the kernels ahead, then the token tiles
-          const int n = min(S, nkb);
-          for (int i = 0; i < n; ++i) load_w(i, kb0 + i);
-          grid_dependency_wait();
-          waited = true;
-          for (int i = 0; i < n; ++i) ptx::tma_load_2d(sX + i * Cfg::kStageX, &tmap_x, (kb0 + i) * kBK, m0, full_bar(i));
-          kb = kb0 + n;
-          s = n % S;
-          if (n == S) phase ^= 1;
-        }
-        for (; kb < kb1; ++kb) {
+        for (int kb = kb0; kb < kb1; ++kb) {
           ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
           if (!ok) break;
-          load_w(s, kb);
+          ptx::mbar_expect_tx(full_bar(s), Cfg::kStage);
+          ptx::tma_load_2d(sW + s * Cfg::kStageW, &tmap_w, kb * kBK, nt * 256, full_bar(s));
+          ptx::tma_load_2d(sW + s * Cfg::kStageW + 128 * kBK, &tmap_w, kb * kBK, nt * 256 + 128, full_bar(s));
           if (!QUANT) ptx::tma_load_2d(sX + s * Cfg::kStageX, &tmap_x, kb * kBK, m0, full_bar(s));
           if (++s == S) s = 0, phase ^= 1;
         }
@@ -188,7 +176,11 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     }
     __syncwarp();
   } else {
-    grid_dependency_wait();  // x and the output buffer belong to the kernels before this one
+    // Every operand and the output buffer belong to the kernels before this one, which may still run. The weight stream
+    // starts all the same, as a prefetch into L2, a row for each thread.
+    const int n_first = item0 / p.t_tiles * 256 + threadIdx.x;
+    if (n_first < p.N) prefetch_weight_row(p.w + (int64_t)n_first * p.K + kb0 * kBK, min(kPrefetchKb, nkb));
+    grid_dependency_wait();
     if constexpr (QUANT) {
       // 8 lanes share the 128-group of one row, 32 groups in flight per round: (K block, row) = group index
       const int chunk = threadIdx.x & 7;
@@ -400,6 +392,7 @@ inline int launch_linear_stream(const void* W, const void* X, LinearStreamParams
     set_error_detail("cannot resolve the device status word");
     return B200_E_LAUNCH;
   }
+  p.w = static_cast<const uint8_t*>(W);
   CUtensorMap tw, tx;
   int rc = make_tmap_u8(&tw, W, (uint64_t)p.N, (uint64_t)p.K, 128, "W");
   if (rc) return rc;

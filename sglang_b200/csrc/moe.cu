@@ -436,7 +436,7 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   }
   if (stream) {
     StreamParams sp = {};
-    sp.expert_ids = expert_ids; sp.num_post_pad = npp; sp.sorted_ids = sorted; sp.numel = (int)numel;
+    sp.expert_ids = expert_ids; sp.num_post_pad = npp; sp.sorted_ids = sorted; sp.numel = (int)numel; sp.experts = E;
     // Every bucket that has rows has at most one partly filled block. The separate align lays out the pairs of other ranks
     // (id -1) as a bucket of its own, in front of the experts'; moe_prep_kernel leaves them out.
     const int64_t buckets = one_launch ? E : E + 1;
