@@ -161,7 +161,8 @@ int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa, int64_t s
  * x [M,K] bf16/f16 row-major (M <= 16), B [N,K] e4m3, Bs fp32 [ceil(N/128), ceil(K/128)],
  * out [M,N] in the dtype of x. K % 16 == 0, K <= 65536, N % 8 == 0, N <= 524288.
  * workspace: b200_w8a8_block_fp8_linear_decode_workspace_bytes(M,N,K) bytes (none at present: the K split
- * is summed on chip). tickets: 4096 zeroed uint32 of one stream, not NULL (left as they are at present).
+ * is summed on chip). tickets: 4096 zeroed uint32 of one stream, not NULL: the library may count in them and
+ * leaves them zero (at present it does not touch them).
  * Anything else: B200_E_UNSUPPORTED (callers fall back to the two-step path). */
 size_t b200_w8a8_block_fp8_linear_decode_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B, const float* Bs,

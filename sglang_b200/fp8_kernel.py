@@ -320,17 +320,12 @@ def w8a8_block_fp8_linear(
     return output.to(dtype=input_2d.dtype).view(*output_shape)
 
 
-# Rows up to which every call takes the one-launch kernel: none, the native path weighs it against quantiser + GEMM by
-# size. (It takes up to 16 rows, and for up to 4 any K that is a multiple of 16.)
-DECODE_FUSED_MAX_M = 0
-
-
-def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weight_scale: torch.Tensor,
-                         max_rows: int = DECODE_FUSED_MAX_M):
-    """A few rows (the kernel takes up to 16, the wrapper sends it up to ``max_rows``) of 16-bit
-    activations: quantiser, GEMM and split-K sum as ONE launch (every CTA
-    quantises the slice of ``x`` it needs; same bytes and scales as ``per_token_group_quant_fp8``). Returns
-    None when the shapes or dtypes are outside that kernel, and the caller takes the two-step path."""
+def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weight_scale: torch.Tensor, max_rows: int):
+    """Up to ``max_rows`` (at most 16) rows of 16-bit activations: quantiser, GEMM and split-K sum as ONE launch (every
+    CTA quantises the slice of ``x`` it needs; same bytes and scales as ``per_token_group_quant_fp8``). Returns
+    None when the shapes or dtypes are outside that kernel, and the caller takes the two-step path. The native path
+    weighs this kernel against quantiser + GEMM by size and takes it itself where K is a multiple of 128; here it
+    serves the few-row calls with any other K."""
     M, K = x.shape
     if not (0 < M <= max_rows and x.is_cuda and x.dtype in (torch.bfloat16, torch.float16)
             and list(block_size) == [128, 128] and weight.dtype == fp8_dtype and weight.dim() == 2
@@ -345,10 +340,11 @@ def _linear_decode_fused(x: torch.Tensor, weight: torch.Tensor, block_size, weig
     out = torch.empty(M, Nn, dtype=x.dtype, device=x.device)
     with N.on_device(x):
         ws_bytes = lib.b200_w8a8_block_fp8_linear_decode_workspace_bytes(M, Nn, K)
+        tickets = torch.zeros(4096, dtype=torch.int32, device=x.device)
         with scratch(x.device, ws_bytes) as ws:
             st = lib.b200_w8a8_block_fp8_linear_decode(
                 N.ptr(x), N.DTYPE_CODE[x.dtype], N.ptr(weight), N.ptr(weight_scale), N.ptr(out), M, Nn, K, 1e-10, N.ptr(ws),
-                ws_bytes, N.ptr(weight_scale), N.current_stream(),  # the ticket array is no longer used: any non-null pointer
+                ws_bytes, N.ptr(tickets), N.current_stream(),
             )
     N.check(st, "w8a8_block_fp8_linear (decode)")
     return out

@@ -201,20 +201,18 @@ def test_llama70b_shard_shapes(name, N, K, kind, tp, M):
 def test_one_launch_decode_linear(M, N, K, dtype):
     """At most 16 rows: quantiser + GEMM + split-K sum run as one kernel. Against the oracle, against the
     two-step path (same quantised bytes and scales, so only the fp32 summation order differs), and called
-    twice in a row (the split-K tickets must be left ready for the next call)."""
+    twice in a row (nothing is left behind for the next call)."""
     import sglang_b200 as S
+    from sglang_b200 import _native, fp8_kernel
     from sglang_b200._native import tuning
-
-    from sglang_b200 import fp8_kernel
 
     x = make_activation(M, K, 2300 + M + K, dtype=dtype)
     wq, ws = make_weight(N, K, 2301 + N)
     ref = O.w8a8_block_fp8_linear(x, wq, ws, output_dtype=torch.float32)
     xd, wd, sd = x.cuda(), wq.cuda(), ws.cuda()
-    # the kernel itself takes up to 16 rows; the public wrapper routes fewer rows to it by default
     out = fp8_kernel._linear_decode_fused(xd, wd, [128, 128], sd, max_rows=16)
     out2 = fp8_kernel._linear_decode_fused(xd, wd, [128, 128], sd, max_rows=16)
-    if M <= fp8_kernel.DECODE_FUSED_MAX_M:
+    if _native.load().b200_w8a8_block_fp8_linear_workspace_bytes(M, N, K) == 0:  # sizes the public call sends there
         assert torch.equal(S.w8a8_block_fp8_linear(xd, wd, [128, 128], sd), out)
     with tuning(linear_decode_fused=0):
         two_step = S.w8a8_block_fp8_linear(xd, wd, [128, 128], sd)
@@ -223,6 +221,21 @@ def test_one_launch_decode_linear(M, N, K, dtype):
     assert torch.equal(out, out2)
     assert O.rel_frobenius(out.float().cpu(), ref) < TOL
     assert float((out.float() - two_step.float()).norm() / two_step.float().norm()) < 2e-3
+
+
+def test_one_launch_decode_linear_lends_no_operand_as_tickets(monkeypatch):
+    """The ticket array is memory that the library may write: 4096 words of its own, not one of the operands."""
+    from sglang_b200 import _native, fp8_kernel
+
+    lib, seen = _native.load(), []
+    real = lib.b200_w8a8_block_fp8_linear_decode
+    monkeypatch.setattr(lib, "b200_w8a8_block_fp8_linear_decode", lambda *a: seen.append(a) or real(*a))
+    x, (wq, ws) = make_activation(3, 400, 1).cuda(), make_weight(264, 400, 2)
+    wq, ws = wq.cuda(), ws.cuda()
+    out = fp8_kernel._linear_decode_fused(x, wq, [128, 128], ws, max_rows=4)
+    (tickets,) = [a[11] for a in seen]
+    for t in (x, wq, ws, out):
+        assert tickets + 4096 * 4 <= t.data_ptr() or tickets >= t.data_ptr() + t.numel() * t.element_size()
 
 
 def test_one_launch_decode_linear_declines_other_shapes():
