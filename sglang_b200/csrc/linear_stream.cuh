@@ -347,9 +347,11 @@ inline bool plan_linear_stream(int64_t M, int64_t N, int64_t K, int sms, int& cs
   // as many ranks per item as bring items x ranks up to the SM count, two K blocks each at least; where a rank could not
   // hold its K range, or the ring not the other ranks' sums, the nearest cluster size that fits
   int64_t want = sms / items;
-  // Clusters of up to 8 where they leave a quarter of the chip free; up to 4 otherwise, which fit its SM groups (16 tiles,
-  // 1 x 4096 x 14336: 19.7 us with clusters of 8, 13.9 with 4; 3 tiles, 1 x 768 x 4096: 5.6 and 6.6)
-  if (want > 4) want = items * 8 * 4 <= (int64_t)sms * 3 + 12 ? 8 : 4;
+  // Clusters of up to 8 as long as they all run at once, at one CTA per SM: the SM groups of this part hold 15 of them
+  // (cudaOccupancyMaxActiveClusters), which depends on the SMs that a part has, so one is left spare. Clusters of 4 (33 fit)
+  // beyond. With weights from HBM, 8 against 4: 13 tiles, 1 x 3328 x 4096 6.1 and 7.3 us, 61 x 3328 x 14336 18.7 and 22.5;
+  // 14 tiles 6.2 and 7.3, 19.1 and 22.8; 15 tiles 6.4 and 7.4, 19.9 and 22.6; 16 tiles 7.7 and 7.7, 32.3 and 22.5.
+  if (want > 4) want = items <= 14 ? 8 : 4;
   if (want > num_kb / 2) want = num_kb / 2;
   if (want < 1) want = 1;
   for (int i = 0; i < 16; ++i) {
