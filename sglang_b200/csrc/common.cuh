@@ -261,4 +261,19 @@ __device__ __forceinline__ float group_max(float v) {
   return v;
 }
 
+// 16 consecutive 16-bit elements of a 128-group that 8 consecutive lanes share: bytes and scale as the stand-alone
+// quantiser gives them. All 8 lanes call.
+template <typename T>
+__device__ __forceinline__ float quant_chunk(const uint4 (&raw)[2], float eps, uint4& out) {
+  const T* v = reinterpret_cast<const T*>(raw);
+  float f[16];
+#pragma unroll
+  for (int i = 0; i < 16; ++i) f[i] = to_f32<T>(v[i]);
+  float amax = 0.f;
+#pragma unroll
+  for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
+  amax = fmaxf(group_max<8>(amax), eps);
+  return quant16(f, amax, B200_QUANT_DIV_CORRECTED, out);
+}
+
 }  // namespace b200

@@ -230,7 +230,7 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     p.split_stride = M * N;
     p.n_dest = 0;  // the partials stay local; the reduction pass fans the sum out
     int rc = wide ? launch_gemm_wide<float>(bn, A, B, p, splits, st)
-                  : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, 0, splits);
+                  : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, splits);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
     if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);

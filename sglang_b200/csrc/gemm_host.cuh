@@ -173,10 +173,9 @@ inline int launch_gemm_inst(const CUtensorMap& ta, const CUtensorMap& tb, const 
 
 // a_rows x K (fp8) times b_rows_total x K (fp8; grouped: experts stacked) -> C.
 // p must be filled except num_kb / n_blocks / n_tiles / m_tiles / group_m / status.
-// m_tiles_hint: expected number of live 128-row tiles when that is decided on the device.
 template <int MODE, typename OutT>
 inline int launch_gemm(const void* A, const void* B, int64_t b_rows_total, GemmParams p, int force_bn,
-                       cudaStream_t st, int64_t m_tiles_hint = 0, int k_splits = 1) {
+                       cudaStream_t st, int k_splits = 1) {
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_blocks = (int)cdiv(p.N, 128);
   p.m_tiles = (int)cdiv(p.M, kBM);
@@ -192,7 +191,6 @@ inline int launch_gemm(const void* A, const void* B, int64_t b_rows_total, GemmP
   // spread over the SMs by split-K instead).
   int bn = 256;
   if (MODE == GEMM_GROUPED_SILU_QUANT) force_bn = 256;  // gate + up halves of one tile
-  (void)m_tiles_hint;
   if (p.N <= 128) bn = 128;
   if (force_bn == 128 || force_bn == 256) bn = force_bn;
   p.n_tiles = MODE == GEMM_GROUPED_SILU_QUANT ? p.N / 128 : (int)cdiv(p.N, bn);

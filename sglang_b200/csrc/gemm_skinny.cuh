@@ -1,6 +1,6 @@
-// Decode-sized block-FP8 GEMM (M <= 64 rows of activations): the roles of the operands are
-// swapped so that the 128 weight rows of a tile fill the 128 lanes of the tensor-core tile
-// and the few tokens are its N dimension:
+// Decode-sized block-FP8 GEMM (up to 32 rows of activations always, up to 256 where plan_gemm finds
+// it the fastest): the roles of the operands are swapped so that the 128 weight rows of a tile fill
+// the 128 lanes of the tensor-core tile and the few tokens are its N dimension:
 //     D[n, m] = sum_k W[n, k] * X[m, k]        (UMMA M = 128 weight rows, N = NT tokens)
 // A thread of the promotion warps then owns ONE weight row and NT (16 or 32) token
 // accumulators instead of 128, so the per-K-block TMEM -> register promotion that bounds the
@@ -222,7 +222,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   if (p.cluster) {
     __syncwarp();
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-    if (Cfg::kSumBytes == 0) ptx::cluster_barrier();  // every ring is idle
+    if (Cfg::kSumBytes == 0) ptx::cluster_sync();  // every ring is idle
     // every split adds up its share of the rows: row t belongs to split t / per
     const int rows = min(NT, p.M - m0), r = threadIdx.x & 127, per = (rows + p.k_splits - 1) / p.k_splits;
     const uint32_t sums_off = Cfg::kSumBytes ? (uint32_t)(reinterpret_cast<uint8_t*>(bars + 32) - smem_al) : 0u;
@@ -230,12 +230,12 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       int owner = 0, j = 0;
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        if (t < rows) ptx::st_cluster_f32(ptx::stream_mapa(smem_base + sums_off, owner) + ((ks * per + j) * 128 + r) * 4, acc[t]);
+        if (t < rows) ptx::st_cluster_f32(ptx::mapa(smem_base + sums_off, owner) + ((ks * per + j) * 128 + r) * 4, acc[t]);
         if (++j == per) j = 0, ++owner;
       }
     }
     __syncwarp();
-    ptx::cluster_barrier();
+    ptx::cluster_sync();
     if (warp < 4 && ok_sum && n0 + r < p.N) {
       const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + r;
       OutT* out = static_cast<OutT*>(p.C) + n0 + r;

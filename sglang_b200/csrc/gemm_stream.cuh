@@ -63,17 +63,8 @@ struct StreamCfg {
 };
 
 namespace ptx {
-__device__ __forceinline__ uint32_t stream_mapa(uint32_t addr, uint32_t rank) {
-  uint32_t out;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(out) : "r"(addr), "r"(rank));
-  return out;
-}
 __device__ __forceinline__ void st_cluster_f32(uint32_t addr, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(addr), "f"(v) : "memory");
-}
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 }  // namespace ptx
 
@@ -387,15 +378,15 @@ stream_gemm_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_cons
   if (csize > 1) {
     // the first CTA's ring is idle once every rank is here; the others add their sums there, [rank - 1][token][row]
     __syncwarp();
-    ptx::cluster_barrier();
+    ptx::cluster_sync();
     const bool live = warp < 8 && my_block >= 0 && sum_ok;
     if (live && rank > 0) {
-      const uint32_t dst = ptx::stream_mapa(smem_base, 0) + (((rank - 1) * NT) * 256 + half * 128 + r) * 4;
+      const uint32_t dst = ptx::mapa(smem_base, 0) + (((rank - 1) * NT) * 256 + half * 128 + r) * 4;
 #pragma unroll
       for (int t = 0; t < NT; ++t) ptx::st_cluster_f32(dst + t * 1024, acc[t]);
     }
     __syncwarp();
-    ptx::cluster_barrier();
+    ptx::cluster_sync();
     if (live && rank == 0) {
       const float* src = reinterpret_cast<const float*>(smem_al) + half * 128 + r;
       for (int c = 1; c < (int)csize; ++c)  // rank order: the same sum on every run

@@ -203,16 +203,8 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
 #pragma unroll
         for (int u = 0; u < R; ++u) {
           if (g0 - (threadIdx.x >> 3) + 32 * u >= groups) break;  // the same for every thread
-          const T* e = reinterpret_cast<const T*>(raw[u]);
-          float f[16];
-#pragma unroll
-          for (int i = 0; i < 16; ++i) f[i] = to_f32<T>(e[i]);
-          float amax = 0.f;
-#pragma unroll
-          for (int i = 0; i < 16; ++i) amax = fmaxf(amax, fabsf(f[i]));
-          amax = fmaxf(group_max<8>(amax), p.eps);
           uint4 q;
-          const float sc = quant16(f, amax, B200_QUANT_DIV_CORRECTED, q);
+          const float sc = quant_chunk<T>(raw[u], p.eps, q);
           if (kb[u] >= 0) {
             *reinterpret_cast<uint4*>(x_ptr + (size_t)kb[u] * NT * kBK + (row[u] >> 3) * 1024 + (row[u] & 7) * 128 +
                                       ((chunk ^ (row[u] & 7)) << 4)) = q;
@@ -291,7 +283,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     // every rank adds up its share of the tokens (token t belongs to rank t / per): [rank][token][row], behind the tables, or
     // in the ring, which is idle once every rank is here
-    if (!p.own_sums) ptx::cluster_barrier();
+    if (!p.own_sums) ptx::cluster_sync();
     const uint32_t sums_off = p.own_sums ? (uint32_t)(reinterpret_cast<uint8_t*>(bs_tab + 2 * cap) - smem_al + 15) & ~15u : 0u;
     const int nt = item0 / p.t_tiles, m0 = (item0 - nt * p.t_tiles) * NT;
     const int rows = min(NT, p.M - m0), per = (rows + (int)csize - 1) / (int)csize, n = half * 128 + r;
@@ -299,12 +291,12 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       int owner = 0, j = 0;
 #pragma unroll
       for (int t = 0; t < NT; ++t) {
-        if (t < rows) ptx::st_cluster_f32(ptx::stream_mapa(smem_base + sums_off, owner) + (((int)rank * per + j) * 256 + n) * 4, acc[t]);
+        if (t < rows) ptx::st_cluster_f32(ptx::mapa(smem_base + sums_off, owner) + (((int)rank * per + j) * 256 + n) * 4, acc[t]);
         if (++j == per) j = 0, ++owner;
       }
     }
     __syncwarp();
-    ptx::cluster_barrier();
+    ptx::cluster_sync();
     if (warp < 8 && sum_ok && nt * 256 + n < p.N) {
       const float* src = reinterpret_cast<const float*>(smem_al + sums_off) + n;
       T* out = static_cast<T*>(p.out) + nt * 256 + n;

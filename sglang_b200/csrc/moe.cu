@@ -54,6 +54,7 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
   const int64_t tok = blockIdx.x;
   for (int j = threadIdx.x; j < min(topk, 64); j += blockDim.x) pos[j] = __ldg(position + tok * topk + j);
   __syncthreads();
+  // more than 64 slots per token: the scatter entry point takes them (fused_experts and the slot sum refuse)
   auto position_of = [&](int j) { return j < 64 ? pos[j] : __ldg(position + tok * topk + j); };
   const int groups = (int)(H / 128);
   for (int c0 = threadIdx.x & ~31; c0 < H / 16; c0 += blockDim.x) {  // whole warps
@@ -68,15 +69,7 @@ __global__ void __launch_bounds__(512) moe_scatter_quant_kernel(
       uint4 raw[2];
       raw[0] = active ? ld_nc_16(hidden + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
       raw[1] = active ? ld_nc_16(hidden + tok * H + chunk * 16 + 8) : make_uint4(0, 0, 0, 0);
-      const T* v = reinterpret_cast<const T*>(raw);
-      float f[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k) f[k] = to_f32<T>(v[k]);
-      float amax = 0.f;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(f[k]));
-      amax = fmaxf(group_max<8>(amax), 1e-10f);
-      scale = quant16(f, amax, B200_QUANT_DIV_CORRECTED, out);  // the stand-alone quantiser's bytes and scales
+      scale = quant_chunk<T>(raw, 1e-10f, out);
     }
     if (!active) continue;
     if ((chunk & 7) == 0 && chunk / 8 < kRowScales) row_s[chunk / 8] = scale;
@@ -165,15 +158,7 @@ __global__ void __launch_bounds__(256) moe_prep_kernel(const T* __restrict__ hid
       uint4 raw[2];
       raw[0] = active ? ld_nc_16(hidden + tok * H + chunk * 16) : make_uint4(0, 0, 0, 0);
       raw[1] = active ? ld_nc_16(hidden + tok * H + chunk * 16 + 8) : make_uint4(0, 0, 0, 0);
-      const T* v = reinterpret_cast<const T*>(raw);
-      float f[16];
-#pragma unroll
-      for (int k = 0; k < 16; ++k) f[k] = to_f32<T>(v[k]);
-      float amax = 0.f;
-#pragma unroll
-      for (int k = 0; k < 16; ++k) amax = fmaxf(amax, fabsf(f[k]));
-      amax = fmaxf(group_max<8>(amax), 1e-10f);
-      scale = quant16(f, amax, B200_QUANT_DIV_CORRECTED, out);  // the stand-alone quantiser's bytes and scales
+      scale = quant_chunk<T>(raw, 1e-10f, out);
     }
     if (!active) continue;
     *reinterpret_cast<uint4*>(q + (int64_t)pos * H + chunk * 16) = out;
@@ -455,8 +440,6 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
                             topk_ids, static_cast<T*>(out), topk, E, H, routed_scale, skip_unrouted, nullptr);
   }
   const int force_bn = tuning().gemm_bn == 128 || tuning().gemm_bn == 256 ? (int)tuning().gemm_bn : 0;
-  // expected live row tiles: every pair once, plus up to one partial tile per expert
-  const int64_t tiles_hint = cdiv(numel, kMoeBlockM) + (numel < E ? numel : E) / 2;
   GemmParams p = {};
   p.expert_ids = expert_ids; p.num_post_pad = npp; p.sorted_ids = sorted; p.numel = (int)numel;
   p.M = (int)L.cap;
@@ -464,7 +447,7 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   p.As = as1; p.as_sm = scales_by_row ? H / 128 : 1; p.as_sk = scales_by_row ? 1 : L.cap; p.Bs = w1_scale; p.C = nullptr; p.ldc = 0;
   p.N = (int)I; p.K = (int)H; p.topk_weights = weight_on_input ? topk_weights : nullptr;
   p.q_out = aq2; p.q_scales = as2; p.q_scale_ld = L.cap;
-  if ((rc = launch_gemm<GEMM_GROUPED_SILU_QUANT, T>(aq1, w1, (int64_t)E * 2 * I, p, 256, st, tiles_hint))) return rc;
+  if ((rc = launch_gemm<GEMM_GROUPED_SILU_QUANT, T>(aq1, w1, (int64_t)E * 2 * I, p, 256, st))) return rc;
   // GEMM 2: [cap, I] x w2[E, H, I]^T -> rows scattered to (token, slot), times the router weight
   p.As = as2; p.as_sm = 1; p.as_sk = L.cap; p.Bs = w2_scale; p.C = c3; p.ldc = H; p.N = (int)H; p.K = (int)I;
   p.topk_weights = weight_on_input ? nullptr : topk_weights;
@@ -476,7 +459,7 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
   }
   if (split) {
     p.split_stride = numel * H;
-    if ((rc = launch_gemm<GEMM_GROUPED_SCATTER, float>(aq2, w2, (int64_t)E * H, p, 256, st, tiles_hint, down_splits)))
+    if ((rc = launch_gemm<GEMM_GROUPED_SCATTER, float>(aq2, w2, (int64_t)E * H, p, 256, st, down_splits)))
       return rc;
     const int64_t rows = no_combine ? numel : T_tokens;
     const int64_t total = rows * (H / 8);
@@ -485,7 +468,7 @@ static int run_fused_experts(const void* hidden, const float* hidden_scale, cons
         numel * H, E, H, no_combine ? 1.0f : routed_scale, skip_unrouted);
     return check_launch("moe_sum_reduce_splits");
   }
-  if ((rc = launch_gemm<GEMM_GROUPED_SCATTER, T>(aq2, w2, (int64_t)E * H, p, force_bn, st, tiles_hint))) return rc;
+  if ((rc = launch_gemm<GEMM_GROUPED_SCATTER, T>(aq2, w2, (int64_t)E * H, p, force_bn, st))) return rc;
   if (!no_combine) {
     moe_sum_reduce_kernel<T><<<(unsigned)T_tokens, 256, 0, st>>>(c3, topk_ids, static_cast<T*>(out), topk, E, H,
                                                                   routed_scale, skip_unrouted, nullptr);
@@ -552,10 +535,10 @@ static int run_masked_experts(const void* hidden_q, const float* hidden_s, const
   // gate_up: row-major input scales [cap][H/128]
   p.As = hidden_s; p.as_sm = H / 128; p.as_sk = 1; p.Bs = w1_scale; p.N = (int)I; p.K = (int)H;
   p.q_out = aq2; p.q_scales = as2; p.q_scale_ld = L.cap;
-  if ((rc = launch_gemm<GEMM_GROUPED_SILU_QUANT, T>(hidden_q, w1, (int64_t)E * 2 * I, p, 256, st, 0))) return rc;
+  if ((rc = launch_gemm<GEMM_GROUPED_SILU_QUANT, T>(hidden_q, w1, (int64_t)E * 2 * I, p, 256, st))) return rc;
   // down: rows stay where they are (identity "scatter"), no router weight
   p.As = as2; p.as_sm = 1; p.as_sk = L.cap; p.Bs = w2_scale; p.C = out; p.ldc = H; p.N = (int)H; p.K = (int)I;
-  return launch_gemm<GEMM_GROUPED_SCATTER, T>(aq2, w2, (int64_t)E * H, p, 0, st, 0);
+  return launch_gemm<GEMM_GROUPED_SCATTER, T>(aq2, w2, (int64_t)E * H, p, 0, st);
 }
 
 }  // namespace b200
