@@ -85,10 +85,25 @@ def test_many_experts_per_token_slot_sum(T, E, topk):
     assert float(out[0].float().abs().max()) == 0.0
 
 
+@pytest.mark.parametrize("moe_decode", [0, -1])
 @pytest.mark.parametrize("T,E,topk,H,I", [(1, 8, 2, 256, 2048), (3, 8, 2, 512, 1024), (5, 16, 4, 256, 1536)])
-def test_few_tokens_split_k_down_gemm(T, E, topk, H, I):
-    """A handful of tokens: the down GEMM splits K = I over the SMs and the slot reduction sums
-    the fp32 partials; with and without the slot reduction, and with ids of other ranks (-1)."""
+def test_few_tokens_split_k_down_gemm(T, E, topk, H, I, moe_decode):
+    """Few tiles to fill the SMs with: the down GEMM splits K = I. On the tile path (knob 0; by itself it takes a few local
+    experts with more than about 27 rows each) the slot reduction sums fp32 partials, on the weight-streaming path, which
+    these shapes take by default, a cluster does. With and without the slot reduction, and with ids of other ranks (-1)."""
+    from sglang_b200._native import tuning
+
+    with tuning(moe_decode=moe_decode):
+        _split_k_down_case(T, E, topk, H, I)
+
+
+@pytest.mark.parametrize("T,E,topk,H,I", [(60, 1, 1, 512, 2048), (70, 4, 2, 768, 1024)])
+def test_split_k_down_gemm_by_default(T, E, topk, H, I):
+    """Shapes that take the tile path and its K split without a knob."""
+    _split_k_down_case(T, E, topk, H, I)
+
+
+def _split_k_down_case(T, E, topk, H, I):
     g = torch.Generator().manual_seed(100 + T)
     x = torch.randn(T, H, generator=g).bfloat16()
     w1, w2, w1_s, w2_s = _weights(E, I, H, 40 + T)
@@ -106,13 +121,16 @@ def test_few_tokens_split_k_down_gemm(T, E, topk, H, I):
     assert O.rel_frobenius(part.float().cpu(), ref_part) < TOL
     nc_part = _run(x, w1, w2, w1_s, w2_s, tw, local, no_combine=True)
     assert nc_part[:, 0].abs().max().item() == 0
+    ref_part = O.fused_experts_fp8(x, w1, w2, w1_s, w2_s, tw, local, [128, 128], no_combine=True)
+    if topk > 1:
+        assert O.rel_frobenius(nc_part.float().cpu(), ref_part) < TOL
 
 
 @pytest.mark.parametrize("T,E,topk,H,I", [(1, 8, 2, 512, 256), (7, 64, 8, 1024, 256), (16, 16, 4, 256, 384), (17, 8, 2, 512, 256),
                                           (32, 256, 8, 512, 128), (40, 8, 2, 256, 1152), (64, 8, 2, 512, 256)])
 def test_few_token_path_vs_oracle_and_tile_path(T, E, topk, H, I):
-    """The swapped-operand kernels for T <= 64 (token tiles of 16 / 32 / 64, no align or gather pass; opt-in
-    with the knob ``moe_decode=1``). Against the oracle, and against the default 128 x 256 tile path on the
+    """The weight-streaming kernels (token blocks of 16 / 32 / 64, chosen by the rows per expert; the knob keeps the
+    larger of these shapes on them). Against the oracle, and against the 128 x 256 tile path on the
     same inputs: both quantise the token rows identically, so they differ only by the intermediate's
     quantisation arithmetic and the summation order."""
     from sglang_b200._native import tuning
@@ -130,7 +148,7 @@ def _few_token_case(T, E, topk, H, I, tuning):
     out = _run(x, w1, w2, w1_s, w2_s, tw, ti)
     assert O.rel_frobenius(out.float().cpu(), ref) < TOL
     with tuning(moe_decode=0):
-        tile = _run(x, w1, w2, w1_s, w2_s, tw, ti)  # the default path
+        tile = _run(x, w1, w2, w1_s, w2_s, tw, ti)
     assert O.rel_frobenius(out.float().cpu(), tile.float().cpu()) < TOL
     # called again: same bits (no state is carried between calls)
     assert torch.equal(_run(x, w1, w2, w1_s, w2_s, tw, ti), out)
@@ -190,6 +208,50 @@ def test_expert_parallel_minus_one_ids_sum_to_full_result():
     # a rank that owns none of the selected experts returns exact zeros
     none = _run(x, w1[:4], w2[:4], w1_s[:4], w2_s[:4], tw, torch.full_like(ti, -1))
     assert none.abs().max().item() == 0
+
+
+@pytest.mark.parametrize("remote", [False, True])
+@pytest.mark.parametrize("block", [16, 32, 64])
+@pytest.mark.parametrize("T,E,topk,H,I", [(600, 16, 2, 256, 256), (131, 40, 8, 512, 128)])
+def test_streaming_experts_behind_the_separate_align(T, E, topk, H, I, block, remote):
+    """More than 1024 pairs: align, scatter and the streaming GEMMs as kernels of their own, with several blocks of rows per
+    expert, at every block size; with a third of the ids on other ranks too."""
+    from sglang_b200._native import tuning
+
+    assert T * topk > 1024
+    g = torch.Generator().manual_seed(800 + T + block)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    w1, w2, w1_s, w2_s = _weights(E, I, H, 90)
+    tw, ti = O.softmax_topk(torch.randn(T, E, generator=g), topk, True)
+    if remote:
+        ti = torch.where(torch.rand(T, topk, generator=g) < 0.33, torch.full_like(ti, -1), ti)
+    with tuning(moe_decode=block):
+        out = _run(x, w1, w2, w1_s, w2_s, tw, ti)
+        nc = _run(x, w1, w2, w1_s, w2_s, tw, ti, no_combine=True)
+    args = (x, w1, w2, w1_s, w2_s, tw, ti, [128, 128])
+    assert O.rel_frobenius(out.float().cpu(), O.fused_experts_fp8(*args)) < TOL
+    assert O.rel_frobenius(nc.float().cpu(), O.fused_experts_fp8(*args, no_combine=True)) < TOL
+
+
+def test_scatter_of_more_than_64_slots():
+    """The scatter entry point takes more slots per token than the slot sum does."""
+    import sglang_b200 as S
+    from sglang_b200 import _native as N
+    from sglang_b200.fused_moe import fused_experts_scatter
+
+    T, E, topk, H, I = 9, 80, 70, 256, 128
+    g = torch.Generator().manual_seed(7)
+    x = torch.randn(T, H, generator=g).bfloat16()
+    w1, w2, w1_s, w2_s = _weights(E, I, H, 8)
+    tw, ti = O.softmax_topk(torch.randn(T, E, generator=g), topk, True)
+    ti[::2, 1::3] = -1
+    q, s = S.per_token_group_quant_fp8(x.cuda(), 128)
+    rows = torch.zeros(T * topk, H, dtype=torch.bfloat16, device="cuda")
+    fused_experts_scatter(q, s, w1.cuda(), w2.cuda(), tw.cuda(), ti.cuda().int(), w1_s.cuda(), w2_s.cuda(),
+                          (N.c_void_p * 1)(rows.data_ptr()), T * topk)
+    _status_ok()
+    ref = O.fused_experts_fp8(x, w1, w2, w1_s, w2_s, tw, ti, [128, 128], no_combine=True)
+    assert O.rel_frobenius(rows.view(T, topk, H).float().cpu(), ref) < TOL
 
 
 @pytest.mark.parametrize("block,T,E,topk", [(16, 263, 8, 4), (32, 262, 20, 4), (64, 275, 40, 6)])
