@@ -146,10 +146,11 @@ __device__ __forceinline__ uint4 ld_nc_16(const void* p) {
 
 // The first n 128-byte K blocks of a weight row into L2. Nothing is read, so a kernel launched as a programmatic dependent
 // may ask for its weights while an earlier kernel still writes them: the write goes to the same L2 line.
-// Depth, in K blocks per CTA of the dense kernels: beyond what fits the gap before the wait ends, the requests hold up the
-// loads behind them. Four projections of 6144..28672 x 4096..14336, 1 / 16 rows: 3 blocks 52.7 / 55.6 us, 4 53.0 / 55.7,
-// 5 53.5 / 56.0, 10 55.3 / 57.7, none 58.5 / 58.7; the same boxes by cp.async.bulk.prefetch.tensor, which queue in front of
-// the loads, 5 blocks 59.5 / 59.7; loads into the ring before the wait, which nothing orders behind a writer, 53.2 / 56.6.
+// Depth, in K blocks per CTA of the dense kernels: what fits the gap before the wait ends; requests beyond that hold up the
+// loads behind them. Four projections (6144..28672 x 4096..14336) in a graph, 1 / 16 / 61 rows: none 52.9 / 55.9 / 73.0 us,
+// 1 block 51.9 / 55.2 / 73.0, 3 blocks 50.9 / 54.3 / 73.0, 5 blocks 50.2 / 54.3 / 73.7; a rank of eight (10240 x 8192 and so
+// on), 61 rows: 1 block 48.9, 3 blocks 49.9, 5 blocks 50.6. Boxes by cp.async.bulk.prefetch.tensor gain nothing, they queue
+// in front of the loads. Loads into the ring before the wait, which nothing would order behind a writer: 51.1 / 53.5 / 70.7.
 constexpr int kPrefetchKb = 3;
 __device__ __forceinline__ void prefetch_weight_row(const uint8_t* row, int n) {
   for (int i = 0; i < n; ++i) asm volatile("prefetch.global.L2 [%0];" ::"l"(row + i * 128) : "memory");

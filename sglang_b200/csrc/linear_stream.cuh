@@ -103,9 +103,10 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
   const uint32_t tmem_base = *tmem_slot;
   // "I have started", waited for before another CTA's shared memory is written at the very end
   if (csize > 1) asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
-  // after the TMEM allocation: a dependent grid's CTA that got its columns first, and then waits for this grid, would
-  // otherwise hold them for ever
-  grid_launch_dependents();
+  // The next kernels may start: at once behind the one-launch kernel (four projections of 1 row, rank of eight, 19.9 us in a
+  // graph, signalled at the end of the K loop 21.5), else there, as in gemm_skinny.cuh. After the TMEM allocation in any
+  // case: a dependent grid's CTA that got its columns first, and then waits for this grid, would otherwise hold them for ever.
+  if (QUANT) grid_launch_dependents();
 
   const int item0 = blockIdx.x / csize, step = gridDim.x / csize;
   const int kb0 = (int)rank * p.kb_per_rank, kb1 = min(p.num_kb, kb0 + p.kb_per_rank);
@@ -275,6 +276,7 @@ linear_stream_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_co
       if (csize > 1) break;  // one item per cluster: finished below
       if (ok) store(item);
     }
+    if (!QUANT) grid_launch_dependents();
     if (csize > 1) sum_ok = !named_bar_any(1, 256, !ok);
   }
 

@@ -14,11 +14,10 @@ __global__ void __launch_bounds__(256) quant_group_kernel(const T* __restrict__ 
                                                           int64_t s_stride_g, float eps, int early) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = c < total_chunks;  // whole lane-groups are active or not (total % LPG == 0)
-  // The GEMM of a linear layer, launched as programmatic dependent, may set itself up and prefetch weights from here on; it
-  // waits for this grid's completion before it reads anything. Admitted earlier, before the kernels ahead are through, it is
-  // in their way: four projections of one row 58.4 us against 53.5. The stand-alone quantiser signals by ending.
-  grid_dependency_wait();  // x, and the readers of the buffers overwritten below
+  // The GEMM of a linear layer, launched as programmatic dependent, may set itself up and prefetch weights now; it waits
+  // for this grid's completion before it reads anything. The stand-alone quantiser signals by ending.
   if (early) grid_launch_dependents();
+  grid_dependency_wait();  // x, and the readers of the buffers overwritten below
   float f[16];
   if (active) {
     Vec16<T>::load(x + c * 16, f);
