@@ -8,15 +8,21 @@
 // Roles per CTA (640 threads):
 //   warps 0-15   promotion: warp w owns TMEM lanes 32 (w % 4).. and columns 64 (w / 4)..; 64 accumulators per thread.
 //                Four warps per SM sub-partition: the TMEM round trip of one hides behind the FMAs of the others.
+//                What the loop costs in instructions is time (the MMA warp waits for the accumulator buffer half of the
+//                time) and, at the power cap, clock: packed FMAs straight on what tcgen05.ld returns, no register copies, one
+//                scale read from shared memory, two K blocks per trip. Four times (16 columns, 8 FMAs) instead of twice
+//                (32, 16) costs 4 %, plain FMAs instead of packed ones 3 %.
 //   warp  16     TMA producer (no multicast: every load has one destination CTA)
 //   warp  17     MMA issuer (leader CTA only)
 //   warps 18-19  scale loaders: products As[row] * Bs[128-column block] of four K blocks at a time into a
-//                shared-memory ring, so a promotion thread reads one float per K block
+//                shared-memory ring [block][row][K block], so a promotion thread reads one float per K block
 // Cross-CTA protocol (rank 0 = leader):
 //   full[s]   (leader's)  2 arrivals (one expect_tx per producer) + the bytes of both CTAs' TMA loads
-//   empty[s]  (each CTA)  arrival of promotion warp 0 once it saw the MMAs of the stage complete
-//   tfull[b]  (each CTA)  arrival from the leader's tcgen05.commit
+//   empty[s]  (each CTA)  arrival from the leader's tcgen05.commit
+//   tfull[b]  (each CTA)  likewise
 //   tempty[b] (leader's)  32 arrivals: the promotion warps of both CTAs
+// Looped, with the copies (120 instructions per warp and K block) and without (97): 8192 x 4096 x 4096 143 -> 134 us,
+// 1027 x 7168 x 8192 78.6 -> 73.3, 203 x 6144 x 4096 (128-wide tiles) 15.1 -> 13.2.
 #pragma once
 
 #include "gemm_host.cuh"
@@ -86,11 +92,17 @@ __device__ __forceinline__ void wide_sync() {
   __syncthreads();
   if constexpr (CTAS == 2) cluster_sync();
 }
-// a += b * s on two packed floats
+// Wait for this thread's outstanding tcgen05.ld. The loaded registers are not operands of the wait (as in tmem_ld_wait):
+// what reads them is volatile too and stays behind it, and the compiler makes no copies of them.
+__device__ __forceinline__ void tmem_ld_wait_all() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
+// a += b * s on two packed floats, b just loaded from TMEM
 __device__ __forceinline__ void ffma2(uint64_t& a, uint32_t b0, uint32_t b1, uint64_t s) {
-  uint64_t b;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(b) : "r"(b0), "r"(b1));
-  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(a) : "l"(b), "l"(s));
+  asm volatile("{.reg .b64 b; mov.b64 b, {%1, %2}; fma.rn.f32x2 %0, b, %3, %0;}" : "+l"(a) : "r"(b0), "r"(b1), "l"(s));
+}
+__device__ __forceinline__ uint64_t pack2(float v) {
+  uint64_t p;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(v));
+  return p;
 }
 }  // namespace ptx
 
@@ -110,8 +122,8 @@ struct Wide {
   static constexpr int kRegsPromotion = 104, kRegsOther = 64;
   static constexpr int kBoxBytes = 32 * kCols * 2;             // a warp's 32 rows of 16-bit output
   static constexpr int kStagingBytes = 16 * 32 * 128;          // at most 128 bytes per row
-  static constexpr int kBlocks = BN == 192 ? 3 : BN / 128;     // 128-column scale blocks a tile touches
-  static constexpr int kScaleSlots = CTAS == 1 ? 2 : 3, kScaleSlotBytes = 4 * kBlocks * 128 * 4;  // four K blocks x blocks x rows
+  static constexpr int kBlocks = BN == 128 ? 1 : 2;            // 128-column scale blocks a tile touches
+  static constexpr int kScaleSlots = 2, kScaleSlotBytes = kBlocks * 128 * 16;  // blocks x rows x four K blocks
   static constexpr int kTmemCols = 512;
   static constexpr size_t kSmemBytes =
       (size_t)kStages * (kStageA + kStageB) + kStagingBytes + kScaleSlots * kScaleSlotBytes + 1024 + 256;
@@ -142,7 +154,7 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * S + 2 * NB + 2 * SQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * S + 2 * NB + 2 * SQ + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const uint32_t rank = CTAS == 2 ? ptx::cluster_ctarank() : 0;
   const bool leader = rank == 0;
 
@@ -226,20 +238,25 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
             if (++s == S) s = 0, phase ^= 1;
           }
         }
+        // the leader's last arrivals on this CTA's empty barriers, before its shared memory may go
+        for (int i = 0; i < S && ok; ++i) {
+          ok = ptx::mbar_wait(empty_bar(s), phase, abort_flag);
+          if (++s == S) s = 0, phase ^= 1;
+        }
       }
       __syncwarp();
     } else if (warp == Cfg::kMmaWarp) {
       if (leader && ptx::elect_one()) {  // ------------------------------------------ MMA issuer (leader only)
         constexpr uint32_t idesc = ptx::idesc_e4m3_f32(kRows, BN);
         int s = 0;
-        uint32_t phase = 0, it = 0;
+        uint32_t phase = 0, tphase = 1;
+        int b = 0;
         bool ok = true;
         for (int item = pair; item < total_items && ok; item += npairs) {
           const Item c = item_of(item);
-          for (int kb = c.kb0; kb < c.kb1; ++kb, ++it) {
-            const int b = it % NB;
-            ok = ptx::mbar_wait(tempty_bar(b), ((it / NB) & 1) ^ 1, abort_flag) &&
-                 ptx::mbar_wait(full_bar(s), phase, abort_flag);
+          for (int kb = c.kb0; kb < c.kb1; ++kb) {
+            // the accumulator buffer comes last of the two as a rule: nothing but its own wake-up in front of the MMAs
+            ok = ptx::mbar_wait(full_bar(s), phase, abort_flag) && ptx::mbar_wait(tempty_bar(b), tphase, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after();
             const uint64_t da = ptx::smem_desc_sw128(sA + s * Cfg::kStageA);
@@ -247,8 +264,14 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
             const uint32_t d = tmem_base + b * Cfg::kAccStride;
 #pragma unroll
             for (int k = 0; k < kBK / 32; ++k) ptx::wide_mma<CTAS>(d, da + 2 * k, db + 2 * k, idesc, k > 0);
-            if constexpr (CTAS == 2) ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
-            else ptx::mma_commit(tfull_bar(b));
+            if constexpr (CTAS == 2) {
+              ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
+              ptx::mma_commit_pair_multicast(empty_bar(s), (uint16_t)3);
+            } else {
+              ptx::mma_commit(tfull_bar(b));
+              ptx::mma_commit(empty_bar(s));
+            }
+            if (++b == NB) b = 0, tphase ^= 1;
             if (++s == S) s = 0, phase ^= 1;
           }
         }
@@ -278,14 +301,14 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
           }
           ok = ptx::mbar_wait(sempty_bar(q), phase, abort_flag);
           if (!ok) break;
-          float* dst = scales + q * (Cfg::kScaleSlotBytes / 4) + tid;
+          float* dst = scales + q * (Cfg::kScaleSlotBytes / 4) + tid * 4;  // [block][row][K block]
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-#pragma unroll
-            for (int n = 0; n < Cfg::kBlocks; ++n) {
-              dst[(j * Cfg::kBlocks + n) * 128] = a[j][0] * b[j][n];
-              dst[(j * Cfg::kBlocks + n) * 128 + 64] = a[j][1] * b[j][n];
-            }
+          for (int n = 0; n < Cfg::kBlocks; ++n) {
+            *reinterpret_cast<float4*>(dst + n * 512) =
+                make_float4(a[0][0] * b[0][n], a[1][0] * b[1][n], a[2][0] * b[2][n], a[3][0] * b[3][n]);
+            *reinterpret_cast<float4*>(dst + n * 512 + 256) =
+                make_float4(a[0][1] * b[0][n], a[1][1] * b[1][n], a[2][1] * b[2][n], a[3][1] * b[3][n]);
+          }
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(sfull_bar(q));
           if (++q == SQ) q = 0, phase ^= 1;
@@ -299,79 +322,67 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     const int quarter = warp & 3, colq = warp >> 2;
     constexpr int kCols = Cfg::kCols, CH = Cfg::kChunks;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + colq * kCols;
-    const uint32_t wstage = staging + warp * Cfg::kBoxBytes;
-    const uint32_t my_scales = ptx::smem_u32(scales) + (quarter * 32 + lane) * 4;
+    const uint32_t my_scales = ptx::smem_u32(scales) + (quarter * 32 + lane) * 16;
     const uint32_t leader_tempty = CTAS == 2 ? ptx::mapa(tempty_bar(0), 0) : tempty_bar(0);
-    uint32_t it = 0;
-    int s = 0, q = 0;
-    uint32_t sphase = 0;
+    uint32_t tphase = 0, sphase = 0;
+    int q = 0, b = 0;
     bool ok = true;
     for (int item = pair; item < total_items && ok; item += npairs) {
       const Item c = item_of(item);
-      // byte offset of the scale block of every 16-column chunk of this warp (a 192-wide tile starts inside a block)
-      uint32_t blk_off[CH];
+      // a 192-wide tile starts inside a scale block, so a warp's 16-column chunks may lie in two of them
+      const int col_in_block = BN == 192 ? c.nt * BN % 128 + colq * kCols : colq * kCols;
+      const int first_blk = col_in_block / 128;
+      bool second[CH];
 #pragma unroll
-      for (int h = 0; h < CH; ++h)
-        blk_off[h] = (BN == 192 ? (c.nt * BN + colq * kCols + 16 * h) / 128 - c.nt * BN / 128 : colq * kCols / 128) * 512;
+      for (int h = 0; h < CH; ++h) second[h] = BN == 192 && (col_in_block + 16 * h) / 128 != first_blk;
       uint64_t acc[kCols / 2];
 #pragma unroll
       for (int j = 0; j < kCols / 2; ++j) acc[j] = 0;
       for (int kbase = c.kb0; kbase < c.kb1 && ok; kbase += 4) {
         ok = ptx::mbar_wait(sfull_bar(q), sphase, abort_flag);
         const int n = min(4, c.kb1 - kbase);
-        for (int j = 0; j < n && ok; ++j, ++it) {
-          const int b = it % NB;
-          uint64_t sc[CH];  // {scale, scale} of every chunk; one value where the tile is aligned to the blocks
-#pragma unroll
-          for (int h = 0; h < CH; ++h) {
-            if (BN == 192 || h == 0) {
-              float v;
-              asm volatile("ld.shared.f32 %0, [%1];"
-                           : "=f"(v)
-                           : "r"(my_scales + q * Cfg::kScaleSlotBytes + j * Cfg::kBlocks * 512 + blk_off[h])
-                           : "memory");
-              asm("mov.b64 %0, {%1, %1};" : "=l"(sc[h]) : "f"(v));
-            } else {
-              sc[h] = sc[0];
-            }
-          }
-          ok = ptx::mbar_wait(tfull_bar(b), (it / NB) & 1, abort_flag);
+#pragma unroll 2
+        for (int j = 0; j < n && ok; ++j) {
+          float sc1, sc2;  // scale in the warp's first scale block and in its second
+          const uint32_t sa = my_scales + q * Cfg::kScaleSlotBytes + first_blk * 2048 + 4 * j;
+          asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc1) : "r"(sa) : "memory");
+          if (BN == 192) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(sc2) : "r"(second[CH - 1] ? sa + 2048 : sa) : "memory");
+          ok = ptx::mbar_wait(tfull_bar(b), tphase, abort_flag);
           if (!ok) break;
           ptx::tc_fence_after();
+          const uint64_t sc = ptx::pack2(sc1);
           const uint32_t ta = lane_base + b * Cfg::kAccStride;
-          uint32_t v[32];
-          ptx::tmem_ld32(ta, v);
-          if (warp == 0 && lane == 0) ptx::mbar_arrive(empty_bar(s));  // the MMAs of this stage have read it
-          if (++s == S) s = 0;
-          ptx::tmem_ld_wait(v);
-          if (kCols > 32) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) ptx::ffma2(acc[i], v[2 * i], v[2 * i + 1], sc[i / 8]);
-            if (kCols == 64) {
-              ptx::tmem_ld32(ta + 32, v);
-              ptx::tmem_ld_wait(v);
-            } else {
-              ptx::tmem_ld16(ta + 32, v);
-              ptx::tmem_ld_wait16(v);
+          for (int h = 0; h < CH; h += 2) {  // 32 columns, or the last 16
+            uint32_t v[32];
+            if (CH - h >= 2) ptx::tmem_ld32(ta + 16 * h, v);
+            else ptx::tmem_ld16(ta + 16 * h, v);
+            ptx::tmem_ld_wait_all();
+            if (h + 2 >= CH) {
+              ptx::tc_fence_before();
+              __syncwarp();
+              if (ptx::elect_one()) {
+                if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(leader_tempty + 8 * b);
+                else ptx::mbar_arrive(leader_tempty + 8 * b);
+              }
+              if (++b == NB) b = 0, tphase ^= 1;
+            }
+#pragma unroll
+            for (int i = 0; i < (CH - h >= 2 ? 2 : 1); ++i) {
+              const uint64_t sch = BN == 192 && second[h + i] ? ptx::pack2(sc2) : sc;
+#pragma unroll
+              for (int k = 0; k < 8; ++k) ptx::ffma2(acc[8 * (h + i) + k], v[16 * i + 2 * k], v[16 * i + 2 * k + 1], sch);
             }
           }
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) {
-            if constexpr (CTAS == 2) ptx::mbar_arrive_cluster(leader_tempty + 8 * b);
-            else ptx::mbar_arrive(leader_tempty + 8 * b);
-          }
-          constexpr int base = kCols > 32 ? 16 : 0;
-#pragma unroll
-          for (int i = 0; i < kCols / 2 - base; ++i) ptx::ffma2(acc[base + i], v[2 * i], v[2 * i + 1], sc[(base + i) / 8]);
         }
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(sempty_bar(q));
+        if (ptx::elect_one()) ptx::mbar_arrive(sempty_bar(q));
         if (++q == SQ) q = 0, sphase ^= 1;
       }
       if (!ok) break;
 
       // ------------------------------------------------------------------------ tile epilogue
+      const uint32_t wstage = staging + warp * Cfg::kBoxBytes;
       const int row0 = c.mt * kRows + (int)rank * kBM + quarter * 32, col0 = c.nt * BN + colq * kCols;
       if constexpr (sizeof(OutT) == 2) {
         if (lane == 0) ptx::tma_store_wait_read();  // the last tile's box has left the staging area
