@@ -143,9 +143,15 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N,
 
 namespace b200 {
 // The decode kernel (gemm_skinny.cuh) with its K split; sp holds the scales.
+// Whether run_skinny writes the result itself (no K split, or one summed within clusters), without partials in memory.
+static bool skinny_direct(int64_t M, int64_t N, int64_t K, int splits) {
+  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;
+  const int nt = skinny_token_tile(M);
+  return splits == 1 || (tuning().gemm_splitk <= 0 && skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) > 1);
+}
 static int run_skinny(const void* A, const void* B, SkinnyParams sp, int splits, void* C, int c_dtype, int64_t M, int64_t N,
                       int64_t K, void* workspace, size_t workspace_bytes, cudaStream_t st, const FanOut& fan) {
-  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16>::kMaxKb) ++splits;  // scales of one item fit its smem table
+  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;  // scales of one item fit its smem table
   sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
   // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
   const int nt = skinny_token_tile(M);
@@ -302,6 +308,17 @@ static bool linear_one_launch(int64_t M, int64_t N, int64_t K) {
   return M <= kLinearStreamMaxM && tuning().linear_decode_fused != 0 &&
          plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages, own) && kb * M <= 32 && N * K < (16 << 20);
 }
+// Quantiser inside the decode GEMM (one launch): up to 8 rows, where the plan takes that kernel and its splits are summed
+// within clusters. The four projections of an unsharded 4096-wide layer, launched one by one, two launches each against one:
+// 1 row 53.7 and 48.0 us, 8 rows 56.2 and 51.0; at 16 rows the quantiser warps no longer keep up with the weights, 56.6 and 65.0
+// (with twice as many of them 56.2, but then 1 row takes 50.3).
+constexpr int64_t kLinearQuantInGemmMaxM = 8;
+static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K) {
+  const Tuning& tune = tuning();
+  if (M > kLinearQuantInGemmMaxM || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
+  const GemmPlan plan = plan_gemm(M, N, K, sm_count() < 148 ? sm_count() : 148, true);
+  return plan.skinny && skinny_direct(M, N, K, plan.splits);
+}
 }  // namespace b200
 
 extern "C" size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
@@ -327,6 +344,15 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
     return B200_E_WORKSPACE;
   }
   if (linear_one_launch(M, N, K)) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
+  if (linear_quant_in_gemm(M, N, K)) {
+    B200_CHECK_ARG(((uintptr_t)out & 15) == 0, "gemm: A, B and C must be 16-byte aligned");
+    B200_UNSUPPORTED(N > 0x7fffff00LL || K > 0x7fffff00LL, "gemm: dimension too large");
+    const int sms = sm_count() < 148 ? sm_count() : 148;
+    SkinnyParams sp = {};
+    sp.x = x; sp.eps = 1e-10f; sp.Bs = Bs;
+    return run_skinny(nullptr, B, sp, plan_gemm(M, N, K, sms, true).splits, out, x_dtype, M, N, K, nullptr, 0,
+                      static_cast<cudaStream_t>(stream), FanOut{});
+  }
   uint8_t* q = static_cast<uint8_t*>(workspace);
   float* s = reinterpret_cast<float*>(q + linear_q_bytes(M, K));
   uint8_t* rest = reinterpret_cast<uint8_t*>(s) + linear_s_bytes(M, K);

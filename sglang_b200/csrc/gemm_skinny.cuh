@@ -23,6 +23,8 @@ struct SkinnyParams {
   const int32_t *sfa, *sfb;
   int64_t sfa_ld, sfb_ld;
   int sfb_step;
+  const void* x;    // QUANT: 16-bit activations [M, K], row-major
+  float eps;        // QUANT: least row-group maximum
   void* C;          // OutT [M, N], or fp32 partials [splits][M, N]
   int M, N, K, num_kb;
   int n_tiles, t_tiles, k_splits, kb_per_split;
@@ -31,12 +33,12 @@ struct SkinnyParams {
   int* status;
 };
 
-template <int NT>
+template <int NT, bool QUANT>
 struct SkinnyCfg {
   static constexpr int kStages = 5;
   static constexpr int kStageW = 128 * kBK;  // 16 KB of weights
   static constexpr int kStageX = NT * kBK;   // 2 or 4 KB of activations
-  static constexpr int kThreads = 6 * 32;    // 4 promotion warps, producer, MMA issuer
+  static constexpr int kQuantWarps = 4, kThreads = (QUANT ? 6 + kQuantWarps : 6) * 32;  // 4 promotion warps, producer, MMA issuer (, quantisers)
   // TMEM accumulator buffers: the tensor core runs this many K blocks ahead of the promotion warps, so the
   // commit -> tcgen05.ld -> arrive round trip (about a microsecond) is off the per-K-block path
   static constexpr int kAccBufs = 4;
@@ -46,14 +48,19 @@ struct SkinnyCfg {
   // room for them and they go to the ring once it is idle
   static constexpr int kSumBytes = NT == 16 ? 21 * 512 : 0;
   static constexpr size_t kSmemBytes =
-      (size_t)kStages * (kStageW + kStageX) + (size_t)kMaxKb * NT * 4 + kSumBytes + 1024 + 256;
+      (size_t)kStages * (kStageW + kStageX) + (size_t)kMaxKb * NT * 4 + kSumBytes + (QUANT ? kMaxKb * 8 : 0) + 1024 + 256;
 };
 
-template <int NT, typename OutT>
-__global__ void __launch_bounds__(SkinnyCfg<NT>::kThreads, 2)
+// QUANT: X is the 16-bit input of a linear layer. Four more warps quantise the CTA's K range of its rows (same bytes and scales as
+// the stand-alone quantiser), one K block after the other into the ring next to the weights, while those stream: quantiser and
+// GEMM in one launch, the quantiser's time hidden behind the weights'. Bound by the weight stream and, between two calls, by the
+// dependency wait, the first rows of x and the fill of the ring (3.7 us a projection). Prefetching more than three K blocks into
+// L2 meanwhile makes it slower (1 row, four projections: 2 or 3 blocks 47.9, 5 49.7, 8 51.9 us).
+template <int NT, bool QUANT, typename OutT>
+__global__ void __launch_bounds__(SkinnyCfg<NT, QUANT>::kThreads, 2)
 block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const __grid_constant__ CUtensorMap tmap_x,
                              const SkinnyParams p) {
-  using Cfg = SkinnyCfg<NT>;
+  using Cfg = SkinnyCfg<NT, QUANT>;
   constexpr int S = Cfg::kStages;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -70,6 +77,8 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   auto tempty_bar = [&](int b) { return bar0 + 8u * (2 * S + NB + b); };
   volatile uint32_t* tmem_slot = reinterpret_cast<volatile uint32_t*>(bars + 2 * S + 2 * NB);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * S + 2 * NB + 1);
+  // QUANT: scales of K block j are in the table (used once, behind the sums of the other splits)
+  auto table_bar = [&](int j) { return bar0 + 256u + (uint32_t)Cfg::kSumBytes + 8u * j; };
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   constexpr int kProducerWarp = 4, kMmaWarp = 5;
@@ -81,10 +90,15 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   const int nt = item / (p.k_splits * p.t_tiles);
   const int kb0 = ks * p.kb_per_split, kb1 = min(p.num_kb, kb0 + p.kb_per_split);
   const int n0 = nt * 128, m0 = tt * NT;
+  // QUANT: rows that the 16 groups of eight lanes take side by side, 4 or 8; the other groups take the next K blocks. Four
+  // K blocks at most are under way: with more than the ring's stages a group would wait for a phase of a stage's barrier that is
+  // two ahead of it, which the parity does not tell from the one before.
+  const int rows = min(NT, p.M - m0);
+  const int q_rows = rows <= 4 ? 4 : 8;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
-      ptx::mbar_init(full_bar(s), 1);
+      ptx::mbar_init(full_bar(s), QUANT ? 1 + q_rows : 1);
       ptx::mbar_init(empty_bar(s), 1);
     }
     for (int b = 0; b < NB; ++b) {
@@ -94,13 +108,15 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     *abort_flag = 0;
     ptx::fence_mbar_init();
   }
+  // a thread each; only waited for within the CTA, so __syncthreads below is all they need
+  if (QUANT && threadIdx.x >= 32 && (int)threadIdx.x - 32 < kb1 - kb0) ptx::mbar_init(table_bar(threadIdx.x - 32), q_rows);
   if (warp == kMmaWarp) {
     ptx::tmem_alloc(ptx::smem_u32(const_cast<uint32_t*>(tmem_slot)), Cfg::kTmemCols);
     ptx::tmem_relinquish();
   }
   if (warp == kProducerWarp && lane == 0) {
     ptx::prefetch_tensormap(&tmap_w);
-    ptx::prefetch_tensormap(&tmap_x);
+    if (!QUANT) ptx::prefetch_tensormap(&tmap_x);
   }
   ptx::tc_fence_before();
   __syncthreads();
@@ -117,7 +133,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       prefetch_weight_row(p.w + (int64_t)(n0 + threadIdx.x) * p.K + kb0 * kBK, min(kPrefetchKb, kb1 - kb0));
     grid_dependency_wait();
     const float* bs_row = p.Bs + (int64_t)nt * p.num_kb;
-    for (int i = threadIdx.x; i < (kb1 - kb0) * NT; i += 128) {
+    for (int i = threadIdx.x; !QUANT && i < (kb1 - kb0) * NT; i += 128) {
       const int kb = kb0 + i / NT, t = i % NT;
       const int m = m0 + t;
       float s = 0.f;
@@ -132,7 +148,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       }
       scales[i] = s;
     }
-    asm volatile("bar.sync 1, 128;" ::: "memory");
+    if (!QUANT) asm volatile("bar.sync 1, 128;" ::: "memory");
   }
 
   float acc[NT];
@@ -146,9 +162,9 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
         const int s = it % S;
         ok = ptx::mbar_wait(empty_bar(s), ((it / S) & 1) ^ 1, abort_flag);
         if (!ok) break;
-        ptx::mbar_expect_tx(full_bar(s), Cfg::kStageW + Cfg::kStageX);
+        ptx::mbar_expect_tx(full_bar(s), Cfg::kStageW + (QUANT ? 0 : Cfg::kStageX));
         ptx::tma_load_2d(sW + s * Cfg::kStageW, &tmap_w, kb * kBK, n0, full_bar(s));
-        ptx::tma_load_2d(sX + s * Cfg::kStageX, &tmap_x, kb * kBK, m0, full_bar(s));
+        if (!QUANT) ptx::tma_load_2d(sX + s * Cfg::kStageX, &tmap_x, kb * kBK, m0, full_bar(s));
       }
     }
     __syncwarp();
@@ -173,6 +189,53 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
       }
     }
     __syncwarp();
+  } else if (QUANT && warp > kMmaWarp) {
+    if constexpr (QUANT) {
+      // Eight lanes hold the 128 values of one (row, K block), 16 each; the groups of a warp have the same K block.
+      static_assert(S >= 4, "the K blocks under way fit the ring");
+      const int tid = threadIdx.x - (kMmaWarp + 1) * 32, chunk = tid & 7, row = (tid >> 3) & (q_rows - 1);
+      const int step = 4 * Cfg::kQuantWarps / q_rows, first = (tid >> 3) / q_rows, nkb = kb1 - kb0;
+      const unsigned group = 0xffu << (lane & 24);
+      const OutT* src = static_cast<const OutT*>(p.x) + (int64_t)(m0 + min(row, rows - 1)) * p.K + (int64_t)kb0 * kBK + chunk * 16;
+      const float* bs = p.Bs + (int64_t)nt * p.num_kb + kb0;
+      constexpr int D = 4;  // K blocks in flight per group
+      uint4 raw[D][2];
+      float b[D];
+      auto request = [&](int j, int u) {
+        j = min(j, nkb - 1);
+        raw[u][0] = ld_nc_16(src + (int64_t)j * kBK);
+        raw[u][1] = ld_nc_16(src + (int64_t)j * kBK + 8);
+        b[u] = __ldg(bs + j);
+      };
+      grid_dependency_wait();
+#pragma unroll
+      for (int u = 0; u < D; ++u) request(first + u * step, u);
+      bool ok = true;
+      for (int j0 = 0; j0 < nkb; j0 += D * step) {
+#pragma unroll
+        for (int u = 0; u < D; ++u) {
+          if (j0 + u * step >= nkb) break;  // the same for the whole warp
+          const int j = j0 + u * step + first;
+          uint4 q;
+          const float scale = quant_chunk<OutT>(raw[u], p.eps, q) * b[u];
+          request(j + D * step, u);
+          if (j >= nkb) continue;
+          const int s = j % S;
+          ok = ok && ptx::mbar_wait(empty_bar(s), ((j / S) & 1) ^ 1, abort_flag);
+          if (ok && row < rows) {
+            const uint32_t dst = sX + s * Cfg::kStageX + (row >> 3) * 1024 + (row & 7) * 128 + ((chunk ^ (row & 7)) << 4);
+            asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(dst), "r"(q.x), "r"(q.y), "r"(q.z), "r"(q.w) : "memory");
+            if (chunk == 0) scales[j * NT + row] = scale;
+            ptx::fence_proxy_async_smem();  // generic-proxy writes -> the tensor core's reads
+          }
+          __syncwarp(group);
+          if (ok && chunk == 0) {
+            ptx::mbar_arrive(full_bar(s));
+            ptx::mbar_arrive(table_bar(j));
+          }
+        }
+      }
+    }
   } else {
     // promotion warps: lane = weight row, columns = tokens
     const int n = n0 + warp * 32 + lane;
@@ -184,6 +247,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     for (int kb = kb0; kb < kb1; ++kb, ++it) {
       const int b = it % NB;
       ok = ptx::mbar_wait(tfull_bar(b), (it / NB) & 1, abort_flag);
+      if (QUANT) ok = ok && ptx::mbar_wait(table_bar(kb - kb0), 0, abort_flag);
       if (!ok) break;
       ptx::tc_fence_after();
       uint32_t v[32];
@@ -225,7 +289,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
     if (Cfg::kSumBytes == 0) ptx::cluster_sync();  // every ring is idle
     // every split adds up its share of the rows: row t belongs to split t / per
-    const int rows = min(NT, p.M - m0), r = threadIdx.x & 127, per = (rows + p.k_splits - 1) / p.k_splits;
+    const int r = threadIdx.x & 127, per = (rows + p.k_splits - 1) / p.k_splits;
     const uint32_t sums_off = Cfg::kSumBytes ? (uint32_t)(reinterpret_cast<uint8_t*>(bars + 32) - smem_al) : 0u;
     if (warp < 4) {
       int owner = 0, j = 0;
@@ -299,18 +363,18 @@ inline int skinny_cluster(int64_t items, int64_t K, int nt, int want) {
   return c;
 }
 
-template <int NT, typename OutT>
+template <int NT, bool QUANT, typename OutT>
 inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, const SkinnyParams& p, cudaStream_t st) {
-  auto k = block_fp8_gemm_skinny_kernel<NT, OutT>;
-  const size_t smem = SkinnyCfg<NT>::kSmemBytes;
+  auto k = block_fp8_gemm_skinny_kernel<NT, QUANT, OutT>;
+  const size_t smem = SkinnyCfg<NT, QUANT>::kSmemBytes;
   if (int rc_smem = allow_smem(k, smem, "GEMM kernel")) return rc_smem;
   // programmatic dependent of the kernel before it (normally the activation quantiser, which
   // signals launch_dependents at once): set-up and the first weight prefetches overlap its tail
-  return launch_dependent(k, dim3((unsigned)(p.n_tiles * p.t_tiles * p.k_splits)), SkinnyCfg<NT>::kThreads, smem, st,
+  return launch_dependent(k, dim3((unsigned)(p.n_tiles * p.t_tiles * p.k_splits)), SkinnyCfg<NT, QUANT>::kThreads, smem, st,
                           p.cluster ? p.k_splits : 1, "block_fp8_gemm_skinny_kernel", tw, tx, p);
 }
 
-// out: OutT [M, N] when splits == 1 or they are a cluster, else fp32 partials [splits][M, N].
+// out: OutT [M, N] when splits == 1 or they are a cluster, else fp32 partials [splits][M, N]. p.x: quantise it (16 rows at most).
 template <typename OutT>
 inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int splits, bool cluster, cudaStream_t st) {
   const int nt = skinny_token_tile(p.M);
@@ -329,10 +393,13 @@ inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int split
   CUtensorMap tw, tx;
   int rc = make_tmap_u8(&tw, W, (uint64_t)p.N, (uint64_t)p.K, 128, "W");
   if (rc) return rc;
+  if constexpr (sizeof(OutT) == 2) {
+    if (p.x != nullptr) return launch_skinny_inst<16, true, OutT>(tw, tw, p, st);
+  }
   rc = make_tmap_u8(&tx, X, (uint64_t)p.M, (uint64_t)p.K, (uint32_t)nt, "X");
   if (rc) return rc;
-  if (nt == 16) return launch_skinny_inst<16, OutT>(tw, tx, p, st);
-  return launch_skinny_inst<32, OutT>(tw, tx, p, st);
+  if (nt == 16) return launch_skinny_inst<16, false, OutT>(tw, tx, p, st);
+  return launch_skinny_inst<32, false, OutT>(tw, tx, p, st);
 }
 
 }  // namespace b200

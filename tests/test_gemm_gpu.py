@@ -223,6 +223,30 @@ def test_one_launch_decode_linear(M, N, K, dtype):
     assert float((out.float() - two_step.float()).norm() / two_step.float().norm()) < 2e-3
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 3, 4, 5, 8, 9, 16])
+@pytest.mark.parametrize("N,K", [(6144, 4096), (28672, 4096), (4096, 14336), (8, 128), (1032, 384), (136, 8192 + 128), (1280, 8192)])
+def test_decode_linear_quantises_in_the_gemm(M, N, K, dtype):
+    """Up to 16 rows the decode GEMM quantises its own input: the same bytes, scales and order of the sums as quantiser and
+    GEMM on their own, so the same bits, also for calls that follow one another without a pause."""
+    import sglang_b200 as S
+    from sglang_b200._native import tuning
+
+    calls = []
+    for i in range(3):
+        wq, ws = make_weight(N, K, 2501 + N + i) if i == 0 or N * K < 1 << 22 else (calls[0][1].cpu(), calls[0][2].cpu())
+        calls.append((make_activation(M, K, 2500 + M + K + i, dtype=dtype).cuda(), wq.cuda(), ws.cuda()))
+    outs = [S.w8a8_block_fp8_linear(x, w, [128, 128], s) for x, w, s in calls for _ in range(2)]
+    with tuning(linear_decode_fused=0):
+        two = [S.w8a8_block_fp8_linear(x, w, [128, 128], s) for x, w, s in calls for _ in range(2)]
+    _status_ok()
+    for o, t in zip(outs, two):
+        if N * K < 16 << 20 and not torch.equal(o, t):  # small weights: one launch of the weight-streaming kernel, other splits
+            assert float((o.float() - t.float()).norm() / t.float().norm()) < 2e-3
+        else:
+            assert torch.equal(o, t)
+
+
 def test_one_launch_decode_linear_lends_no_operand_as_tickets(monkeypatch):
     """The ticket array is memory that the library may write: 4096 words of its own, not one of the operands."""
     from sglang_b200 import _native, fp8_kernel
