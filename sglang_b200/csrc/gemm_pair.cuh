@@ -21,6 +21,9 @@
 //   empty[s]  (each CTA)  arrival from the leader's tcgen05.commit
 //   tfull[b]  (each CTA)  likewise
 //   tempty[b] (leader's)  32 arrivals: the promotion warps of both CTAs
+// The MMA warp's own trip (two polls, four MMAs, two commits) bounds the 128-wide tile; both barriers are polled at once.
+// Shared memory is next: a K block writes 24 KB and reads 24 to 32 KB (128 wide), 375 to 440 clocks at 128 B/clk, against 430 measured.
+// Polled one after the other, and with 5 stages instead of 7: 203 x 8192 x 7168 20.8 -> 18.7 us, 512 x 4096 x 14336 35.0 -> 32.4.
 // Looped, with the copies (120 instructions per warp and K block) and without (97): 8192 x 4096 x 4096 143 -> 134 us,
 // 1027 x 7168 x 8192 78.6 -> 73.3, 203 x 6144 x 4096 (128-wide tiles) 15.1 -> 13.2.
 #pragma once
@@ -113,7 +116,6 @@ template <int CTAS, int BN>
 struct Wide {
   static constexpr int kStageA = kBM * kBK;       // this CTA's 128 rows of A
   static constexpr int kStageB = (BN / CTAS) * kBK;  // this CTA's share of the B tile
-  static constexpr int kStages = CTAS == 1 ? 3 : BN == 256 ? 4 : 5;
   static constexpr int kAccBufs = BN == 128 ? 4 : 2, kAccStride = BN == 128 ? 128 : 256;  // TMEM accumulator buffers
   static constexpr int kPromWarps = 16, kProducerWarp = 16, kMmaWarp = 17, kScaleWarp = 18;
   static constexpr int kCols = BN / 4, kChunks = kCols / 16;  // columns of one promotion warp, in 16-column chunks
@@ -121,12 +123,14 @@ struct Wide {
   // 20 warps start with 96 registers each (5 per sub-partition); 4 x 104 + 64 = 5 x 96
   static constexpr int kRegsPromotion = 104, kRegsOther = 64;
   static constexpr int kBoxBytes = 32 * kCols * 2;             // a warp's 32 rows of 16-bit output
-  static constexpr int kStagingBytes = 16 * 32 * 128;          // at most 128 bytes per row
+  static constexpr int kStagingBytes = 16 * kBoxBytes;
   static constexpr int kBlocks = BN == 128 ? 1 : 2;            // 128-column scale blocks a tile touches
   static constexpr int kScaleSlots = 2, kScaleSlotBytes = kBlocks * 128 * 16;  // blocks x rows x four K blocks
   static constexpr int kTmemCols = 512;
-  static constexpr size_t kSmemBytes =
-      (size_t)kStages * (kStageA + kStageB) + kStagingBytes + kScaleSlots * kScaleSlotBytes + 1024 + 256;
+  static constexpr int kFixed = kStagingBytes + kScaleSlots * kScaleSlotBytes + 1024 + 256;
+  // as many stages as fit: 3 (single CTAs), 4, 6 and 7 (pairs, 256 / 192 / 128 wide)
+  static constexpr int kFit = (232448 - kFixed) / (kStageA + kStageB), kStages = kFit < 8 ? kFit : 8;
+  static constexpr size_t kSmemBytes = (size_t)kStages * (kStageA + kStageB) + kFixed;
 };
 
 // OutT: 16-bit output [M, N], or fp32 (C + split * split_stride: partial sums of a K split, or an fp32 result)
@@ -248,19 +252,19 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     } else if (warp == Cfg::kMmaWarp) {
       if (leader && ptx::elect_one()) {  // ------------------------------------------ MMA issuer (leader only)
         constexpr uint32_t idesc = ptx::idesc_e4m3_f32(kRows, BN);
-        int s = 0;
+        const uint64_t da0 = ptx::smem_desc_sw128(sA), db0 = ptx::smem_desc_sw128(sB);
+        int s = 0, b = 0;
         uint32_t phase = 0, tphase = 1;
-        int b = 0;
         bool ok = true;
         for (int item = pair; item < total_items && ok; item += npairs) {
           const Item c = item_of(item);
-          for (int kb = c.kb0; kb < c.kb1; ++kb) {
-            // the accumulator buffer comes last of the two as a rule: nothing but its own wake-up in front of the MMAs
-            ok = ptx::mbar_wait(full_bar(s), phase, abort_flag) && ptx::mbar_wait(tempty_bar(b), tphase, abort_flag);
+#pragma unroll 1
+          for (int n = c.kb1 - c.kb0; n > 0; --n) {
+            ok = ptx::mbar_wait2(full_bar(s), phase, tempty_bar(b), tphase, abort_flag);
             if (!ok) break;
             ptx::tc_fence_after();
-            const uint64_t da = ptx::smem_desc_sw128(sA + s * Cfg::kStageA);
-            const uint64_t db = ptx::smem_desc_sw128(sB + s * Cfg::kStageB);
+            // a stage further = its bytes >> 4 in the address field, which does not overflow: shared memory ends below 2^18
+            const uint64_t da = da0 + (uint32_t)(s * (Cfg::kStageA >> 4)), db = db0 + (uint32_t)(s * (Cfg::kStageB >> 4));
             const uint32_t d = tmem_base + b * Cfg::kAccStride;
 #pragma unroll
             for (int k = 0; k < kBK / 32; ++k) ptx::wide_mma<CTAS>(d, da + 2 * k, db + 2 * k, idesc, k > 0);
