@@ -76,57 +76,70 @@ struct GemmPlan {
   int pair_bn;  // 0: single-CTA 128 x 256 tiles, else CTA pairs with 256 x pair_bn tiles
   bool skinny;  // swapped-operand decode kernel
   bool stream;  // weight-streaming kernel, token tiles of 64
+  bool csum;    // the K splits of a pair's tile are one cluster and summed there
   double us;    // modelled time (0: not modelled, decode sizes)
 };
 
-// Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up
-// (4.5 us), then whole waves of tiles: microseconds per 128-K block of a tile and 0.8 us for its epilogue; K splits add a
-// reduction pass (0.5 us and their fp32 partials, written and read at about 2 TB/s); nothing is faster than reading the
-// weights (6.2 TB/s). The decode kernel re-reads the weights for every 32 rows at the L2's 10.5 TB/s. The constants are
-// fits to measurements at 10 weight shapes (1280..28672 x 1024..14336) and 8 row counts (72..1027), where the plan is
-// within 10 % of the best configuration; what they decide is mostly wave counts, e.g. 203 x 6144 x 4096: single 22.3 us,
-// pair 256 wide 19.5, pair 128 wide 15.8; 1027 x 8192 x 3584: single 35.3, pair 44.3 and up.
+// Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up, then
+// whole waves of tiles, each its 128-K blocks and an epilogue; nothing is faster than reading the weights (6.2 TB/s). The decode
+// kernel re-reads the weights for every 32 rows at the L2's 9.5 TB/s. Where the tiles of 128-wide pairs leave half of the chip idle
+// their K range is split 2 or 4 ways within clusters, of which this part holds 33 and 15 at once; the sum costs 2 to 3 us. The
+// constants are fits to measurements at 16 weight shapes (1280..28672 x 1024..14336) and 17 row counts (33..2200), where the plan
+// is 0.3 % behind the best kernel on average; e.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, split in clusters
+// of 4 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
 static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair) {
   const Tuning& tune = tuning();
   const int64_t num_kb = cdiv(K, 128);
   const int64_t skinny_max = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
   const bool skinny_ok = may_pair && tune.gemm_skinny != 0;
-  if (may_pair && tune.gemm_stream > 0) return {1, 0, false, true, 0.0};
-  if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, 0.0};
-  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : tune.gemm_2cta == 2 ? 0 : (int)tune.gemm_2cta, false, false, 0.0};
-  GemmPlan best = {1, 0, false, false, 1e30};
+  if (may_pair && tune.gemm_stream > 0) return {1, 0, false, true, false, 0.0};
+  if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, false, 0.0};
+  if (may_pair && (tune.gemm_2cta == 1282 || tune.gemm_2cta == 1284) && N >= 256) return {(int)tune.gemm_2cta % 10, 128, false, false, true, 0.0};
+  if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : tune.gemm_2cta == 2 ? 0 : (int)tune.gemm_2cta, false, false, false, 0.0};
+  GemmPlan best = {1, 0, false, false, false, 1e30};
   const double stream_us = (double)N * (double)K / 6.2e6;
-  auto consider = [&](int bm, int bn, int slots, double us_per_kb, int pair_bn) {
+  auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int max_splits) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
-    for (int s = 1; s <= 8 && (s == 1 || num_kb >= 4 * s); ++s) {
+    for (int s = 1; s <= max_splits && (s == 1 || num_kb >= 4 * s); ++s) {
       const double waves = (double)cdiv(tiles * s, slots);
-      double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + 0.8);
+      double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + epilogue);
       if (work < stream_us) work = stream_us;
-      const double us = 4.5 + work + (s > 1 ? 0.5 + 16.0 * s * (double)M * (double)N / 4e6 : 0.0);
-      if (us < best.us) best = {s, pair_bn, false, false, us};
+      // through memory: a reduction pass and the fp32 partials, written and read at about 2 TB/s
+      const double us = base + work + (s > 1 ? 0.5 + 16.0 * s * (double)M * (double)N / 4e6 : 0.0);
+      if (us < best.us) best = {s, pair_bn, false, false, false, us};
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
-  consider(128, N > 128 ? 256 : 128, sms, 0.51, 0);
-  if (may_pair && tune.gemm_2cta != 0 && N >= 256) {
-    consider(256, 256, sms / 2, 0.47, 256);
-    consider(256, 192, sms / 2, 0.44, 192);
-    consider(256, 128, sms / 2, 0.34, 128);
+  const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256;
+  consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, pairs ? 1 : 8);
+  if (pairs) {
+    consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1);
+    consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, 1);
+    consider(256, 128, sms / 2, 4.25, 0.22, 0.8, 128, 1);
+    const int64_t tiles = cdiv(M, 256) * cdiv(N, 128);
+    for (int s = 2; s <= 4; s += 2) {
+      if (sms < 148 || tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
+      double work = (double)cdiv(num_kb, s) * (s == 2 ? 0.21 : 0.18);
+      if (work < stream_us) work = stream_us;
+      const double us = (s == 2 ? 6.5 : 7.75) + work;
+      if (us < best.us) best = {s, 128, false, false, true, us};
+    }
   }
   if (may_pair && tune.gemm_stream != 0 && M > 32 && M <= 128) {
     int csize, kb, stages, own;
     if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own)) {
-      // 0.49 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more
+      // 0.44 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more, and clusters fill 132 SMs
+      // at most (80 x 6144 x 4096 in clusters of 3: 24.8 us, two waves)
       const int64_t items = cdiv(N, 256) * cdiv(M, 64);
-      double work = (double)cdiv(items * csize, sms) * kb * 0.49;
+      double work = (double)cdiv(items * csize, csize > 1 ? sms - 16 : sms) * kb * 0.44;
       if (work < (double)N * (double)K / 6.4e6) work = (double)N * (double)K / 6.4e6;
-      const double us = 6.0 + (csize > 1 ? 1.0 : 0.0) + work;
-      if (us < best.us) best = {1, 0, false, true, us};
+      const double us = 7.5 + (csize > 1 ? 1.0 : 0.0) + work;
+      if (us < best.us) best = {1, 0, false, true, false, us};
     }
   }
-  const double skinny_us = 4.5 + (double)cdiv(M, 32) * (double)N * (double)K / 10.5e6;
+  const double skinny_us = 5.0 + (double)cdiv(M, 32) * (double)N * (double)K / 9.5e6;
   if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM) && skinny_us < best.us)
-    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, skinny_us};
+    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, false, skinny_us};
   return best;
 }
 }
@@ -225,6 +238,11 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
   const int bn = plan.pair_bn;
   // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
   const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
+  if (plan.csum && wide && fan.n == 0 && tune.gemm_splitk <= 0) {
+    if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, splits, true, st);
+    if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, splits, true, st);
+    return launch_gemm_wide<float>(bn, A, B, p, splits, true, st);
+  }
   if (splits > 1) {
     // few tiles: fp32 partials per K split in the workspace, then one reduction pass
     const size_t need = (size_t)splits * (size_t)M * (size_t)N * sizeof(float);
@@ -235,7 +253,7 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     p.C = workspace;
     p.split_stride = M * N;
     p.n_dest = 0;  // the partials stay local; the reduction pass fans the sum out
-    int rc = wide ? launch_gemm_wide<float>(bn, A, B, p, splits, st)
+    int rc = wide ? launch_gemm_wide<float>(bn, A, B, p, splits, false, st)
                   : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, splits);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
@@ -244,9 +262,9 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
   if (wide && fan.n == 0) {
-    if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, 1, st);
-    if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, 1, st);
-    return launch_gemm_wide<float>(bn, A, B, p, 1, st);
+    if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, 1, false, st);
+    if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, 1, false, st);
+    return launch_gemm_wide<float>(bn, A, B, p, 1, false, st);
   }
   switch (c_dtype) {
     case B200_BF16: return launch_gemm<GEMM_DENSE, __nv_bfloat16>(A, B, N, p, force_bn, st);
@@ -381,12 +399,12 @@ extern "C" int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, con
 }
 
 namespace b200 {
-// Modelled time of the block-scaled kernels (see plan_gemm): a 128-K block takes about 0.36 us for a CTA's 128 x 224 tile
-// and for a pair's 256 x 240 one, so the pair does twice the work per SM clock where whole waves allow it (3000 x 4096 x
-// 14336: 2759 against 2244 TFLOP/s; 1027 x 7168 x 8192, three waves instead of two: 1849 against 2288).
+// Modelled time of the block-scaled kernels (see plan_gemm; fitted to 14 weight shapes x 12 row counts, 70..3000): a CTA's 128 x 224
+// tile takes 0.38 us per 128-K block, a pair's 256 x 240 one 0.34, so the pair does twice the work per SM clock where whole waves
+// allow it (3000 x 4096 x 14336: 2759 against 2244 TFLOP/s); it starts 2 us later (400 x 8192 x 1024: single 8.1 us, pair 9.8).
 static double block_scaled_us(int64_t M, int64_t N, int64_t K, int sms, bool pair) {
   const int64_t tiles = pair ? cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN) : cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN);
-  return 4.5 + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * 0.36 + 0.3) * (pair ? 0.97 : 1.0);
+  return (pair ? 6.0 : 4.0) + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * (pair ? 0.34 : 0.38) + 1.2);
 }
 }  // namespace b200
 
@@ -452,12 +470,14 @@ __global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __res
 }
 
 // Whether the block-scaled kernels (scales applied by the tensor core, no K split) beat the promotion kernels on unpacked
-// scales: below 65 rows the weight stream decides, then wave counts (unpacking takes 2 us).
+// scales: below 65 rows the weight stream decides, then wave counts. Unpacking takes 2.5 us, and long problems run at the power
+// cap, where applying scales in the tensor core pays beyond the model (1500 x 4096 x 14336: 75.7 us against 85.5). With this margin
+// the choice is 0.2 % behind the best on those sizes (203 x 4096 x 14336: 46 us block-scaled, 25 promoted).
 static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
   if (tuning().gemm_ue8m0 > 0) return true;
   if (M <= 64) return false;
   const double one = block_scaled_us(M, N, K, sms, false), two = block_scaled_us(M, N, K, sms, true);
-  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true).us + 2.0;
+  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true).us * 1.08 + 3.0;
 }
 static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
 static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }

@@ -55,6 +55,7 @@ struct GemmParams {
   const float* As;  // A scales: As[m*as_sm + kb*as_sk]
   int64_t as_sm, as_sk;
   const float* Bs;  // [experts][n_blocks][num_kb]
+  const uint8_t* w;  // the weights B, for prefetches (16-warp kernel)
   void* C;
   int64_t ldc;     // elements
   int M, N, K;     // M = rows of A (grouped: capacity of the sorted layout)

@@ -102,6 +102,17 @@ __device__ __forceinline__ void tmem_ld_wait_all() { asm volatile("tcgen05.wait:
 __device__ __forceinline__ void ffma2(uint64_t& a, uint32_t b0, uint32_t b1, uint64_t s) {
   asm volatile("{.reg .b64 b; mov.b64 b, {%1, %2}; fma.rn.f32x2 %0, b, %3, %0;}" : "+l"(a) : "r"(b0), "r"(b1), "l"(s));
 }
+__device__ __forceinline__ uint64_t fadd2(uint64_t a, uint64_t b) {
+  uint64_t p;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(p) : "l"(a), "l"(b));
+  return p;
+}
+__device__ __forceinline__ void st_cluster_2x64(uint32_t addr, uint64_t a, uint64_t b) {
+  asm volatile("st.shared::cluster.v2.b64 [%0], {%1, %2};" ::"r"(addr), "l"(a), "l"(b) : "memory");
+}
+__device__ __forceinline__ void lds_2x64(uint32_t addr, uint64_t& a, uint64_t& b) {
+  asm volatile("ld.shared.v2.b64 {%0, %1}, [%2];" : "=l"(a), "=l"(b) : "r"(addr) : "memory");
+}
 __device__ __forceinline__ uint64_t pack2(float v) {
   uint64_t p;
   asm("mov.b64 %0, {%1, %1};" : "=l"(p) : "f"(v));
@@ -133,12 +144,28 @@ struct Wide {
   static constexpr size_t kSmemBytes = (size_t)kStages * (kStageA + kStageB) + kFixed;
 };
 
+// The weights that CTA `rank` of pair `pair` loads first, a row per thread.
+template <int CTAS, int BN>
+__device__ __forceinline__ void prefetch_first_weights(const GemmParams& p, int pair, int rank) {
+  const int t = fast_div(pair, p.k_splits_div), ks = pair - t * p.k_splits, kb0 = ks * p.kb_per_split;
+  int mt, nt;
+  tile_coords(t, p.m_tiles, p.n_tiles, p.group_m, p.per_group_div, mt, nt);
+  const int row = nt * BN + rank * (BN / CTAS) + (int)threadIdx.x;
+  if (t < p.m_tiles * p.n_tiles && row < p.N)
+    prefetch_weight_row(p.w + (int64_t)row * p.K + (int64_t)kb0 * kBK, min(kPrefetchKb, min(p.num_kb, kb0 + p.kb_per_split) - kb0));
+}
+
 // OutT: 16-bit output [M, N], or fp32 (C + split * split_stride: partial sums of a K split, or an fp32 result)
-template <int CTAS, int BN, typename OutT>
-__global__ void __cluster_dims__(CTAS, 1, 1) __launch_bounds__(Wide<CTAS, BN>::kThreads, 1)
+// CS > 0: the K splits of a tile, CS of them (2 or 4), are one cluster. Each of them sums and stores its share of the columns; the
+// others hand theirs over through distributed shared memory, in the ring, which is idle by then. 64 KB move at most per CTA, and no
+// fp32 partials in memory nor a reduction launch: 203 x 4096 x 4096 12.5 us unsplit -> 10.3 with 2 splits, 203 x 4096 x 14336 24.5
+// with partials in memory -> 19.7.
+template <int CTAS, int BN, int CS, typename OutT>
+__global__ void __cluster_dims__(CTAS * (CS ? CS : 1), 1, 1) __launch_bounds__(Wide<CTAS, BN>::kThreads, 1)
 block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_constant__ CUtensorMap tmap_b,
                            const __grid_constant__ CUtensorMap tmap_c, const GemmParams p) {
   using Cfg = Wide<CTAS, BN>;
+  constexpr bool CSUM = CS > 0;
   constexpr int S = Cfg::kStages, NB = Cfg::kAccBufs, SQ = Cfg::kScaleSlots, kRows = CTAS * kBM;
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (ptx::smem_u32(smem_raw) + 1023u) & ~1023u;
@@ -159,7 +186,9 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
   volatile int* abort_flag = reinterpret_cast<volatile int*>(bars + 2 * S + 2 * NB + 2 * SQ + 1);
 
   const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
-  const uint32_t rank = CTAS == 2 ? ptx::cluster_ctarank() : 0;
+  const uint32_t cluster_rank = CTAS == 2 || CSUM ? ptx::cluster_ctarank() : 0;
+  // rank in the pair, and the pair's leader in the cluster (a constant where it can be one: it is on the MMA warp's trip)
+  const uint32_t rank = CSUM ? cluster_rank & (CTAS - 1) : cluster_rank, leader_rank = CSUM ? cluster_rank - rank : 0u;
   const bool leader = rank == 0;
 
   if (threadIdx.x == 0) {
@@ -194,10 +223,13 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     ptx::prefetch_tensormap(&tmap_c);
   }
   ptx::tc_fence_before();
-  ptx::wide_sync<CTAS>();  // the peer's barriers are initialised before anything signals them
+  ptx::wide_sync<CSUM ? 2 : CTAS>();  // the peer's barriers are initialised before anything signals them
   ptx::tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
   grid_launch_dependents();
+  // What is read and overwritten below belongs to the kernels before, which may still run; the weights of the first K blocks are
+  // asked for all the same, as a prefetch into L2, a row each.
+  if (warp < Cfg::kPromWarps && (int)threadIdx.x < BN / CTAS) prefetch_first_weights<CTAS, BN>(p, blockIdx.x / CTAS, (int)rank);
   grid_dependency_wait();
 
   const int S_k = p.k_splits;
@@ -232,7 +264,7 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
             if (!ok) break;
             uint32_t lf = full_bar(s);
             if constexpr (CTAS == 2) {
-              lf = ptx::mapa(lf, 0);
+              lf = ptx::mapa(lf, leader_rank);
               ptx::mbar_expect_tx_cluster(lf, Cfg::kStageA + Cfg::kStageB);
             } else {
               ptx::mbar_expect_tx(lf, Cfg::kStageA + Cfg::kStageB);
@@ -269,8 +301,8 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
 #pragma unroll
             for (int k = 0; k < kBK / 32; ++k) ptx::wide_mma<CTAS>(d, da + 2 * k, db + 2 * k, idesc, k > 0);
             if constexpr (CTAS == 2) {
-              ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)3);
-              ptx::mma_commit_pair_multicast(empty_bar(s), (uint16_t)3);
+              ptx::mma_commit_pair_multicast(tfull_bar(b), (uint16_t)(3u << leader_rank));
+              ptx::mma_commit_pair_multicast(empty_bar(s), (uint16_t)(3u << leader_rank));
             } else {
               ptx::mma_commit(tfull_bar(b));
               ptx::mma_commit(empty_bar(s));
@@ -327,7 +359,7 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     constexpr int kCols = Cfg::kCols, CH = Cfg::kChunks;
     const uint32_t lane_base = tmem_base + ((uint32_t)(quarter * 32) << 16) + colq * kCols;
     const uint32_t my_scales = ptx::smem_u32(scales) + (quarter * 32 + lane) * 16;
-    const uint32_t leader_tempty = CTAS == 2 ? ptx::mapa(tempty_bar(0), 0) : tempty_bar(0);
+    const uint32_t leader_tempty = CTAS == 2 ? ptx::mapa(tempty_bar(0), leader_rank) : tempty_bar(0);
     uint32_t tphase = 0, sphase = 0;
     int q = 0, b = 0;
     bool ok = true;
@@ -383,11 +415,51 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
         if (ptx::elect_one()) ptx::mbar_arrive(sempty_bar(q));
         if (++q == SQ) q = 0, sphase ^= 1;
       }
-      if (!ok) break;
-
-      // ------------------------------------------------------------------------ tile epilogue
+      if (!CSUM && !ok) break;
       const uint32_t wstage = staging + warp * Cfg::kBoxBytes;
       const int row0 = c.mt * kRows + (int)rank * kBM + quarter * 32, col0 = c.nt * BN + colq * kCols;
+      if constexpr (CSUM) {  // the only item of this CTA; a warp whose wait gave up takes part all the same
+        constexpr int G = kCols / 8;  // groups of 8 columns; split s owns G / S_k of them
+        constexpr int per = G / (CSUM ? CS : 1);
+        const int me = c.ks;
+        __syncwarp();
+        ptx::cluster_sync();  // every ring is idle
+        auto slot = [&](uint32_t base, int src, int g, int half) {
+          return base + (uint32_t)(((src * per + g % per) * 2 + half) * Cfg::kPromWarps * 32 + (int)threadIdx.x) * 16;
+        };
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          const int owner = g / per;
+          if (owner == me) continue;
+          const uint32_t base = ptx::mapa(smem_base, (uint32_t)owner * CTAS + rank);
+          ptx::st_cluster_2x64(slot(base, me, g, 0), acc[4 * g], acc[4 * g + 1]);
+          ptx::st_cluster_2x64(slot(base, me, g, 1), acc[4 * g + 2], acc[4 * g + 3]);
+        }
+        __syncwarp();
+        ptx::cluster_sync();
+#pragma unroll
+        for (int g = 0; g < G; ++g) {
+          if (g / per != me) continue;
+          uint64_t sum[4] = {0, 0, 0, 0};
+          for (int src = 0; src < CS; ++src) {  // split order: the same sum on every run
+            uint64_t v[4] = {acc[4 * g], acc[4 * g + 1], acc[4 * g + 2], acc[4 * g + 3]};
+            if (src != me) {
+              ptx::lds_2x64(slot(smem_base, src, g, 0), v[0], v[1]);
+              ptx::lds_2x64(slot(smem_base, src, g, 1), v[2], v[3]);
+            }
+#pragma unroll
+            for (int i = 0; i < 4; ++i) sum[i] = ptx::fadd2(sum[i], v[i]);
+          }
+          float t[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) t[i] = __uint_as_float((uint32_t)(sum[i / 2] >> (32 * (i & 1))));
+          if (ok && row0 + lane < p.M && col0 + g * 8 < p.N)
+            store8<OutT>(static_cast<OutT*>(p.C) + (int64_t)(row0 + lane) * p.ldc + col0 + g * 8, t);
+        }
+        break;
+      }
+
+      // ------------------------------------------------------------------------ tile epilogue
       if constexpr (sizeof(OutT) == 2) {
         if (lane == 0) ptx::tma_store_wait_read();  // the last tile's box has left the staging area
         __syncwarp();
@@ -423,6 +495,11 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     }
     if (sizeof(OutT) == 2 && lane == 0) ptx::tma_store_wait_all();
   }
+  if (CSUM && warp >= Cfg::kPromWarps) {  // the other warps' share of the two cluster barriers above
+    __syncwarp();
+    ptx::cluster_sync();
+    ptx::cluster_sync();
+  }
 
   // ---------------------------------------------------------------------- teardown
   if (*abort_flag) {
@@ -430,7 +507,7 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
     while (ptx::globaltimer_ns() - t0 < 2000000ull) __nanosleep(1000);
   }
   ptx::tc_fence_before();
-  ptx::wide_sync<CTAS>();  // neither CTA leaves while the other may still signal its barriers or use its smem
+  ptx::wide_sync<CSUM ? 2 : CTAS>();  // neither CTA leaves while the other may still signal its barriers or use its smem
   if (threadIdx.x == 0 && *abort_flag) atomicCAS(p.status, 0, 1);
   if (warp == Cfg::kMmaWarp) {
     ptx::tc_fence_after();
@@ -440,7 +517,7 @@ block_fp8_gemm_wide_kernel(const __grid_constant__ CUtensorMap tmap_a, const __g
 }
 
 // p.M/N/K/As/Bs/C/ldc (and split_stride) filled by the caller.
-template <int CTAS, int BN, typename OutT>
+template <int CTAS, int BN, int CS, typename OutT>
 inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_splits, cudaStream_t st) {
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_blocks = (int)cdiv(p.N, 128);
@@ -451,6 +528,7 @@ inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_sp
   p.kb_per_split = (int)cdiv(p.num_kb, k_splits);
   p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);
   p.k_splits_div = make_fastdiv(p.k_splits);
+  p.w = static_cast<const uint8_t*>(B);
   p.status = device_status_word();
   if (!p.status) {
     set_error_detail("cannot resolve the device status word");
@@ -459,29 +537,30 @@ inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_sp
   const int64_t items = (int64_t)p.m_tiles * p.n_tiles * p.k_splits;
   if (items == 0) return B200_OK;
   const int slots = sm_count() / CTAS;
-  const int units = (int)(items < slots ? items : slots);
+  const int units = (int)(CS > 0 || items < slots ? items : slots);
   CUtensorMap ta, tb, tc;
   int rc = make_tmap_u8(&ta, A, (uint64_t)p.M, (uint64_t)p.K, kBM, "A");
   if (rc) return rc;
   rc = make_tmap_u8(&tb, B, (uint64_t)p.N, (uint64_t)p.K, BN / CTAS, "B");
   if (rc) return rc;
   tc = ta;
-  if (sizeof(OutT) == 2) {
+  if (sizeof(OutT) == 2 && CS == 0) {
     rc = make_tmap_out(&tc, p.C, 1, (uint64_t)p.M, (uint64_t)p.N, 2, std::is_same<OutT, __nv_bfloat16>::value, "C", BN / 4);
     if (rc) return rc;
   }
-  auto k = block_fp8_gemm_wide_kernel<CTAS, BN, OutT>;
+  auto k = block_fp8_gemm_wide_kernel<CTAS, BN, CS, OutT>;
   if (int rc_smem = allow_smem(k, Wide<CTAS, BN>::kSmemBytes, "block_fp8_gemm_wide_kernel")) return rc_smem;
   return launch_dependent(k, dim3((unsigned)(CTAS * units)), Wide<CTAS, BN>::kThreads, Wide<CTAS, BN>::kSmemBytes, st, 1,
                           "block_fp8_gemm_wide_kernel", ta, tb, tc, p);
 }
-// bn: columns of a pair's tile, or 0: single CTAs
+// bn: columns of a pair's tile, or 0: single CTAs. csum: the K splits (2 or 4) are summed within clusters (128-wide pairs).
 template <typename OutT>
-inline int launch_gemm_wide(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, cudaStream_t st) {
-  if (bn == 0) return launch_gemm_wide<1, 256, OutT>(A, B, p, k_splits, st);
-  if (bn == 128) return launch_gemm_wide<2, 128, OutT>(A, B, p, k_splits, st);
-  if (bn == 192) return launch_gemm_wide<2, 192, OutT>(A, B, p, k_splits, st);
-  return launch_gemm_wide<2, 256, OutT>(A, B, p, k_splits, st);
+inline int launch_gemm_wide(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, bool csum, cudaStream_t st) {
+  if (csum) return k_splits == 2 ? launch_gemm_wide<2, 128, 2, OutT>(A, B, p, 2, st) : launch_gemm_wide<2, 128, 4, OutT>(A, B, p, 4, st);
+  if (bn == 0) return launch_gemm_wide<1, 256, 0, OutT>(A, B, p, k_splits, st);
+  if (bn == 128) return launch_gemm_wide<2, 128, 0, OutT>(A, B, p, k_splits, st);
+  if (bn == 192) return launch_gemm_wide<2, 192, 0, OutT>(A, B, p, k_splits, st);
+  return launch_gemm_wide<2, 256, 0, OutT>(A, B, p, k_splits, st);
 }
 
 }  // namespace b200

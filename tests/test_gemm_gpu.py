@@ -340,6 +340,28 @@ def test_cta_pair_widths(M, N, K, bn, splitk):
             _case(M, N, K, 900 + M, out_dtype=dt, col_major=True)
 
 
+@pytest.mark.parametrize("out_dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("knob", [1282, 1284])
+@pytest.mark.parametrize("M,N,K", [(1, 256, 128), (33, 264, 640), (129, 1288, 2048 + 16), (203, 4096, 1024), (256, 384, 8192), (300, 640, 1920)])
+def test_k_splits_summed_in_clusters(M, N, K, knob, out_dtype):
+    """CTA pairs whose K splits are one cluster: an empty last split, ragged rows and columns, whole row quarters behind the last row;
+    fp32 against the oracle to 1e-5 (only the order of the sums differs), and twice the same."""
+    import sglang_b200 as S
+    from sglang_b200._native import tuning
+
+    A, B = _rand_fp8((M, K), 61 + M), _rand_fp8((N, K), 62 + N)
+    g = torch.Generator().manual_seed(63)
+    kt, nt = (K + 127) // 128, (N + 127) // 128
+    As, Bs = torch.rand(M, kt, generator=g) * 1e-2, torch.rand(nt, kt, generator=g) * 1e-2
+    args = A.cuda(), B.cuda(), As.t().contiguous().cuda().t(), Bs.cuda(), [128, 128], out_dtype
+    with tuning(gemm_2cta=knob, gemm_skinny=0):
+        C, again = S.w8a8_block_fp8_matmul(*args), S.w8a8_block_fp8_matmul(*args)
+    _status_ok()
+    assert torch.equal(C, again)
+    ref = O.w8a8_block_fp8_matmul(A, B, As, Bs, [128, 128], torch.float32)
+    assert O.rel_frobenius(C.float().cpu(), ref) < (1e-5 if out_dtype == torch.float32 else TOL)
+
+
 @pytest.mark.parametrize("M,N,K", [(1, 8, 128), (33, 256, 1408), (64, 1032, 4096), (65, 392, 528), (130, 7168, 2048),
                                    (64, 45056, 256)])
 def test_dense_weight_streaming_kernel(M, N, K):
