@@ -523,7 +523,7 @@ inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_sp
   p.n_blocks = (int)cdiv(p.N, 128);
   p.n_tiles = (int)cdiv(p.N, BN);
   p.m_tiles = (int)cdiv(p.M, CTAS * kBM);
-  p.group_m = 16 / CTAS;  // 2048 rows swept per column tile
+  p.group_m = row_group(p.M, p.K, CTAS * kBM);
   p.k_splits = k_splits;
   p.kb_per_split = (int)cdiv(p.num_kb, k_splits);
   p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);

@@ -307,7 +307,7 @@ inline int launch_gemm_ue8m0(const void* A, const void* B, Ue8m0Params p, cudaSt
   p.num_kb = (int)cdiv(p.K, kBK);
   p.m_tiles = (int)cdiv(p.M, kBM);
   p.n_tiles = (int)cdiv(p.N, Ue8m0Cfg::BN);
-  p.group_m = 16;
+  p.group_m = row_group(p.M, p.K, kBM);
   p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);
   p.status = device_status_word();
   if (!p.status) {

@@ -279,7 +279,7 @@ inline int launch_gemm_ue8m0_pair(const void* A, const void* B, Ue8m0Params p, c
   p.num_kb = (int)cdiv(p.K, kBK);
   p.m_tiles = (int)cdiv(p.M, 2 * kBM);
   p.n_tiles = (int)cdiv(p.N, Cfg::BN);
-  p.group_m = 8;
+  p.group_m = row_group(p.M, p.K, 2 * kBM);
   p.per_group_div = make_fastdiv(p.group_m * p.n_tiles);
   p.status = device_status_word();
   if (!p.status) {
