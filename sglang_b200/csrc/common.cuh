@@ -136,6 +136,26 @@ __device__ __forceinline__ __nv_bfloat16 from_f32<__nv_bfloat16>(float v) { retu
 template <>
 __device__ __forceinline__ __half from_f32<__half>(float v) { return __float2half_rn(v); }
 
+// Division by a divisor fixed at launch as a multiply-high and a shift (exact for 0 <= n < 2^31): the 32-bit
+// integer division of the hardware is a ~25-instruction dependent chain, and three of them in a row sat on the
+// critical path between two tiles of the promotion warps.
+struct FastDiv {
+  uint32_t mul, shr;
+};
+inline FastDiv make_fastdiv(int d) {
+  FastDiv f = {0u, 0u};
+  if (d <= 1) return f;  // mul == 0 marks "divide by one"
+  int l = 0;
+  while ((1ll << l) < d) ++l;  // ceil(log2 d)
+  const int p = 31 + l;
+  f.mul = (uint32_t)(((1ull << p) + (uint64_t)d - 1) / (uint64_t)d);
+  f.shr = (uint32_t)(p - 32);
+  return f;
+}
+__device__ __forceinline__ int fast_div(int n, FastDiv f) {
+  return f.mul == 0u ? n : (int)(__umulhi((uint32_t)n, f.mul) >> f.shr);
+}
+
 // 16-byte read-only global load (bypasses L1 allocation: streamed once).
 __device__ __forceinline__ uint4 ld_nc_16(const void* p) {
   uint4 v;

@@ -31,26 +31,6 @@ namespace b200 {
 
 enum { GEMM_DENSE = 0, GEMM_GROUPED_SILU_QUANT = 1, GEMM_GROUPED_SCATTER = 2 };
 
-// Division by a divisor fixed at launch as a multiply-high and a shift (exact for 0 <= n < 2^31): the 32-bit
-// integer division of the hardware is a ~25-instruction dependent chain, and three of them in a row sat on the
-// critical path between two tiles of the promotion warps.
-struct FastDiv {
-  uint32_t mul, shr;
-};
-inline FastDiv make_fastdiv(int d) {
-  FastDiv f = {0u, 0u};
-  if (d <= 1) return f;  // mul == 0 marks "divide by one"
-  int l = 0;
-  while ((1ll << l) < d) ++l;  // ceil(log2 d)
-  const int p = 31 + l;
-  f.mul = (uint32_t)(((1ull << p) + (uint64_t)d - 1) / (uint64_t)d);
-  f.shr = (uint32_t)(p - 32);
-  return f;
-}
-__device__ __forceinline__ int fast_div(int n, FastDiv f) {
-  return f.mul == 0u ? n : (int)(__umulhi((uint32_t)n, f.mul) >> f.shr);
-}
-
 struct GemmParams {
   const float* As;  // A scales: As[m*as_sm + kb*as_sk]
   int64_t as_sm, as_sk;

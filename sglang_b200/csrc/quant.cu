@@ -7,10 +7,12 @@
 
 namespace b200 {
 
+// Row of a chunk by a multiplication: the division of 64-bit numbers was a good part of the instructions (8192 x 14336 bf16
+// 66.0 -> 63.2 us, 203 x 4096 2.03 -> 1.95). Two chunks per thread, both loaded ahead, are slower (78 us).
 template <typename T, int LPG, int FORMULA>
 __global__ void __launch_bounds__(256) quant_group_kernel(const T* __restrict__ x, uint8_t* __restrict__ q,
                                                           float* __restrict__ s, int64_t total_chunks,
-                                                          int chunks_per_row, int64_t s_stride_m,
+                                                          int chunks_per_row, FastDiv row_div, int64_t s_stride_m,
                                                           int64_t s_stride_g, float eps, int early) {
   const int64_t c = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const bool active = c < total_chunks;  // whole lane-groups are active or not (total % LPG == 0)
@@ -34,7 +36,7 @@ __global__ void __launch_bounds__(256) quant_group_kernel(const T* __restrict__ 
   if (active) {
     *reinterpret_cast<uint4*>(q + c * 16) = out;
     if ((threadIdx.x & (LPG - 1)) == 0) {
-      const int64_t row = c / chunks_per_row;
+      const int64_t row = total_chunks < (1ll << 31) ? fast_div((int)c, row_div) : c / chunks_per_row;
       const int g = (int)(c - row * chunks_per_row) / LPG;
       s[row * s_stride_m + g * s_stride_g] = scale;
     }
@@ -55,7 +57,7 @@ static int launch_quant(const void* x, void* q, float* s, int64_t M, int64_t K, 
   const int cpr = (int)(K / 16);
 #define B200_Q_LAUNCH_F(LPG, F)                                                                                            \
   return launch_dependent(quant_group_kernel<T, LPG, F>, dim3((unsigned)blocks), threads, 0, st, 1, "per_token_group_quant_fp8", \
-                          static_cast<const T*>(x), static_cast<uint8_t*>(q), s, total, cpr, ssm, ssg, eps, 0)
+                          static_cast<const T*>(x), static_cast<uint8_t*>(q), s, total, cpr, make_fastdiv(cpr), ssm, ssg, eps, 0)
 #define B200_Q_LAUNCH(LPG)                                                        \
   switch (formula) {                                                              \
     case B200_QUANT_RECIP: B200_Q_LAUNCH_F(LPG, B200_QUANT_RECIP);                \
@@ -83,7 +85,7 @@ static int launch_quant_for_linear(const void* x, void* q, float* s, int64_t M, 
   const int64_t total = M * (K / 16);
   return launch_dependent(quant_group_kernel<T, 8, B200_QUANT_DIV_CORRECTED>, dim3((unsigned)cdiv(total, 256)), 256, 0, st, 1,
                           "per_token_group_quant_fp8", static_cast<const T*>(x), static_cast<uint8_t*>(q), s, total,
-                          (int)(K / 16), 1, M, 1e-10f, 1);
+                          (int)(K / 16), make_fastdiv((int)(K / 16)), 1, M, 1e-10f, 1);
 }
 
 int quant_for_linear(const void* x, int x_dtype, void* q, float* s, int64_t M, int64_t K, cudaStream_t st) {
