@@ -10,6 +10,7 @@ import importlib.util
 import os
 import threading
 from ctypes import c_char_p, c_float, c_int, c_int32, c_int64, c_long, c_size_t, c_uint32, c_void_p, POINTER
+from typing import NamedTuple
 
 import torch
 
@@ -25,6 +26,10 @@ SIGNATURES = {
     "b200_read_device_status": (c_int, [POINTER(c_int), c_void_p]),
     "b200_set_tuning": (c_int, [c_char_p, c_long]),
     "b200_get_tuning": (c_int, [c_char_p, POINTER(c_long)]),
+    "b200_plan_dense": (
+        c_int,
+        [c_int, c_int64, c_int64, c_int64, c_int, POINTER(c_int), POINTER(c_int), POINTER(c_int), POINTER(c_int)],
+    ),
     "b200_per_token_group_quant_fp8": (
         c_int,
         [c_void_p, c_int, c_void_p, c_void_p, c_int64, c_int64, c_int, c_int64, c_int64, c_float, c_int, c_void_p],
@@ -256,6 +261,26 @@ def get_tuning(name: str) -> int:
     v = c_long(0)
     check(load().b200_get_tuning(name.encode(), ctypes.byref(v)), "get_tuning")
     return v.value
+
+
+PLAN_ENTRIES = {"gemm": 0, "fanout": 1, "linear": 2}
+KERNELS = ("tile", "wide", "skinny", "stream", "skinny_quant", "stream_quant")
+SUMS = ("none", "memory", "cluster")
+
+
+class DensePlan(NamedTuple):
+    kernel: str  # one of KERNELS
+    tile_n: int
+    splits: int
+    sum: str  # one of SUMS
+
+
+def plan_dense(entry: str, M: int, N: int, K: int, sms: int = 0) -> DensePlan:
+    """The kernel that a dense call of this size takes (``b200_plan_dense``); sms = 0: on the current device."""
+    v = [c_int(0) for _ in range(4)]
+    check(load().b200_plan_dense(PLAN_ENTRIES[entry], M, N, K, sms, *map(ctypes.byref, v)), "plan_dense")
+    kernel, tile_n, splits, total = (x.value for x in v)
+    return DensePlan(KERNELS[kernel], tile_n, splits, SUMS[total])
 
 
 def read_device_status() -> int:

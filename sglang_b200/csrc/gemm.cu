@@ -80,6 +80,9 @@ struct GemmPlan {
   double us;    // modelled time (0: not modelled, decode sizes)
 };
 
+// SMs that plans are made for
+static int plan_sms() { return sm_count() < 148 ? sm_count() : 148; }
+
 // Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up, then
 // whole waves of tiles, each its 128-K blocks and an epilogue; nothing is faster than reading the weights (6.2 TB/s). The decode
 // kernel re-reads the weights for every 32 rows at the L2's 9.5 TB/s. Where the tiles of 128-wide pairs leave half of the chip idle
@@ -155,22 +158,56 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N,
 }
 
 namespace b200 {
-// The decode kernel (gemm_skinny.cuh) with its K split; sp holds the scales.
-// Whether run_skinny writes the result itself (no K split, or one summed within clusters), without partials in memory.
-static bool skinny_direct(int64_t M, int64_t N, int64_t K, int splits) {
-  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;
-  const int nt = skinny_token_tile(M);
-  return splits == 1 || (tuning().gemm_splitk <= 0 && skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) > 1);
-}
-static int run_skinny(const void* A, const void* B, SkinnyParams sp, int splits, void* C, int c_dtype, int64_t M, int64_t N,
-                      int64_t K, void* workspace, size_t workspace_bytes, cudaStream_t st, const FanOut& fan) {
+// K splits of the decode kernel (gemm_skinny.cuh) when `splits` are asked for, and whether they are summed within clusters.
+struct SkinnySplit {
+  int splits;
+  bool cluster;
+  bool direct() const { return splits == 1 || cluster; }  // the kernel writes the result itself, without partials in memory
+};
+static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
   while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;  // scales of one item fit its smem table
-  sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
-  // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
   const int nt = skinny_token_tile(M);
   const int cluster = splits > 1 && tuning().gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
-  if (cluster > 1) splits = cluster;
-  if (fan.n == 0 && (splits == 1 || cluster > 1)) {
+  return cluster > 1 ? SkinnySplit{cluster, true} : SkinnySplit{splits, false};
+}
+
+// What a dense problem runs: kernel, columns of its tile, K splits and where they are summed (the codes of b200_plan_dense).
+// gemm_impl and the linear layer launch it, b200_plan_dense reports it.
+struct GemmRoute {
+  int kernel, tile_n, splits, sum;
+};
+static GemmRoute skinny_route(int64_t M, int64_t N, int64_t K, int splits, bool fanout, int kernel) {
+  // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
+  const SkinnySplit s = skinny_split(M, N, K, splits);
+  return {kernel, 128, s.splits, s.direct() && !fanout ? (s.splits > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE) : B200_SUM_MEMORY};
+}
+static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, bool fanout) {
+  const Tuning& tune = tuning();
+  const int force_bn = tune.gemm_bn == 128 || tune.gemm_bn == 256 ? (int)tune.gemm_bn : 0;
+  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0);
+  int splits = plan.splits;
+  if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
+  if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
+  if (plan.stream && !fanout && tune.gemm_splitk <= 0) {
+    int csize = 1, kb, stages, own;
+    plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own);
+    return {B200_KERNEL_STREAM, 256, csize, csize > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE};
+  }
+  if (plan.skinny) return skinny_route(M, N, K, splits, fanout, B200_KERNEL_SKINNY);
+  // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
+  const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
+  if (plan.csum && wide && !fanout && tune.gemm_splitk <= 0) return {B200_KERNEL_WIDE, plan.pair_bn, splits, B200_SUM_CLUSTER};
+  const int sum = splits > 1 ? B200_SUM_MEMORY : B200_SUM_NONE;
+  if (wide && (splits > 1 || !fanout)) return {B200_KERNEL_WIDE, plan.pair_bn, splits, sum};
+  return {B200_KERNEL_TILE, force_bn, splits, sum};
+}
+
+// The decode kernel as skinny_route laid it out; sp holds the scales (or the input to quantise).
+static int run_skinny(const void* A, const void* B, SkinnyParams sp, const GemmRoute& r, void* C, int c_dtype, int64_t M, int64_t N,
+                      int64_t K, void* workspace, size_t workspace_bytes, cudaStream_t st, const FanOut& fan) {
+  sp.M = (int)M; sp.N = (int)N; sp.K = (int)K;
+  const int splits = r.splits;
+  if (r.sum != B200_SUM_MEMORY) {
     sp.C = C;
     if (c_dtype == B200_BF16) return launch_skinny<__nv_bfloat16>(A, B, sp, splits, splits > 1, st);
     if (c_dtype == B200_F16) return launch_skinny<__half>(A, B, sp, splits, splits > 1, st);
@@ -210,19 +247,12 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
   p.M = (int)M; p.N = (int)N; p.K = (int)K;
   p.n_dest = fan.n; p.dest_by_tile = fan.by_tile;
   for (int d = 0; d < fan.n; ++d) p.dest[d] = fan.dest[d];
-  const Tuning& tune = tuning();
-  const int force_bn = tune.gemm_bn == 128 || tune.gemm_bn == 256 ? (int)tune.gemm_bn : 0;
-
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   B200_CHECK_ARG(c_dtype == B200_BF16 || c_dtype == B200_F16 || c_dtype == B200_F32, "gemm: unknown output dtype code %d",
                  c_dtype);
-  const int sms = sm_count() < 148 ? sm_count() : 148;
-  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0);
-  const bool skinny = plan.skinny;
-  int splits = plan.splits;
-  if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
-  if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
-  if (plan.stream && fan.n == 0 && tune.gemm_splitk <= 0) {
+  const GemmRoute r = route_gemm(M, N, K, plan_sms(), fan.n > 0);
+  const int splits = r.splits, bn = r.tile_n;
+  if (r.kernel == B200_KERNEL_STREAM) {
     LinearStreamParams lp = {};
     lp.As = As; lp.as_sm = as_stride_m; lp.as_sk = as_stride_k; lp.Bs = Bs; lp.out = C;
     lp.M = (int)M; lp.N = (int)N; lp.K = (int)K;
@@ -230,15 +260,13 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     if (c_dtype == B200_F16) return launch_linear_stream<64, false, __half>(B, A, lp, st);
     return launch_linear_stream<64, false, float>(B, A, lp, st);
   }
-  if (skinny) {
+  if (r.kernel == B200_KERNEL_SKINNY) {
     SkinnyParams sp = {};
     sp.As = As; sp.as_sm = as_stride_m; sp.as_sk = as_stride_k; sp.Bs = Bs;
-    return run_skinny(A, B, sp, splits, C, c_dtype, M, N, K, workspace, workspace_bytes, st, fan);
+    return run_skinny(A, B, sp, r, C, c_dtype, M, N, K, workspace, workspace_bytes, st, fan);
   }
-  const int bn = plan.pair_bn;
-  // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
-  const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
-  if (plan.csum && wide && fan.n == 0 && tune.gemm_splitk <= 0) {
+  const bool wide = r.kernel == B200_KERNEL_WIDE;
+  if (r.sum == B200_SUM_CLUSTER) {
     if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, splits, true, st);
     if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, splits, true, st);
     return launch_gemm_wide<float>(bn, A, B, p, splits, true, st);
@@ -254,22 +282,22 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
     p.split_stride = M * N;
     p.n_dest = 0;  // the partials stay local; the reduction pass fans the sum out
     int rc = wide ? launch_gemm_wide<float>(bn, A, B, p, splits, false, st)
-                  : launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st, splits);
+                  : launch_gemm<GEMM_DENSE, float>(A, B, N, p, bn, st, splits);
     if (rc) return rc;
     const float* part = static_cast<const float*>(workspace);
     if (c_dtype == B200_BF16) return launch_reduce<__nv_bfloat16>(part, C, M * N, splits, st, fan, N);
     if (c_dtype == B200_F16) return launch_reduce<__half>(part, C, M * N, splits, st, fan, N);
     return launch_reduce<float>(part, C, M * N, splits, st, fan, N);
   }
-  if (wide && fan.n == 0) {
+  if (wide) {
     if (c_dtype == B200_BF16) return launch_gemm_wide<__nv_bfloat16>(bn, A, B, p, 1, false, st);
     if (c_dtype == B200_F16) return launch_gemm_wide<__half>(bn, A, B, p, 1, false, st);
     return launch_gemm_wide<float>(bn, A, B, p, 1, false, st);
   }
   switch (c_dtype) {
-    case B200_BF16: return launch_gemm<GEMM_DENSE, __nv_bfloat16>(A, B, N, p, force_bn, st);
-    case B200_F16: return launch_gemm<GEMM_DENSE, __half>(A, B, N, p, force_bn, st);
-    default: return launch_gemm<GEMM_DENSE, float>(A, B, N, p, force_bn, st);
+    case B200_BF16: return launch_gemm<GEMM_DENSE, __nv_bfloat16>(A, B, N, p, bn, st);
+    case B200_F16: return launch_gemm<GEMM_DENSE, __half>(A, B, N, p, bn, st);
+    default: return launch_gemm<GEMM_DENSE, float>(A, B, N, p, bn, st);
   }
 }
 }  // namespace b200
@@ -321,28 +349,55 @@ static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M 
 // (16 x 768 x 4096: 6.6 against 5.2) and for larger weights (1 x 8192 x 3584: 8.3 against 7.2); with small weights the GPU
 // finishes before the host, which pays 4.7 us for one launch and 7 for two.
 constexpr int64_t kLinearStreamMaxM = 16;
-static bool linear_one_launch(int64_t M, int64_t N, int64_t K) {
+static bool linear_one_launch(int64_t M, int64_t N, int64_t K, int sms, int* ranks = nullptr) {
   int csize, kb, stages, own;
-  return M <= kLinearStreamMaxM && tuning().linear_decode_fused != 0 &&
-         plan_linear_stream<16, true>(M, N, K, sm_count(), csize, kb, stages, own) && kb * M <= 32 && N * K < (16 << 20);
+  if (M > kLinearStreamMaxM || tuning().linear_decode_fused == 0 || !plan_linear_stream<16, true>(M, N, K, sms, csize, kb, stages, own) ||
+      kb * M > 32 || N * K >= (16 << 20))
+    return false;
+  if (ranks) *ranks = csize;
+  return true;
 }
 // Quantiser inside the decode GEMM (one launch): up to 8 rows, where the plan takes that kernel and its splits are summed
 // within clusters. The four projections of an unsharded 4096-wide layer, launched one by one, two launches each against one:
 // 1 row 53.7 and 48.0 us, 8 rows 56.2 and 51.0; at 16 rows the quantiser warps no longer keep up with the weights, 56.6 and 65.0
 // (with twice as many of them 56.2, but then 1 row takes 50.3).
 constexpr int64_t kLinearQuantInGemmMaxM = 8;
-static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K) {
+static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K, int sms, GemmRoute* route) {
   const Tuning& tune = tuning();
   if (M > kLinearQuantInGemmMaxM || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
-  const GemmPlan plan = plan_gemm(M, N, K, sm_count() < 148 ? sm_count() : 148, true);
-  return plan.skinny && skinny_direct(M, N, K, plan.splits);
+  const GemmPlan plan = plan_gemm(M, N, K, sms, true);
+  if (!plan.skinny || !skinny_split(M, N, K, plan.splits).direct()) return false;
+  *route = skinny_route(M, N, K, plan.splits, false, B200_KERNEL_SKINNY_QUANT);
+  return true;
+}
+// A linear layer: one of the two kernels that quantise their input themselves, or the quantiser and what route_gemm says.
+static GemmRoute route_linear(int64_t M, int64_t N, int64_t K, int sms) {
+  GemmRoute r;
+  int ranks;
+  if (linear_one_launch(M, N, K, sms, &ranks))
+    return {B200_KERNEL_STREAM_QUANT, 256, ranks, ranks > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE};
+  const int gemm_sms = sms < 148 ? sms : 148;
+  if (linear_quant_in_gemm(M, N, K, gemm_sms, &r)) return r;
+  return route_gemm(M, N, K, gemm_sms, false);
 }
 }  // namespace b200
+
+extern "C" int b200_plan_dense(int entry, int64_t M, int64_t N, int64_t K, int sms, int* kernel, int* tile_n, int* splits, int* sum) {
+  using namespace b200;
+  B200_CHECK_ARG(entry >= B200_PLAN_GEMM && entry <= B200_PLAN_LINEAR, "plan: unknown entry point code %d", entry);
+  B200_CHECK_ARG(M > 0 && N > 0 && K > 0 && sms >= 0, "plan: bad shape");
+  B200_CHECK_ARG(kernel && tile_n && splits && sum, "plan: null pointer");
+  if (sms == 0) sms = sm_count();
+  const GemmRoute r = entry == B200_PLAN_LINEAR ? route_linear(M, N, K, sms)
+                                                : route_gemm(M, N, K, sms < 148 ? sms : 148, entry == B200_PLAN_GEMM_FANOUT);
+  *kernel = r.kernel, *tile_n = r.tile_n, *splits = r.splits, *sum = r.sum;
+  return B200_OK;
+}
 
 extern "C" size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  if (linear_one_launch(M, N, K)) return 0;
+  if (linear_one_launch(M, N, K, sm_count())) return 0;
   return linear_q_bytes(M, K) + linear_s_bytes(M, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
 }
 
@@ -361,15 +416,14 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
     set_error_detail("linear: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
   }
-  if (linear_one_launch(M, N, K)) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
-  if (linear_quant_in_gemm(M, N, K)) {
+  const GemmRoute r = route_linear(M, N, K, sm_count());
+  if (r.kernel == B200_KERNEL_STREAM_QUANT) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
+  if (r.kernel == B200_KERNEL_SKINNY_QUANT) {
     B200_CHECK_ARG(((uintptr_t)out & 15) == 0, "gemm: A, B and C must be 16-byte aligned");
     B200_UNSUPPORTED(N > 0x7fffff00LL || K > 0x7fffff00LL, "gemm: dimension too large");
-    const int sms = sm_count() < 148 ? sm_count() : 148;
     SkinnyParams sp = {};
     sp.x = x; sp.eps = 1e-10f; sp.Bs = Bs;
-    return run_skinny(nullptr, B, sp, plan_gemm(M, N, K, sms, true).splits, out, x_dtype, M, N, K, nullptr, 0,
-                      static_cast<cudaStream_t>(stream), FanOut{});
+    return run_skinny(nullptr, B, sp, r, out, x_dtype, M, N, K, nullptr, 0, static_cast<cudaStream_t>(stream), FanOut{});
   }
   uint8_t* q = static_cast<uint8_t*>(workspace);
   float* s = reinterpret_cast<float*>(q + linear_q_bytes(M, K));
@@ -507,15 +561,15 @@ extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa
     set_error_detail("gemm_packed: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
   }
-  const GemmPlan plan = plan_gemm(M, N, K, sm_count() < 148 ? sm_count() : 148, tuning().gemm_bn < 0);
-  if (plan.skinny && tuning().gemm_splitk <= 0) {  // a few rows: the decode kernel reads the packed words itself
+  const GemmRoute r = route_gemm(M, N, K, plan_sms(), false);
+  if (r.kernel == B200_KERNEL_SKINNY && tuning().gemm_splitk <= 0) {  // a few rows: the decode kernel reads the packed words itself
     B200_CHECK_ARG(A && B && C && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B & 15) == 0 && ((uintptr_t)C & 15) == 0,
                    "gemm_packed: A, B and C must be 16-byte aligned");
     B200_CHECK_ARG(c_dtype == B200_BF16 || c_dtype == B200_F16 || c_dtype == B200_F32, "gemm_packed: unknown output dtype code %d", c_dtype);
     B200_UNSUPPORTED(K % 16 != 0 || N % 8 != 0, "gemm_packed: K=%lld must be a multiple of 16, N=%lld of 8", (long long)K, (long long)N);
     SkinnyParams sp = {};
     sp.sfa = sfa; sp.sfb = sfb; sp.sfa_ld = sfa_ld; sp.sfb_ld = sfb_ld; sp.sfb_step = 128 / sfb_rows_per_word;
-    return run_skinny(A, B, sp, plan.splits, C, c_dtype, M, N, K, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), FanOut{});
+    return run_skinny(A, B, sp, r, C, c_dtype, M, N, K, workspace, workspace_bytes, static_cast<cudaStream_t>(stream), FanOut{});
   }
   float* as = static_cast<float*>(workspace);
   uint8_t* bs = static_cast<uint8_t*>(workspace) + packed_as_bytes(M, K);
