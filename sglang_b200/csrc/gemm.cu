@@ -113,7 +113,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
-  const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256;
+  const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256 && sms >= 2;
   consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, pairs ? 1 : 8);
   if (pairs) {
     consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1);
@@ -131,10 +131,10 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (may_pair && tune.gemm_stream != 0 && M > 32 && M <= 128) {
     int csize, kb, stages, own;
     if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own)) {
-      // 0.44 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more, and clusters fill 132 SMs
-      // at most (80 x 6144 x 4096 in clusters of 3: 24.8 us, two waves)
+      // 0.44 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more, and clusters fill 132 of
+      // 148 SMs at most (80 x 6144 x 4096 in clusters of 3: 24.8 us, two waves)
       const int64_t items = cdiv(N, 256) * cdiv(M, 64);
-      double work = (double)cdiv(items * csize, csize > 1 ? sms - 16 : sms) * kb * 0.44;
+      double work = (double)cdiv(items * csize, csize > 1 && sms >= 148 ? sms - 16 : sms) * kb * 0.44;
       if (work < (double)N * (double)K / 6.4e6) work = (double)N * (double)K / 6.4e6;
       const double us = 7.5 + (csize > 1 ? 1.0 : 0.0) + work;
       if (us < best.us) best = {1, 0, false, true, false, us};
@@ -458,6 +458,7 @@ namespace b200 {
 // allow it (3000 x 4096 x 14336: 2759 against 2244 TFLOP/s); it starts 2 us later (400 x 8192 x 1024: single 8.1 us, pair 9.8).
 static double block_scaled_us(int64_t M, int64_t N, int64_t K, int sms, bool pair) {
   const int64_t tiles = pair ? cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN) : cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN);
+  if (pair && sms < 2) return 1e30;
   return (pair ? 6.0 : 4.0) + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * (pair ? 0.34 : 0.38) + 1.2);
 }
 }  // namespace b200
