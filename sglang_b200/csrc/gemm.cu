@@ -114,11 +114,14 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
     }
   };
   const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256 && sms >= 2;
-  consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, pairs ? 1 : 8);
+  // Splits of pairs go through memory on partitions of the part only: all of it sums them in clusters (below), whose numbers at
+  // once are known for 148 SMs.
+  const int max_splits = pairs && sms >= 148 ? 1 : 8;
+  consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, max_splits);
   if (pairs) {
-    consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1);
-    consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, 1);
-    consider(256, 128, sms / 2, 4.25, 0.22, 0.8, 128, 1);
+    consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, max_splits);
+    consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, max_splits);
+    consider(256, 128, sms / 2, 4.25, 0.22, 0.8, 128, max_splits);
     const int64_t tiles = cdiv(M, 256) * cdiv(N, 128);
     for (int s = 2; s <= 4; s += 2) {
       if (sms < 148 || tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
@@ -149,9 +152,9 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
 
 extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  // sized for the split that 148 SMs pick (or the tuning knobs force)
+  // sized for the split that this device's SMs pick, 148 without a device (or the tuning knobs force)
   const b200::Tuning& tune = b200::tuning();
-  int s = b200::plan_gemm(M, N, K, 148, tune.gemm_bn < 0).splits;
+  int s = b200::plan_gemm(M, N, K, b200::plan_sms(), tune.gemm_bn < 0).splits;
   if (tune.gemm_splitk > s) s = (int)tune.gemm_splitk;
   if (tune.gemm_skinny_max_m >= 0 && s < 16) s = 16;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
@@ -540,7 +543,7 @@ static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(c
 
 extern "C" size_t b200_w8a8_block_fp8_gemm_packed_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
-  if (M <= 0 || N <= 0 || K <= 0 || block_scaled_wins(M, N, K, 148)) return 0;
+  if (M <= 0 || N <= 0 || K <= 0 || block_scaled_wins(M, N, K, plan_sms())) return 0;
   return packed_as_bytes(M, K) + packed_bs_bytes(N, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
 }
 

@@ -27,3 +27,12 @@ for sms in range(1, 149):
 """
     r = subprocess.run([sys.executable, "-c", code], cwd=ROOT, capture_output=True, text=True)
     assert r.returncode == 0, (r.returncode, r.stderr[-2000:])
+
+
+def test_few_tiles_split_k_on_a_partition():
+    """Half of the part: four to eight tiles of a long K are not left to four CTAs or pairs (the whole part splits them in clusters)."""
+    for sms in (36, 74, 132):
+        for M, n, k in [(300, 512, 16384), (512, 256, 16384), (300, 512, 8192)]:
+            p = _plan("gemm", M, n, k, sms)
+            assert p.kernel == "wide" and p.splits > 1 and p.sum == "memory", (sms, M, n, k, p)
+    assert _plan("gemm", 512, 256, 16384, 148).sum == "cluster"
