@@ -80,16 +80,44 @@ struct GemmPlan {
   double us;    // modelled time (0: not modelled, decode sizes)
 };
 
+// K splits of the decode kernel (gemm_skinny.cuh) when `splits` are asked for, and whether they are summed within clusters.
+struct SkinnySplit {
+  int splits;
+  bool cluster;
+  bool direct() const { return splits == 1 || cluster; }  // the kernel writes the result itself, without partials in memory
+};
+static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
+  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;  // scales of one item fit its smem table
+  const int nt = skinny_token_tile(M);
+  const int cluster = splits > 1 && tuning().gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
+  return cluster > 1 ? SkinnySplit{cluster, true} : SkinnySplit{splits, false};
+}
+
+// Modelled time of the decode kernel. Its CTAs run two to an SM: one that has its SM to itself takes 0.20 us per 128-K block, one
+// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (5 TB/s) or, once per 32 rows, from
+// L2 (10.7 TB/s). Over 370 sizes of 33 to 256 rows it is within 6 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most
+// of it where K is short: 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
+static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
+  const int64_t t_tiles = cdiv(M, skinny_token_tile(M)), ctas = cdiv(N, 128) * t_tiles * s.splits;
+  const double kb = (double)cdiv(cdiv(K, 128), s.splits);
+  double work = (double)(cdiv(ctas, 2 * sms) - 1) * (kb * 0.385 + 2.0) + kb * (ctas <= sms ? 0.20 : 0.385);
+  const double memory = (double)N * (double)K / 5.0e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
+  if (work < memory) work = memory;
+  if (work < l2) work = l2;
+  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.28 * s.splits * (double)M * (double)N / 1e6;
+  return 2.9 + work + sum;
+}
+
 // SMs that plans are made for
 static int plan_sms() { return sm_count() < 148 ? sm_count() : 148; }
 
 // Kernel, tile and K split of a dense problem: the one whose modelled time is least. The model is launch and set-up, then
-// whole waves of tiles, each its 128-K blocks and an epilogue; nothing is faster than reading the weights (6.2 TB/s). The decode
-// kernel re-reads the weights for every 32 rows at the L2's 9.5 TB/s. Where the tiles of 128-wide pairs leave half of the chip idle
-// their K range is split 2 or 4 ways within clusters, of which this part holds 33 and 15 at once; the sum costs 2 to 3 us. The
-// constants are fits to measurements at 16 weight shapes (1280..28672 x 1024..14336) and 17 row counts (33..2200), where the plan
-// is 0.3 % behind the best kernel on average; e.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, split in clusters
-// of 4 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
+// whole waves of tiles, each its 128-K blocks and an epilogue; nothing is faster than reading the weights (6.2 TB/s). Where the
+// tiles of 128-wide pairs leave half of the chip idle their K range is split 2 or 4 ways within clusters, of which this part holds
+// 33 and 15 at once; the sum costs 2 to 3 us. The constants are fits to every kernel's time at 632 sizes, 16 weight shapes (1280..28672
+// x 1024..14336) times 17 row counts (33..2200) and as many spread over 17..2200 x 136..16384 x 256..16384: the plan is
+// 0.6 % behind the best kernel on average. E.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, their K split two ways
+// 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
 static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair) {
   const Tuning& tune = tuning();
   const int64_t num_kb = cdiv(K, 128);
@@ -121,7 +149,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (pairs) {
     consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, max_splits);
     consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, max_splits);
-    consider(256, 128, sms / 2, 4.25, 0.22, 0.8, 128, max_splits);
+    consider(256, 128, sms / 2, 3.8, 0.22, 0.85, 128, max_splits);
     const int64_t tiles = cdiv(M, 256) * cdiv(N, 128);
     for (int s = 2; s <= 4; s += 2) {
       if (sms < 148 || tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
@@ -143,9 +171,11 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       if (us < best.us) best = {1, 0, false, true, false, us};
     }
   }
-  const double skinny_us = 5.0 + (double)cdiv(M, 32) * (double)N * (double)K / 9.5e6;
-  if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM) && skinny_us < best.us)
-    best = {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, false, skinny_us};
+  if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM)) {
+    const int splits = skinny_k_splits(M, N, K, skinny_token_tile(M), sms);
+    const double us = skinny_us(M, N, K, sms, skinny_split(M, N, K, splits));
+    if (us < best.us) best = {splits, 0, true, false, false, us};
+  }
   return best;
 }
 }
@@ -161,19 +191,6 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N,
 }
 
 namespace b200 {
-// K splits of the decode kernel (gemm_skinny.cuh) when `splits` are asked for, and whether they are summed within clusters.
-struct SkinnySplit {
-  int splits;
-  bool cluster;
-  bool direct() const { return splits == 1 || cluster; }  // the kernel writes the result itself, without partials in memory
-};
-static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
-  while (cdiv(cdiv(K, 128), splits) > SkinnyCfg<16, false>::kMaxKb) ++splits;  // scales of one item fit its smem table
-  const int nt = skinny_token_tile(M);
-  const int cluster = splits > 1 && tuning().gemm_splitk <= 0 ? skinny_cluster(cdiv(N, 128) * cdiv(M, nt), K, nt, splits) : 1;
-  return cluster > 1 ? SkinnySplit{cluster, true} : SkinnySplit{splits, false};
-}
-
 // What a dense problem runs: kernel, columns of its tile, K splits and where they are summed (the codes of b200_plan_dense).
 // gemm_impl and the linear layer launch it, b200_plan_dense reports it.
 struct GemmRoute {
