@@ -77,17 +77,19 @@ int b200_set_tuning(const char* name, long value);
 int b200_get_tuning(const char* name, long* value);
 
 /* Which kernel a dense call of this size takes under the present knobs, and how: for tests and tuning sweeps. Host arithmetic
- * only, no GPU needed. entry: the plain GEMM (fp32 scales), the fan-out GEMM or the linear layer. sms: multiprocessors to plan
+ * only, no GPU needed. entry: the plain GEMM (fp32 scales), the fan-out GEMM, the linear layer or the GEMM on packed scales. sms: multiprocessors to plan
  * for; 0 = those of the current device. *tile_n: columns of the tile (wide kernel: 0 = single CTAs with 256, else of a CTA pair;
  * tile kernel: 0 = by N). *splits: K splits, *sum: where they are summed. Returns B200_E_BAD_ARG for an empty shape. */
-enum { B200_PLAN_GEMM = 0, B200_PLAN_GEMM_FANOUT = 1, B200_PLAN_LINEAR = 2 };
+enum { B200_PLAN_GEMM = 0, B200_PLAN_GEMM_FANOUT = 1, B200_PLAN_LINEAR = 2, B200_PLAN_GEMM_PACKED = 3 };
 enum {
   B200_KERNEL_TILE = 0,         /* 8 promotion warps (gemm_kernel.cuh) */
   B200_KERNEL_WIDE = 1,         /* 16 promotion warps, single CTAs or pairs (gemm_pair.cuh) */
   B200_KERNEL_SKINNY = 2,       /* decode, swapped operands (gemm_skinny.cuh) */
   B200_KERNEL_STREAM = 3,       /* weight-streaming, token tiles of 64 (linear_stream.cuh) */
   B200_KERNEL_SKINNY_QUANT = 4, /* linear: decode kernel that quantises its own input */
-  B200_KERNEL_STREAM_QUANT = 5  /* linear: weight-streaming kernel that quantises its own input */
+  B200_KERNEL_STREAM_QUANT = 5, /* linear: weight-streaming kernel that quantises its own input */
+  B200_KERNEL_BLOCK_SCALED = 6, /* packed scales: scales applied by the tensor core (gemm_ue8m0.cuh) */
+  B200_KERNEL_BLOCK_SCALED_PAIR = 7 /* the same on CTA pairs (gemm_ue8m0_pair.cuh) */
 };
 enum { B200_SUM_NONE = 0, B200_SUM_MEMORY = 1, B200_SUM_CLUSTER = 2 };
 int b200_plan_dense(int entry, int64_t M, int64_t N, int64_t K, int sms, int* kernel, int* tile_n, int* splits, int* sum);

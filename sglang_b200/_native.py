@@ -263,8 +263,8 @@ def get_tuning(name: str) -> int:
     return v.value
 
 
-PLAN_ENTRIES = {"gemm": 0, "fanout": 1, "linear": 2}
-KERNELS = ("tile", "wide", "skinny", "stream", "skinny_quant", "stream_quant")
+PLAN_ENTRIES = {"gemm": 0, "fanout": 1, "linear": 2, "packed": 3}
+KERNELS = ("tile", "wide", "skinny", "stream", "skinny_quant", "stream_quant", "block_scaled", "block_scaled_pair")
 SUMS = ("none", "memory", "cluster")
 
 

@@ -118,7 +118,8 @@ static int plan_sms() { return sm_count() < 148 ? sm_count() : 148; }
 // x 1024..14336) times 17 row counts (33..2200) and as many spread over 17..2200 x 136..16384 x 256..16384: the plan is
 // 0.6 % behind the best kernel on average. E.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, their K split two ways
 // 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
-static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair) {
+// unpack_us: what every kernel but the decode kernel waits for first (packed scales, which that one reads itself).
+static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair, double unpack_us = 0.0) {
   const Tuning& tune = tuning();
   const int64_t num_kb = cdiv(K, 128);
   const int64_t skinny_max = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
@@ -127,7 +128,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (M <= skinny_max && skinny_ok) return {skinny_k_splits(M, N, K, skinny_token_tile(M), sms), 0, true, false, false, 0.0};
   if (may_pair && (tune.gemm_2cta == 1282 || tune.gemm_2cta == 1284) && N >= 256) return {(int)tune.gemm_2cta % 10, 128, false, false, true, 0.0};
   if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : tune.gemm_2cta == 2 ? 0 : (int)tune.gemm_2cta, false, false, false, 0.0};
-  GemmPlan best = {1, 0, false, false, false, 1e30};
+  GemmPlan best = {1, 0, false, false, false, 1e30};  // its time without unpacking
   const double stream_us = (double)N * (double)K / 6.2e6;
   auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int max_splits) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
@@ -174,20 +175,26 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM)) {
     const int splits = skinny_k_splits(M, N, K, skinny_token_tile(M), sms);
     const double us = skinny_us(M, N, K, sms, skinny_split(M, N, K, splits));
-    if (us < best.us) best = {splits, 0, true, false, false, us};
+    if (us < best.us + unpack_us) best = {splits, 0, true, false, false, us};
   }
+  if (!best.skinny) best.us += unpack_us;
   return best;
 }
 }
 
-extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
-  if (M <= 0 || N <= 0 || K <= 0) return 0;
-  // sized for the split that this device's SMs pick, 148 without a device (or the tuning knobs force)
-  const b200::Tuning& tune = b200::tuning();
-  int s = b200::plan_gemm(M, N, K, b200::plan_sms(), tune.gemm_bn < 0).splits;
+namespace b200 {
+// fp32 partials of the split that this device's SMs pick, 148 without a device (or the tuning knobs force)
+static size_t partial_bytes(int64_t M, int64_t N, int64_t K, double unpack_us = 0.0) {
+  const Tuning& tune = tuning();
+  int s = plan_gemm(M, N, K, plan_sms(), tune.gemm_bn < 0, unpack_us).splits;
   if (tune.gemm_splitk > s) s = (int)tune.gemm_splitk;
   if (tune.gemm_skinny_max_m >= 0 && s < 16) s = 16;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
+}
+}  // namespace b200
+
+extern "C" size_t b200_w8a8_block_fp8_gemm_workspace_bytes(int64_t M, int64_t N, int64_t K) {
+  return M <= 0 || N <= 0 || K <= 0 ? 0 : b200::partial_bytes(M, N, K);
 }
 
 namespace b200 {
@@ -201,10 +208,10 @@ static GemmRoute skinny_route(int64_t M, int64_t N, int64_t K, int splits, bool 
   const SkinnySplit s = skinny_split(M, N, K, splits);
   return {kernel, 128, s.splits, s.direct() && !fanout ? (s.splits > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE) : B200_SUM_MEMORY};
 }
-static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, bool fanout) {
+static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, bool fanout, double unpack_us = 0.0) {
   const Tuning& tune = tuning();
   const int force_bn = tune.gemm_bn == 128 || tune.gemm_bn == 256 ? (int)tune.gemm_bn : 0;
-  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0);
+  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0, unpack_us);
   int splits = plan.splits;
   if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
   if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
@@ -402,18 +409,6 @@ static GemmRoute route_linear(int64_t M, int64_t N, int64_t K, int sms) {
 }
 }  // namespace b200
 
-extern "C" int b200_plan_dense(int entry, int64_t M, int64_t N, int64_t K, int sms, int* kernel, int* tile_n, int* splits, int* sum) {
-  using namespace b200;
-  B200_CHECK_ARG(entry >= B200_PLAN_GEMM && entry <= B200_PLAN_LINEAR, "plan: unknown entry point code %d", entry);
-  B200_CHECK_ARG(M > 0 && N > 0 && K > 0 && sms >= 0, "plan: bad shape");
-  B200_CHECK_ARG(kernel && tile_n && splits && sum, "plan: null pointer");
-  if (sms == 0) sms = sm_count();
-  const GemmRoute r = entry == B200_PLAN_LINEAR ? route_linear(M, N, K, sms)
-                                                : route_gemm(M, N, K, sms < 148 ? sms : 148, entry == B200_PLAN_GEMM_FANOUT);
-  *kernel = r.kernel, *tile_n = r.tile_n, *splits = r.splits, *sum = r.sum;
-  return B200_OK;
-}
-
 extern "C" size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -473,13 +468,18 @@ extern "C" int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, con
 }
 
 namespace b200 {
-// Modelled time of the block-scaled kernels (see plan_gemm; fitted to 14 weight shapes x 12 row counts, 70..3000): a CTA's 128 x 224
-// tile takes 0.38 us per 128-K block, a pair's 256 x 240 one 0.34, so the pair does twice the work per SM clock where whole waves
-// allow it (3000 x 4096 x 14336: 2759 against 2244 TFLOP/s); it starts 2 us later (400 x 8192 x 1024: single 8.1 us, pair 9.8).
+// Modelled time of the block-scaled kernels (see plan_gemm; fitted to 560 sizes of 65..2200 rows): a CTA's 128 x 224 tile takes
+// 0.40 us per 128-K block, a pair's 256 x 240 one 0.32, so the pair does more than twice the work per SM clock where whole waves
+// allow it (3000 x 4096 x 14336: 2759 against 2244 TFLOP/s); it starts 2 us later (400 x 8192 x 1024: single 8.1 us, pair 9.8;
+// 160 x 14336 x 4096 18.8 and 17.8).
 static double block_scaled_us(int64_t M, int64_t N, int64_t K, int sms, bool pair) {
   const int64_t tiles = pair ? cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN) : cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN);
   if (pair && sms < 2) return 1e30;
-  return (pair ? 6.0 : 4.0) + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * (pair ? 0.34 : 0.38) + 1.2);
+  return (pair ? 6.0 : 4.0) + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * (pair ? 0.32 : 0.40) + 1.2);
+}
+static bool block_scaled_pair(int64_t M, int64_t N, int64_t K, int sms) {
+  const long knob = tuning().gemm_ue8m0;
+  return knob == 2 || (knob != 1 && block_scaled_us(M, N, K, sms, true) <= block_scaled_us(M, N, K, sms, false));
 }
 }  // namespace b200
 
@@ -501,9 +501,7 @@ extern "C" int b200_w8a8_block_fp8_gemm_ue8m0(const void* A, const int32_t* sfa,
   p.sfa = sfa; p.sfb = sfb; p.sfa_ld = sfa_ld; p.sfb_ld = sfb_ld; p.sfb_rows_per_word = sfb_rows_per_word;
   p.C = C; p.M = (int)M; p.N = (int)N; p.K = (int)K;
   cudaStream_t st = static_cast<cudaStream_t>(stream);
-  const long knob = tuning().gemm_ue8m0;
-  const bool pair = knob == 2 || (knob != 1 && block_scaled_us(M, N, K, sm_count(), true) <= block_scaled_us(M, N, K, sm_count(), false));
-  if (pair) {
+  if (block_scaled_pair(M, N, K, plan_sms())) {
     switch (c_dtype) {
       case B200_BF16: return launch_gemm_ue8m0_pair<__nv_bfloat16>(A, B, p, st);
       case B200_F16: return launch_gemm_ue8m0_pair<__half>(A, B, p, st);
@@ -544,15 +542,17 @@ __global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __res
   }
 }
 
+constexpr double kUnpackUs = 1.1;
 // Whether the block-scaled kernels (scales applied by the tensor core, no K split) beat the promotion kernels on unpacked
-// scales: below 65 rows the weight stream decides, then wave counts. Unpacking takes 2.5 us, and long problems run at the power
-// cap, where applying scales in the tensor core pays beyond the model (1500 x 4096 x 14336: 75.7 us against 85.5). With this margin
-// the choice is 0.2 % behind the best on those sizes (203 x 4096 x 14336: 46 us block-scaled, 25 promoted).
+// scales, or the decode kernel, which reads the packed words itself: below 65 rows the weight stream decides, then wave counts.
+// Long problems run at the power cap, where applying scales in the tensor core pays beyond the model (1500 x 4096 x 14336: 75.7 us
+// against 85.5). With this margin the choice is 0.6 % behind the best on those sizes (203 x 4096 x 14336: 46 us block-scaled, 25
+// promoted; 96 x 5120 x 1536 9.4 and 7.2 in the decode kernel; 204 x 336 x 1152 6.6 and 4.9).
 static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
   if (tuning().gemm_ue8m0 > 0) return true;
   if (M <= 64) return false;
   const double one = block_scaled_us(M, N, K, sms, false), two = block_scaled_us(M, N, K, sms, true);
-  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true).us * 1.08 + 3.0;
+  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true, kUnpackUs).us * 1.04 + 1.0;
 }
 static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
 static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }
@@ -561,7 +561,9 @@ static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(c
 extern "C" size_t b200_w8a8_block_fp8_gemm_packed_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || block_scaled_wins(M, N, K, plan_sms())) return 0;
-  return packed_as_bytes(M, K) + packed_bs_bytes(N, K) + b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
+  // the decode kernel takes its partials first, the others run on unpacked scales with the plain plan
+  const size_t partials = partial_bytes(M, N, K), decode = partial_bytes(M, N, K, kUnpackUs);
+  return packed_as_bytes(M, K) + packed_bs_bytes(N, K) + (partials > decode ? partials : decode);
 }
 
 extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa, int64_t sfa_ld, const void* B,
@@ -582,7 +584,7 @@ extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa
     set_error_detail("gemm_packed: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
   }
-  const GemmRoute r = route_gemm(M, N, K, plan_sms(), false);
+  const GemmRoute r = route_gemm(M, N, K, plan_sms(), false, kUnpackUs);
   if (r.kernel == B200_KERNEL_SKINNY && tuning().gemm_splitk <= 0) {  // a few rows: the decode kernel reads the packed words itself
     B200_CHECK_ARG(A && B && C && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B & 15) == 0 && ((uintptr_t)C & 15) == 0,
                    "gemm_packed: A, B and C must be 16-byte aligned");
@@ -603,4 +605,23 @@ extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa
   if (rc) return rc;
   return gemm_impl(A, as, 1, M, B, reinterpret_cast<const float*>(bs), C, c_dtype, M, N, K, rest,
                    need - (size_t)(rest - static_cast<uint8_t*>(workspace)), stream, FanOut{});
+}
+
+extern "C" int b200_plan_dense(int entry, int64_t M, int64_t N, int64_t K, int sms, int* kernel, int* tile_n, int* splits, int* sum) {
+  using namespace b200;
+  B200_CHECK_ARG(entry >= B200_PLAN_GEMM && entry <= B200_PLAN_GEMM_PACKED, "plan: unknown entry point code %d", entry);
+  B200_CHECK_ARG(M > 0 && N > 0 && K > 0 && sms >= 0, "plan: bad shape");
+  B200_CHECK_ARG(kernel && tile_n && splits && sum, "plan: null pointer");
+  if (sms == 0) sms = sm_count();
+  const int gemm_sms = sms < 148 ? sms : 148;
+  GemmRoute r;
+  if (entry == B200_PLAN_LINEAR)
+    r = route_linear(M, N, K, sms);
+  else if (entry == B200_PLAN_GEMM_PACKED && block_scaled_wins(M, N, K, gemm_sms))
+    r = block_scaled_pair(M, N, K, gemm_sms) ? GemmRoute{B200_KERNEL_BLOCK_SCALED_PAIR, Ue8m0PairCfg::BN, 1, B200_SUM_NONE}
+                                             : GemmRoute{B200_KERNEL_BLOCK_SCALED, Ue8m0Cfg::BN, 1, B200_SUM_NONE};
+  else
+    r = route_gemm(M, N, K, gemm_sms, entry == B200_PLAN_GEMM_FANOUT, entry == B200_PLAN_GEMM_PACKED ? kUnpackUs : 0.0);
+  *kernel = r.kernel, *tile_n = r.tile_n, *splits = r.splits, *sum = r.sum;
+  return B200_OK;
 }

@@ -19,7 +19,7 @@ from sglang_b200 import _native as N
 for sms in range(1, 149):
     for M, n, k in [(1, 1536, 4096), (8, 4096, 4096), (33, 512, 1024), (64, 256, 8192), (100, 2048, 7168), (203, 4096, 4096),
                     (300, 200, 8192), (1027, 7168, 8192), (3000, 4096, 14336)]:
-        for entry in ("gemm", "fanout", "linear"):
+        for entry in ("gemm", "fanout", "linear", "packed"):
             p = N.plan_dense(entry, M, n, k, sms)
             assert 1 <= p.splits <= k // 128, (entry, M, n, k, sms, p)
             if sms < 2:
@@ -50,3 +50,35 @@ def test_short_weights_of_some_rows_take_the_decode_kernel():
     assert _plan("gemm", 203, 28672, 4096, 148).kernel == "wide"
     assert _plan("gemm", 61, 14336, 8192, 148).kernel == "stream"
     assert _plan("gemm", 957, 288, 256, 148) == ("wide", 128, 1, "none")
+
+
+def test_packed_scales_take_the_decode_kernel_where_it_saves_the_unpacking():
+    """The decode kernel reads packed words itself, every other kernel on fp32 scales waits for their unpacking. Measured:
+    96 x 5120 x 1536 9.4 us block-scaled, 7.2 in the decode kernel; 204 x 336 x 1152 6.6 and 4.9; 64 x 16384 x 1024 8.9 on
+    unpacked scales, 6.3."""
+    for m, n, k in [(40, 16384, 1024), (64, 16384, 1024), (204, 336, 1152), (193, 312, 1024), (65, 5120, 1536), (80, 5120, 1536),
+                    (96, 5120, 1536), (74, 264, 1024), (107, 816, 896), (57, 13560, 4736), (112, 1536, 7168)]:
+        assert _plan("packed", m, n, k, 148).kernel == "skinny", (m, n, k)
+    # CTA pairs where their start is paid back by K: 17.1 us against 17.9 of single CTAs; and where it is not
+    for m in (100, 160, 203, 256):
+        assert _plan("packed", m, 14336, 4096, 148).kernel == "block_scaled_pair", m
+    assert _plan("packed", 400, 8192, 1024, 148).kernel == "block_scaled"
+    assert _plan("packed", 3000, 4096, 14336, 148).kernel == "block_scaled_pair"
+    assert _plan("packed", 203, 4096, 14336, 148).kernel == "wide"
+
+
+def test_packed_workspace_covers_either_plan():
+    """Partials of the decode kernel, or scales and partials of the plan on unpacked ones."""
+    from sglang_b200 import _native as N
+
+    lib = N.load()
+    for m in (1, 33, 64, 100, 144, 200, 256, 300):
+        for n, k in [(4096, 1024), (1536, 7168), (5120, 1536), (16384, 1024), (264, 8192), (4096, 14336)]:
+            have = lib.b200_w8a8_block_fp8_gemm_packed_workspace_bytes(m, n, k)
+            p = _plan("packed", m, n, k)
+            need = p.splits * m * n * 4 if p.sum == "memory" else 0
+            if p.kernel.startswith("block_scaled"):
+                assert have == 0
+            else:
+                scales = 0 if p.kernel == "skinny" else 4 * (m + -(-n // 128)) * -(-k // 128)
+                assert have >= need + scales and have > 0, (m, n, k, p)
