@@ -94,14 +94,14 @@ static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
 }
 
 // Modelled time of the decode kernel. Its CTAs run two to an SM: one that has its SM to itself takes 0.20 us per 128-K block, one
-// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (5 TB/s) or, once per 32 rows, from
+// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (4.6 TB/s) or, once per 32 rows, from
 // L2 (10.7 TB/s). Over 370 sizes of 33 to 256 rows it is within 6 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most
 // of it where K is short: 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
 static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
   const int64_t t_tiles = cdiv(M, skinny_token_tile(M)), ctas = cdiv(N, 128) * t_tiles * s.splits;
   const double kb = (double)cdiv(cdiv(K, 128), s.splits);
   double work = (double)(cdiv(ctas, 2 * sms) - 1) * (kb * 0.385 + 2.0) + kb * (ctas <= sms ? 0.20 : 0.385);
-  const double memory = (double)N * (double)K / 5.0e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
+  const double memory = (double)N * (double)K / 4.6e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
   if (work < memory) work = memory;
   if (work < l2) work = l2;
   const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.28 * s.splits * (double)M * (double)N / 1e6;

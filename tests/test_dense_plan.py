@@ -65,6 +65,9 @@ def test_packed_scales_take_the_decode_kernel_where_it_saves_the_unpacking():
     assert _plan("packed", 400, 8192, 1024, 148).kernel == "block_scaled"
     assert _plan("packed", 3000, 4096, 14336, 148).kernel == "block_scaled_pair"
     assert _plan("packed", 203, 4096, 14336, 148).kernel == "wide"
+    # large weights: unpacking is paid back by the weight-streaming kernel, 32 us against 35
+    for m in (33, 48, 64):
+        assert _plan("packed", m, 14336, 8192, 148).kernel == "stream", m
 
 
 def test_packed_workspace_covers_either_plan():
