@@ -332,7 +332,8 @@ int b200_route_topk_softmax_capped(const void* logits, int logits_dtype, float s
  * array of device pointers, which may be peer GPUs' memory mapped into this process) while the
  * GEMM is still running. dest_by_tile != 0: the tile of 128-row block mt goes only to
  * dest[mt % n_dest] (reduce-scatter by row block). Workspace as for the plain GEMM, sized by
- * b200_w8a8_block_fp8_gemm_fanout_workspace_bytes.
+ * b200_w8a8_block_fp8_gemm_fanout_workspace_bytes. Its K splits are planned for the kernels that can fan out, so sums may be
+ * grouped otherwise than the plain GEMM's of the same size (with equal splits the bytes are equal).
  * b200_allreduce_finish: n_ranks slots of slot_stride elements each (LOCAL memory; slot r holds
  * the [M,N] partial written by rank r's fan-out GEMM; bf16/f16). Handshake with all ranks (flag arrays of 2*8 uint32, zero before the
  * first call, epoch strictly increasing by call and identical on all ranks; my_flags local,

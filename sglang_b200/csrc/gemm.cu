@@ -97,15 +97,18 @@ static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
 // that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (4.6 TB/s) or, once per 32 rows, from
 // L2 (10.7 TB/s). Over 370 sizes of 33 to 256 rows it is within 6 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most
 // of it where K is short: 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
-static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
+static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s, double sum) {
   const int64_t t_tiles = cdiv(M, skinny_token_tile(M)), ctas = cdiv(N, 128) * t_tiles * s.splits;
   const double kb = (double)cdiv(cdiv(K, 128), s.splits);
   double work = (double)(cdiv(ctas, 2 * sms) - 1) * (kb * 0.385 + 2.0) + kb * (ctas <= sms ? 0.20 : 0.385);
   const double memory = (double)N * (double)K / 4.6e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
   if (work < memory) work = memory;
   if (work < l2) work = l2;
-  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.28 * s.splits * (double)M * (double)N / 1e6;
   return 2.9 + work + sum;
+}
+static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
+  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.28 * s.splits * (double)M * (double)N / 1e6;
+  return skinny_us(M, N, K, sms, s, sum);
 }
 
 // SMs that plans are made for
@@ -118,8 +121,17 @@ static int plan_sms() { return sm_count() < 148 ? sm_count() : 148; }
 // x 1024..14336) times 17 row counts (33..2200) and as many spread over 17..2200 x 136..16384 x 256..16384: the plan is
 // 0.6 % behind the best kernel on average. E.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, their K split two ways
 // 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
-// unpack_us: what every kernel but the decode kernel waits for first (packed scales, which that one reads itself).
-static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair, double unpack_us = 0.0) {
+//
+// A fan-out (its result goes to several buffers) is planned from what can do that: the 8-warp tile kernel unsplit, or the decode
+// and 16-warp kernels with fp32 partials, whose reduction pass writes to the buffers (1.5 us and 4.5 us per million partials; no
+// clusters, no weight streaming). Fitted to 567 sizes of 33..1200 rows with the buffers on this GPU, 0.5 % behind the best;
+// e.g. 72 x 6144 x 4096: decode kernel 11.4 us, tile kernel unsplit 22.2; 300 x 4096 x 14336: unsplit 64, 2 splits of 128-wide
+// pairs 35; 112 x 5120 x 1536: 8.7 and 11.8.
+struct PlanFor {
+  bool fanout = false;
+  double unpack_us = 0.0;  // what every kernel but the decode kernel waits for first (packed scales, which that one reads itself)
+};
+static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pair, PlanFor use = {}) {
   const Tuning& tune = tuning();
   const int64_t num_kb = cdiv(K, 128);
   const int64_t skinny_max = tune.gemm_skinny_max_m >= 0 ? tune.gemm_skinny_max_m : kSkinnyMaxM;
@@ -130,37 +142,46 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (may_pair && tune.gemm_2cta > 0 && N >= 256) return {1, tune.gemm_2cta == 1 ? 256 : tune.gemm_2cta == 2 ? 0 : (int)tune.gemm_2cta, false, false, false, 0.0};
   GemmPlan best = {1, 0, false, false, false, 1e30};  // its time without unpacking
   const double stream_us = (double)N * (double)K / 6.2e6;
-  auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int max_splits) {
+  // K splits through memory: a reduction pass and the fp32 partials, written and read at about 2 TB/s
+  auto memory_sum = [&](int s) { return use.fanout ? 1.5 + 4.5 * s * (double)M * (double)N / 1e6 : 0.5 + 4.0 * s * (double)M * (double)N / 1e6; };
+  auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int first, int last) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
-    for (int s = 1; s <= max_splits && (s == 1 || num_kb >= 4 * s); ++s) {
+    for (int s = 1; s <= last && (s == 1 || num_kb >= 4 * s); ++s) {
       const double waves = (double)cdiv(tiles * s, slots);
       double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + epilogue);
       if (work < stream_us) work = stream_us;
-      // through memory: a reduction pass and the fp32 partials, written and read at about 2 TB/s
-      const double us = base + work + (s > 1 ? 0.5 + 16.0 * s * (double)M * (double)N / 4e6 : 0.0);
-      if (us < best.us) best = {s, pair_bn, false, false, false, us};
+      const double us = base + work + (s > 1 ? memory_sum(s) : 0.0);
+      if (s >= first && us < best.us) best = {s, pair_bn, false, false, false, us};
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
   const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256 && sms >= 2;
-  // Splits of pairs go through memory on partitions of the part only: all of it sums them in clusters (below), whose numbers at
-  // once are known for 148 SMs.
-  const int max_splits = pairs && sms >= 148 ? 1 : 8;
-  consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, max_splits);
-  if (pairs) {
-    consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, max_splits);
-    consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, max_splits);
-    consider(256, 128, sms / 2, 3.8, 0.22, 0.85, 128, max_splits);
+  if (use.fanout) {
+    consider(128, N > 128 ? 256 : 128, sms, 4.0, 0.64, 1.5, 0, 1, 1);
+    consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.55, 1.0, 0, 2, 8);
+    if (pairs) consider(256, 128, sms / 2, 3.8, 0.225, 0.85, 128, 2, 8);
+  } else {
+    // Splits of pairs go through memory on partitions of the part only: all of it sums them in clusters (below), whose numbers at
+    // once are known for 148 SMs.
+    const int max_splits = pairs && sms >= 148 ? 1 : 8;
+    consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, 1, max_splits);
+    if (pairs) {
+      consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1, max_splits);
+      consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, 1, max_splits);
+      consider(256, 128, sms / 2, 3.8, 0.22, 0.85, 128, 1, max_splits);
+    }
+  }
+  if (pairs && !use.fanout && sms >= 148) {
     const int64_t tiles = cdiv(M, 256) * cdiv(N, 128);
     for (int s = 2; s <= 4; s += 2) {
-      if (sms < 148 || tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
+      if (tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
       double work = (double)cdiv(num_kb, s) * (s == 2 ? 0.21 : 0.18);
       if (work < stream_us) work = stream_us;
       const double us = (s == 2 ? 6.5 : 7.75) + work;
       if (us < best.us) best = {s, 128, false, false, true, us};
     }
   }
-  if (may_pair && tune.gemm_stream != 0 && M > 32 && M <= 128) {
+  if (may_pair && !use.fanout && tune.gemm_stream != 0 && M > 32 && M <= 128) {
     int csize, kb, stages, own;
     if (plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own)) {
       // 0.44 us per 128-K block of 256 weight rows x 64 tokens; a cluster's sum costs a microsecond more, and clusters fill 132 of
@@ -174,19 +195,21 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   }
   if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM)) {
     const int splits = skinny_k_splits(M, N, K, skinny_token_tile(M), sms);
-    const double us = skinny_us(M, N, K, sms, skinny_split(M, N, K, splits));
-    if (us < best.us + unpack_us) best = {splits, 0, true, false, false, us};
+    const SkinnySplit split = skinny_split(M, N, K, splits);
+    const double us = use.fanout ? skinny_us(M, N, K, sms, split, 0.0) + 1.2 + 1.27 * split.splits * (double)M * (double)N / 1e6
+                                 : skinny_us(M, N, K, sms, split);
+    if (us < best.us + use.unpack_us) best = {splits, 0, true, false, false, us};
   }
-  if (!best.skinny) best.us += unpack_us;
+  if (!best.skinny) best.us += use.unpack_us;
   return best;
 }
 }
 
 namespace b200 {
 // fp32 partials of the split that this device's SMs pick, 148 without a device (or the tuning knobs force)
-static size_t partial_bytes(int64_t M, int64_t N, int64_t K, double unpack_us = 0.0) {
+static size_t partial_bytes(int64_t M, int64_t N, int64_t K, PlanFor use = {}) {
   const Tuning& tune = tuning();
-  int s = plan_gemm(M, N, K, plan_sms(), tune.gemm_bn < 0, unpack_us).splits;
+  int s = plan_gemm(M, N, K, plan_sms(), tune.gemm_bn < 0, use).splits;
   if (tune.gemm_splitk > s) s = (int)tune.gemm_splitk;
   if (tune.gemm_skinny_max_m >= 0 && s < 16) s = 16;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
@@ -204,28 +227,28 @@ struct GemmRoute {
   int kernel, tile_n, splits, sum;
 };
 static GemmRoute skinny_route(int64_t M, int64_t N, int64_t K, int splits, bool fanout, int kernel) {
-  // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM
+  // a fan-out takes the same splits through memory, so its sums are those of the plain GEMM where that runs the decode kernel too
   const SkinnySplit s = skinny_split(M, N, K, splits);
   return {kernel, 128, s.splits, s.direct() && !fanout ? (s.splits > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE) : B200_SUM_MEMORY};
 }
-static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, bool fanout, double unpack_us = 0.0) {
+static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, PlanFor use = {}) {
   const Tuning& tune = tuning();
   const int force_bn = tune.gemm_bn == 128 || tune.gemm_bn == 256 ? (int)tune.gemm_bn : 0;
-  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0, unpack_us);
+  const GemmPlan plan = plan_gemm(M, N, K, sms, force_bn == 0, use);
   int splits = plan.splits;
   if (tune.gemm_splitk > 0) splits = (int)tune.gemm_splitk;
   if (splits > (int)cdiv(K, 128)) splits = (int)cdiv(K, 128);
-  if (plan.stream && !fanout && tune.gemm_splitk <= 0) {
+  if (plan.stream && !use.fanout && tune.gemm_splitk <= 0) {
     int csize = 1, kb, stages, own;
     plan_linear_stream<64, false>(M, N, K, sms, csize, kb, stages, own);
     return {B200_KERNEL_STREAM, 256, csize, csize > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE};
   }
-  if (plan.skinny) return skinny_route(M, N, K, splits, fanout, B200_KERNEL_SKINNY);
+  if (plan.skinny) return skinny_route(M, N, K, splits, use.fanout, B200_KERNEL_SKINNY);
   // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
   const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
-  if (plan.csum && wide && !fanout && tune.gemm_splitk <= 0) return {B200_KERNEL_WIDE, plan.pair_bn, splits, B200_SUM_CLUSTER};
+  if (plan.csum && wide && !use.fanout && tune.gemm_splitk <= 0) return {B200_KERNEL_WIDE, plan.pair_bn, splits, B200_SUM_CLUSTER};
   const int sum = splits > 1 ? B200_SUM_MEMORY : B200_SUM_NONE;
-  if (wide && (splits > 1 || !fanout)) return {B200_KERNEL_WIDE, plan.pair_bn, splits, sum};
+  if (wide && (splits > 1 || !use.fanout)) return {B200_KERNEL_WIDE, plan.pair_bn, splits, sum};
   return {B200_KERNEL_TILE, force_bn, splits, sum};
 }
 
@@ -277,7 +300,7 @@ static int gemm_impl(const void* A, const float* As, int64_t as_stride_m, int64_
   cudaStream_t st = static_cast<cudaStream_t>(stream);
   B200_CHECK_ARG(c_dtype == B200_BF16 || c_dtype == B200_F16 || c_dtype == B200_F32, "gemm: unknown output dtype code %d",
                  c_dtype);
-  const GemmRoute r = route_gemm(M, N, K, plan_sms(), fan.n > 0);
+  const GemmRoute r = route_gemm(M, N, K, plan_sms(), PlanFor{fan.n > 0});
   const int splits = r.splits, bn = r.tile_n;
   if (r.kernel == B200_KERNEL_STREAM) {
     LinearStreamParams lp = {};
@@ -338,10 +361,10 @@ extern "C" int b200_w8a8_block_fp8_gemm(const void* A, const float* As, int64_t 
 
 extern "C" size_t b200_w8a8_block_fp8_gemm_fanout_workspace_bytes(int64_t M, int64_t N, int64_t K) {
   if (M <= 0 || N <= 0 || K <= 0) return 0;
-  const size_t plain = b200_w8a8_block_fp8_gemm_workspace_bytes(M, N, K);
+  const size_t partials = b200::partial_bytes(M, N, K, b200::PlanFor{true});
   // the decode kernel always goes through an fp32 partial when its result is fanned out
   const size_t one = M <= b200::kSkinnyPlanMaxM ? (size_t)M * (size_t)N * sizeof(float) : 0;
-  return plain > one ? plain : one;
+  return partials > one ? partials : one;
 }
 
 extern "C" int b200_w8a8_block_fp8_gemm_fanout(const void* A, const float* As, int64_t as_stride_m, int64_t as_stride_k,
@@ -405,7 +428,7 @@ static GemmRoute route_linear(int64_t M, int64_t N, int64_t K, int sms) {
     return {B200_KERNEL_STREAM_QUANT, 256, ranks, ranks > 1 ? B200_SUM_CLUSTER : B200_SUM_NONE};
   const int gemm_sms = sms < 148 ? sms : 148;
   if (linear_quant_in_gemm(M, N, K, gemm_sms, &r)) return r;
-  return route_gemm(M, N, K, gemm_sms, false);
+  return route_gemm(M, N, K, gemm_sms);
 }
 }  // namespace b200
 
@@ -552,7 +575,7 @@ static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
   if (tuning().gemm_ue8m0 > 0) return true;
   if (M <= 64) return false;
   const double one = block_scaled_us(M, N, K, sms, false), two = block_scaled_us(M, N, K, sms, true);
-  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true, kUnpackUs).us * 1.04 + 1.0;
+  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true, PlanFor{false, kUnpackUs}).us * 1.04 + 1.0;
 }
 static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
 static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }
@@ -562,7 +585,7 @@ extern "C" size_t b200_w8a8_block_fp8_gemm_packed_workspace_bytes(int64_t M, int
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0 || block_scaled_wins(M, N, K, plan_sms())) return 0;
   // the decode kernel takes its partials first, the others run on unpacked scales with the plain plan
-  const size_t partials = partial_bytes(M, N, K), decode = partial_bytes(M, N, K, kUnpackUs);
+  const size_t partials = partial_bytes(M, N, K), decode = partial_bytes(M, N, K, PlanFor{false, kUnpackUs});
   return packed_as_bytes(M, K) + packed_bs_bytes(N, K) + (partials > decode ? partials : decode);
 }
 
@@ -584,7 +607,7 @@ extern "C" int b200_w8a8_block_fp8_gemm_packed(const void* A, const int32_t* sfa
     set_error_detail("gemm_packed: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
     return B200_E_WORKSPACE;
   }
-  const GemmRoute r = route_gemm(M, N, K, plan_sms(), false, kUnpackUs);
+  const GemmRoute r = route_gemm(M, N, K, plan_sms(), PlanFor{false, kUnpackUs});
   if (r.kernel == B200_KERNEL_SKINNY && tuning().gemm_splitk <= 0) {  // a few rows: the decode kernel reads the packed words itself
     B200_CHECK_ARG(A && B && C && ((uintptr_t)A & 15) == 0 && ((uintptr_t)B & 15) == 0 && ((uintptr_t)C & 15) == 0,
                    "gemm_packed: A, B and C must be 16-byte aligned");
@@ -621,7 +644,7 @@ extern "C" int b200_plan_dense(int entry, int64_t M, int64_t N, int64_t K, int s
     r = block_scaled_pair(M, N, K, gemm_sms) ? GemmRoute{B200_KERNEL_BLOCK_SCALED_PAIR, Ue8m0PairCfg::BN, 1, B200_SUM_NONE}
                                              : GemmRoute{B200_KERNEL_BLOCK_SCALED, Ue8m0Cfg::BN, 1, B200_SUM_NONE};
   else
-    r = route_gemm(M, N, K, gemm_sms, entry == B200_PLAN_GEMM_FANOUT, entry == B200_PLAN_GEMM_PACKED ? kUnpackUs : 0.0);
+    r = route_gemm(M, N, K, gemm_sms, PlanFor{entry == B200_PLAN_GEMM_FANOUT, entry == B200_PLAN_GEMM_PACKED ? kUnpackUs : 0.0});
   *kernel = r.kernel, *tile_n = r.tile_n, *splits = r.splits, *sum = r.sum;
   return B200_OK;
 }

@@ -85,3 +85,34 @@ def test_packed_workspace_covers_either_plan():
             else:
                 scales = 0 if p.kernel == "skinny" else 4 * (m + -(-n // 128)) * -(-k // 128)
                 assert have >= need + scales and have > 0, (m, n, k, p)
+
+
+def test_fanout_is_planned_from_kernels_that_can_fan_out():
+    """No sums in clusters, no weight streaming, and no kernel's time that the call does not run. Measured with the buffers on one
+    GPU: 72 x 6144 x 4096 11.4 us in the decode kernel, 22.2 as the unsplit tile kernel that a plan for the streaming kernel ends in;
+    320 x 2112 x 7168 34 unsplit, 17 in two splits."""
+    for m, n, k in [(72, 6144, 4096), (112, 5120, 1536), (72, 8192, 3584), (128, 4096, 4096), (160, 3584, 4096), (65, 8192, 2048),
+                    (128, 7168, 2048), (72, 4096, 4096), (160, 2560, 4096), (203, 2560, 4096)]:
+        assert _plan("fanout", m, n, k, 148).kernel == "skinny", (m, n, k)
+    for m, n, k in [(320, 2112, 7168), (384, 2112, 7168), (300, 4096, 14336), (158, 6912, 14336)]:
+        assert _plan("fanout", m, n, k, 148) == ("wide", 128, 2, "memory"), (m, n, k)
+    assert _plan("fanout", 1027, 8192, 3584, 148).kernel == "tile"
+    for sms in (36, 148):
+        for m in (1, 16, 33, 64, 100, 128, 200, 300, 512, 1027):
+            for n, k in [(128, 8192), (200, 4096), (1024, 8192), (4096, 1792), (8192, 3584), (4096, 14336), (14336, 8192)]:
+                p = _plan("fanout", m, n, k, sms)
+                assert p.kernel in ("tile", "wide", "skinny") and p.sum != "cluster", p
+                assert p.sum == "memory" or p.kernel == "tile", p  # the others write to the buffers in the reduction pass
+                if p.kernel != "skinny":
+                    assert (p.sum == "memory") == (p.splits > 1), p
+
+
+def test_fanout_workspace_covers_its_plan():
+    from sglang_b200 import _native as N
+
+    lib = N.load()
+    for m in (1, 16, 33, 100, 256, 300, 700):
+        for n, k in [(128, 8192), (200, 4096), (1024, 8192), (4096, 1792), (2112, 7168), (4096, 14336)]:
+            p = _plan("fanout", m, n, k)
+            need = p.splits * m * n * 4 if p.sum == "memory" else 0
+            assert lib.b200_w8a8_block_fp8_gemm_fanout_workspace_bytes(m, n, k) >= need, (m, n, k, p)
