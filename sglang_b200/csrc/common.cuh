@@ -56,7 +56,7 @@ struct Tuning {
   long gemm_2cta = -1;          // 0: never the 16-warp kernel, 1 / 2: always, on pairs / single CTAs; 128, 192, 256: pairs of that width;
                                 // 1282, 1284: pairs, 128 wide, 2 or 4 K splits summed in clusters
   long gemm_ue8m0 = -1;          // 0: packed power-of-two scales never take the block-scaled MMA kernel
-  long linear_decode_fused = -1; // 0: callers keep quantiser + GEMM as separate launches at decode sizes
+  long linear_decode_fused = -1; // 0: quantiser + GEMM as separate launches at decode sizes, 2: quantiser in the decode GEMM wherever it runs
   long moe_decode = -1;         // 0 / 1: never / always the weight-streaming experts; 16, 32, 64: with that row block
   long moe_down_splitk = -1;    // 0: the down GEMM never splits K
   long moe_zero_pads = -1;      // 0 / 1: whether the gather pass zeroes pad rows

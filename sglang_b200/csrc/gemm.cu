@@ -401,22 +401,35 @@ static size_t linear_s_bytes(int64_t M, int64_t K) { return align_up((size_t)(M 
 constexpr int64_t kLinearStreamMaxM = 16;
 static bool linear_one_launch(int64_t M, int64_t N, int64_t K, int sms, int* ranks = nullptr) {
   int csize, kb, stages, own;
-  if (M > kLinearStreamMaxM || tuning().linear_decode_fused == 0 || !plan_linear_stream<16, true>(M, N, K, sms, csize, kb, stages, own) ||
+  if (M > kLinearStreamMaxM || tuning().linear_decode_fused == 0 || tuning().linear_decode_fused == 2 ||
+      !plan_linear_stream<16, true>(M, N, K, sms, csize, kb, stages, own) ||
       kb * M > 32 || N * K >= (16 << 20))
     return false;
   if (ranks) *ranks = csize;
   return true;
 }
 // Quantiser inside the decode GEMM (one launch): up to 8 rows, where the plan takes that kernel and its splits are summed
-// within clusters. The four projections of an unsharded 4096-wide layer, launched one by one, two launches each against one:
-// 1 row 53.7 and 48.0 us, 8 rows 56.2 and 51.0; at 16 rows the quantiser warps no longer keep up with the weights, 56.6 and 65.0
-// (with twice as many of them 56.2, but then 1 row takes 50.3).
+// within clusters, and where every CTA's share of the quantising hides behind its weights. It does while no two CTAs share an SM
+// (clusters fill 132 of 148): 4096 x 4096, 1 row, called one by one 6.5 us against 7.6 with a launch of its own (in a graph
+// 6.5 and 6.6), 4096 x 14336 13.0 and 14.2 (13.4).
+// A few SMs with two CTAs hold all others up (160 CTAs, 8 x 5120 x 5120 10.1 and 9.0; 144, 8 x 4608 x 7168 11.4 and 10.2), and short K
+// ranges leave nothing to hide behind (4 x 25416 x 1152 10.5 and 8.7). Where most SMs have two and K is long it wins again:
+// 8 x 28672 x 4096 21.6 and 22.3, 8 x 8192 x 28672 38.0 and 41.8; one or two rows are less work: 1 x 6144 x 4096 8.8 and 9.1. Over
+// 401 sizes of 1..8 rows, in a graph and one by one, this rule gains 4 % where it takes the kernel and is nowhere more than 5 % behind.
+// At 16 rows the quantiser warps no longer keep up with the weights at all: four projections of a 4096-wide layer 56.6 and 65.0 us
+// (with twice as many of them 56.2, but then 1 row takes 50.3 instead of 48.0).
+static bool quant_in_gemm_wins(int64_t M, int64_t N, int64_t K, int sms, int splits) {
+  const int64_t ctas = cdiv(N, 128) * splits, kb = cdiv(cdiv(K, 128), splits);
+  return ctas <= sms - 16 || (3 * ctas > 4 * sms && kb >= 15) || (M <= 2 && 9 * ctas > 10 * sms && kb >= (splits > 1 ? 7 : 15));
+}
 constexpr int64_t kLinearQuantInGemmMaxM = 8;
 static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K, int sms, GemmRoute* route) {
   const Tuning& tune = tuning();
   if (M > kLinearQuantInGemmMaxM || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
   const GemmPlan plan = plan_gemm(M, N, K, sms, true);
-  if (!plan.skinny || !skinny_split(M, N, K, plan.splits).direct()) return false;
+  const SkinnySplit split = skinny_split(M, N, K, plan.splits);
+  if (!plan.skinny || !split.direct()) return false;
+  if (tune.linear_decode_fused != 2 && !quant_in_gemm_wins(M, N, K, sms, split.splits)) return false;
   *route = skinny_route(M, N, K, plan.splits, false, B200_KERNEL_SKINNY_QUANT);
   return true;
 }

@@ -116,3 +116,14 @@ def test_fanout_workspace_covers_its_plan():
             p = _plan("fanout", m, n, k)
             need = p.splits * m * n * 4 if p.sum == "memory" else 0
             assert lib.b200_w8a8_block_fp8_gemm_fanout_workspace_bytes(m, n, k) >= need, (m, n, k, p)
+
+
+def test_quantiser_in_the_decode_gemm_where_it_hides():
+    """Measured against a quantiser of its own: ahead with at most one CTA per SM or two on nearly all and a long K, behind with
+    a few SMs that have two CTAs (8 x 5120 x 5120 10.1 us and 9.0) or a short K (4 x 25416 x 1152 10.5 and 8.7)."""
+    for m, n, k in [(1, 4096, 4096), (8, 4096, 4096), (8, 4096, 14336), (8, 28672, 4096), (1, 6144, 4096), (2, 6144, 4096), (8, 8192, 28672),
+                    (8, 57344, 8192), (1, 8192, 3584), (8, 14336, 8192)]:
+        assert _plan("linear", m, n, k, 148).kernel == "skinny_quant", (m, n, k)
+    for m, n, k in [(8, 5120, 5120), (4, 5120, 5120), (2, 5120, 5120), (8, 4608, 7168), (8, 6144, 4096), (8, 8192, 3584), (4, 22336, 1152),
+                    (1, 22400, 896), (4, 24576, 1536), (1, 32768, 512), (1, 16384, 1024), (9, 4096, 4096)]:
+        assert _plan("linear", m, n, k, 148).kernel == "skinny", (m, n, k)

@@ -25,14 +25,21 @@ def _same_bits(a, b):
 
 
 def _takes_it(M, N, K):
-    """Both routes, checked: the kernel with the quantiser, and the decode kernel with the same splits behind a quantiser."""
+    """Both routes, checked: the kernel with the quantiser (which the plan takes where it is the faster one, here everywhere), and
+    the decode kernel with the same splits behind a quantiser."""
     from sglang_b200 import _native as N_
 
-    fused = N_.plan_dense("linear", M, N, K)
+    with N_.tuning(linear_decode_fused=2):
+        fused = N_.plan_dense("linear", M, N, K)
     with N_.tuning(linear_decode_fused=0):
         apart = N_.plan_dense("linear", M, N, K)
     assert fused.kernel == "skinny_quant" and apart == fused._replace(kernel="skinny")
-    return fused
+
+
+def _fused():
+    from sglang_b200 import _native as N_
+
+    return N_.tuning(linear_decode_fused=2)
 
 
 # unsplit with one wave and with two, the largest scale table (64 K blocks a CTA), clusters of 2 to 8, a short last split,
@@ -46,15 +53,17 @@ def test_same_bits_as_quantiser_and_gemm(M, N, K, dtype):
 
     _takes_it(M, N, K)
     x, (w, s) = make_activation(M, K, M + K, dtype=dtype).cuda(), _weight(N, K, N + K)
-    out = S.w8a8_block_fp8_linear(x, w, [128, 128], s)
+    with _fused():
+        out = S.w8a8_block_fp8_linear(x, w, [128, 128], s)
     with N_.tuning(linear_decode_fused=0):
         apart = S.w8a8_block_fp8_linear(x, w, [128, 128], s)
     assert N_.read_device_status() == 0
     assert out.dtype == dtype and _same_bits(out, apart) and bool(out.float().abs().max() > 0)
 
 
-# small weights take it where a rank of the weight-streaming kernel would quantise more than 32 (row, K block) groups
-@pytest.mark.parametrize("M,N,K", [(4, 136, 8320), (8, 136, 8320), (5, 1280, 8192), (8, 1280, 8192), (8, 520, 16384)])
+# small weights: clusters of 5 to 8, a last split of one K block, one K block in all, fewer columns than a tile
+@pytest.mark.parametrize("M,N,K", [(4, 136, 8320), (8, 136, 8320), (5, 1280, 8192), (8, 1280, 8192), (8, 520, 16384), (8, 8, 128),
+                                   (3, 1032, 384), (7, 2048, 2176)])
 def test_same_bits_with_small_weights(M, N, K):
     test_same_bits_as_quantiser_and_gemm(M, N, K, torch.bfloat16)
 
@@ -71,9 +80,10 @@ def test_input_written_right_before_the_call(M, N, K):
     want = [S.w8a8_block_fp8_linear(x, w, [128, 128], s) for x in kept]
     torch.cuda.synchronize()
     x, wrong = torch.empty_like(kept[0]), []
-    for i in range(40):
-        x.copy_(kept[i % 2])
-        wrong.append((S.w8a8_block_fp8_linear(x, w, [128, 128], s) != want[i % 2]).sum())
+    with _fused():
+        for i in range(40):
+            x.copy_(kept[i % 2])
+            wrong.append((S.w8a8_block_fp8_linear(x, w, [128, 128], s) != want[i % 2]).sum())
     assert int(torch.stack(wrong).sum()) == 0
     assert N_.read_device_status() == 0
 
@@ -103,7 +113,8 @@ def test_chain_through_two_buffers(M):
         return bufs[steps % 2]
 
     for steps in (2, 3, 10, 31):
-        got = chain(steps, pause=False)
+        with _fused():
+            got = chain(steps, pause=False)
         with N_.tuning(linear_decode_fused=0):
             want = chain(steps, pause=True)
         assert _same_bits(got, want), steps
