@@ -143,7 +143,10 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   GemmPlan best = {1, 0, false, false, false, 1e30};  // its time without unpacking
   const double stream_us = (double)N * (double)K / 6.2e6;
   // K splits through memory: a reduction pass and the fp32 partials, written and read at about 2 TB/s
-  auto memory_sum = [&](int s) { return use.fanout ? 1.5 + 4.5 * s * (double)M * (double)N / 1e6 : 0.5 + 4.0 * s * (double)M * (double)N / 1e6; };
+  auto memory_sum = [&](int s) {
+    const double partials = s * (double)M * (double)N / 1e6;
+    return use.fanout ? 1.5 + 4.5 * partials : N <= 128 ? 2.2 + 2.3 * partials : 3.6 + 2.6 * partials;
+  };
   auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int first, int last) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
     for (int s = 1; s <= last && (s == 1 || num_kb >= 4 * s); ++s) {
@@ -164,7 +167,13 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
     // Splits of pairs go through memory on partitions of the part only: all of it sums them in clusters (below), whose numbers at
     // once are known for 148 SMs.
     const int max_splits = pairs && sms >= 148 ? 1 : 8;
-    consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.44, 1.0, 0, 1, max_splits);
+    if (N >= 256) {
+      consider(128, 256, sms, 3.5, 0.44, 1.0, 0, 1, max_splits);
+    } else if (N > 128) {  // 502 x 192 x 1536: unsplit 7.8 us, three splits 11.5, which the costs of the line above would take
+      consider(128, 256, sms, 3.1, 0.35, 0.7, 0, 1, max_splits);
+    } else {
+      consider(128, 128, sms, 3.1, 0.27, 0.05, 0, 1, max_splits);
+    }
     if (pairs) {
       consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1, max_splits);
       consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, 1, max_splits);

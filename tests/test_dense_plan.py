@@ -127,3 +127,14 @@ def test_quantiser_in_the_decode_gemm_where_it_hides():
     for m, n, k in [(8, 5120, 5120), (4, 5120, 5120), (2, 5120, 5120), (8, 4608, 7168), (8, 6144, 4096), (8, 8192, 3584), (4, 22336, 1152),
                     (1, 22400, 896), (4, 24576, 1536), (1, 32768, 512), (1, 16384, 1024), (9, 4096, 4096)]:
         assert _plan("linear", m, n, k, 148).kernel == "skinny", (m, n, k)
+
+
+def test_narrow_outputs_are_not_split_for_nothing():
+    """Fewer than 256 columns: a reduction pass costs 2 to 4 us, so 12 K blocks stay whole (502 x 192 x 1536 7.8 us, three splits
+    11.5; packed 502 x 120 x 1536 8.6 in splits), 64 do not (300 x 128 x 8192 20.6 us whole, 9.2 in eight splits)."""
+    for n in (64, 120, 128, 136, 192, 248):
+        for m in (300, 502, 959):
+            assert _plan("gemm", m, n, 1536, 148).splits == 1
+            assert _plan("gemm", m, n, 8192, 148).splits >= 4
+            p = _plan("packed", m, n, 1536, 148)
+            assert p.kernel == "block_scaled" or p.splits == 1
