@@ -94,20 +94,20 @@ static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
 }
 
 // Modelled time of the decode kernel. Its CTAs run two to an SM: one that has its SM to itself takes 0.20 us per 128-K block, one
-// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (4.6 TB/s) or, once per 32 rows, from
+// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (4.8 TB/s) or, once per 32 rows, from
 // L2 (10.7 TB/s). Over 370 sizes of 33 to 256 rows it is within 6 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most
 // of it where K is short: 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
 static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s, double sum) {
   const int64_t t_tiles = cdiv(M, skinny_token_tile(M)), ctas = cdiv(N, 128) * t_tiles * s.splits;
   const double kb = (double)cdiv(cdiv(K, 128), s.splits);
   double work = (double)(cdiv(ctas, 2 * sms) - 1) * (kb * 0.385 + 2.0) + kb * (ctas <= sms ? 0.20 : 0.385);
-  const double memory = (double)N * (double)K / 4.6e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
+  const double memory = (double)N * (double)K / 4.8e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
   if (work < memory) work = memory;
   if (work < l2) work = l2;
   return 2.9 + work + sum;
 }
 static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
-  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.28 * s.splits * (double)M * (double)N / 1e6;
+  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.2 * s.splits * (double)M * (double)N / 1e6;
   return skinny_us(M, N, K, sms, s, sum);
 }
 
@@ -205,8 +205,10 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   if (skinny_ok && M <= (tune.gemm_skinny_max_m >= 0 ? skinny_max : kSkinnyPlanMaxM)) {
     const int splits = skinny_k_splits(M, N, K, skinny_token_tile(M), sms);
     const SkinnySplit split = skinny_split(M, N, K, splits);
-    const double us = use.fanout ? skinny_us(M, N, K, sms, split, 0.0) + 1.2 + 1.27 * split.splits * (double)M * (double)N / 1e6
-                                 : skinny_us(M, N, K, sms, split);
+    double us = use.fanout ? skinny_us(M, N, K, sms, split, 0.0) + 1.2 + 1.27 * split.splits * (double)M * (double)N / 1e6
+                           : skinny_us(M, N, K, sms, split);
+    // packed words are staged by each CTA before its first sum: 64 x 14336 x 8192, 64 K blocks, 35 us (30 on fp32 scales)
+    if (use.unpack_us > 0.0) us += 0.02 * (double)cdiv(num_kb, split.splits);
     if (us < best.us + use.unpack_us) best = {splits, 0, true, false, false, us};
   }
   if (!best.skinny) best.us += use.unpack_us;
