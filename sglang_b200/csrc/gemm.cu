@@ -93,21 +93,24 @@ static SkinnySplit skinny_split(int64_t M, int64_t N, int64_t K, int splits) {
   return cluster > 1 ? SkinnySplit{cluster, true} : SkinnySplit{splits, false};
 }
 
-// Modelled time of the decode kernel. Its CTAs run two to an SM: one that has its SM to itself takes 0.20 us per 128-K block, one
-// that shares it 0.385, whole waves add up, and nothing is faster than the weights from memory (4.8 TB/s) or, once per 32 rows, from
-// L2 (10.7 TB/s). Over 370 sizes of 33 to 256 rows it is within 6 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most
-// of it where K is short: 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
+// Modelled time of the decode kernel. Its CTAs run two to an SM: one that has its SM to itself takes 0.22 us per 128-K block, one
+// that shares it 0.39. More CTAs than places are partly whole waves and partly fill in as others end (long K ranges drift apart);
+// nothing is faster than the weights from memory (5.4 TB/s; 4.4 where they nearly fill the L2, which the next token tile then misses:
+// 64 x 8192 x 7168 16.0 us, x 14336 31.3) or, once per 32 rows, from L2 (12.5 TB/s). Over 450 sizes of 34 to 256
+// rows it is within 5 % on average; a rate per byte alone (9.5 TB/s) was 12 % off, most of it where K is short:
+// 65..128 x 8192 x 512 4.3 us, 8.5 modelled, so the plan took pairs at 5.4.
 static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s, double sum) {
   const int64_t t_tiles = cdiv(M, skinny_token_tile(M)), ctas = cdiv(N, 128) * t_tiles * s.splits;
-  const double kb = (double)cdiv(cdiv(K, 128), s.splits);
-  double work = (double)(cdiv(ctas, 2 * sms) - 1) * (kb * 0.385 + 2.0) + kb * (ctas <= sms ? 0.20 : 0.385);
-  const double memory = (double)N * (double)K / 4.8e6, l2 = (double)t_tiles * (double)N * (double)K / 10.7e6;
+  const double kb = (double)cdiv(cdiv(K, 128), s.splits), places = 2.0 * sms, waves = (double)cdiv(ctas, 2 * sms);
+  double work = ctas <= sms ? kb * 0.222 : kb * 0.389;
+  if (waves > 1.0) work = kb * 0.389 * (0.56 * waves + 0.44 * (double)ctas / places) + 2.6 * (waves - 1.0);
+  const double memory = (double)N * (double)K / (N * K > (96 << 20) ? 4.4e6 : 5.4e6), l2 = (double)t_tiles * (double)N * (double)K / 12.5e6;
   if (work < memory) work = memory;
   if (work < l2) work = l2;
-  return 2.9 + work + sum;
+  return 2.67 + work + sum;
 }
 static double skinny_us(int64_t M, int64_t N, int64_t K, int sms, SkinnySplit s) {
-  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.1 : 0.7 + 1.2 * s.splits * (double)M * (double)N / 1e6;
+  const double sum = s.splits == 1 ? 0.0 : s.cluster ? 2.0 : 0.78 + 1.52 * s.splits * (double)M * (double)N / 1e6;
   return skinny_us(M, N, K, sms, s, sum);
 }
 
@@ -147,37 +150,41 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
     const double partials = s * (double)M * (double)N / 1e6;
     return use.fanout ? 1.5 + 4.5 * partials : N <= 128 ? 2.2 + 2.3 * partials : 3.6 + 2.6 * partials;
   };
-  auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, int pair_bn, int first, int last) {
+  // crowd: what tiles side by side cost one another when every slot has one (256 x 4096 x 1024, 32 pairs, 5.4 us; 64 x 8192 x 1024, 64
+  // pairs, 7.1)
+  auto consider = [&](int bm, int bn, int slots, double base, double us_per_kb, double epilogue, double crowd, int pair_bn, int first,
+                      int last) {
     const int64_t tiles = cdiv(M, bm) * cdiv(N, bn);
+    const double busy = tiles < slots ? (double)tiles / slots : 1.0;
     for (int s = 1; s <= last && (s == 1 || num_kb >= 4 * s); ++s) {
       const double waves = (double)cdiv(tiles * s, slots);
       double work = waves * ((double)cdiv(num_kb, s) * us_per_kb + epilogue);
       if (work < stream_us) work = stream_us;
-      const double us = base + work + (s > 1 ? memory_sum(s) : 0.0);
+      const double us = base + crowd * busy + work + (s > 1 ? memory_sum(s) : 0.0);
       if (s >= first && us < best.us) best = {s, pair_bn, false, false, false, us};
       if (tiles * s >= slots) break;  // every slot is busy: more splits only add partials
     }
   };
   const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256 && sms >= 2;
   if (use.fanout) {
-    consider(128, N > 128 ? 256 : 128, sms, 4.0, 0.64, 1.5, 0, 1, 1);
-    consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.55, 1.0, 0, 2, 8);
-    if (pairs) consider(256, 128, sms / 2, 3.8, 0.225, 0.85, 128, 2, 8);
+    consider(128, N > 128 ? 256 : 128, sms, 4.0, 0.64, 1.5, 0.0, 0, 1, 1);
+    consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.55, 1.0, 0.0, 0, 2, 8);
+    if (pairs) consider(256, 128, sms / 2, 3.8, 0.225, 0.85, 0.0, 128, 2, 8);
   } else {
     // Splits of pairs go through memory on partitions of the part only: all of it sums them in clusters (below), whose numbers at
     // once are known for 148 SMs.
     const int max_splits = pairs && sms >= 148 ? 1 : 8;
     if (N >= 256) {
-      consider(128, 256, sms, 3.5, 0.44, 1.0, 0, 1, max_splits);
+      consider(128, 256, sms, 3.5, 0.44, 1.0, 0.0, 0, 1, max_splits);
     } else if (N > 128) {  // 502 x 192 x 1536: unsplit 7.8 us, three splits 11.5, which the costs of the line above would take
-      consider(128, 256, sms, 3.1, 0.35, 0.7, 0, 1, max_splits);
+      consider(128, 256, sms, 3.1, 0.35, 0.7, 0.0, 0, 1, max_splits);
     } else {
-      consider(128, 128, sms, 3.1, 0.27, 0.05, 0, 1, max_splits);
+      consider(128, 128, sms, 3.1, 0.27, 0.05, 0.0, 0, 1, max_splits);
     }
     if (pairs) {
-      consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 256, 1, max_splits);
-      consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 192, 1, max_splits);
-      consider(256, 128, sms / 2, 3.8, 0.22, 0.85, 128, 1, max_splits);
+      consider(256, 256, sms / 2, 3.5, 0.38, 1.8, 0.0, 256, 1, max_splits);
+      consider(256, 192, sms / 2, 4.25, 0.35, 1.2, 0.0, 192, 1, max_splits);
+      consider(256, 128, sms / 2, 3.1, 0.225, 0.85, 1.0, 128, 1, max_splits);
     }
   }
   if (pairs && !use.fanout && sms >= 148) {
@@ -186,7 +193,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       if (tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
       double work = (double)cdiv(num_kb, s) * (s == 2 ? 0.21 : 0.18);
       if (work < stream_us) work = stream_us;
-      const double us = (s == 2 ? 6.5 : 7.75) + work;
+      const double us = (s == 2 ? 5.97 : 7.4) + work;
       if (us < best.us) best = {s, 128, false, false, true, us};
     }
   }
@@ -431,7 +438,8 @@ static bool linear_one_launch(int64_t M, int64_t N, int64_t K, int sms, int* ran
 // (with twice as many of them 56.2, but then 1 row takes 50.3 instead of 48.0).
 static bool quant_in_gemm_wins(int64_t M, int64_t N, int64_t K, int sms, int splits) {
   const int64_t ctas = cdiv(N, 128) * splits, kb = cdiv(cdiv(K, 128), splits);
-  return ctas <= sms - 16 || (3 * ctas > 4 * sms && kb >= 15) || (M <= 2 && 9 * ctas > 10 * sms && kb >= (splits > 1 ? 7 : 15));
+  return ctas <= sms - 16 || (3 * ctas > 4 * sms && kb >= 15) || 
+         (M <= 2 && ((ctas > sms && kb >= 15) || (splits > 1 && 9 * ctas > 10 * sms && kb >= 7)));
 }
 constexpr int64_t kLinearQuantInGemmMaxM = 8;
 static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K, int sms, GemmRoute* route) {
@@ -515,14 +523,17 @@ extern "C" int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, con
 }
 
 namespace b200 {
-// Modelled time of the block-scaled kernels (see plan_gemm; fitted to 560 sizes of 65..2200 rows): a CTA's 128 x 224 tile takes
-// 0.40 us per 128-K block, a pair's 256 x 240 one 0.32, so the pair does more than twice the work per SM clock where whole waves
-// allow it (3000 x 4096 x 14336: 2759 against 2244 TFLOP/s); it starts 2 us later (400 x 8192 x 1024: single 8.1 us, pair 9.8;
-// 160 x 14336 x 4096 18.8 and 17.8).
+// Modelled time of the block-scaled kernels (see plan_gemm; fitted to 590 sizes of 65..2200 rows, within 8 %): launch and set-up, whole
+// waves of tiles, a CTA's 128 x 224 at 0.34 us per 128-K block, a pair's 256 x 240 at 0.30, and the operands, of which a pair halves
+// what it reads of the weights: 160 x 14336 x 4096 18.8 and 17.8 us, 3000 x 4096 x 14336 2244 and 2759 TFLOP/s; 1500 x 2560 x 4096
+// 15.7 and 16.6, 400 x 8192 x 1024 8.1 and 9.8.
 static double block_scaled_us(int64_t M, int64_t N, int64_t K, int sms, bool pair) {
-  const int64_t tiles = pair ? cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN) : cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN);
   if (pair && sms < 2) return 1e30;
-  return (pair ? 6.0 : 4.0) + (double)cdiv(tiles, pair ? sms / 2 : sms) * ((double)cdiv(K, 128) * (pair ? 0.32 : 0.40) + 1.2);
+  const double num_kb = (double)cdiv(K, 128), weights = (double)N * (double)K / 1e6, rows = (double)M * (double)K / 1e6;
+  if (N < 256) return (pair ? 4.4 : 3.0) + (N > 128 ? 1.0 : 0.0) + num_kb * 0.26;  // narrow, few tiles: 2135 x 80 x 256 3.5 us
+  if (pair)
+    return 4.73 + (double)cdiv(cdiv(M, 256) * cdiv(N, Ue8m0PairCfg::BN), sms / 2) * (num_kb * 0.303 + 0.99) + 0.019 * weights + 0.051 * rows;
+  return 3.46 + (double)cdiv(cdiv(M, 128) * cdiv(N, Ue8m0Cfg::BN), sms) * (num_kb * 0.343 + 0.96) + 0.027 * weights;
 }
 static bool block_scaled_pair(int64_t M, int64_t N, int64_t K, int sms) {
   const long knob = tuning().gemm_ue8m0;
@@ -591,15 +602,15 @@ __global__ void __launch_bounds__(256) unpack_scales_kernel(const int32_t* __res
 
 constexpr double kUnpackUs = 1.1;
 // Whether the block-scaled kernels (scales applied by the tensor core, no K split) beat the promotion kernels on unpacked
-// scales, or the decode kernel, which reads the packed words itself: below 65 rows the weight stream decides, then wave counts.
-// Long problems run at the power cap, where applying scales in the tensor core pays beyond the model (1500 x 4096 x 14336: 75.7 us
-// against 85.5). With this margin the choice is 0.6 % behind the best on those sizes (203 x 4096 x 14336: 46 us block-scaled, 25
-// promoted; 96 x 5120 x 1536 9.4 and 7.2 in the decode kernel; 204 x 336 x 1152 6.6 and 4.9).
+// scales, or the decode kernel, which reads the packed words itself: below 65 rows the weight stream decides, then the modelled
+// times (which know nothing of the power cap, at which applying scales in the tensor core pays: 4 %). The choice is 0.6 % behind
+// the best on those sizes (203 x 4096 x 14336: 46 us block-scaled, 25 promoted; 96 x 5120 x 1536 9.4 and 7.2 in the decode
+// kernel; 204 x 336 x 1152 6.6 and 4.9; 1500 x 4096 x 14336 75.7 and 85.5).
 static bool block_scaled_wins(int64_t M, int64_t N, int64_t K, int sms) {
   if (tuning().gemm_ue8m0 > 0) return true;
   if (M <= 64) return false;
   const double one = block_scaled_us(M, N, K, sms, false), two = block_scaled_us(M, N, K, sms, true);
-  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true, PlanFor{false, kUnpackUs}).us * 1.04 + 1.0;
+  return (one < two ? one : two) <= plan_gemm(M, N, K, sms, true, PlanFor{false, kUnpackUs}).us * (N < 256 ? 1.0 : 1.04);
 }
 static size_t packed_as_bytes(int64_t M, int64_t K) { return align_up((size_t)(M * cdiv(K, 128)) * 4, 256); }
 static size_t packed_bs_bytes(int64_t N, int64_t K) { return align_up((size_t)(cdiv(N, 128) * cdiv(K, 128)) * 4, 256); }
