@@ -264,7 +264,8 @@ static GemmRoute route_gemm(int64_t M, int64_t N, int64_t K, int sms, PlanFor us
   if (plan.skinny) return skinny_route(M, N, K, splits, use.fanout, B200_KERNEL_SKINNY);
   // the 8-warp tile kernel keeps the 128-wide tile (N <= 128) and the fan-out epilogue
   const bool wide = force_bn == 0 && N > 128 && tune.gemm_2cta != 0;
-  if (plan.csum && wide && !use.fanout && tune.gemm_splitk <= 0) return {B200_KERNEL_WIDE, plan.pair_bn, splits, B200_SUM_CLUSTER};
+  // as many splits as the cluster has pairs, some of them empty where K has fewer blocks
+  if (plan.csum && wide && !use.fanout && tune.gemm_splitk <= 0) return {B200_KERNEL_WIDE, plan.pair_bn, plan.splits, B200_SUM_CLUSTER};
   const int sum = splits > 1 ? B200_SUM_MEMORY : B200_SUM_NONE;
   if (wide && (splits > 1 || !use.fanout)) return {B200_KERNEL_WIDE, plan.pair_bn, splits, sum};
   return {B200_KERNEL_TILE, force_bn, splits, sum};

@@ -556,7 +556,11 @@ inline int launch_gemm_wide(const void* A, const void* B, GemmParams p, int k_sp
 // bn: columns of a pair's tile, or 0: single CTAs. csum: the K splits (2 or 4) are summed within clusters (128-wide pairs).
 template <typename OutT>
 inline int launch_gemm_wide(int bn, const void* A, const void* B, const GemmParams& p, int k_splits, bool csum, cudaStream_t st) {
-  if (csum) return k_splits == 2 ? launch_gemm_wide<2, 128, 2, OutT>(A, B, p, 2, st) : launch_gemm_wide<2, 128, 4, OutT>(A, B, p, 4, st);
+  if (csum) {
+    B200_UNSUPPORTED(bn != 128 || (k_splits != 2 && k_splits != 4), "gemm: clusters sum 2 or 4 K splits of 128-wide pairs, not %d of %d",
+                     k_splits, bn);
+    return k_splits == 2 ? launch_gemm_wide<2, 128, 2, OutT>(A, B, p, 2, st) : launch_gemm_wide<2, 128, 4, OutT>(A, B, p, 4, st);
+  }
   if (bn == 0) return launch_gemm_wide<1, 256, 0, OutT>(A, B, p, k_splits, st);
   if (bn == 128) return launch_gemm_wide<2, 128, 0, OutT>(A, B, p, k_splits, st);
   if (bn == 192) return launch_gemm_wide<2, 192, 0, OutT>(A, B, p, k_splits, st);

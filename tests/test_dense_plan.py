@@ -129,6 +129,16 @@ def test_quantiser_in_the_decode_gemm_where_it_hides():
         assert _plan("linear", m, n, k, 148).kernel == "skinny", (m, n, k)
 
 
+def test_clusters_have_the_splits_that_were_asked_for():
+    """Two or four pairs, whatever K has: a split without K blocks adds zeros."""
+    from sglang_b200 import _native as N
+
+    for knob, splits in [(1282, 2), (1284, 4)]:
+        for k in (128, 256, 384, 640, 4096):
+            with N.tuning(gemm_2cta=knob, gemm_skinny=0):
+                assert _plan("gemm", 200, 264, k, 148) == ("wide", 128, splits, "cluster"), (knob, k)
+
+
 def test_narrow_outputs_are_not_split_for_nothing():
     """Fewer than 256 columns: a reduction pass costs 2 to 4 us, so 12 K blocks stay whole (502 x 192 x 1536 7.8 us, three splits
     11.5; packed 502 x 120 x 1536 8.6 in splits), 64 do not (300 x 128 x 8192 20.6 us whole, 9.2 in eight splits)."""
