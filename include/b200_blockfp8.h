@@ -193,9 +193,11 @@ int b200_w8a8_block_fp8_linear_decode(const void* x, int x_dtype, const void* B,
  * w8a8_block_fp8_linear: quantise + GEMM of one linear layer in one call, any M
  * replaces: python/sglang/srt/layers/quantization/fp8_utils.py:814-834 (the same composition)
  * out = the result of b200_per_token_group_quant_fp8 (group 128) followed by b200_w8a8_block_fp8_gemm,
- * with the kernels chained as programmatic dependents (a few rows: the one-launch kernel above).
- * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out as above.
- * workspace: b200_w8a8_block_fp8_linear_workspace_bytes(M,N,K) bytes, 256-byte aligned. */
+ * with the kernels chained as programmatic dependents.
+ * x [M,K] bf16/f16 row-major, K % 128 == 0, N % 8 == 0; B, Bs, out as above. Up to 16 rows one kernel may do it all: the one-launch kernel above for
+ * small weights, the decode GEMM that quantises its own input (up to 8 rows) where that is faster (b200_plan_dense says which).
+ * workspace: b200_w8a8_block_fp8_linear_workspace_bytes(M,N,K) bytes, 256-byte aligned; a call that runs as one kernel does not
+ * look at it, whatever the query says. */
 size_t b200_w8a8_block_fp8_linear_workspace_bytes(int64_t M, int64_t N, int64_t K);
 int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void* B, const float* Bs, void* out,
                                int64_t M, int64_t N, int64_t K, void* workspace, size_t workspace_bytes,

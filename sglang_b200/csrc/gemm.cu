@@ -227,7 +227,8 @@ namespace b200 {
 // fp32 partials of the split that this device's SMs pick, 148 without a device (or the tuning knobs force)
 static size_t partial_bytes(int64_t M, int64_t N, int64_t K, PlanFor use = {}) {
   const Tuning& tune = tuning();
-  int s = plan_gemm(M, N, K, plan_sms(), tune.gemm_bn < 0, use).splits;
+  const GemmPlan plan = plan_gemm(M, N, K, plan_sms(), tune.gemm_bn < 0, use);
+  int s = plan.csum && !use.fanout ? 1 : plan.splits;  // summed in clusters
   if (tune.gemm_splitk > s) s = (int)tune.gemm_splitk;
   if (tune.gemm_skinny_max_m >= 0 && s < 16) s = 16;
   return s > 1 ? (size_t)s * (size_t)M * (size_t)N * sizeof(float) : 0;
@@ -482,11 +483,6 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
   B200_CHECK_ARG(x && B && Bs && out, "linear: null pointer");
   B200_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)B & 15) == 0, "linear: x and B must be 16-byte aligned");
   B200_UNSUPPORTED(N % 8 != 0, "linear: N=%lld must be a multiple of 8", (long long)N);
-  const size_t need = b200_w8a8_block_fp8_linear_workspace_bytes(M, N, K);
-  if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0)) {
-    set_error_detail("linear: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
-    return B200_E_WORKSPACE;
-  }
   const GemmRoute r = route_linear(M, N, K, sm_count());
   if (r.kernel == B200_KERNEL_STREAM_QUANT) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
   if (r.kernel == B200_KERNEL_SKINNY_QUANT) {
@@ -495,6 +491,11 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
     SkinnyParams sp = {};
     sp.x = x; sp.eps = 1e-10f; sp.Bs = Bs;
     return run_skinny(nullptr, B, sp, r, out, x_dtype, M, N, K, nullptr, 0, static_cast<cudaStream_t>(stream), FanOut{});
+  }
+  const size_t need = b200_w8a8_block_fp8_linear_workspace_bytes(M, N, K);
+  if (need && (!workspace || workspace_bytes < need || ((uintptr_t)workspace & 255) != 0)) {
+    set_error_detail("linear: workspace %zu < %zu bytes or not 256-byte aligned", workspace_bytes, need);
+    return B200_E_WORKSPACE;
   }
   uint8_t* q = static_cast<uint8_t*>(workspace);
   float* s = reinterpret_cast<float*>(q + linear_q_bytes(M, K));

@@ -111,6 +111,8 @@ def test_fanout_workspace_covers_its_plan():
     from sglang_b200 import _native as N
 
     lib = N.load()
+    with N.tuning(gemm_2cta=1284, gemm_skinny=0):  # clusters asked for: a fan-out takes as many splits through memory
+        assert lib.b200_w8a8_block_fp8_gemm_fanout_workspace_bytes(300, 1024, 4096) >= 4 * 300 * 1024 * 4
     for m in (1, 16, 33, 100, 256, 300, 700):
         for n, k in [(128, 8192), (200, 4096), (1024, 8192), (4096, 1792), (2112, 7168), (4096, 14336)]:
             p = _plan("fanout", m, n, k)
@@ -148,3 +150,28 @@ def test_narrow_outputs_are_not_split_for_nothing():
             assert _plan("gemm", m, n, 8192, 148).splits >= 4
             p = _plan("packed", m, n, 1536, 148)
             assert p.kernel == "block_scaled" or p.splits == 1
+
+
+def test_workspace_of_sums_in_clusters():
+    """CTA pairs that sum their K splits in clusters write no partials; everything else is covered by the query."""
+    from sglang_b200 import _native as N
+
+    lib = N.load()
+    for m, n, k in [(203, 4096, 4096), (203, 4096, 14336), (512, 1280, 8192), (300, 512, 16384)]:
+        assert _plan("gemm", m, n, k).sum == "cluster" and _plan("gemm", m, n, k).kernel == "wide"
+        assert lib.b200_w8a8_block_fp8_gemm_workspace_bytes(m, n, k) == 0, (m, n, k)
+    for m in (1, 16, 33, 64, 100, 203, 256, 300, 700, 2000):
+        for n, k in [(64, 8192), (200, 4096), (1024, 8192), (4096, 1792), (2112, 7168), (4096, 14336), (28672, 4096)]:
+            p = _plan("gemm", m, n, k)
+            need = p.splits * m * n * 4 if p.sum == "memory" else 0
+            assert lib.b200_w8a8_block_fp8_gemm_workspace_bytes(m, n, k) >= need, (m, n, k, p)
+
+
+def test_linear_wants_a_workspace_only_for_two_launches():
+    """Without one, a size that runs as quantiser and GEMM is refused before anything is launched."""
+    from sglang_b200 import _native as N
+
+    lib, fake = N.load(), 1 << 20  # never read
+    for m, n, k in [(9, 4096, 4096), (8, 5120, 5120), (203, 4096, 4096), (1027, 4096, 4096)]:
+        assert not _plan("linear", m, n, k).kernel.endswith("quant")
+        assert lib.b200_w8a8_block_fp8_linear(fake, N.BF16, fake, fake, fake, m, n, k, None, 0, None) == N.E_WORKSPACE

@@ -88,6 +88,21 @@ def test_input_written_right_before_the_call(M, N, K):
     assert N_.read_device_status() == 0
 
 
+@pytest.mark.parametrize("M,N,K", [(1, 4096, 4096), (8, 4096, 14336), (1, 1536, 4096)])
+def test_one_kernel_needs_no_workspace(M, N, K):
+    import sglang_b200 as S
+    from sglang_b200 import _native as N_
+
+    assert N_.plan_dense("linear", M, N, K).kernel.endswith("quant")
+    x, (w, s) = make_activation(M, K, 6).cuda(), _weight(N, K, 7)
+    out = torch.empty(M, N, dtype=x.dtype, device="cuda")
+    st = N_.load().b200_w8a8_block_fp8_linear(x.data_ptr(), N_.BF16, w.data_ptr(), s.data_ptr(), out.data_ptr(), M, N, K, None, 0,
+                                              N_.current_stream())
+    N_.check(st, "linear")
+    assert _same_bits(out, S.w8a8_block_fp8_linear(x, w, [128, 128], s))
+    assert N_.read_device_status() == 0
+
+
 @pytest.mark.parametrize("M", [1, 8])
 def test_chain_through_two_buffers(M):
     """Linears that read what the one before has written and overwrite what it has read: each starts while the one before, and
