@@ -440,17 +440,17 @@ static bool linear_one_launch(int64_t M, int64_t N, int64_t K, int sms, int* ran
 // (with twice as many of them 56.2, but then 1 row takes 50.3 instead of 48.0).
 static bool quant_in_gemm_wins(int64_t M, int64_t N, int64_t K, int sms, int splits) {
   const int64_t ctas = cdiv(N, 128) * splits, kb = cdiv(cdiv(K, 128), splits);
-  return ctas <= sms - 16 || (3 * ctas > 4 * sms && kb >= 15) || 
+  return ctas <= sms - 16 || (3 * ctas > 4 * sms && kb >= 15) ||
          (M <= 2 && ((ctas > sms && kb >= 15) || (splits > 1 && 9 * ctas > 10 * sms && kb >= 7)));
 }
-constexpr int64_t kLinearQuantInGemmMaxM = 8;
 static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K, int sms, GemmRoute* route) {
   const Tuning& tune = tuning();
-  if (M > kLinearQuantInGemmMaxM || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
+  const bool forced = tune.linear_decode_fused == 2;  // the launch refuses what the kernel cannot take
+  if ((M > SkinnyCfg<16, true>::kQuantRows && !forced) || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
   const GemmPlan plan = plan_gemm(M, N, K, sms, true);
   const SkinnySplit split = skinny_split(M, N, K, plan.splits);
   if (!plan.skinny || !split.direct()) return false;
-  if (tune.linear_decode_fused != 2 && !quant_in_gemm_wins(M, N, K, sms, split.splits)) return false;
+  if (!forced && !quant_in_gemm_wins(M, N, K, sms, split.splits)) return false;
   *route = skinny_route(M, N, K, plan.splits, false, B200_KERNEL_SKINNY_QUANT);
   return true;
 }

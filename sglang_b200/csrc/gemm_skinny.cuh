@@ -43,6 +43,7 @@ struct SkinnyCfg {
   static constexpr int kStages = 5;
   static constexpr int kStageW = 128 * kBK;  // 16 KB of weights
   static constexpr int kStageX = NT * kBK;   // 2 or 4 KB of activations
+  static constexpr int kQuantRows = 8;  // QUANT: rows that the quantiser warps cover
   static constexpr int kQuantWarps = 4, kThreads = (QUANT ? 6 + kQuantWarps : 6) * 32;  // 4 promotion warps, producer, MMA issuer (, quantisers)
   // TMEM accumulator buffers: the tensor core runs this many K blocks ahead of the promotion warps, so the
   // commit -> tcgen05.ld -> arrive round trip (about a microsecond) is off the per-K-block path
@@ -99,7 +100,7 @@ block_fp8_gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_w, const _
   // K blocks at most are under way: with more than the ring's stages a group would wait for a phase of a stage's barrier that is
   // two ahead of it, which the parity does not tell from the one before.
   const int rows = min(NT, p.M - m0);
-  const int q_rows = rows <= 4 ? 4 : 8;
+  const int q_rows = rows <= 4 ? 4 : Cfg::kQuantRows;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < S; ++s) {
@@ -379,9 +380,12 @@ inline int launch_skinny_inst(const CUtensorMap& tw, const CUtensorMap& tx, cons
                           p.cluster ? p.k_splits : 1, "block_fp8_gemm_skinny_kernel", tw, tx, p);
 }
 
-// out: OutT [M, N] when splits == 1 or they are a cluster, else fp32 partials [splits][M, N]. X null: p.x is quantised (16 rows at most).
+// out: OutT [M, N] when splits == 1 or they are a cluster, else fp32 partials [splits][M, N]. X null: p.x is quantised.
 template <typename OutT>
 inline int launch_skinny(const void* X, const void* W, SkinnyParams p, int splits, bool cluster, cudaStream_t st) {
+  constexpr int kQuantRows = SkinnyCfg<16, true>::kQuantRows;
+  B200_UNSUPPORTED(X == nullptr && (p.M > kQuantRows || sizeof(OutT) != 2),
+                   "gemm: the decode kernel quantises %d rows of 16-bit input at most, not %d", kQuantRows, p.M);
   const int nt = skinny_token_tile(p.M);
   p.num_kb = (int)cdiv(p.K, kBK);
   p.n_tiles = (int)cdiv(p.N, 128);

@@ -75,3 +75,14 @@ def test_tuning_knobs_round_trip_without_a_gpu():
     with N.tuning(gemm_splitk=4):
         assert lib.b200_w8a8_block_fp8_gemm_workspace_bytes(4096, 4096, 4096) == 4 * 4096 * 4096 * 4
     assert lib.b200_w8a8_block_fp8_gemm_workspace_bytes(4096, 4096, 4096) == plain
+
+
+def test_the_decode_kernel_refuses_rows_that_it_does_not_quantise():
+    """Its quantiser warps cover eight rows; a ninth is refused by the launch itself, not left unwritten."""
+    from sglang_b200 import _native as N
+
+    lib, fake = N.load(), 1 << 20  # never read: without a workspace no other route gets as far as a launch
+    for m in (9, 12, 16):
+        with N.tuning(linear_decode_fused=2):
+            st = lib.b200_w8a8_block_fp8_linear(fake, N.BF16, fake, fake, fake, m, 4096, 4096, None, 0, None)
+        assert st == N.E_UNSUPPORTED and b"8 rows" in lib.b200_last_error_detail(), (m, st)
