@@ -346,7 +346,8 @@ block_fp8_gemm_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_c
         if (MODE != GEMM_DENSE && p.expert_ids[mt] < 0) continue;
         for (int kb = kb0; kb < kb1; ++kb, ++it) {
           const int s = it % S, b = it & 1;
-          // looped, polled one after the other: 16384 tokens through 256 experts 8540 us, together 8410
+          // looped, polled one after the other: 16384 tokens through 256 experts 8540 us, together 8410 (1.5 %, as much as
+          // repeats of the whole pass differ)
           ok = ptx::mbar_wait2(full_bar(s), (it / S) & 1, tempty_bar(b), ((it >> 1) & 1) ^ 1, abort_flag);
           if (!ok) break;
           ptx::tc_fence_after();

@@ -22,7 +22,8 @@
 //   tfull[b]  (each CTA)  likewise
 //   tempty[b] (leader's)  32 arrivals: the promotion warps of both CTAs
 // The MMA warp's own trip (two polls, four MMAs, two commits) bounds the 128-wide tile; both barriers are polled at once.
-// Shared memory is next: a K block writes 24 KB and reads 24 to 32 KB (128 wide), 375 to 440 clocks at 128 B/clk, against 430 measured.
+// Shared memory is next: a K block writes 24 KB and reads 24 to 32 KB (128 wide), 384 to 448 clocks at 128 B/clk, against 430 measured.
+// The scale reads take four wavefronts each (lanes 8 apart share a bank): 64 of those clocks, 16 without the conflict.
 // Polled one after the other, and with 5 stages instead of 7: 203 x 8192 x 7168 20.8 -> 18.7 us, 512 x 4096 x 14336 35.0 -> 32.4.
 // Looped, with the copies (120 instructions per warp and K block) and without (97): 8192 x 4096 x 4096 143 -> 134 us,
 // 1027 x 7168 x 8192 78.6 -> 73.3, 203 x 6144 x 4096 (128-wide tiles) 15.1 -> 13.2.
@@ -157,8 +158,8 @@ __device__ __forceinline__ void prefetch_first_weights(const GemmParams& p, int 
 
 // OutT: 16-bit output [M, N], or fp32 (C + split * split_stride: partial sums of a K split, or an fp32 result)
 // CS > 0: the K splits of a tile, CS of them (2 or 4), are one cluster. Each of them sums and stores its share of the columns; the
-// others hand theirs over through distributed shared memory, in the ring, which is idle by then. 64 KB move at most per CTA, and no
-// fp32 partials in memory nor a reduction launch: 203 x 4096 x 4096 12.5 us unsplit -> 10.3 with 2 splits, 203 x 4096 x 14336 24.5
+// others hand theirs over through distributed shared memory, in the ring, which is idle by then: 32 or 48 of the 64 KB that a CTA holds, and no
+// fp32 partials in memory nor a reduction launch: 203 x 4096 x 4096 12.5 us unsplit -> 10.3 in two splits, 203 x 4096 x 14336 24.5
 // with partials in memory -> 19.7.
 template <int CTAS, int BN, int CS, typename OutT>
 __global__ void __cluster_dims__(CTAS * (CS ? CS : 1), 1, 1) __launch_bounds__(Wide<CTAS, BN>::kThreads, 1)
