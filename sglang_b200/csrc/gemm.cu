@@ -167,7 +167,9 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
   };
   const bool pairs = may_pair && tune.gemm_2cta != 0 && N >= 256 && sms >= 2;
   if (use.fanout) {
-    consider(128, N > 128 ? 256 : 128, sms, 4.0, 0.64, 1.5, 0.0, 0, 1, 1);
+    if (N >= 256) consider(128, 256, sms, 4.0, 0.64, 1.5, 0.0, 0, 1, 1);
+    else if (N > 128) consider(128, 256, sms, 3.7, 0.45, 1.5, 0.0, 0, 1, 1);
+    else consider(128, 128, sms, 3.7, 0.30, 0.5, 0.0, 0, 1, 1);
     consider(128, N > 128 ? 256 : 128, sms, 3.5, 0.55, 1.0, 0.0, 0, 2, 8);
     if (pairs) consider(256, 128, sms / 2, 3.8, 0.225, 0.85, 0.0, 128, 2, 8);
   } else {
@@ -193,7 +195,7 @@ static GemmPlan plan_gemm(int64_t M, int64_t N, int64_t K, int sms, bool may_pai
       if (tiles > (s == 2 ? 33 : 15) || num_kb < 4 * s) continue;
       double work = (double)cdiv(num_kb, s) * (s == 2 ? 0.21 : 0.18);
       if (work < stream_us) work = stream_us;
-      const double us = (s == 2 ? 5.97 : 7.4) + work;
+      const double us = (s == 2 ? 5.2 + 1.5 * (double)(2 * tiles) / 74.0 : 7.4) + work;
       if (us < best.us) best = {s, 128, false, false, true, us};
     }
   }
