@@ -122,7 +122,7 @@ static int plan_sms() { return sm_count() < 148 ? sm_count() : 148; }
 // tiles of 128-wide pairs leave half of the chip idle their K range is split 2 or 4 ways within clusters, of which this part holds
 // 33 and 15 at once; the sum costs 2 to 3 us. The constants are fits to every kernel's time at 632 sizes, 16 weight shapes (1280..28672
 // x 1024..14336) times 17 row counts (33..2200) and as many spread over 17..2200 x 136..16384 x 256..16384: the plan is
-// 0.6 % behind the best kernel on average. E.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, their K split two ways
+// 0.4 % behind the best kernel on average up to 256 rows, 1 % over all (at the power cap repeats of one kernel differ by more). E.g. 203 x 4096 x 4096: decode kernel 14.1 us, pairs 128 wide 12.5, their K split two ways
 // 10.3; 203 x 4096 x 14336: 24.5 with partials through memory, 19.7; 512 x 1280 x 8192 16.6 and 13.9.
 //
 // A fan-out (its result goes to several buffers) is planned from what can do that: the 8-warp tile kernel unsplit, or the decode
