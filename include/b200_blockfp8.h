@@ -69,7 +69,7 @@ int b200_read_device_status(int* out, void* stream);
  * 128 / 192 / 256 = always on pairs with that tile width, 1282 / 1284 = always on 128-wide pairs whose 2 / 4 K splits are summed
  * in clusters), "gemm_ue8m0" (0 = packed power-of-two scales are unpacked and take the fp32-scale kernels, 1 / 2 = always the
  * single-CTA / CTA-pair block-scaled kernel), "linear_decode_fused" (0 = never a kernel that quantises its own input, 2 = the
- * linear takes the decode kernel that does wherever that runs; more than its 8 rows: B200_E_UNSUPPORTED), "moe_decode"
+ * linear takes the decode kernel that does wherever that runs; 9 to 16 rows: B200_E_UNSUPPORTED), "moe_decode"
  * (0 = never the weight-streaming MoE kernels, 1 = always, 16 / 32 / 64 = always with that row block), "moe_down_splitk" (0 = never),
  * "moe_zero_pads" (0 / 1), "peer_wait_ms" (limit of a device-side wait for another GPU, 100 .. 60000).
  * No counterpart in the reference (its Triton launchers read tuned JSON configs instead,

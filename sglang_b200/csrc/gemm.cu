@@ -448,7 +448,7 @@ static bool quant_in_gemm_wins(int64_t M, int64_t N, int64_t K, int sms, int spl
 static bool linear_quant_in_gemm(int64_t M, int64_t N, int64_t K, int sms, GemmRoute* route) {
   const Tuning& tune = tuning();
   const bool forced = tune.linear_decode_fused == 2;  // the launch refuses what the kernel cannot take
-  if ((M > SkinnyCfg<16, true>::kQuantRows && !forced) || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
+  if (M > (forced ? kLinearStreamMaxM : SkinnyCfg<16, true>::kQuantRows) || tune.linear_decode_fused == 0 || tune.gemm_splitk > 0 || tune.gemm_bn >= 0) return false;
   const GemmPlan plan = plan_gemm(M, N, K, sms, true);
   const SkinnySplit split = skinny_split(M, N, K, plan.splits);
   if (!plan.skinny || !split.direct()) return false;
@@ -485,7 +485,8 @@ extern "C" int b200_w8a8_block_fp8_linear(const void* x, int x_dtype, const void
   B200_CHECK_ARG(x && B && Bs && out, "linear: null pointer");
   B200_CHECK_ARG(((uintptr_t)x & 15) == 0 && ((uintptr_t)B & 15) == 0, "linear: x and B must be 16-byte aligned");
   B200_UNSUPPORTED(N % 8 != 0, "linear: N=%lld must be a multiple of 8", (long long)N);
-  const GemmRoute r = route_linear(M, N, K, sm_count());
+  GemmRoute r = {};
+  if (M <= kLinearStreamMaxM) r = route_linear(M, N, K, sm_count());  // no kernel takes more rows as they come
   if (r.kernel == B200_KERNEL_STREAM_QUANT) return run_linear_stream(x, x_dtype, B, Bs, out, M, N, K, 1e-10f, static_cast<cudaStream_t>(stream));
   if (r.kernel == B200_KERNEL_SKINNY_QUANT) {
     B200_CHECK_ARG(((uintptr_t)out & 15) == 0, "gemm: A, B and C must be 16-byte aligned");
